@@ -1,56 +1,68 @@
 // Dequant-fused small-M GEMM on the fifth-generation tensor cores: the product
 // behind Projections::Apply (GgufProjections::MatMul,
-// src/models/qwen35/gguf_projections.cpp:239-286 in the reference) when 16 to
-// 128 token rows share one weight read - the ragged verify batch, where every
-// sequence brings a few draft tokens and the packed rows form one matrix.
+// src/models/qwen35/gguf_projections.cpp:239-286 in the reference) when many
+// token rows share one weight read - the ragged verify batch, where every
+// sequence brings a few draft tokens, and the rows of a prompt.
 //
-// One thread block multiplies 256 weight rows by all the tokens over a range
-// of K:
-//   D[128 token rows][256 weight rows] (fp32, tensor memory) += X[128][64] * W[256][64]^T
-// per 64 columns. The tokens sit on the MMA's M (the tensor core spends M cycles
-// per instruction whatever N is, measured here: 128 x 32 x 16 took as long as
-// 128 x 128 x 16), the weight rows fill its N = 256.
-//   - six loader warps copy one block of each of the 256 rows per stage (Q4_K:
-//     its 144 bytes; Q6_K: 208 bytes from the three planes of the device
-//     arrangement plus the slab's d values) with 16-byte cp.async whose
-//     completion arrives on an mbarrier (tiled TMA boxes this narrow, 144 B wide,
-//     ran no faster);
-//   - one loader thread brings the activation tiles with one bulk copy
-//     (cp.async.bulk) each: the activations were converted once per product into
-//     fp16 tile images that already carry the shared-memory swizzle;
-//   - sixteen dequant warps, two threads per weight row: w = d*sc*q - dmin*m
-//     (DequantQ4_K, src/core/quant.cpp:33-59) in packed fp16 arithmetic (two
-//     weights per instruction, as d*sc*(q - 8) + (8*d*sc - dmin*m)) or
-//     w = d*sc*(q - 32) (DequantQ6_K, :98-125), likewise two per instruction,
-//     stored in the 128-byte-swizzled K-major layout the MMA reads; all sixteen
-//     warps work on one tile at a time, in the order the MMA consumes them;
-//   - one thread issues tcgen05.mma (kind::f16, M = 128, N = 256, K = 16, four
-//     per tile) and tcgen05.commit hands the tile buffers back;
-//   - four epilogue warps read the accumulator with tcgen05.ld (lane = token,
-//     column = weight row) and store y[token][row] while the other warps are
-//     already on the next unit of work: thread blocks are persistent, walk their
-//     (row tile, K range) units round-robin, and tensor memory holds two
-//     accumulators.
+//   D[128 weight rows][N token columns] (fp32, tensor memory)
+//       += W[128][64] (fp16, tensor memory) * X[N][64]^T (fp16, shared memory)
+//
+// per 64 columns of K; N is the tokens of a group rounded up to 16. The weights
+// sit on the MMA's M and reach it through TENSOR MEMORY: a dequant thread owns
+// one weight row, i.e. one lane of tensor memory, and leaves its 64 fp16 weights
+// there with two tcgen05.st - no address arithmetic, no swizzle, no proxy fence,
+// and none of the shared-memory bandwidth that bound the form this replaces
+// (weights written to and read back from swizzled shared-memory tiles: 7 bytes
+// of shared-memory traffic per weight, 16 weights per cycle and SM). An
+// instruction of this shape spends N / 2 cycles, so the tensor core's time falls
+// with the tokens instead of being that of 128 of them.
+//
+// Roles of the 23 warps of a thread block (one per SM):
+//   - sixteen dequant warps in four groups of four; group p turns pair p of a
+//     block (64 of its 256 values) of 128 rows into tensor memory slot p:
+//     w = d*sc*q - dmin*m (DequantQ4_K, src/core/quant.cpp:33-59) in packed fp16
+//     arithmetic, as d*sc*(q - 8) + (8*d*sc - dmin*m), or w = d*sc*(q - 32)
+//     (DequantQ6_K, :98-125). While the tensor core reads a slot, its group is at
+//     the arithmetic of the next block;
+//   - one thread brings the raw blocks of 128 rows with tiled TMA (Q4_K: one box
+//     of 144 bytes a row, whose row pitch is free of bank conflicts as it is;
+//     Q6_K: boxes of its four planes, the wide ones swizzled);
+//   - one thread brings the activation tiles, converted once per product into
+//     fp16 tile images that already carry the swizzle (StageHalfKernel);
+//   - one thread issues tcgen05.mma and hands the slots back with
+//     tcgen05.commit;
+//   - four epilogue warps read the accumulators with tcgen05.ld (lane = weight
+//     row, column = token: a store instruction of a warp covers 32 adjacent
+//     rows of one token) while the others are on the next tile: tensor memory
+//     holds two accumulators beside the four weight slots.
+//
+// Work split. A unit is a tile of 128 weight rows against one group of tokens; it
+// takes `blocks` steps of one 256-value block. The launch's units times steps are
+// cut into equal contiguous ranges, one per thread block, so the SMs finish
+// together whatever the number of tiles (2 x 9728 rows are 152 tiles for 148 SMs)
+// where that saves more than the cuts cost (PlanTc). A tile that a cut goes through
+// is finished by whichever of its thread blocks comes last, which adds the others'
+// partial sums (left in scratch) to its own in block order, so the result does not
+// depend on who that is. Nobody waits for another block.
+//
+// What bounds it: the dequantization's instructions (about 4500 warp instructions
+// a step, issue slots 60-65 % busy) up to about 100 tokens, then the activation
+// tiles' shared memory (a step of 128 tokens holds 64 KB of them: two and a half
+// steps in flight) and the tensor core. Measured (activation staging included): 2 x
+// 9728 x 2560 Q4_K, 32 / 128 / 512 tokens 29 / 33 / 131 -> 17 / 24 / 58 us (875
+// TFLOP/s at 512); 248320 x 2560 Q6_K, 32 / 79 / 128 tokens 229 / 245 / 266 -> 127 /
+// 144 / 190 us (4.4 TB/s at 32).
+//
 // Each activation row is scaled by a power of two into fp16 range first and the
 // outputs scaled back, so range never costs precision. Rounding w and x to
-// fp16 (11 significant bits) bounds the relative L2 error of y near 2e-4.
-//
-// Roofline: weights stream once from HBM (0.5625 B per weight); a tile costs
-// 4 MMAs of 128 cycles for 256 x 64 weights, 32 weights per cycle per SM, and
-// about 4 instructions per weight of dequant arithmetic. What binds today is
-// shared-memory bandwidth: every weight is written as fp16 (2 B) and read by
-// the MMA (2 B), its Q4_K bytes pass through shared memory (1.1 B), and the
-// activation tile of 16 KiB is written and read once per 16384 weights (2 B):
-// about 7 B per weight against 128 B per cycle, 16 to 18 weights per cycle per
-// SM, which is what the kernel measures. Matrices with few row tiles split K
-// over thread blocks when the modelled time says so; the partial sums are
-// added in a fixed order by a second kernel.
+// fp16 (11 significant bits) bounds the relative L2 error of y near 4e-4.
 //
 // Every wait on an mbarrier is bounded: a wait that runs out records an error
 // code, raises a block-wide abort flag that ends all other waits, and the
 // kernel still frees its tensor memory and returns.
 #include "gemm_tc.cuh"
 
+#include <cuda.h>
 #include <cuda_fp16.h>
 
 #include <vector>
@@ -59,140 +71,93 @@ namespace gufo {
 
 namespace {
 
-constexpr int kTileRows = 256;             // weight rows per thread block (the MMA's N)
-constexpr int kTokenRows = 128;            // token rows per tile image (the MMA's M)
-constexpr int kTileK = 64;                 // values per tile (one swizzle row of fp16)
-constexpr int kWTileBytes = kTileRows * kTileK * 2;    // 32 KiB
-constexpr int kXTileBytes = kTokenRows * kTileK * 2;   // 16 KiB
-// What differs between the block formats: how one block of a row is copied into
-// shared memory (16-byte chunks) and how deep the rings are.
+constexpr int kTileRows = 128;      // weight rows of one MMA (its M)
+constexpr int kTileK = 64;          // values per activation tile (one swizzle row of fp16)
+constexpr int kGroups = 4;          // dequant groups = tensor memory slots = pairs of a block
+constexpr int kSlotColumns = kTileK / 2;               // 32-bit columns of a slot: two fp16 each
+constexpr int kAccColumn = kGroups * kSlotColumns;     // the accumulators' first column
+constexpr int kTmemColumns = 512;
+constexpr int kAccColumns = kTmemColumns - kAccColumn;
+constexpr int kMaxN = kAccColumns / 2;                 // 192 token columns
+constexpr int kDequantWarps = 4 * kGroups;
+constexpr int kEpilogueWarp = kDequantWarps;           // four, one per lane quarter
+constexpr int kRawWarp = kEpilogueWarp + 4;
+constexpr int kXWarp = kRawWarp + 1;
+constexpr int kMmaWarp = kXWarp + 1;
+constexpr int kTcThreads = (kMmaWarp + 1) * 32;
+constexpr int kMaxStages = 10;
+constexpr long long kWaitCycles = 1ll << 31;           // about a second of SM clocks
+constexpr int kHeaderBytes = 4096;                     // of the scratch: error word, counters of cut tiles
+constexpr size_t kScratchFloor = 32u << 20;            // of the scratch: one allocation serves most shapes
+constexpr int kSharedLimit = 227 * 1024;
+
+// The raw bytes of one block of 128 rows in shared memory.
 template <int TYPE>
 struct Quant;
-
 template <>
 struct Quant<GUFO_CUDA_Q4_K> {
-  static constexpr int kRowBytes = kQ4KBytes;   // shared memory per row and block
-  static constexpr int kWStages = 3, kXStages = 3, kRawStages = 2;
-  static constexpr int kLoaders = 3;            // loader warps at work (of kLoaderWarps)
-  // Chunk `chunk` of block `block` of a row: the GGUF bytes as they are.
-  __device__ static const uint8_t* Source(const uint8_t* row, int blocks, int block, int chunk) {
-    (void)blocks;
-    return row + static_cast<size_t>(block) * kQ4KBytes + chunk * 16;
-  }
+  static constexpr int kMaps = 1;
+  static constexpr int kRawBytes = kTileRows * kQ4KBytes;
+  static constexpr int kRawStride = kRawBytes;
 };
-
 template <>
 struct Quant<GUFO_CUDA_Q6_K> {
-  // ql 128 | qh 64 | scales 16 | the 16 bytes that hold the slab's d values | 16
-  // unused: rows 240 bytes apart, so that the 16-byte reads of eight consecutive
-  // rows fall into different banks (224 put rows r and r + 4 into the same).
-  static constexpr int kRowBytes = 240;
-  static constexpr int kWStages = 2, kXStages = 2, kRawStages = 2;
-  static constexpr int kLoaders = 6;
-  // The planar device arrangement (Q6KBlockAt): a slab of n blocks stores
-  // ql n x 128 | qh n x 64 | scales n x 16 | d n x 2.
-  __device__ static const uint8_t* Source(const uint8_t* row, int blocks, int block, int chunk) {
-    const int slab = block / kQ6KSlabBlocks;
-    const int j = block - slab * kQ6KSlabBlocks;
-    const int left = blocks - slab * kQ6KSlabBlocks;
-    const int n = left < kQ6KSlabBlocks ? left : kQ6KSlabBlocks;
-    const uint8_t* base = row + static_cast<size_t>(slab) * kQ6KSlabBlocks * kQ6KBytes;
-    if (chunk < 8) {
-      return base + 128 * j + 16 * chunk;
-    }
-    if (chunk < 12) {
-      return base + 128 * n + 64 * j + 16 * (chunk - 8);
-    }
-    if (chunk == 12) {
-      return base + 192 * n + 16 * j;
-    }
-    return base + 208 * n;   // all of the slab's d values; the row stride covers the 16 bytes
-  }
-};
-constexpr int kDequantThreads = 2 * kTileRows;         // two threads per weight row
-constexpr int kEpilogueWarp = kDequantThreads / 32;    // four epilogue warps, one per lane quarter
-constexpr int kEpilogueWarps = 4;
-constexpr int kLoaderWarp = kEpilogueWarp + kEpilogueWarps;   // and the next: weight loaders
-// Up to six of them (Quant<TYPE>::kLoaders at work): with two, in-kernel cycle
-// counters showed the loaders issuing copies 70 % (Q4_K) and 98 % (Q6_K) of the
-// time while every other role waited.
-constexpr int kLoaderWarps = 6;
-constexpr int kMmaWarp = kLoaderWarp + kLoaderWarps;
-constexpr int kTileLoaderWarp = kMmaWarp + 1;
-constexpr int kTcThreads = (kTileLoaderWarp + 1) * 32;
-constexpr int kTmemColumns = 512;                      // two accumulators of 256 columns
-constexpr long long kWaitCycles = 1ll << 31;   // about a second of SM clocks
-
-// Dynamic shared memory, from a 1024-byte aligned base.
-template <int TYPE>
-struct Smem {
-  using Q = Quant<TYPE>;
-  static constexpr int kRawBytes = kTileRows * Q::kRowBytes;   // one block of every row
-  static constexpr int kW = 0;
-  static constexpr int kX = kW + Q::kWStages * kWTileBytes;
-  static constexpr int kRaw = kX + Q::kXStages * kXTileBytes;
-  static constexpr int kBars = kRaw + Q::kRawStages * kRawBytes;
-  // raw_full, raw_empty, w_full, w_empty, x_full, x_empty (per stage), acc_full[2], acc_empty[2]
-  static constexpr int kBarCount = 2 * Q::kRawStages + 2 * Q::kWStages + 2 * Q::kXStages + 4;
-  static constexpr int kTmemSlot = kBars + kBarCount * 8;
-  static constexpr int kAbort = kTmemSlot + 4;
-  static constexpr int kBytes = kAbort + 4 + 1024;   // + room to align the base
-  static_assert(kX % 1024 == 0 && kRaw % 1024 == 0, "swizzled tiles need 1024-byte alignment");
-  static_assert(kBytes <= 227 * 1024, "beyond the shared memory of a thread block");
+  static constexpr int kMaps = 3;   // boxes 128, 64 and 16 bytes wide
+  static constexpr int kQl = 0, kQh = kTileRows * 128, kSc = kQh + kTileRows * 64, kD = kSc + kTileRows * 16;
+  static constexpr int kRawBytes = kD + kTileRows * 16;
+  static constexpr int kRawStride = kRawBytes;   // 28 KiB: a multiple of 1024
 };
 
 constexpr int kTcMaxParts = 4;
 
 struct TcPart {
-  const uint8_t* w;        // first row
   int rows;
-  int row_bytes;
-  int tiles;               // 256-row tiles of this part
-  float* out;              // ksplit == 1: y + offset; else partial sums [ksplit][tokens][rows]
-  int out_stride;          // floats between token rows of out
-  size_t split_stride;     // floats between the K ranges' partial sums
+  int tiles;               // tiles of 128 rows
+  float* out;              // y + the part's first column
 };
 
 struct TcGemmArgs {
+  CUtensorMap maps[kTcMaxParts * 3];   // [part][map]
   TcPart parts[kTcMaxParts];
   int nparts;
-  int blocks;              // Q4_K blocks per row
-  int blocks_per_unit;     // K range of one unit of work
-  int ksplit;
-  int total_units;         // tiles * ksplit, dealt round-robin to the thread blocks
-  int tile_rows;           // weight rows per tile: a multiple of 16 up to kTileRows (the MMA's N)
-  const uint8_t* xh;       // activation tile images [blocks * 4][128][64] fp16, swizzled
-  const float* unscale;    // [128]: factor that undoes the row's power-of-two scale
+  int blocks;              // 256-value blocks per row: the steps of a unit
+  int groups;              // token groups
+  int n;                   // token columns of a group, a multiple of 16
+  int units;               // tiles * groups
+  int per, extra;          // steps of a thread block: per, one more for the first `extra`
+  int raw_stages, x_stages;
+  const uint8_t* xh;       // activation tile images [group][blocks * 4][n][64] fp16, swizzled
+  const float* unscale;    // [groups * n]: factor that undoes a row's power-of-two scale
+  float* partial;          // [thread block][2][n][128]: sums of tiles that a cut goes through
+  unsigned* counters;      // [thread block]: arrivals at the tile that starts there
   int tokens;
+  int out_stride;          // floats between token rows of y
   int* error;              // device int: 0, or the code of the first wait that ran out
 };
 
-__device__ __forceinline__ uint32_t SharedAddress(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void MbarInit(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
 __device__ __forceinline__ void MbarArrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void MbarArriveExpectTx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool MbarTryWait(uint32_t bar, uint32_t parity) {
+
+// The same test, suspended by the hardware for up to kSuspendNs first: most warps
+// of the kernel wait most of the time, and polling took as many issue slots as the
+// dequantization.
+constexpr uint32_t kSuspendNs = 20000;
+__device__ __forceinline__ bool MbarTrySuspended(uint32_t bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+      : "=r"(done) : "r"(bar), "r"(parity), "r"(kSuspendNs) : "memory");
   return done != 0;
 }
 
 // Waits for the phase with `parity` to complete, for at most kWaitCycles and
 // only while no thread of the block has given up. Returns false when it did
-// not see the phase complete.
+// not see the phase complete. PATIENT: suspended in between (loaders and
+// epilogue, whose waits are long; waking up takes longer).
+template <bool PATIENT = false>
 __device__ __forceinline__ bool BoundedWait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                             int* error, int code) {
   if (MbarTryWait(bar, parity)) {
@@ -200,7 +165,7 @@ __device__ __forceinline__ bool BoundedWait(uint32_t bar, uint32_t parity, volat
   }
   const long long start = clock64();
   while (clock64() - start < kWaitCycles) {
-    if (MbarTryWait(bar, parity)) {
+    if (PATIENT ? MbarTrySuspended(bar, parity) : MbarTryWait(bar, parity)) {
       return true;
     }
     if (*abort_flag != 0) {
@@ -212,9 +177,21 @@ __device__ __forceinline__ bool BoundedWait(uint32_t bar, uint32_t parity, volat
   return false;
 }
 
-__device__ __forceinline__ void BulkCopy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+// One thread of a converged warp. Instructions of the asynchronous units take
+// their operands from uniform registers; behind this predicate the compiler knows
+// that there is one thread, behind `lane == 0` it does not and walks the warp for
+// every operand (measured: 112 cycles to issue an MMA or a commit, whatever its
+// size, against N / 2 and about 25).
+__device__ __forceinline__ bool ElectOne() {
+  uint32_t elected;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+  return elected != 0;
+}
+
+// A box of 128 rows at byte column x, row y of a matrix (x is a multiple of 16).
+__device__ __forceinline__ void TileCopy(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 
 // Shared-memory matrix descriptor of a K-major tile with 128-byte rows and the
@@ -230,18 +207,28 @@ __device__ __forceinline__ uint64_t TileDescriptor(uint32_t shared_address) {
   return desc;
 }
 
-__device__ __forceinline__ void MmaF16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+// D (tensor memory) += A (tensor memory) * B (shared memory).
+__device__ __forceinline__ void MmaF16(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
                                        uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0) : "memory");
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 __device__ __forceinline__ void MmaCommit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
+}
+
+__device__ __forceinline__ void TmemStore16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
 }
 
 __device__ __forceinline__ void TmemLoad16(uint32_t taddr, float (&v)[16]) {
@@ -260,71 +247,156 @@ __device__ __forceinline__ void TmemLoad16(uint32_t taddr, float (&v)[16]) {
 }
 
 // Within every four consecutive values of K the tiles hold them in the order
-// (0, 2, 1, 3): a Q4_K word yields the nibbles of its bytes 0 and 2 together (and
-// 1 and 3), so this order lets a pair leave the arithmetic as it arrives. The
-// activation tiles (StageHalfKernel) and the Q6_K tiles follow the same order;
-// a contraction does not care how K is numbered.
+// (0, 2, 1, 3): a word yields the codes of its bytes 0 and 2 together (and 1 and
+// 3), so this order lets a pair leave the arithmetic as it arrives. The
+// activation tiles (StageHalfKernel) follow the same order; a contraction does
+// not care how K is numbered.
 //
-// Eight weights from two words of a sub-block pair's nibble bytes, in packed
-// fp16 arithmetic. A nibble is masked in place under an fp16
-// exponent whose mantissa bit there is worth 1 (1024 + code for bits 0-3,
-// 64 + code for bits 4-7: one logic instruction for two codes); subtracting the
-// power of two plus 8 leaves code - 8 exactly, and one fused multiply-add per
-// pair gives w = scale * (code - 8) + (8 * scale - offset). Centring the code
-// keeps both terms of the size of w itself, so rounding the scale and the
-// constant to fp16 costs about what rounding w does; scale * code - offset
-// loses three more bits to cancellation (measured relative L2 of a product:
-// 7e-4 that way, 3.8e-4 centred, 2e-4 with fp32 arithmetic rounded once).
-__device__ __forceinline__ uint32_t HalfPairFma(uint32_t biased, uint32_t bias, uint32_t scale, uint32_t constant) {
-  const __half2 code = __hsub2(*reinterpret_cast<const __half2*>(&biased), *reinterpret_cast<const __half2*>(&bias));
-  const __half2 w = __hfma2(code, *reinterpret_cast<const __half2*>(&scale), *reinterpret_cast<const __half2*>(&constant));
-  return *reinterpret_cast<const uint32_t*>(&w);
+// Four codes under the bits of kMask in the bytes of w, in packed fp16
+// arithmetic: a code is masked in place under an fp16 exponent whose mantissa bit
+// there is worth 1 (1024 + code for bits 0-5, 64 + code for bits 4-7: one logic
+// instruction for two codes), and subtracting that power of two plus the centre
+// leaves code - centre exactly.
+__device__ __forceinline__ __half2 Centred(uint32_t w, uint32_t mask, uint32_t one, uint32_t bias) {
+  const uint32_t biased = (w & mask) | one;
+  return __hsub2(*reinterpret_cast<const __half2*>(&biased), *reinterpret_cast<const __half2*>(&bias));
 }
+__device__ __forceinline__ uint32_t HalfBits(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
 
-// HIGH = false: the low nibbles of the eight bytes of w0 and w1 (eight values of
-// sub-block 2t); HIGH = true: the high nibbles (of sub-block 2t + 1).
+// Q4_K: scale * (code - 8) + (8 * scale - offset) of 32 nibbles (HIGH: the high
+// ones) of eight words. Centring the code keeps both terms of the size of w
+// itself, so rounding the scale and the constant to fp16 costs about what
+// rounding w does; scale * code - offset loses three more bits to cancellation
+// (measured relative L2 of a product: 7e-4 that way, 3.8e-4 centred, 2e-4 with
+// fp32 arithmetic rounded once).
 template <bool HIGH>
-__device__ __forceinline__ uint4 EightWeights(uint32_t w0, uint32_t w1, uint32_t scale, uint32_t constant) {
+__device__ __forceinline__ void Nibbles(const uint32_t (&w)[8], __half2 scale, __half2 constant, uint32_t (&out)[16]) {
   constexpr uint32_t kMask = HIGH ? 0x00F000F0u : 0x000F000Fu;
   constexpr uint32_t kOne = HIGH ? 0x54005400u : 0x64006400u;    // 64 or 1024 as fp16 pairs
   constexpr uint32_t kBias = HIGH ? 0x54805480u : 0x64086408u;   // 72 or 1032
-  const uint32_t s0 = w0 >> 8, s1 = w1 >> 8;
-  return make_uint4(HalfPairFma((w0 & kMask) | kOne, kBias, scale, constant),    // bytes 0 and 2
-                    HalfPairFma((s0 & kMask) | kOne, kBias, scale, constant),    // bytes 1 and 3
-                    HalfPairFma((w1 & kMask) | kOne, kBias, scale, constant),
-                    HalfPairFma((s1 & kMask) | kOne, kBias, scale, constant));
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    out[2 * c] = HalfBits(__hfma2(Centred(w[c], kMask, kOne, kBias), scale, constant));
+    out[2 * c + 1] = HalfBits(__hfma2(Centred(w[c] >> 8, kMask, kOne, kBias), scale, constant));
+  }
 }
 
-// Eight Q6_K weights from the codes in the bytes of two words, as four fp16
-// pairs, in packed fp16 arithmetic: the codes of bytes 0 and 2 (and 1 and 3) are
-// masked in place under the fp16 exponent of 1024, 1024 + 32 is subtracted
-// exactly, and one multiply per pair applies the group's scale, itself rounded
-// to fp16: w = scale * (code - 32).
-__device__ __forceinline__ uint4 EightCodes(uint32_t w0, uint32_t w1, float scale) {
-  constexpr uint32_t kMask = 0x003F003Fu, kOne = 0x64006400u, kBias = 0x64206420u;   // 1024, 1056
-  const __half2 s2 = __float2half2_rn(scale);
-  auto two = [&](uint32_t w) {
-    const uint32_t biased = (w & kMask) | kOne;
-    const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&biased), *reinterpret_cast<const __half2*>(&kBias)), s2);
-    return *reinterpret_cast<const uint32_t*>(&v);
-  };
-  // Bytes (0, 2) and (1, 3) of each word: the tiles' order of K.
-  return make_uint4(two(w0), two(w0 >> 8), two(w1), two(w1 >> 8));
+// Q6_K: scale * (code - 32) of the 32 values whose low nibbles are bits 0-3 of
+// the bytes of lo and whose high bits are bits 4-5 of the bytes of hi (bits 6-7
+// zero); the first sixteen take scale a, the others b. The code byte is complete
+// and clean, so one byte permute puts two of them under the exponent of 1024.
+__device__ __forceinline__ void SixBits(const uint32_t (&lo)[8], const uint32_t (&hi)[8], __half2 a, __half2 b,
+                                        uint32_t (&out)[16]) {
+  constexpr uint32_t kBias = 0x64206420u;   // 1024 + 32
+  const __half2 bias = *reinterpret_cast<const __half2*>(&kBias);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const uint32_t code = (lo[c] & 0x0F0F0F0Fu) | (hi[c] & ~0x0F0F0F0Fu);
+    const uint32_t even = __byte_perm(code, 0x64646464u, 0x4240u), odd = __byte_perm(code, 0x64646464u, 0x4341u);
+    const __half2 scale = c < 4 ? a : b;
+    out[2 * c] = HalfBits(__hmul2(__hsub2(*reinterpret_cast<const __half2*>(&even), bias), scale));
+    out[2 * c + 1] = HalfBits(__hmul2(__hsub2(*reinterpret_cast<const __half2*>(&odd), bias), scale));
+  }
 }
 
-// Where unit `u` of a launch works: its part, weight rows and K range.
+// The raw bytes that one dequant thread needs of a block of its row, the 64
+// values of pair p, and their fp16 weights. p stays a run-time value: sixteen
+// warps in one piece of code (a copy of the loop per group ran 15 % slower, out of
+// the instruction cache).
+template <int TYPE>
+struct Pair;
+
+template <>
+struct Pair<GUFO_CUDA_Q4_K> {
+  uint4 head, q0, q1;
+  __device__ __forceinline__ void Load(const uint8_t* raw, int row, int p, int b) {
+    (void)b;
+    const uint8_t* block = raw + row * kQ4KBytes;
+    head = *reinterpret_cast<const uint4*>(block);
+    q0 = *reinterpret_cast<const uint4*>(block + 16 + 32 * p);
+    q1 = *reinterpret_cast<const uint4*>(block + 32 + 32 * p);
+  }
+  __device__ __forceinline__ void Weights(int p, uint32_t (&lo)[16], uint32_t (&hi)[16]) const {
+    const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    const float d = HalfBitsToFloat(static_cast<uint16_t>(head.x & 0xFFFF));
+    const float dmin = HalfBitsToFloat(static_cast<uint16_t>(head.x >> 16));
+    // Scales and mins of sub-blocks 2p and 2p + 1 (ScaleMinK4) in bytes 0 and 1.
+    uint32_t sc = head.y & 0x3F3F3F3Fu, mn = head.z & 0x3F3F3F3Fu;
+    if (p >= 2) {
+      sc = (head.w & 0x0F0F0F0Fu) | ((head.y >> 2) & 0x30303030u);
+      mn = ((head.w >> 4) & 0x0F0F0F0Fu) | ((head.z >> 2) & 0x30303030u);
+    }
+    sc >>= 16 * (p & 1);
+    mn >>= 16 * (p & 1);
+    auto prepare = [&](uint32_t scale_byte, uint32_t min_byte, __half2& scale2, __half2& constant2) {
+      const float scale = d * static_cast<float>(scale_byte);
+      scale2 = __float2half2_rn(scale);
+      constant2 = __float2half2_rn(fmaf(8.0f, scale, -dmin * static_cast<float>(min_byte)));
+    };
+    __half2 s, c;
+    prepare(sc & 0xFFu, mn & 0xFFu, s, c);
+    Nibbles<false>(words, s, c, lo);
+    prepare((sc >> 8) & 0xFFu, (mn >> 8) & 0xFFu, s, c);
+    Nibbles<true>(words, s, c, hi);
+  }
+};
+
+// Pair p: runs k = j and k = j + 2 (j = p & 1) of half h = p / 2, which share their
+// 32 ql bytes: values 128 h + 32 k .. + 31, low nibbles for the first run and high
+// ones for the second, two bits of the half's qh bytes at 2 k.
+template <>
+struct Pair<GUFO_CUDA_Q6_K> {
+  using Q = Quant<GUFO_CUDA_Q6_K>;
+  uint4 l0, l1, h0, h1;
+  uint2 sc8;
+  uint32_t d;
+  __device__ __forceinline__ void Load(const uint8_t* raw, int row, int p, int b) {
+    const int h = p >> 1;
+    const uint8_t* ql = raw + Q::kQl + row * 128;
+    const uint8_t* qh = raw + Q::kQh + row * 64;
+    const int c0 = 4 * h + 2 * (p & 1);
+    const int swz = row & 7, swz_h = (row >> 1) & 3;   // of the boxes' 128- and 64-byte swizzles
+    l0 = *reinterpret_cast<const uint4*>(ql + ((c0 ^ swz) << 4));
+    l1 = *reinterpret_cast<const uint4*>(ql + (((c0 + 1) ^ swz) << 4));
+    h0 = *reinterpret_cast<const uint4*>(qh + (((2 * h) ^ swz_h) << 4));
+    h1 = *reinterpret_cast<const uint4*>(qh + (((2 * h + 1) ^ swz_h) << 4));
+    sc8 = *reinterpret_cast<const uint2*>(raw + Q::kSc + row * 16 + 8 * h);
+    d = *reinterpret_cast<const uint16_t*>(raw + Q::kD + row * 16 + 2 * (b & (kQ6KSlabBlocks - 1)));
+  }
+  __device__ __forceinline__ void Weights(int p, uint32_t (&lo)[16], uint32_t (&hi)[16]) const {
+    const float scale = HalfBitsToFloat(static_cast<uint16_t>(d));
+    const int j = p & 1;
+    // int8 scales of 16-value groups 2j, 2j + 1 (first run) and 2j + 4, 2j + 5 of this half.
+    const uint32_t first = sc8.x >> (16 * j), second = sc8.y >> (16 * j);
+    auto of = [&](uint32_t byte) { return __float2half2_rn(scale * static_cast<float>(static_cast<int8_t>(byte))); };
+    const uint32_t low[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+    const uint32_t high[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+    uint32_t nib[8], up[8], bits[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      bits[c] = (high[c] >> (2 * j)) & 0x33333333u;   // both runs' bits, at 0-1 and 4-5
+      up[c] = bits[c] << 4;
+      nib[c] = low[c] >> 4;
+    }
+    SixBits(low, up, of(first), of(first >> 8), lo);
+    SixBits(nib, bits, of(second), of(second >> 8), hi);
+  }
+};
+
+// First step of thread block c's range: the first `extra` ranges are a step longer.
+__device__ __forceinline__ int RangeStart(const TcGemmArgs& a, int c) { return c * a.per + min(c, a.extra); }
+
+// Where a unit works: its part, first weight row and token group.
 struct Unit {
   int part;
   int row0;
-  int split;
-  int first_block;
-  int blocks;
+  int group;
 };
 
 __device__ __forceinline__ Unit LocateUnit(const TcGemmArgs& a, int u) {
   Unit unit;
-  int tile = u / a.ksplit;
-  unit.split = u - tile * a.ksplit;
+  int tile = u / a.groups;   // groups of one tile follow one another: its weights are in L2 by then
+  unit.group = u - tile * a.groups;
   unit.part = 0;
 #pragma unroll
   for (int p = 0; p < kTcMaxParts - 1; ++p) {
@@ -333,244 +405,350 @@ __device__ __forceinline__ Unit LocateUnit(const TcGemmArgs& a, int u) {
       unit.part = p + 1;
     }
   }
-  unit.row0 = tile * a.tile_rows;
-  unit.first_block = unit.split * a.blocks_per_unit;
-  unit.blocks = min(a.blocks_per_unit, a.blocks - unit.first_block);   // >= 1 by construction
+  unit.row0 = tile * kTileRows;
   return unit;
 }
 
-// Row of the MMA's M that token t occupies: tokens are dealt round-robin to the
-// four 32-lane quarters of tensor memory, so that all four epilogue warps (each
-// can read one quarter) share the work of a small batch.
-__host__ __device__ __forceinline__ int TokenRow(int t) { return (t & 3) * 32 + (t >> 2); }
+// The thread blocks that share a cut tile (the unit of `blocks` steps from step
+// `begin` on), from one of them.
+struct CutTile {
+  int from, to;
+};
+__device__ __forceinline__ CutTile LocateCut(const TcGemmArgs& a, int self, int begin) {
+  CutTile cut{self, self};
+  while (RangeStart(a, cut.from) > begin) {
+    --cut.from;
+  }
+  while (RangeStart(a, cut.to + 1) < begin + a.blocks) {
+    ++cut.to;
+  }
+  return cut;
+}
+// Which of block c's partial slots holds its share: only the first of the tile's
+// blocks can have begun elsewhere.
+__device__ __forceinline__ int CutSlot(const TcGemmArgs& a, const CutTile& cut, int c, int begin) {
+  return c == cut.from && RangeStart(a, c) < begin ? 1 : 0;
+}
+
+// Column `col` (128 rows) of a thread block's partial sums.
+__device__ __forceinline__ float* PartialColumn(const TcGemmArgs& a, int block, int slot, int col) {
+  return a.partial + ((static_cast<size_t>(block) * 2 + slot) * a.n + col) * kTileRows;
+}
+
+// A cut tile whose shares are all in scratch, by the first twenty warps: a column
+// of 128 rows a warp, in block order.
+__device__ __noinline__ void AddShares(const TcGemmArgs& a, int u, const CutTile& cut) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int begin = u * a.blocks;
+  __threadfence();
+  const Unit unit = LocateUnit(a, u);
+  const TcPart& part = a.parts[unit.part];
+  const int token0 = unit.group * a.n;
+  const int columns = min(a.n, a.tokens - token0);
+  const bool vectors = a.out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(part.out) & 15) == 0;
+#pragma unroll 4
+  for (int col = warp; col < columns; col += kDequantWarps + 4) {
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float f = __ldcg(a.unscale + token0 + col);
+#pragma unroll 4
+    for (int c = cut.from; c <= cut.to; ++c) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(PartialColumn(a, c, CutSlot(a, cut, c, begin), col)) + lane);
+      sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+    }
+    const int row = unit.row0 + 4 * lane;
+    float* to = part.out + static_cast<size_t>(token0 + col) * a.out_stride + row;
+    if (vectors && row + 4 <= part.rows) {
+      *reinterpret_cast<float4*>(to) = make_float4(sum.x * f, sum.y * f, sum.z * f, sum.w * f);
+    } else {
+      const float v[4] = {sum.x * f, sum.y * f, sum.z * f, sum.w * f};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (row + i < part.rows) {
+          to[i] = v[i];
+        }
+      }
+    }
+  }
+  if (threadIdx.x == 0) {
+    a.counters[cut.from] = 0;   // for the next launch
+  }
+}
+
+// What a dequant warp of group p works with.
+struct DequantPlace {
+  uint32_t raw_full, raw_empty;   // stage 0; eight bytes apart
+  uint32_t w_full, w_empty;       // the group's slot
+  const uint8_t* raw;             // stage 0
+  uint32_t slot;                  // the warp's lanes of the slot
+  int row;                        // this thread's row of the tile
+  int p;
+};
+
+// The steps [first, last) of one dequant warp.
+template <int TYPE>
+__device__ __forceinline__ void DequantSteps(const TcGemmArgs& a, const DequantPlace& at, int first, int last,
+                                             volatile int* abort_flag) {
+  const bool leader = (threadIdx.x & 31) == 0;
+  int stage = 0;
+  uint32_t phase = 0, w_phase = 1;
+  int b = first % a.blocks;
+  const uint8_t* raw = at.raw;
+  for (int step = first; step < last; ++step) {
+    BoundedWait(at.raw_full + 8 * stage, phase, abort_flag, a.error, 4);
+    Pair<TYPE> pair;
+    pair.Load(raw, at.row, at.p, b);
+    __syncwarp();
+    if (leader) {
+      MbarArrive(at.raw_empty + 8 * stage);
+    }
+    uint32_t lo[16], hi[16];
+    pair.Weights(at.p, lo, hi);
+    // The tensor core has read the slot's weights of the block before.
+    BoundedWait(at.w_empty, w_phase, abort_flag, a.error, 5);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    TmemStore16(at.slot, lo);
+    TmemStore16(at.slot + 16, hi);
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (leader) {
+      MbarArrive(at.w_full);
+    }
+    w_phase ^= 1u;
+    raw += Quant<TYPE>::kRawStride;
+    if (++stage == a.raw_stages) {
+      stage = 0;
+      phase ^= 1u;
+      raw = at.raw;
+    }
+    if (++b == a.blocks) {
+      b = 0;
+    }
+  }
+}
 
 template <int TYPE>
 __global__ void __launch_bounds__(kTcThreads, 1)
 GemmTc(const __grid_constant__ TcGemmArgs a) {
   using Q = Quant<TYPE>;
-  using Smem = Smem<TYPE>;
-  constexpr int kWStages = Q::kWStages, kXStages = Q::kXStages, kRawStages = Q::kRawStages;
-  constexpr int kRawBytes = Smem::kRawBytes;
   extern __shared__ uint8_t smem_raw[];
-  // The swizzled tiles need a 1024-byte aligned base.
+  __shared__ __align__(8) uint64_t bar_mem[4 * kMaxStages + 2 * kGroups + 4];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_word;
+  __shared__ float factor[kMaxN];    // what undoes the scales of the unit's token rows
+  __shared__ int finish;             // a cut tile whose shares are all in scratch and that is left to this block (unit + 1)
+  __shared__ int others_done;
+  // The swizzled tiles need a 1024-byte aligned base: activation tiles, then raw blocks.
   const uint32_t base = (SharedAddress(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - SharedAddress(smem_raw));
-  const uint32_t bars = base + Smem::kBars;
+  const int x_bytes = 2 * a.n * kTileK * 2;   // a stage of two activation tiles
+  const uint32_t raw_at = static_cast<uint32_t>(a.x_stages * x_bytes);
+  const uint32_t bars = SharedAddress(bar_mem);
   auto raw_full = [&](int s) { return bars + 8u * s; };
-  auto raw_empty = [&](int s) { return bars + 8u * (kRawStages + s); };
-  auto w_full = [&](int s) { return bars + 8u * (2 * kRawStages + s); };
-  auto w_empty = [&](int s) { return bars + 8u * (2 * kRawStages + kWStages + s); };
-  auto x_full = [&](int s) { return bars + 8u * (2 * kRawStages + 2 * kWStages + s); };
-  auto x_empty = [&](int s) { return bars + 8u * (2 * kRawStages + 2 * kWStages + kXStages + s); };
-  auto acc_full = [&](int s) { return bars + 8u * (2 * kRawStages + 2 * kWStages + 2 * kXStages + s); };
-  auto acc_empty = [&](int s) { return bars + 8u * (2 * kRawStages + 2 * kWStages + 2 * kXStages + 2 + s); };
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + Smem::kTmemSlot);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Smem::kAbort);
+  auto raw_empty = [&](int s) { return bars + 8u * (kMaxStages + s); };
+  auto x_full = [&](int s) { return bars + 8u * (2 * kMaxStages + s); };
+  auto x_empty = [&](int s) { return bars + 8u * (3 * kMaxStages + s); };
+  auto w_full = [&](int g) { return bars + 8u * (4 * kMaxStages + g); };
+  auto w_empty = [&](int g) { return bars + 8u * (4 * kMaxStages + kGroups + g); };
+  auto acc_full = [&](int s) { return bars + 8u * (4 * kMaxStages + 2 * kGroups + s); };
+  auto acc_empty = [&](int s) { return bars + 8u * (4 * kMaxStages + 2 * kGroups + 2 + s); };
+  volatile int* abort_flag = &abort_word;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int units = a.total_units;
+  const int first = RangeStart(a, blockIdx.x);
+  const int last = RangeStart(a, blockIdx.x + 1);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kRawStages; ++s) {
-      MbarInit(raw_full(s), 32 * Q::kLoaders);
-      MbarInit(raw_empty(s), kDequantThreads / 32);
+    for (int s = 0; s < a.raw_stages; ++s) {
+      MbarInit(raw_full(s), 1);
+      MbarInit(raw_empty(s), kDequantWarps);
     }
-    for (int s = 0; s < kWStages; ++s) {
-      MbarInit(w_full(s), kDequantThreads / 32);
-      MbarInit(w_empty(s), 1);
-    }
-    for (int s = 0; s < kXStages; ++s) {
+    for (int s = 0; s < a.x_stages; ++s) {
       MbarInit(x_full(s), 1);
       MbarInit(x_empty(s), 1);
     }
+    for (int g = 0; g < kGroups; ++g) {
+      MbarInit(w_full(g), 4);
+      MbarInit(w_empty(g), 1);
+    }
     for (int s = 0; s < 2; ++s) {
       MbarInit(acc_full(s), 1);
-      MbarInit(acc_empty(s), kEpilogueWarps);
+      MbarInit(acc_empty(s), 4);
     }
-    *abort_flag = 0;
+    abort_word = 0;
+    finish = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 0) {
+  if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(base + Smem::kTmemSlot), "r"(kTmemColumns) : "memory");
+                 ::"r"(SharedAddress(&tmem_slot)), "r"(kTmemColumns) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_slot);
   // The weights never depend on earlier kernels; the activation tiles and the
   // outputs do.
   GridLaunchDependents();
 
-  // Every role walks the same units, blockIdx.x, blockIdx.x + gridDim.x, ...;
-  // the stage counters run on across units, so the pipeline never drains
-  // between them.
-  if (warp >= kLoaderWarp && warp < kLoaderWarp + Q::kLoaders) {
-    // ---- weight loaders: the 16-byte chunks of one block of every row (Q4_K: 9
-    // per row, one 144-byte run; Q6_K: 14 per row from its four planes), split
-    // between the loader warps; consecutive lanes take consecutive chunks -------
-    const int which = warp - kLoaderWarp;
-    constexpr int kChunksPerRow = Q::kRowBytes / 16;
-    const int kChunks = a.tile_rows * kChunksPerRow;
-    int i = 0;   // blocks requested so far
-    for (int u = blockIdx.x; u < units; u += gridDim.x) {
-      const Unit unit = LocateUnit(a, u);
-      const TcPart& part = a.parts[unit.part];
-      for (int b = 0; b < unit.blocks; ++b, ++i) {
-        const int s = i % kRawStages;
-        const uint32_t phase = (i / kRawStages) & 1u;
-        BoundedWait(raw_empty(s), phase ^ 1u, abort_flag, a.error, 1);
-        const uint32_t to = base + Smem::kRaw + s * kRawBytes;
-        if constexpr (TYPE == GUFO_CUDA_Q4_K) {
-#pragma unroll 6
-          for (int c = which * 32 + lane; c < kChunks; c += 32 * Q::kLoaders) {
-            const int r = c / kChunksPerRow;
-            const int chunk = c - r * kChunksPerRow;
-            // Rows past the end repeat the last row; their sums are never stored.
-            const int row = min(unit.row0 + r, part.rows - 1);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + c * 16),
-                         "l"(Q::Source(part.w + static_cast<size_t>(row) * part.row_bytes, a.blocks,
-                                       unit.first_block + b, chunk)) : "memory");
-          }
-        } else {
-          // Plane by plane (ql: 8 chunks a row, qh: 4, scales: 1, the slab's d values: 1),
-          // so that a warp's lanes never part ways over which plane a chunk is in and the
-          // offsets of a plane are computed once a block.
-          const int block = unit.first_block + b;
-          const int slab = block / kQ6KSlabBlocks;
-          const int j = block - slab * kQ6KSlabBlocks;
-          const int left = a.blocks - slab * kQ6KSlabBlocks;
-          const int n = left < kQ6KSlabBlocks ? left : kQ6KSlabBlocks;
-          const uint8_t* from = part.w + static_cast<size_t>(slab) * kQ6KSlabBlocks * kQ6KBytes;
-          const int last = part.rows - 1 - unit.row0;
-          auto plane = [&](int src_at, int dst_at, int shift) {
-            // 1 << shift chunks a row.
-            const int items = a.tile_rows << shift;
-#pragma unroll 4
-            for (int c = which * 32 + lane; c < items; c += 32 * Q::kLoaders) {
-              const int r = c >> shift;
-              const int chunk = c & ((1 << shift) - 1);
-              const int row = unit.row0 + min(r, last);
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + r * Q::kRowBytes + dst_at + 16 * chunk),
-                           "l"(from + static_cast<size_t>(row) * part.row_bytes + src_at + 16 * chunk) : "memory");
+  // Every role walks the steps [first, last); the stage counters run on across
+  // units, so the pipeline never drains between them.
+  if (warp == kRawWarp) {
+    // ---- raw blocks ----------------------------------------------------------
+    if (ElectOne()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int step = first; step < last;) {
+        const int u = step / a.blocks;
+        const Unit unit = LocateUnit(a, u);
+        const CUtensorMap* map = &a.maps[unit.part * 3];
+        for (int b = step - u * a.blocks; b < a.blocks && step < last; ++b, ++step) {
+          {
+            BoundedWait<true>(raw_empty(stage), phase ^ 1u, abort_flag, a.error, 1);
+            const uint32_t to = base + raw_at + stage * Q::kRawStride;
+            const uint32_t bar = raw_full(stage);
+            MbarArriveExpectTx(bar, Q::kRawBytes);
+            // Rows past the end of the part arrive as zeros.
+            const int row = unit.row0;
+            if constexpr (TYPE == GUFO_CUDA_Q4_K) {
+              TileCopy(to, map, b * kQ4KBytes, row, bar);
+            } else {
+              // The planar device arrangement (Q6KBlockAt): a slab of n blocks stores
+              // ql n x 128 | qh n x 64 | scales n x 16 | d n x 2.
+              const int slab = b / kQ6KSlabBlocks;
+              const int j = b - slab * kQ6KSlabBlocks;
+              const int n = min(a.blocks - slab * kQ6KSlabBlocks, kQ6KSlabBlocks);
+              const int at = slab * kQ6KSlabBlocks * kQ6KBytes;
+              TileCopy(to + Quant<GUFO_CUDA_Q6_K>::kQl, map, at + 128 * j, row, bar);
+              TileCopy(to + Quant<GUFO_CUDA_Q6_K>::kQh, map + 1, at + 128 * n + 64 * j, row, bar);
+              TileCopy(to + Quant<GUFO_CUDA_Q6_K>::kSc, map + 2, at + 192 * n + 16 * j, row, bar);
+              TileCopy(to + Quant<GUFO_CUDA_Q6_K>::kD, map + 2, at + 208 * n, row, bar);   // the slab's d values
             }
-          };
-          plane(128 * j, 0, 3);
-          plane(128 * n + 64 * j, 128, 2);
-          plane(192 * n + 16 * j, 192, 0);
-          plane(208 * n, 208, 0);
+            if (++stage == a.raw_stages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+          }
         }
-        // Arrives on the stage's barrier once this thread's copies have landed.
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(raw_full(s)) : "memory");
       }
     }
-  } else if (warp == kTileLoaderWarp) {
-    // ---- activation tile loader ------------------------------------------------
+  } else if (warp == kXWarp) {
+    // ---- activation tiles, two (half a step's) per stage ------------------------
     GridDependencyWait();
-    int stage = 0;
-    uint32_t phase = 0;
-    for (int u = blockIdx.x; u < units; u += gridDim.x) {
-      const Unit unit = LocateUnit(a, u);
-      for (int i = 0; i < unit.blocks * 4; ++i) {
-        BoundedWait(x_empty(stage), phase ^ 1u, abort_flag, a.error, 2);
-        if (lane == 0) {
-          MbarArriveExpectTx(x_full(stage), kXTileBytes);
-          BulkCopy(base + Smem::kX + stage * kXTileBytes,
-                   a.xh + (static_cast<size_t>(unit.first_block) * 4 + i) * kXTileBytes, kXTileBytes, x_full(stage));
-        }
-        if (++stage == kXStages) {
-          stage = 0;
-          phase ^= 1u;
+    if (ElectOne()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int step = first; step < last; ++step) {
+        const int u = step / a.blocks;
+        const int group = u % a.groups;
+        const uint8_t* from = a.xh + (static_cast<size_t>(group) * a.blocks + (step - u * a.blocks)) * 2 * x_bytes;
+        for (int t = 0; t < 2; ++t) {
+          BoundedWait<true>(x_empty(stage), phase ^ 1u, abort_flag, a.error, 2);
+          MbarArriveExpectTx(x_full(stage), x_bytes);
+          BulkCopy(base + stage * x_bytes, from + static_cast<size_t>(t) * x_bytes, x_bytes, x_full(stage));
+          if (++stage == a.x_stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
         }
       }
     }
   } else if (warp == kMmaWarp) {
     // ---- MMA issue ---------------------------------------------------------
-    // kind::f16, fp32 accumulate, fp16 A and B, both K-major, N = 256, M = 128.
-    const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(a.tile_rows >> 3) << 17) |
-                           (static_cast<uint32_t>(kTokenRows >> 4) << 24);
-    int ws = 0, xs = 0;
-    uint32_t w_phase = 0, x_phase = 0;
-    int n = 0;   // units done
-    for (int u = blockIdx.x; u < units; u += gridDim.x, ++n) {
-      const Unit unit = LocateUnit(a, u);
-      const int buffer = n & 1;
-      // The epilogue of the unit before last has read this accumulator.
-      BoundedWait(acc_empty(buffer), ((n >> 1) & 1u) ^ 1u, abort_flag, a.error, 8);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t accumulator = tmem + static_cast<uint32_t>(buffer * kTileRows);
-      for (int i = 0; i < unit.blocks * 4; ++i) {
-        BoundedWait(w_full(ws), w_phase, abort_flag, a.error, 3);
-        BoundedWait(x_full(xs), x_phase, abort_flag, a.error, 7);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (lane == 0) {
-          const uint64_t desc_x = TileDescriptor(base + Smem::kX + xs * kXTileBytes);
-          const uint64_t desc_w = TileDescriptor(base + Smem::kW + ws * kWTileBytes);
+    // kind::f16, fp32 accumulate, fp16 A and B, both K-major, M = 128.
+    if (ElectOne()) {
+      const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(a.n >> 3) << 17) |
+                             (static_cast<uint32_t>(kTileRows >> 4) << 24);
+      int xs = 0;              // stage of the step's first two activation tiles
+      uint32_t x_phase = 0;
+      uint32_t w_phase = 0;    // slots are filled once per block: they flip together
+      int acc = 0;
+      uint32_t acc_phase = 0;
+      for (int step = first; step < last;) {
+        const int end = min((step / a.blocks + 1) * a.blocks, last);
+        // The epilogue has read what this accumulator held before.
+        BoundedWait(acc_empty(acc), acc_phase ^ 1u, abort_flag, a.error, 8);
+        const uint32_t accumulator = tmem + kAccColumn + static_cast<uint32_t>(acc * a.n);
+        for (uint32_t more = 0; step < end; ++step, more = 1) {
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            BoundedWait(x_full(xs), x_phase, abort_flag, a.error, 7);
+            const uint64_t desc_x = TileDescriptor(base + xs * x_bytes);
 #pragma unroll
-          for (int k = 0; k < kTileK / 16; ++k) {
-            // 16 values = 32 bytes further along K inside the swizzled rows.
-            MmaF16(accumulator, desc_x + 2u * k, desc_w + 2u * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+            for (int t = 0; t < 2; ++t) {
+              const int g = 2 * half + t;
+              BoundedWait(w_full(g), w_phase, abort_flag, a.error, 3);
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint32_t slot = tmem + static_cast<uint32_t>(g * kSlotColumns);
+              const uint64_t desc = desc_x + static_cast<uint64_t>(t * (x_bytes >> 5));   // 16-byte units
+#pragma unroll
+              for (int k = 0; k < kTileK / 16; ++k) {
+                // 16 values: eight columns of the slot, 32 bytes of the swizzled rows.
+                MmaF16(accumulator, slot + 8u * k, desc + 2u * k, idesc, k > 0 || g > 0 ? 1u : more);
+              }
+              // A commit arrives once everything issued so far has retired.
+              MmaCommit(w_empty(g));
+            }
+            MmaCommit(x_empty(xs));
+            if (++xs == a.x_stages) {
+              xs = 0;
+              x_phase ^= 1u;
+            }
           }
-          // Each commit arrives once everything issued so far has retired.
-          MmaCommit(w_empty(ws));
-          MmaCommit(x_empty(xs));
-          if (i == unit.blocks * 4 - 1) {
-            MmaCommit(acc_full(buffer));
-          }
-        }
-        __syncwarp();
-        if (++ws == kWStages) {
-          ws = 0;
           w_phase ^= 1u;
         }
-        if (++xs == kXStages) {
-          xs = 0;
-          x_phase ^= 1u;
-        }
+        MmaCommit(acc_full(acc));
+        acc ^= 1;
+        acc_phase ^= acc == 0 ? 1u : 0u;
       }
     }
-  } else if (warp >= kEpilogueWarp && warp < kEpilogueWarp + kEpilogueWarps) {
-    // ---- epilogue: lane of tensor memory = token row, column = weight row;
-    // warp q reads quarter q, i.e. tokens q, q + 4, q + 8, ... -------------------
+  } else if (warp >= kEpilogueWarp && warp < kEpilogueWarp + 4) {
+    // ---- epilogue: warp q reads lanes 32 q .. 32 q + 31, i.e. weight rows ------
+    GridDependencyWait();
     const int quarter = warp - kEpilogueWarp;
-    const int token = lane * 4 + quarter;
-    int n = 0;
-    for (int u = blockIdx.x; u < units; u += gridDim.x, ++n) {
+    const int local = quarter * 32 + lane;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int step = first; step < last;) {
+      const int u = step / a.blocks;
       const Unit unit = LocateUnit(a, u);
       const TcPart& part = a.parts[unit.part];
-      const int buffer = n & 1;
-      const bool ready = BoundedWait(acc_full(buffer), (n >> 1) & 1u, abort_flag, a.error, 6);
+      const int begin = u * a.blocks;
+      const int end = min(begin + a.blocks, last);
+      const bool whole = step == begin && end == begin + a.blocks;
+      const int token0 = unit.group * a.n;
+      const int columns = min(a.n, a.tokens - token0);
+      asm volatile("bar.sync 1, 128;" ::: "memory");   // the factors of the unit before have been read
+      for (int i = local; i < columns; i += 128) {
+        factor[i] = __ldcg(a.unscale + token0 + i);
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      const bool ready = BoundedWait<true>(acc_full(acc), acc_phase, abort_flag, a.error, 6);
+      if (!whole && end == last) {
+        break;   // the share of a cut tile that ends the range: by all warps, below
+      }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const bool live = ready && token < a.tokens;
-      const float unscale = live ? a.unscale[token] : 0.f;
-      float* out = part.out + static_cast<size_t>(unit.split) * part.split_stride +
-                   static_cast<size_t>(token) * part.out_stride + unit.row0;
-      // 16-byte stores where the output rows allow them.
-      const bool vector_stores = (reinterpret_cast<uintptr_t>(part.out) & 15) == 0 && part.out_stride % 4 == 0 &&
-                                 part.split_stride % 4 == 0;
-      // A quarter without tokens is skipped (uniform over the warp, as
-      // tcgen05.ld requires).
-      if (quarter < a.tokens) {
-        for (int col0 = 0; col0 < a.tile_rows; col0 += 16) {
-          float v[16];
-          TmemLoad16(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + buffer * kTileRows + col0, v);
-          if (live) {
-            if (vector_stores && unit.row0 + col0 + 16 <= part.rows) {
+      const uint32_t from = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kAccColumn +
+                            static_cast<uint32_t>(acc * a.n);
+      const int row = unit.row0 + local;
+      float* to = part.out + static_cast<size_t>(token0) * a.out_stride + row;
+      float* partial = PartialColumn(a, blockIdx.x, 0, 0) + local;
+      for (int col0 = 0; col0 < columns; col0 += 16) {
+        float v[16];
+        TmemLoad16(from + col0, v);
+        if (!whole) {
 #pragma unroll
-              for (int j = 0; j < 16; j += 4) {
-                *reinterpret_cast<float4*>(out + col0 + j) =
-                    make_float4(v[j] * unscale, v[j + 1] * unscale, v[j + 2] * unscale, v[j + 3] * unscale);
-              }
-            } else {
+          for (int j = 0; j < 16; ++j) {
+            __stcg(partial + (col0 + j) * kTileRows, v[j]);
+          }
+        } else if (ready && row < part.rows) {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                if (unit.row0 + col0 + j < part.rows) {
-                  out[col0 + j] = v[j] * unscale;
-                }
-              }
+          for (int j = 0; j < 16; ++j) {
+            if (col0 + j < columns) {
+              to[static_cast<size_t>(col0 + j) * a.out_stride] = v[j] * factor[col0 + j];
             }
           }
         }
@@ -579,153 +757,177 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
-        MbarArrive(acc_empty(buffer));
+        MbarArrive(acc_empty(acc));
       }
-    }
-  } else if (warp < kDequantThreads / 32) {
-    // ---- dequant: threads r and r + 256 own weight row r; all sixteen warps
-    // work on the same tile, in the order the MMA consumes them (the first
-    // thread takes the first half of each tile row, the second the other).
-    // Tile g = 4 * block + t of the thread block's stream lands in buffer g % stages.
-    const int r = threadIdx.x & (kTileRows - 1);
-    const int half = threadIdx.x / kTileRows;
-    const bool active = r < a.tile_rows;   // rows past the tile's height: the barriers only
-    int i = 0;   // blocks done so far
-    for (int u = blockIdx.x; u < units; u += gridDim.x) {
-      const Unit unit = LocateUnit(a, u);
-      for (int b = 0; b < unit.blocks; ++b, ++i) {
-        const int s = i % kRawStages;
-        const uint32_t phase = (i / kRawStages) & 1u;
-        BoundedWait(raw_full(s), phase, abort_flag, a.error, 4);
-        if constexpr (TYPE == GUFO_CUDA_Q4_K) {
-          const uint8_t* block = smem + Smem::kRaw + s * kRawBytes + r * Q::kRowBytes;
-          const uint4 head = *reinterpret_cast<const uint4*>(block);
-          const float d = HalfBitsToFloat(static_cast<uint16_t>(head.x & 0xFFFF));
-          const float dmin = HalfBitsToFloat(static_cast<uint16_t>(head.x >> 16));
-  #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const int g = 4 * i + t;
-            const int ws = g % kWStages;
-            const uint32_t w_phase = static_cast<uint32_t>(g / kWStages) & 1u;
-            // This thread's sub-block of the pair: its scale and the constant
-            // 8 * scale - offset, each doubled into an fp16 pair.
-            int sc, m;
-            ScaleMinK4(2 * t + half, head.y, head.z, head.w, &sc, &m);
-            auto pair = [](float v) {
-              const __half2 h = __float2half2_rn(v);
-              return *reinterpret_cast<const uint32_t*>(&h);
-            };
-            const float scale = d * static_cast<float>(sc);
-            const uint32_t scale2 = pair(scale);
-            const uint32_t constant2 = pair(fmaf(8.0f, scale, -dmin * static_cast<float>(m)));
-            const uint4 q0 = *reinterpret_cast<const uint4*>(block + 16 + 32 * t);
-            const uint4 q1 = *reinterpret_cast<const uint4*>(block + 32 + 32 * t);
-            const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-            BoundedWait(w_empty(ws), w_phase ^ 1u, abort_flag, a.error, 5);
-            uint8_t* tile_row = smem + Smem::kW + ws * kWTileBytes + r * 128;
-  #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              // Chunk c: values 8c .. 8c + 7 of the low sub-block; chunk 4 + c: of the high one.
-              if (active) {
-                const uint4 eight = half == 0 ? EightWeights<false>(words[2 * c], words[2 * c + 1], scale2, constant2)
-                                              : EightWeights<true>(words[2 * c], words[2 * c + 1], scale2, constant2);
-                *reinterpret_cast<uint4*>(tile_row + (((4 * half + c) ^ (r & 7)) << 4)) = eight;
-              }
-            }
-            // Make the generic-proxy stores visible to the tensor core's reads; one
-            // lane then arrives for the warp.
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-              MbarArrive(w_full(ws));
-            }
-          }
-        } else {
-          // Tile t of the block holds values 64t .. 64t + 63: half n = t / 2 of
-          // the block, the low (t even) or high nibbles of its 64 ql bytes, two
-          // bits of its 32 qh bytes: w = d * sc * (code - 32), code = nibble |
-          // two bits of qh << 4 (DequantQ6_K, src/core/quant.cpp:98-125). This
-          // thread takes chunks 4 * half .. 4 * half + 3 of every tile: ql bytes
-          // 32 * half .. + 31 of the tile's half.
-          const uint8_t* block = smem + Smem::kRaw + s * kRawBytes + r * Q::kRowBytes;
-          const float d = HalfBitsToFloat(*reinterpret_cast<const uint16_t*>(
-              block + 208 + 2 * ((unit.first_block + b) % kQ6KSlabBlocks)));
-#pragma unroll
-          for (int n = 0; n < 2; ++n) {
-            const uint4 l0 = *reinterpret_cast<const uint4*>(block + 64 * n + 32 * half);
-            const uint4 l1 = *reinterpret_cast<const uint4*>(block + 64 * n + 32 * half + 16);
-            const uint4 h0 = *reinterpret_cast<const uint4*>(block + 128 + 32 * n);
-            const uint4 h1 = *reinterpret_cast<const uint4*>(block + 128 + 32 * n + 16);
-            const uint2 sc8 = *reinterpret_cast<const uint2*>(block + 192 + 8 * n);
-            const uint32_t ql[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-            const uint32_t qh[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-            // Scale of 16-value group j of this half of the block (int8).
-            auto scale = [&](int j) {
-              const uint32_t word = j < 4 ? sc8.x : sc8.y;
-              return d * static_cast<float>(static_cast<int>(word << (24 - 8 * (j & 3))) >> 24);
-            };
-#pragma unroll
-            for (int tt = 0; tt < 2; ++tt) {
-              const int g = 4 * i + 2 * n + tt;
-              const int ws = g % kWStages;
-              const uint32_t w_phase = static_cast<uint32_t>(g / kWStages) & 1u;
-              BoundedWait(w_empty(ws), w_phase ^ 1u, abort_flag, a.error, 5);
-              uint8_t* tile_row = smem + Smem::kW + ws * kWTileBytes + r * 128;
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                // Chunk 4 * half + k: values from ql bytes 32 * half + 8k .., their two
-                // high bits from qh bytes 8k .. at bit 2 * (2 tt + half).
-                const int shift = 2 * (2 * tt + half);
-                const uint32_t q0 = ql[2 * k], q1 = ql[2 * k + 1];
-                const uint32_t n0 = tt == 0 ? (q0 & 0x0F0F0F0Fu) : ((q0 >> 4) & 0x0F0F0F0Fu);
-                const uint32_t n1 = tt == 0 ? (q1 & 0x0F0F0F0Fu) : ((q1 >> 4) & 0x0F0F0F0Fu);
-                const uint32_t b0 = shift <= 4 ? (qh[2 * k] << (4 - shift)) : (qh[2 * k] >> (shift - 4));
-                const uint32_t b1 = shift <= 4 ? (qh[2 * k + 1] << (4 - shift)) : (qh[2 * k + 1] >> (shift - 4));
-                const float sc = scale(4 * tt + 2 * half + (k >> 1));
-                if (active) {
-                  *reinterpret_cast<uint4*>(tile_row + (((4 * half + k) ^ (r & 7)) << 4)) =
-                      EightCodes(n0 | (b0 & 0x30303030u), n1 | (b1 & 0x30303030u), sc);
-                }
-              }
-              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-              __syncwarp();
-              if (lane == 0) {
-                MbarArrive(w_full(ws));
-              }
-            }
+      acc ^= 1;
+      acc_phase ^= acc == 0 ? 1u : 0u;
+      if (!whole) {
+        // The share of a cut tile that opens the range: left in scratch.
+        __threadfence();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (local == 0) {
+          const CutTile cut = LocateCut(a, blockIdx.x, begin);
+          if (atomicAdd(a.counters + cut.from, 1u) == static_cast<unsigned>(cut.to - cut.from)) {
+            finish = u + 1;
           }
         }
-        __syncwarp();
-        if (lane == 0) {
-          MbarArrive(raw_empty(s));
-        }
       }
+      step = end;
     }
+  } else if (warp < kDequantWarps) {
+    // ---- dequant: group p takes pair p of every block; a thread owns one row ------
+    const DequantPlace at{raw_full(0), raw_empty(0), w_full(warp >> 2), w_empty(warp >> 2), smem + raw_at,
+                          tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) +
+                              static_cast<uint32_t>((warp >> 2) * kSlotColumns),
+                          (warp & 3) * 32 + lane, warp >> 2};
+    DequantSteps<TYPE>(a, at, first, last, abort_flag);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) {
+  // Cut tiles. Most are cut in two: the second share opens its block's range and
+  // is long in scratch when the first, which ends its block's range, is complete in
+  // tensor memory; all warps then add the one to the other.
+  const int tail_unit = (last - 1) / a.blocks;
+  const int tail_begin = tail_unit * a.blocks;
+  const bool tail_opens = first >= tail_begin;   // the block's only share
+  if ((first > tail_begin || last < tail_begin + a.blocks) && warp < kDequantWarps + 4) {
+    const Unit unit = LocateUnit(a, tail_unit);
+    const TcPart& part = a.parts[unit.part];
+    const CutTile cut = LocateCut(a, blockIdx.x, tail_begin);
+    const unsigned others = static_cast<unsigned>(cut.to - cut.from);
+    if (threadIdx.x == 0) {
+      unsigned seen;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.counters + cut.from) : "memory");
+      others_done = seen == others;
+    }
+    asm volatile("bar.sync 2, %0;" ::"n"((kDequantWarps + 4) * 32) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const bool finishes = *const_cast<volatile int*>(&others_done) != 0;
+    const int token0 = unit.group * a.n;
+    const int columns = min(a.n, a.tokens - token0);
+    const int local = (warp & 3) * 32 + lane;
+    const int row = unit.row0 + local;
+    const int acc = (tail_unit - first / a.blocks) & 1;
+    const uint32_t from = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kAccColumn +
+                          static_cast<uint32_t>(acc * a.n);
+    for (int col0 = (warp >> 2) * 16; col0 < columns; col0 += 16 * (kGroups + 1)) {
+      float v[16];
+      TmemLoad16(from + col0, v);
+      if (!finishes) {
+        float* partial = PartialColumn(a, blockIdx.x, tail_opens ? 0 : 1, col0) + local;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          __stcg(partial + j * kTileRows, v[j]);
+        }
+        continue;
+      }
+      // In block order, this block's own share at its place.
+      float sum[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        sum[j] = 0.f;
+      }
+      for (int c = cut.from; c <= cut.to; ++c) {
+        if (c == static_cast<int>(blockIdx.x)) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            sum[j] += v[j];
+          }
+        } else {
+          const float* add = PartialColumn(a, c, CutSlot(a, cut, c, tail_begin), col0) + local;
+          float w[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            w[j] = __ldcg(add + j * kTileRows);
+          }
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            sum[j] += w[j];
+          }
+        }
+      }
+      if (*abort_flag == 0 && row < part.rows) {
+        float* to = part.out + static_cast<size_t>(token0) * a.out_stride + row;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (col0 + j < columns) {
+            to[static_cast<size_t>(col0 + j) * a.out_stride] = sum[j] * factor[col0 + j];
+          }
+        }
+      }
+    }
+    if (finishes) {
+      if (threadIdx.x == 0) {
+        a.counters[cut.from] = 0;   // for the next launch
+      }
+    } else {
+      __threadfence();
+      asm volatile("bar.sync 2, %0;" ::"n"((kDequantWarps + 4) * 32) : "memory");
+      if (threadIdx.x == 0) {
+        others_done = atomicAdd(a.counters + cut.from, 1u) == others ? 2 : 0;
+      }
+      asm volatile("bar.sync 2, %0;" ::"n"((kDequantWarps + 4) * 32) : "memory");
+      if (*const_cast<volatile int*>(&others_done) == 2) {
+        AddShares(a, tail_unit, cut);
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  __syncthreads();
+  if (finish != 0 && warp < kDequantWarps + 4) {
+    AddShares(a, finish - 1, LocateCut(a, blockIdx.x, (finish - 1) * a.blocks));
+  }
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemColumns) : "memory");
   }
 }
 
 // One block per token row: scales the row by a power of two so that its largest
 // magnitude lands in [2^13, 2^14), rounds to fp16 and writes the row into every
-// tile image at its swizzled place. Rows past `tokens` are zero.
-__global__ void __launch_bounds__(256)
-StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int npad, uint8_t* __restrict__ xh,
+// tile image of its group at its swizzled place. Rows past `tokens` are zero.
+// `six`: tile 2 h + j of a block holds Q6_K's runs j and j + 2 of half h (the
+// pair a dequant group turns out together), else values 64 t .. 64 t + 63.
+__global__ void __launch_bounds__(1024)
+StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int group_rows, int six, uint8_t* __restrict__ xh,
                 float* __restrict__ unscale) {
-  __shared__ uint32_t warp_top[8];
+  __shared__ uint32_t warp_top[32];
+  const int threads = static_cast<int>(blockDim.x);
+  GridLaunchDependents();
   GridDependencyWait();
-  const int n = blockIdx.x;                  // token
-  const int image_row = TokenRow(n);        // its row of the MMA's M
+  const int token = blockIdx.x;
+  const int group = token / group_rows;
+  const int image_row = token - group * group_rows;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
+  const float4* row = reinterpret_cast<const float4*>(x + static_cast<size_t>(token) * cols);
+  // A thread's first chunks of eight values stay in registers between the two passes.
+  constexpr int kKeep = 2;
+  float4 keep[kKeep][2];
   float up = 1.0f;
-  if (n < tokens) {
+  if (token < tokens) {
     uint32_t top = 0;
-    for (int i = threadIdx.x; i < cols; i += 256) {
-      top = max(top, __float_as_uint(x[static_cast<size_t>(n) * cols + i]) & 0x7FFFFFFFu);
+    auto see = [&](const float4& v) {
+      top = max(max(top, __float_as_uint(v.x) & 0x7FFFFFFFu), __float_as_uint(v.y) & 0x7FFFFFFFu);
+      top = max(max(top, __float_as_uint(v.z) & 0x7FFFFFFFu), __float_as_uint(v.w) & 0x7FFFFFFFu);
+    };
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i) {
+      const int chunk = threadIdx.x + threads * i;
+      if (chunk < cols / 8) {
+        keep[i][0] = row[2 * chunk];
+        keep[i][1] = row[2 * chunk + 1];
+      } else {
+        keep[i][0] = keep[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+    for (int i = threadIdx.x + 2 * threads * kKeep; i < cols / 4; i += threads) {
+      see(row[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i) {
+      see(keep[i][0]);
+      see(keep[i][1]);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -736,8 +938,7 @@ StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int npad, uin
     }
     __syncthreads();
     top = warp_top[0];
-#pragma unroll
-    for (int w = 1; w < 8; ++w) {
+    for (int w = 1; w < threads / 32; ++w) {
       top = max(top, warp_top[w]);
     }
     // Biased exponent e of the maximum: |x| < 2^(e - 126). Scale by 2^(140 - e)
@@ -748,46 +949,39 @@ StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int npad, uin
     shift = max(-126, min(126, shift));
     up = __uint_as_float(static_cast<uint32_t>(127 + shift) << 23);
     if (threadIdx.x == 0) {
-      unscale[n] = __uint_as_float(static_cast<uint32_t>(127 - shift) << 23);
+      unscale[token] = __uint_as_float(static_cast<uint32_t>(127 - shift) << 23);
     }
   } else if (threadIdx.x == 0) {
-    unscale[n] = 0.f;
+    unscale[token] = 0.f;
   }
-  const size_t tile_bytes = static_cast<size_t>(npad) * (kTileK * 2);
-  for (int chunk = threadIdx.x; chunk < cols / 8; chunk += 256) {
-    const int k = chunk * 8;
-    uint4 packed = make_uint4(0u, 0u, 0u, 0u);
-    if (n < tokens) {
-      const float4 v0 = *reinterpret_cast<const float4*>(x + static_cast<size_t>(n) * cols + k);
-      const float4 v1 = *reinterpret_cast<const float4*>(x + static_cast<size_t>(n) * cols + k + 4);
-      // Values (0, 2, 1, 3) of every four: the order of K the weight tiles use.
-      const __half2 h0 = __floats2half2_rn(v0.x * up, v0.z * up), h1 = __floats2half2_rn(v0.y * up, v0.w * up);
-      const __half2 h2 = __floats2half2_rn(v1.x * up, v1.z * up), h3 = __floats2half2_rn(v1.y * up, v1.w * up);
-      packed = make_uint4(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1),
-                          *reinterpret_cast<const uint32_t*>(&h2), *reinterpret_cast<const uint32_t*>(&h3));
+  const size_t tile_bytes = static_cast<size_t>(group_rows) * (kTileK * 2);
+  uint8_t* image = xh + static_cast<size_t>(group) * (cols / kTileK) * tile_bytes + static_cast<size_t>(image_row) * 128;
+  auto put = [&](int chunk, const float4& v0, const float4& v1) {
+    // Values (0, 2, 1, 3) of every four: the order of K the weights use.
+    const __half2 h0 = __floats2half2_rn(v0.x * up, v0.z * up), h1 = __floats2half2_rn(v0.y * up, v0.w * up);
+    const __half2 h2 = __floats2half2_rn(v1.x * up, v1.z * up), h3 = __floats2half2_rn(v1.y * up, v1.w * up);
+    const uint4 packed = make_uint4(HalfBits(h0), HalfBits(h1), HalfBits(h2), HalfBits(h3));
+    int tile = chunk >> 3;   // of eight chunks
+    int c = chunk & 7;
+    if (six != 0) {
+      const int in_block = chunk & 31;               // 32 chunks a block
+      const int h = in_block >> 4, k = (in_block >> 2) & 3;
+      tile = (chunk >> 5) * 4 + 2 * h + (k & 1);
+      c = 4 * (k >> 1) + (in_block & 3);
     }
-    const int tile = k / kTileK;
-    const int c = (k % kTileK) / 8;
-    *reinterpret_cast<uint4*>(xh + tile * tile_bytes + static_cast<size_t>(image_row) * 128 +
-                              ((c ^ (image_row & 7)) << 4)) = packed;
+    *reinterpret_cast<uint4*>(image + tile * tile_bytes + ((c ^ (image_row & 7)) << 4)) = packed;
+  };
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < kKeep; ++i) {
+    const int chunk = threadIdx.x + threads * i;
+    if (chunk < cols / 8) {
+      put(chunk, token < tokens ? keep[i][0] : zero, token < tokens ? keep[i][1] : zero);
+    }
   }
-}
-
-// y[t][row] = sum over the K ranges, in order, of their partial sums.
-__global__ void __launch_bounds__(256)
-SumSplitsKernel(const float* __restrict__ partial, int ksplit, size_t split_stride, int rows, int tokens,
-                float* __restrict__ y, int y_stride) {
-  GridDependencyWait();
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t = blockIdx.y;
-  if (row >= rows || t >= tokens) {
-    return;
+  for (int chunk = threadIdx.x + threads * kKeep; chunk < cols / 8; chunk += threads) {
+    put(chunk, token < tokens ? row[2 * chunk] : zero, token < tokens ? row[2 * chunk + 1] : zero);
   }
-  float total = 0.f;
-  for (int s = 0; s < ksplit; ++s) {
-    total += partial[static_cast<size_t>(s) * split_stride + static_cast<size_t>(t) * rows + row];
-  }
-  y[static_cast<size_t>(t) * y_stride + row] = total;
 }
 
 int ReserveTc(gufo_cuda_ctx* ctx, size_t bytes) {
@@ -796,14 +990,179 @@ int ReserveTc(gufo_cuda_ctx* ctx, size_t bytes) {
   }
   // An outgrown block is kept (a captured graph may hold it); its error word
   // is not carried over: a failure is read from the current block.
-  const int rc = ctx->GrowScratch(&ctx->tc_scratch, &ctx->tc_scratch_bytes, bytes, 1u << 20, "tcgen05 gemm");
+  const int rc = ctx->GrowScratch(&ctx->tc_scratch, &ctx->tc_scratch_bytes, bytes, kScratchFloor, "tcgen05 gemm");
   if (rc != GUFO_CUDA_OK) {
     return rc;
   }
-  GUFO_CUDA_TRY(cudaMemsetAsync(ctx->tc_scratch, 0, 256, ctx->stream));
+  GUFO_CUDA_TRY(cudaMemsetAsync(ctx->tc_scratch, 0, kHeaderBytes, ctx->stream));
   return GUFO_CUDA_OK;
 }
 
+// cuTensorMapEncodeTiled, a host function of the driver (looked up once).
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiled TensorMapEncoder() {
+  static const EncodeTiled encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) !=
+            cudaSuccess || found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<EncodeTiled>(fn);
+  }();
+  return encode;
+}
+
+// A map of `rows` rows of `row_bytes` bytes whose boxes are 128 rows of `width` bytes.
+int EncodeRows(CUtensorMap* map, const uint8_t* data, int rows, int row_bytes, int width, CUtensorMapSwizzle swizzle) {
+  const EncodeTiled encode = TensorMapEncoder();
+  if (encode == nullptr) {
+    return Fail(GUFO_CUDA_RUNTIME, "tcgen05 gemm: the driver has no cuTensorMapEncodeTiled");
+  }
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(row_bytes), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(width), kTileRows};
+  const cuuint32_t ones[2] = {1, 1};
+  const CUresult e = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(data), dims, strides, box, ones,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return e == CUDA_SUCCESS ? GUFO_CUDA_OK
+                           : Fail(GUFO_CUDA_RUNTIME, "tcgen05 gemm: tensor map of " + std::to_string(rows) + " x " +
+                                                         std::to_string(row_bytes) + " bytes: error " +
+                                                         std::to_string(static_cast<int>(e)));
+}
+
+// How a product of `tokens` rows is cut: token groups of n columns, thread blocks.
+struct Plan {
+  int groups, n, grid, units;
+};
+
+// Cycles of a step (256 values of 128 rows): the slower of the tensor core (16
+// MMAs of n / 2 cycles) and the dequantization with its hand-overs (measured).
+double StepCycles(int type, int n) {
+  const double mma = 8.0 * n + 120;
+  const double dequant = (type == GUFO_CUDA_Q4_K ? 1450 : 2000) + 4.0 * n;
+  return mma > dequant ? mma : dequant;
+}
+
+Plan PlanTc(const GemvArgs& base, const std::vector<int>& parts, int type, int tokens, int sm_count) {
+  const int blocks = base.cols / kSuperBlock;
+  int tiles = 0;
+  for (int p : parts) {
+    tiles += (base.parts[p].rows + kTileRows - 1) / kTileRows;
+  }
+  Plan best{};
+  double best_cost = 1e30;
+  const int least = (tokens + kMaxN - 1) / kMaxN;
+  for (int groups = least; groups <= least + 3; ++groups) {
+    const int n = ((tokens + groups - 1) / groups + 15) / 16 * 16;
+    if ((groups - 1) * n >= tokens) {
+      continue;   // a group without tokens
+    }
+    const int units = tiles * groups;
+    const int64_t total = static_cast<int64_t>(units) * blocks;
+    auto consider = [&](int grid) {
+      if (grid < 1 || grid > sm_count || grid > total) {
+        return;
+      }
+      // Thread blocks that share a tile: one more than the even share where the cuts
+      // do not fall on tile ends. Two shares of which one is complete early cost
+      // little; others end together, and their sums go through scratch (measured
+      // for 96 tiles on 148 blocks and 20 tiles on 40 to 148).
+      const int sharing = units % grid == 0 ? 1 : (grid % units == 0 ? grid / units : (grid + units - 1) / units + 1);
+      const double fix = sharing <= 1 ? 0 : (units > grid ? 1500 : 9000 + 60.0 * n + 500.0 * sharing);
+      const double cost = static_cast<double>((total + grid - 1) / grid) * StepCycles(type, n) + fix + 30.0 * n;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = Plan{groups, n, grid, units};
+      }
+    };
+    consider(sm_count);
+    for (int share = 1; share * units <= sm_count; ++share) {
+      consider(share * units);
+    }
+    for (int rounds = 2; rounds <= 4; ++rounds) {
+      if (units % rounds == 0) {
+        consider(units / rounds);
+      }
+    }
+  }
+  return best;
+}
+
+template <int TYPE>
+int LaunchPlan(gufo_cuda_ctx* ctx, const GemvArgs& base, const std::vector<int>& group, int tokens) {
+  using Q = Quant<TYPE>;
+  static bool configured[16] = {};
+  if (!configured[ctx->device & 15]) {
+    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemmTc<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit - 3072));
+    configured[ctx->device & 15] = true;
+  }
+  const int cols = base.cols;
+  const int blocks = cols / kSuperBlock;
+  const Plan plan = PlanTc(base, group, TYPE, tokens, ctx->sm_count);
+  // Scratch: header (error word, counters), tile images, unscale factors, partial sums.
+  const size_t rows = static_cast<size_t>(plan.groups) * plan.n;
+  const size_t unscale_at = kHeaderBytes + rows * cols * 2;
+  const size_t partial_at = (unscale_at + rows * 4 + 255) / 256 * 256;
+  const size_t partial_bytes = static_cast<size_t>(plan.grid) * 2 * kTileRows * plan.n * 4;
+  int rc = ReserveTc(ctx, partial_at + partial_bytes);
+  if (rc != GUFO_CUDA_OK) {
+    return rc;
+  }
+  TcGemmArgs args{};
+  args.blocks = blocks;
+  args.groups = plan.groups;
+  args.n = plan.n;
+  args.units = plan.units;
+  args.per = plan.units * blocks / plan.grid;
+  args.extra = plan.units * blocks % plan.grid;
+  args.xh = ctx->tc_scratch + kHeaderBytes;
+  args.unscale = reinterpret_cast<float*>(ctx->tc_scratch + unscale_at);
+  args.partial = reinterpret_cast<float*>(ctx->tc_scratch + partial_at);
+  args.counters = reinterpret_cast<unsigned*>(ctx->tc_scratch + 256);
+  args.tokens = tokens;
+  args.out_stride = base.y_stride;
+  args.error = reinterpret_cast<int*>(ctx->tc_scratch);
+  for (int p : group) {
+    const GemvPart& part = base.parts[p];
+    const int at = args.nparts++;
+    args.parts[at] = {part.rows, (part.rows + kTileRows - 1) / kTileRows, base.y + part.out_offset};
+    CUtensorMap* maps = &args.maps[at * 3];
+    if (TYPE == GUFO_CUDA_Q4_K) {
+      rc = EncodeRows(maps, part.data, part.rows, part.row_bytes, kQ4KBytes, CU_TENSOR_MAP_SWIZZLE_NONE);
+    } else {
+      rc = EncodeRows(maps, part.data, part.rows, part.row_bytes, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+      rc = rc != GUFO_CUDA_OK ? rc : EncodeRows(maps + 1, part.data, part.rows, part.row_bytes, 64, CU_TENSOR_MAP_SWIZZLE_64B);
+      rc = rc != GUFO_CUDA_OK ? rc : EncodeRows(maps + 2, part.data, part.rows, part.row_bytes, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
+    }
+    if (rc != GUFO_CUDA_OK) {
+      return rc;
+    }
+  }
+  // Raw blocks (one a step) and activation stages (two a step), as deep in time.
+  const int x_bytes = 2 * plan.n * kTileK * 2;
+  const int room = kSharedLimit - 4096;
+  args.raw_stages = kMaxStages;
+  do {
+    --args.raw_stages;
+    args.x_stages = (room - args.raw_stages * Q::kRawStride) / x_bytes;
+    args.x_stages = args.x_stages < kMaxStages ? args.x_stages : kMaxStages;
+  } while (args.raw_stages > 2 && args.x_stages < 2 * args.raw_stages);
+  const size_t smem = 1024 + static_cast<size_t>(args.x_stages) * x_bytes + static_cast<size_t>(args.raw_stages) * Q::kRawStride;
+  // A thread for every two chunks of eight values of a row.
+  const int stage_threads = cols <= 4096 ? 256 : (cols <= 8192 ? 512 : 1024);
+  GUFO_CUDA_TRY(LaunchOverlapped(StageHalfKernel, dim3(static_cast<unsigned>(rows)), dim3(stage_threads), 0, ctx->stream, 1, base.x,
+                                 tokens, cols, plan.n, TYPE == GUFO_CUDA_Q6_K ? 1 : 0, const_cast<uint8_t*>(args.xh),
+                                 const_cast<float*>(args.unscale)));
+  GUFO_CUDA_TRY(LaunchOverlapped(GemmTc<TYPE>, dim3(plan.grid), dim3(kTcThreads), smem, ctx->stream, 1, args));
+  ctx->launches.fetch_add(2);
+  return GUFO_CUDA_OK;
+}
 
 }  // namespace
 
@@ -812,175 +1171,30 @@ bool TcGemmRuns(const gufo_cuda_ctx* ctx, int type, int cols, int tokens) {
     return false;
   }
   // "tc_gemm" = 2 sends every product of 16 or more rows here (tests).
-  const int least = ctx->tc_gemm_all ? 16 : (type == GUFO_CUDA_Q6_K ? kTcMinTokensQ6K : kTcMinTokens);
+  const int least = ctx->tc_gemm_all ? 16 : kTcMinTokens;
   return (type == GUFO_CUDA_Q4_K || type == GUFO_CUDA_Q6_K) && tokens >= least;
 }
 
-// Scratch layout: [0, 256) error word; then the tile images, the unscale
-// factors, and the partial sums of a split product.
 int LaunchGemmTc(gufo_cuda_ctx* ctx, const GemvArgs& base, int tokens) {
-  const int cols = base.cols;
-  const int blocks = cols / kSuperBlock;
-  static bool configured[16] = {};
-  if (!configured[ctx->device & 15]) {
-    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemmTc<GUFO_CUDA_Q4_K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       Smem<GUFO_CUDA_Q4_K>::kBytes));
-    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemmTc<GUFO_CUDA_Q6_K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       Smem<GUFO_CUDA_Q6_K>::kBytes));
-    configured[ctx->device & 15] = true;
+  for (int p = 0; p < base.nparts; ++p) {
+    if ((reinterpret_cast<uintptr_t>(base.parts[p].data) & 15) != 0 || base.parts[p].row_bytes % 16 != 0) {
+      return Fail(GUFO_CUDA_BAD_ARGUMENT, "tcgen05 gemm: weight rows must be 16-byte aligned");
+    }
   }
-  // Launch groups: parts of one block format, up to kTcMaxParts each.
-  std::vector<std::vector<int>> groups;
+  // Parts of one block format share a launch, up to kTcMaxParts each.
   for (int type : {GUFO_CUDA_Q4_K, GUFO_CUDA_Q6_K}) {
     std::vector<int> group;
-    for (int p = 0; p < base.nparts; ++p) {
-      if ((reinterpret_cast<uintptr_t>(base.parts[p].data) & 15) != 0 || base.parts[p].row_bytes % 16 != 0) {
-        return Fail(GUFO_CUDA_BAD_ARGUMENT, "tcgen05 gemm: weight rows must be 16-byte aligned");
+    for (int p = 0; p <= base.nparts; ++p) {
+      if (p < base.nparts && base.parts[p].type == type) {
+        group.push_back(p);
       }
-      if (base.parts[p].type != type) {
-        continue;
-      }
-      group.push_back(p);
-      if (static_cast<int>(group.size()) == kTcMaxParts) {
-        groups.push_back(group);
+      if (!group.empty() && (p == base.nparts || static_cast<int>(group.size()) == kTcMaxParts)) {
+        const int rc = type == GUFO_CUDA_Q4_K ? LaunchPlan<GUFO_CUDA_Q4_K>(ctx, base, group, tokens)
+                                              : LaunchPlan<GUFO_CUDA_Q6_K>(ctx, base, group, tokens);
+        if (rc != GUFO_CUDA_OK) {
+          return rc;
+        }
         group.clear();
-      }
-    }
-    if (!group.empty()) {
-      groups.push_back(group);
-    }
-  }
-  // K ranges per 256-row tile; up to kTcMaxParts parts share a launch and its split.
-  // The split with the least modelled time: rounds of units over the persistent
-  // thread blocks, each a K range plus a little for the accumulator hand-over;
-  // a split pays for its partial sums; ties go to the smaller split.
-  auto splits_for = [&](int tiles, int m) {
-    // In units of one block's time on one SM (about 1.5 us): what the partial
-    // sums of one more K range cost in HBM traffic, written once and read once.
-    const double range_cost = 2.0 * m * (static_cast<double>(tiles) * kTileRows) * 4.0 / 6.0e6 / 1.5;
-    int best = 1;
-    double best_cost = 1e30;
-    for (int ksplit = 1; ksplit <= blocks; ++ksplit) {
-      const int per = (blocks + ksplit - 1) / ksplit;
-      const int ranges = (blocks + per - 1) / per;   // no empty K range
-      if (ranges != ksplit) {
-        continue;
-      }
-      const int rounds = (tiles * ksplit + ctx->sm_count - 1) / ctx->sm_count;
-      const double cost = rounds * (per + 0.3) + (ksplit > 1 ? 2.0 + ksplit * range_cost : 0.0);
-      if (cost < best_cost - 1e-9) {
-        best_cost = cost;
-        best = ksplit;
-      }
-    }
-    return best;
-  };
-  // Weight rows per tile for a group of parts: the height (a multiple of 16, up
-  // to 256) with the least modelled time over the persistent thread blocks. A
-  // unit's time falls with its rows until the tensor core's share (it spends as
-  // long on a narrow tile as on a wide one) takes over at about half height.
-  auto tiles_of = [&](const std::vector<int>& group, int tile_rows) {
-    int tiles = 0;
-    for (int p : group) {
-      tiles += (base.parts[p].rows + tile_rows - 1) / tile_rows;
-    }
-    return tiles;
-  };
-  auto tile_rows_for = [&](const std::vector<int>& group) {
-    int best = kTileRows;
-    double best_cost = 1e30;
-    for (int tr = kTileRows; tr >= 64; tr -= 16) {
-      const int tiles = tiles_of(group, tr);
-      const int rounds = (tiles + ctx->sm_count - 1) / ctx->sm_count;
-      const double unit = tr / static_cast<double>(kTileRows);
-      const double cost = rounds * (unit > 0.55 ? unit : 0.55);
-      if (cost < best_cost - 1e-9) {
-        best_cost = cost;
-        best = tr;
-      }
-    }
-    return best;
-  };
-  for (int t0 = 0; t0 < tokens; t0 += kTcMaxTokens) {
-    const int m = tokens - t0 < kTcMaxTokens ? tokens - t0 : kTcMaxTokens;
-    const size_t image_bytes = static_cast<size_t>(blocks) * 4 * kXTileBytes;
-    // Worst case for the partial sums: every part split into blocks / 2 ranges.
-    size_t partial_floats = 0;
-    for (const std::vector<int>& group : groups) {
-      size_t rows = 0;
-      for (int p : group) {
-        rows += base.parts[p].rows;
-      }
-      const int tiles = tiles_of(group, tile_rows_for(group));
-      const int ksplit = splits_for(tiles, m);
-      if (ksplit > 1) {
-        const size_t need = static_cast<size_t>(ksplit) * m * rows;
-        partial_floats = need > partial_floats ? need : partial_floats;
-      }
-    }
-    const size_t images_at = 256;
-    const size_t unscale_at = images_at + (image_bytes + 255) / 256 * 256;
-    const size_t partial_at = unscale_at + 1024;
-    const int rc = ReserveTc(ctx, partial_at + partial_floats * 4);
-    if (rc != GUFO_CUDA_OK) {
-      return rc;
-    }
-    uint8_t* xh = ctx->tc_scratch + images_at;
-    float* unscale = reinterpret_cast<float*>(ctx->tc_scratch + unscale_at);
-    float* partial = reinterpret_cast<float*>(ctx->tc_scratch + partial_at);
-    const float* x = base.x + static_cast<size_t>(t0) * cols;
-    GUFO_CUDA_TRY(LaunchOverlapped(StageHalfKernel, dim3(kTokenRows), dim3(256), 0, ctx->stream, 1, x, m, cols,
-                                   kTokenRows, xh, unscale));
-    ctx->launches.fetch_add(1);
-    for (const std::vector<int>& group : groups) {
-      TcGemmArgs args{};
-      args.blocks = blocks;
-      args.xh = xh;
-      args.unscale = unscale;
-      args.tokens = m;
-      args.error = reinterpret_cast<int*>(ctx->tc_scratch);
-      args.tile_rows = tile_rows_for(group);
-      const int tiles = tiles_of(group, args.tile_rows);
-      args.ksplit = splits_for(tiles, m);
-      args.blocks_per_unit = (blocks + args.ksplit - 1) / args.ksplit;
-      float* next_partial = partial;
-      for (int p : group) {
-        const GemvPart& part = base.parts[p];
-        TcPart& to = args.parts[args.nparts++];
-        to.w = part.data;
-        to.rows = part.rows;
-        to.row_bytes = part.row_bytes;
-        to.tiles = (part.rows + args.tile_rows - 1) / args.tile_rows;
-        if (args.ksplit == 1) {
-          to.out = base.y + static_cast<size_t>(t0) * base.y_stride + part.out_offset;
-          to.out_stride = base.y_stride;
-          to.split_stride = 0;
-        } else {
-          to.out = next_partial;
-          to.out_stride = part.rows;
-          to.split_stride = static_cast<size_t>(m) * part.rows;
-          next_partial += static_cast<size_t>(args.ksplit) * m * part.rows;
-        }
-      }
-      args.total_units = tiles * args.ksplit;
-      const int grid = args.total_units < ctx->sm_count ? args.total_units : ctx->sm_count;
-      if (base.parts[group[0]].type == GUFO_CUDA_Q4_K) {
-        GUFO_CUDA_TRY(LaunchOverlapped(GemmTc<GUFO_CUDA_Q4_K>, dim3(grid), dim3(kTcThreads),
-                                       Smem<GUFO_CUDA_Q4_K>::kBytes, ctx->stream, 1, args));
-      } else {
-        GUFO_CUDA_TRY(LaunchOverlapped(GemmTc<GUFO_CUDA_Q6_K>, dim3(grid), dim3(kTcThreads),
-                                       Smem<GUFO_CUDA_Q6_K>::kBytes, ctx->stream, 1, args));
-      }
-      ctx->launches.fetch_add(1);
-      if (args.ksplit > 1) {
-        for (int i = 0; i < args.nparts; ++i) {
-          const GemvPart& part = base.parts[group[i]];
-          float* y = base.y + static_cast<size_t>(t0) * base.y_stride + part.out_offset;
-          GUFO_CUDA_TRY(LaunchOverlapped(SumSplitsKernel, dim3((part.rows + 255) / 256, m), dim3(256), 0, ctx->stream,
-                                         1, static_cast<const float*>(args.parts[i].out), args.ksplit,
-                                         args.parts[i].split_stride, part.rows, m, y, base.y_stride));
-          ctx->launches.fetch_add(1);
-        }
       }
     }
   }
@@ -994,9 +1208,11 @@ int TcGemmError(gufo_cuda_ctx* ctx, int* code) {
   }
   GUFO_CUDA_TRY(cudaMemcpyAsync(code, ctx->tc_scratch, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   GUFO_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (*code != 0) {
+    // A kernel that gave up may have left counters behind.
+    GUFO_CUDA_TRY(cudaMemsetAsync(ctx->tc_scratch, 0, kHeaderBytes, ctx->stream));
+  }
   return GUFO_CUDA_OK;
 }
 
 }  // namespace gufo
-
-

@@ -1,5 +1,4 @@
-// Launch interface of the tcgen05 small-M GEMM (16 to 128 token rows per
-// weight read).
+// Launch interface of the tcgen05 small-M GEMM (16 or more token rows).
 #pragma once
 
 #include "gemv.cuh"
@@ -7,14 +6,11 @@
 
 namespace gufo {
 
-// Fewest token rows that take this path; below, the GEMV kernels re-read the
-// weights once per 8 tokens and are faster. Measured: 2 x 9728 x 2560 Q4_K costs
-// 27 us per 8-token pass against 31 us here whatever the rows (so from a second
-// pass on this path wins, and the third is where it is taken); 248320 x 2560
-// Q6_K 330 us per pass against 670 us here (from a third pass on).
-constexpr int kTcMinTokens = 17;       // Q4_K parts
-constexpr int kTcMinTokensQ6K = 17;    // Q6_K parts
-constexpr int kTcMaxTokens = 128;   // token rows per pass (the MMA's N)
+// Fewest token rows that take this path: a third pass over the weights on the
+// eight-token GEMV kernels. Those keep the activations to 24 bits and this path
+// rounds them to fp16, so the line stays where it is although two passes are
+// slower than this.
+constexpr int kTcMinTokens = 17;
 
 // Whether a product of `tokens` rows against parts of `type` runs on this path.
 bool TcGemmRuns(const gufo_cuda_ctx* ctx, int type, int cols, int tokens);
