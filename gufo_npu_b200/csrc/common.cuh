@@ -261,7 +261,7 @@ struct gufo_cuda_ctx {
   size_t tc_scratch_bytes = 0;
   // Scratch blocks that were outgrown: a CUDA graph captured earlier may still
   // hold their addresses, so they stay allocated until the context goes.
-  std::vector<void*> retired;
+  std::vector<std::pair<uint8_t*, size_t>> retired;
   // Products of 16 or more token rows run on the tcgen05 GEMM (option "tc_gemm").
   bool tc_gemm = true;
   bool tc_gemm_all = false;   // option value 2: from 16 rows on, whatever is faster

@@ -4,6 +4,7 @@
 
 #include <cstring>
 #include <new>
+#include <vector>
 
 namespace gufo {
 
@@ -111,6 +112,81 @@ int RepackQ6KRows(gufo_cuda_ctx* ctx, const uint8_t* raw, int64_t rows, int64_t 
   return GUFO_CUDA_OK;
 }
 
+// Scratch blocks of destroyed contexts, kept for the next one while the process
+// has a context on the device (a cudaMalloc or cudaFree takes a millisecond or
+// more here, and a new context's first products need several): at most kKeep
+// blocks of kKeepBytes in all per device, freed with the device's last context.
+namespace {
+
+struct ScratchPool {
+  static constexpr size_t kKeep = 8;
+  static constexpr size_t kKeepBytes = 256u << 20;
+  struct Block {
+    uint8_t* data;
+    size_t bytes;
+  };
+  struct Device {
+    int contexts = 0;
+    std::vector<Block> blocks;
+  };
+  std::mutex mutex;
+  std::unordered_map<int, Device> devices;
+
+  void Enter(int device) {
+    std::lock_guard<std::mutex> lock(mutex);
+    ++devices[device].contexts;
+  }
+  // The device is current; no work that uses a kept block is left.
+  void Leave(int device) {
+    std::lock_guard<std::mutex> lock(mutex);
+    Device& d = devices[device];
+    if (--d.contexts == 0) {
+      for (const Block& b : d.blocks) {
+        cudaFree(b.data);
+      }
+      d.blocks.clear();
+    }
+  }
+  // The smallest kept block of at least `want` bytes and at most four times that.
+  bool Take(int device, size_t want, uint8_t** data, size_t* bytes) {
+    std::lock_guard<std::mutex> lock(mutex);
+    std::vector<Block>& blocks = devices[device].blocks;
+    size_t best = blocks.size();
+    for (size_t i = 0; i < blocks.size(); ++i) {
+      if (blocks[i].bytes >= want && blocks[i].bytes <= 4 * want && (best == blocks.size() || blocks[i].bytes < blocks[best].bytes)) {
+        best = i;
+      }
+    }
+    if (best == blocks.size()) {
+      return false;
+    }
+    *data = blocks[best].data;
+    *bytes = blocks[best].bytes;
+    blocks.erase(blocks.begin() + best);
+    return true;
+  }
+  void Give(int device, uint8_t* data, size_t bytes) {
+    std::lock_guard<std::mutex> lock(mutex);
+    std::vector<Block>& blocks = devices[device].blocks;
+    size_t held = bytes;
+    for (const Block& b : blocks) {
+      held += b.bytes;
+    }
+    if (blocks.size() >= kKeep || held > kKeepBytes) {
+      cudaFree(data);
+      return;
+    }
+    blocks.push_back({data, bytes});
+  }
+};
+
+ScratchPool& Pool() {
+  static ScratchPool* pool = new ScratchPool();   // outlives every context
+  return *pool;
+}
+
+}  // namespace
+
 }  // namespace gufo
 
 int gufo_cuda_ctx::Reserve(float** buffer, size_t* have, size_t want) {
@@ -179,6 +255,7 @@ int gufo_cuda_ctx_create(int device, void* stream, gufo_cuda_ctx** out) {
     }
     ctx->own_stream = true;
   }
+  gufo::Pool().Enter(device);
   *out = ctx;
   return GUFO_CUDA_OK;
 }
@@ -193,11 +270,13 @@ int gufo_cuda_ctx::GrowScratch(uint8_t** block, size_t* have, size_t want, size_
                       std::string(what) + ": the context's scratch must grow for this product, which a stream "
                                           "capture cannot do; run the product once before capturing");
   }
-  const size_t grown = want < floor ? floor : want;
+  size_t grown = want < floor ? floor : want;
   uint8_t* fresh = nullptr;
-  GUFO_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&fresh), grown));
+  if (!gufo::Pool().Take(device, grown, &fresh, &grown)) {
+    GUFO_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&fresh), grown));
+  }
   if (*block != nullptr) {
-    retired.push_back(*block);   // a graph captured earlier may still use it
+    retired.emplace_back(*block, *have);   // a graph captured earlier may still use it
   }
   *block = fresh;
   *have = grown;
@@ -209,7 +288,7 @@ int gufo_cuda_ctx_destroy(gufo_cuda_ctx* ctx) {
     return GUFO_CUDA_OK;
   }
   cudaSetDevice(ctx->device);
-  cudaStreamSynchronize(ctx->stream);
+  cudaDeviceSynchronize();   // also work on a stream that set_stream replaced
   for (auto& kv : ctx->matrices) {
     if (kv.second.owned) {
       cudaFree(const_cast<uint8_t*>(kv.second.data));
@@ -223,11 +302,14 @@ int gufo_cuda_ctx_destroy(gufo_cuda_ctx* ctx) {
   }
   cudaFree(ctx->stage_x);
   cudaFree(ctx->stage_y);
-  cudaFree(ctx->image);
-  cudaFree(ctx->tc_scratch);
-  for (void* block : ctx->retired) {
-    cudaFree(block);
+  ctx->retired.emplace_back(ctx->image, ctx->image_bytes);
+  ctx->retired.emplace_back(ctx->tc_scratch, ctx->tc_scratch_bytes);
+  for (const auto& block : ctx->retired) {
+    if (block.first != nullptr) {
+      gufo::Pool().Give(ctx->device, block.first, block.second);
+    }
   }
+  gufo::Pool().Leave(ctx->device);
   if (ctx->own_stream) {
     cudaStreamDestroy(ctx->stream);
   }

@@ -88,7 +88,7 @@ constexpr int kTcThreads = (kMmaWarp + 1) * 32;
 constexpr int kMaxStages = 10;
 constexpr long long kWaitCycles = 1ll << 31;           // about a second of SM clocks
 constexpr int kHeaderBytes = 4096;                     // of the scratch: error word, counters of cut tiles
-constexpr size_t kScratchFloor = 32u << 20;            // of the scratch: one allocation serves most shapes
+constexpr size_t kScratchFloor = 48u << 20;            // of the scratch: one allocation serves most shapes
 constexpr int kSharedLimit = 227 * 1024;
 
 // The raw bytes of one block of 128 rows in shared memory.
@@ -1109,7 +1109,8 @@ int LaunchPlan(gufo_cuda_ctx* ctx, const GemvArgs& base, const std::vector<int>&
   const size_t rows = static_cast<size_t>(plan.groups) * plan.n;
   const size_t unscale_at = kHeaderBytes + rows * cols * 2;
   const size_t partial_at = (unscale_at + rows * 4 + 255) / 256 * 256;
-  const size_t partial_bytes = static_cast<size_t>(plan.grid) * 2 * kTileRows * plan.n * 4;
+  const bool cuts = plan.units % plan.grid != 0;
+  const size_t partial_bytes = cuts ? static_cast<size_t>(plan.grid) * 2 * kTileRows * plan.n * 4 : 0;
   int rc = ReserveTc(ctx, partial_at + partial_bytes);
   if (rc != GUFO_CUDA_OK) {
     return rc;
