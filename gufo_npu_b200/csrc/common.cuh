@@ -211,15 +211,10 @@ int LaunchGemvQ4KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
 // Whether the image of `tokens` rows of `cols` values fits in shared memory.
 bool Q4KFastFits(int cols, int tokens);
 bool FastSwiGluPairsFit(const gufo_cuda_ctx* ctx, int type, int cols, int tokens, int pairs);
-// One Mixer::Linear step per sequence; the caller holds ctx->mu.
-// `early_state`: the states and conv windows were not written by the kernels
-// shortly before this one in the stream (several may be in flight at once), so
-// their loads may run ahead of the dependency wait.
 // The F32 alpha / beta rows of a DeltaNet layer's input product, for a step
 // that computes the two gates inside the mixer kernel instead of reading them
 // from the product's output: a = alpha_w[head] . x, b = beta_w[head] . x.
 struct DeltaNetGateRows {
-  const float* x;         // the layer's normed input [cols] (every sequence's, unless xs is given)
   const float* alpha_w;   // [value heads][cols]
   const float* beta_w;
   int cols;               // a multiple of 4
@@ -227,12 +222,33 @@ struct DeltaNetGateRows {
   // vec::RmsNorm (src/core/vec.hpp:57-63) with these weights first.
   const float* norm_w;
   float eps;
-  // Per-sequence inputs (launch order), overriding x when non-null.
-  const float* const* xs;
 };
-int EnqueueDeltaNetLinear(gufo_cuda_ctx* ctx, const DeltaNetLayer& layer,
-                          const gufo_cuda_linear_seq* seqs, int nseq, bool early_state,
-                          const DeltaNetGateRows* gate_rows = nullptr);
+// One sequence of a Mixer::Linear launch: `tokens` rows through the layer. The
+// state after the token before the last goes to `ssm` (two or more tokens), the one
+// after the last to `ssm_last`; likewise the conv windows.
+struct DeltaNetSeq {
+  const float* in;         // [tokens], in_stride floats apart
+  const float* x;          // the gate rows' input [tokens], x_stride apart
+  const float* conv_in;
+  float* conv_saved;       // two or more tokens: the window before the last one
+  float* conv_out;
+  const float* ssm_in;
+  float* ssm;
+  float* ssm_last;
+  float* y;                // [tokens], y_stride apart
+  int64_t in_stride, x_stride, y_stride;
+  int tokens;
+};
+inline DeltaNetSeq OneTokenSeq(const float* in, const float* x, const float* conv_in, float* conv_out, const float* ssm_in,
+                               float* ssm_out, float* y) {
+  return {in, x, conv_in, nullptr, conv_out, ssm_in, nullptr, ssm_out, y, 0, 0, 0, 1};
+}
+// Mixer::Linear for every sequence (1 to 4 tokens each); the caller holds ctx->mu.
+// `early_state`: the states and conv windows were not written by the kernels
+// shortly before this one in the stream (several may be in flight at once), so
+// their loads may run ahead of the dependency wait.
+int EnqueueDeltaNetLinear(gufo_cuda_ctx* ctx, const DeltaNetLayer& layer, const DeltaNetSeq* seqs, int nseq,
+                          bool early_state, const DeltaNetGateRows* gate_rows = nullptr);
 // The same for Q6_K parts (image with group sums of 16).
 int LaunchGemvQ6KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
 bool Q6KFastFits(int cols, int tokens);

@@ -592,27 +592,21 @@ int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens, 
     cur ^= 1;
     const size_t in_width = static_cast<size_t>(l.in.y_stride);
     const size_t mixed_width = static_cast<size_t>(l.out.cols);
-    for (int t = 0; t < tokens; ++t) {
-      const float* in = d->in + t * in_width;
-      float* mixed = d->mixed + t * mixed_width;
-      if (l.attention) {
-        AttnArgs a{c.heads, c.kv_heads, c.head_dim, c.rope_dim, c.max_positions, c.rms_eps,
-                   d->position_dev, in, l.q_norm, l.k_norm, d->inv_freq, l.keys, l.values,
-                   d->queries, d->partials, mixed, t};
-        GUFO_STEP_TRY(EnqueueAttention(ctx, a));
-      } else {
-        // One token: window to window, state in place. Two: the first goes to
-        // conv_saved, the second from there to the other window and ssm_spec.
-        const bool last = t == tokens - 1;
-        const float* conv_from = t == 0 ? l.conv[parity] : l.conv_saved;
-        float* conv_to = last ? l.conv[parity ^ 1] : l.conv_saved;
-        gufo_cuda_linear_seq seq{in, conv_from, conv_to, l.ssm, t > 0 ? l.ssm_spec : nullptr, mixed};
-        gufo::DeltaNetGateRows gate_rows = l.gate_rows;
-        gate_rows.x = d->normed + t * hidden;
-        // A second token reads the state the launch before it wrote: no early loads.
-        GUFO_STEP_TRY(EnqueueDeltaNetLinear(ctx, l.linear, &seq, 1, t == 0,
-                                            gate_rows.alpha_w != nullptr ? &gate_rows : nullptr));
-      }
+    for (int t = 0; l.attention && t < tokens; ++t) {
+      AttnArgs a{c.heads, c.kv_heads, c.head_dim, c.rope_dim, c.max_positions, c.rms_eps,
+                 d->position_dev, d->in + t * in_width, l.q_norm, l.k_norm, d->inv_freq, l.keys, l.values,
+                 d->queries, d->partials, d->mixed + t * mixed_width, t};
+      GUFO_STEP_TRY(EnqueueAttention(ctx, a));
+    }
+    if (!l.attention) {
+      // One token: window to window, state in place. Two: the window and the state
+      // after the first stay in conv_saved and ssm, the second's go to the other
+      // window and ssm_spec.
+      const DeltaNetSeq seq{d->in, d->normed, l.conv[parity], l.conv_saved, l.conv[parity ^ 1], l.ssm, l.ssm,
+                            tokens == 2 ? l.ssm_spec : l.ssm, d->mixed, static_cast<int64_t>(in_width),
+                            static_cast<int64_t>(hidden), static_cast<int64_t>(mixed_width), tokens};
+      GUFO_STEP_TRY(EnqueueDeltaNetLinear(ctx, l.linear, &seq, 1, true,
+                                          l.gate_rows.alpha_w != nullptr ? &l.gate_rows : nullptr));
     }
     Mark(d, l.attention ? GUFO_CUDA_TIMELINE_ATTENTION : GUFO_CUDA_TIMELINE_DELTANET);
     Input plain{kProloguePlain};

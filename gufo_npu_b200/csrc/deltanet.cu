@@ -25,7 +25,8 @@ namespace gufo {
 
 constexpr int kMaxHeadDim = 128;
 constexpr int kDeltaThreads = kMaxHeadDim;            // one thread per column
-constexpr int kMaxSeqs = 16;                          // descriptors per launch
+constexpr int kMaxSeqs = 64;                          // descriptors per launch
+constexpr int kMaxRunTokens = 4;                      // tokens of a sequence per launch
 
 struct DeltaRuleArgs {
   gufo_cuda_delta_seq seq[kMaxSeqs];
@@ -35,8 +36,7 @@ struct DeltaRuleArgs {
   int early_state;   // as in LinearArgs below
 };
 
-struct LinearArgs {
-  gufo_cuda_linear_seq seq[kMaxSeqs];
+struct LinearShape {
   int key_heads;
   int value_heads;
   int head_dim;
@@ -51,19 +51,16 @@ struct LinearArgs {
   int early_state;
   // Non-null alpha_w: the gates come from these rows instead of the input row.
   DeltaNetGateRows gate_rows;
-  const float* gate_x[kMaxSeqs];   // per sequence, or null for gate_rows.x
+};
+
+// A launch of up to SEQS sequences (a decode step's one travels light).
+template <int SEQS>
+struct LinearArgs {
+  LinearShape shape;
+  DeltaNetSeq seq[SEQS];
 };
 
 namespace {
-
-struct DeltaShared {
-  float q[kMaxHeadDim];
-  float k[kMaxHeadDim];
-  float v[kMaxHeadDim];
-  float y[kMaxHeadDim];
-  float gate[2];                              // decay, beta
-  float scratch[5 * (2 * kDeltaThreads / 32)];   // up to five sums a warp (BlockSum5)
-};
 
 // A warp's tile of COLS (8 or 16) adjacent columns of a head's state: a lane
 // holds rows ig, ig + 32 / G, ... (ig = lane / G, G = COLS / 4) of four adjacent
@@ -105,26 +102,26 @@ __device__ __forceinline__ float4 NarrowColumnSum(float4 v) {
   return v;
 }
 
-// The delta rule on this warp's column tile. sh.q, sh.k, sh.v and sh.gate are
-// ready. Writes S' to dst and the tile's outputs to sh.y (no barrier); with
-// `squares`, lane 0 also leaves the sum of the squares of the tile's outputs there.
+// The delta rule on this warp's column tile, which becomes S'. Writes S' to dst
+// (may be null) and the tile's outputs to out (no barrier); with `squares`, lane 0
+// also leaves the sum of the squares of the tile's outputs there. q, k, v: the
+// head's vectors in shared memory.
 template <int COLS>
 __device__ __forceinline__ void NarrowDeltaTile(NarrowTile<COLS>& tile, float* __restrict__ dst, int dk,
-                                                int tile_index, DeltaShared& sh, float* squares = nullptr) {
+                                                int tile_index, const float* q, const float* k, const float* v_in,
+                                                float decay, float beta, float* out, float* squares = nullptr) {
   using T = NarrowTile<COLS>;
   const int lane = threadIdx.x & 31;
   const int col = tile_index * COLS + 4 * (lane % T::kGroups);
   const int ig = lane / T::kGroups;
   const int rows = dk / T::kRowGroups;
-  const float decay = sh.gate[0];
-  const float beta = sh.gate[1];
   float4 (&s)[T::kRowsPerLane] = tile.s;
   // Pass 1: u_j = sum_i S_ij * (k_i * decay).
   float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int r = 0; r < T::kRowsPerLane; ++r) {
     if (r < rows) {
-      const float ki = sh.k[r * T::kRowGroups + ig] * decay;
+      const float ki = k[r * T::kRowGroups + ig] * decay;
       u.x = fmaf(s[r].x, ki, u.x);
       u.y = fmaf(s[r].y, ki, u.y);
       u.z = fmaf(s[r].z, ki, u.z);
@@ -132,7 +129,7 @@ __device__ __forceinline__ void NarrowDeltaTile(NarrowTile<COLS>& tile, float* _
     }
   }
   u = NarrowColumnSum<COLS>(u);
-  const float4 v = *reinterpret_cast<const float4*>(&sh.v[col]);
+  const float4 v = *reinterpret_cast<const float4*>(&v_in[col]);
   float4 delta;
   delta.x = beta * (v.x - u.x);
   delta.y = beta * (v.y - u.y);
@@ -144,14 +141,17 @@ __device__ __forceinline__ void NarrowDeltaTile(NarrowTile<COLS>& tile, float* _
   for (int r = 0; r < T::kRowsPerLane; ++r) {
     if (r < rows) {
       const int i = r * T::kRowGroups + ig;
-      const float ki = sh.k[i];
-      const float qi = sh.q[i];
+      const float ki = k[i];
+      const float qi = q[i];
       float4 n;
       n.x = fmaf(s[r].x, decay, ki * delta.x);
       n.y = fmaf(s[r].y, decay, ki * delta.y);
       n.z = fmaf(s[r].z, decay, ki * delta.z);
       n.w = fmaf(s[r].w, decay, ki * delta.w);
-      *reinterpret_cast<float4*>(dst + static_cast<size_t>(i) * dk + col) = n;
+      if (dst != nullptr) {
+        *reinterpret_cast<float4*>(dst + static_cast<size_t>(i) * dk + col) = n;
+      }
+      s[r] = n;
       y.x = fmaf(n.x, qi, y.x);
       y.y = fmaf(n.y, qi, y.y);
       y.z = fmaf(n.z, qi, y.z);
@@ -160,7 +160,7 @@ __device__ __forceinline__ void NarrowDeltaTile(NarrowTile<COLS>& tile, float* _
   }
   y = NarrowColumnSum<COLS>(y);
   if (ig == 0) {
-    *reinterpret_cast<float4*>(&sh.y[col]) = y;
+    *reinterpret_cast<float4*>(&out[col]) = y;
   }
   if (squares != nullptr) {
     // Lanes 0 .. kGroups - 1 hold the tile's COLS outputs.
@@ -184,7 +184,7 @@ constexpr int kRuleCols = 16;   // and in the stand-alone delta rule (8: 4.9 us 
 // (16-column tiles: 1024 warps for eight sequences of sixteen heads).
 __global__ void __launch_bounds__(32)
 DeltaRuleKernel(const __grid_constant__ DeltaRuleArgs args) {
-  __shared__ __align__(16) DeltaShared sh;
+  __shared__ __align__(16) float q[kMaxHeadDim], k[kMaxHeadDim], v[kMaxHeadDim], y[kMaxHeadDim];
   const gufo_cuda_delta_seq& seq = args.seq[blockIdx.z];
   const int head = blockIdx.y;
   const int tile = blockIdx.x;
@@ -202,22 +202,19 @@ DeltaRuleKernel(const __grid_constant__ DeltaRuleArgs args) {
     LoadNarrowTile(state, seq.state + state_at, dk, tile);
   }
   for (int i = lane; i < dk; i += 32) {
-    sh.q[i] = seq.q[kh * dk + i];
-    sh.k[i] = seq.k[kh * dk + i];
+    q[i] = seq.q[kh * dk + i];
+    k[i] = seq.k[kh * dk + i];
   }
   if (lane < kRuleCols) {
-    sh.v[tile * kRuleCols + lane] = seq.v[head * dk + tile * kRuleCols + lane];
+    v[tile * kRuleCols + lane] = seq.v[head * dk + tile * kRuleCols + lane];
   }
-  if (lane == 0) {
-    sh.gate[0] = seq.decay[head];
-    sh.gate[1] = seq.beta[head];
-  }
+  const float decay = seq.decay[head], beta = seq.beta[head];
   __syncwarp();
   float* dst = (seq.state_out != nullptr ? seq.state_out : seq.state) + state_at;
-  NarrowDeltaTile(state, dst, dk, tile, sh);
+  NarrowDeltaTile(state, dst, dk, tile, q, k, v, decay, beta, y);
   __syncwarp();
   if (lane < kRuleCols) {
-    seq.y[head * dk + tile * kRuleCols + lane] = sh.y[tile * kRuleCols + lane];
+    seq.y[head * dk + tile * kRuleCols + lane] = y[tile * kRuleCols + lane];
   }
 }
 
@@ -227,141 +224,120 @@ __device__ __forceinline__ float Softplus(float x) {
   return x > 20.0f ? x : log1pf(expf(x));
 }
 
-// Block-wide sums of two values per thread at once; results to every thread.
-__device__ __forceinline__ void BlockSum2(float& a, float& b, DeltaShared& sh, int warps) {
-  a = WarpSum(a);
-  b = WarpSum(b);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) {
-    sh.scratch[2 * (threadIdx.x >> 5)] = a;
-    sh.scratch[2 * (threadIdx.x >> 5) + 1] = b;
-  }
-  __syncthreads();
-  a = 0.f;
-  b = 0.f;
-  for (int w = 0; w < warps; ++w) {
-    a += sh.scratch[2 * w];
-    b += sh.scratch[2 * w + 1];
-  }
-}
-
-// The same for five values (the decode step's one reduction ahead of the delta
-// rule: the input's sum of squares, the two gate dots, the q and k norms).
-__device__ __forceinline__ void BlockSum5(float (&v)[5], DeltaShared& sh, int warps) {
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    v[i] = WarpSum(v[i]);
-  }
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      sh.scratch[5 * (threadIdx.x >> 5) + i] = v[i];
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    v[i] = 0.f;
-  }
-  for (int w = 0; w < warps; ++w) {
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      v[i] += sh.scratch[5 * w + i];
-    }
-  }
-}
-
-// Mixer::Linear for one (sequence, value head). grid = (value_heads,
-// sequences), 2 * dk threads: thread t < dk owns channel t of the head's q and k
-// and output t of the epilogue, thread dk + t channel t of v; warp w owns columns
-// 16 w .. 16 w + 15 of the state. (With dk threads and 32 columns per warp the
-// kernel spent 6.5 us per layer of the decode step on four warps' worth of
+// Mixer::Linear for one (sequence, value head), up to TOK tokens. grid =
+// (value_heads, sequences), 2 * dk threads: thread t < dk owns channel t of the
+// head's q and k and output t of the epilogue, thread dk + t channel t of v; warp w
+// owns columns 16 w .. 16 w + 15 of the state. (With dk threads and 32 columns per
+// warp the kernel spent 6.5 us per layer of the decode step on four warps' worth of
 // dependent instructions.)
-__global__ void __launch_bounds__(2 * kDeltaThreads)
-DeltaNetLinearKernel(const __grid_constant__ LinearArgs args) {
-  __shared__ __align__(16) DeltaShared sh;
-  const gufo_cuda_linear_seq& seq = args.seq[blockIdx.y];
+//
+// All that does not need the state - convolutions, gates, norms of every token -
+// is done first, for all tokens at once and under the state's load; the tokens then
+// follow one another on the state in registers with no block barrier between them
+// (a warp's columns need nothing from the others'), and the gated norms of all
+// tokens close the block. The state is read once and written once (a draft's once
+// more) whatever the tokens: as a launch per token index, 32 sequences of 32 heads
+// with one to four tokens took 110 us and moved the states up to eight times.
+template <int TOK>
+struct LinearShared {
+  float q[TOK][kMaxHeadDim];
+  float k[TOK][kMaxHeadDim];
+  float v[TOK][kMaxHeadDim];
+  float y[TOK][kMaxHeadDim];
+  float gate[TOK][2];                                  // decay, beta
+  float scratch[(2 * kDeltaThreads / 32) * 5 * TOK];   // five sums a token and warp
+};
+
+template <int TOK, int WIN, int SEQS>
+__global__ void __launch_bounds__(2 * kDeltaThreads, SEQS > 2 ? 2 : 1)
+DeltaNetLinearKernel(const __grid_constant__ LinearArgs<SEQS> args) {
+  __shared__ __align__(16) LinearShared<TOK> sh;
+  const LinearShape& a = args.shape;
+  const DeltaNetSeq& seq = args.seq[blockIdx.y];
+  const int n = TOK == 1 ? 1 : seq.tokens;
   const int head = blockIdx.x;
-  const int hk = args.key_heads;
-  const int hv = args.value_heads;
-  const int dk = args.head_dim;
+  const int hk = a.key_heads;
+  const int hv = a.value_heads;
+  const int dk = a.head_dim;
   const int threads = 2 * dk;
   const int warps = threads / 32;
   const int key_dim = hk * dk;
   const int value_dim = hv * dk;
   const int channels = 2 * key_dim + value_dim;
-  const int kernel = args.conv_kernel;
-  const int window = kernel - 1;
+  const int kernel = a.conv_kernel;
+  const int window = kernel - 1;      // at most WIN
   const int kh = head % hk;
   const int tid = threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31;
   const bool lower = tid < dk;        // q and k channels, the epilogue
   const int ch = lower ? tid : tid - dk;
-  const float* x = seq.in;
   const size_t state_at = static_cast<size_t>(head) * dk * dk;
   NarrowTile<kStepCols> state_tile;
-  // Causal depthwise conv + SiLU of a channel; also advances that channel's
-  // window when this block is the one that owns it. All loads of a thread's
-  // channels are issued before the first store, so they overlap.
-  constexpr int kMaxWindow = 7;
+  // Causal depthwise conv + SiLU of a channel; its window moves on in registers.
+  // All loads of a thread's channels are issued before the first store, so they
+  // overlap.
   struct Taps {
-    float cur;
-    float old[kMaxWindow];
-    float w[kMaxWindow + 1];
+    float old[WIN];
+    float w[WIN + 1];
   };
   // The layer's weights never depend on the kernels before this one.
   auto fetch_weights = [&](int c, Taps& taps) {
-    const float* kw = args.conv + static_cast<size_t>(c) * kernel;
+    const float* kw = a.conv + static_cast<size_t>(c) * kernel;
 #pragma unroll
-    for (int t = 0; t < kMaxWindow; ++t) {
-      if (t < window) {
-        taps.w[t] = kw[t];
-      }
+    for (int t = 0; t < WIN; ++t) {
+      taps.w[t] = t < window ? kw[t] : 0.f;
     }
-    taps.w[kMaxWindow] = kw[window];
+    taps.w[WIN] = kw[window];
   };
   // The window is state: written a step ago (early_state) or by the launch
   // just before this one.
   auto fetch_window = [&](int c, Taps& taps) {
 #pragma unroll
-    for (int t = 0; t < kMaxWindow; ++t) {
-      if (t < window) {
-        taps.old[t] = seq.conv_in[static_cast<size_t>(t) * channels + c];
-      }
+    for (int t = 0; t < WIN; ++t) {
+      taps.old[t] = t < window ? seq.conv_in[static_cast<size_t>(t) * channels + c] : 0.f;
     }
   };
-  auto conv = [&](int c, const Taps& taps, bool owner) -> float {
-    float acc = taps.w[kMaxWindow] * taps.cur;
+  auto conv = [&](Taps& taps, float cur) -> float {
+    float acc = taps.w[WIN] * cur;
 #pragma unroll
-    for (int t = 0; t < kMaxWindow; ++t) {
+    for (int t = 0; t < WIN; ++t) {
       if (t < window) {
         acc = fmaf(taps.w[t], taps.old[t], acc);
-        if (owner && t > 0) {
-          seq.conv_out[static_cast<size_t>(t - 1) * channels + c] = taps.old[t];
-        }
       }
     }
-    if (owner) {
-      seq.conv_out[static_cast<size_t>(window - 1) * channels + c] = taps.cur;
+#pragma unroll
+    for (int t = 0; t < WIN; ++t) {
+      taps.old[t] = t == window - 1 ? cur : (t + 1 < WIN ? taps.old[t + 1] : cur);
     }
     return Silu(acc);
+  };
+  auto store_window = [&](float* to, int c, const Taps& taps) {
+#pragma unroll
+    for (int t = 0; t < WIN; ++t) {
+      if (t < window) {
+        to[static_cast<size_t>(t) * channels + c] = taps.old[t];
+      }
+    }
   };
   // The window of the key head's q and k channels is advanced by the first
   // value head that reads the key head; every head advances its own v.
   // A lower thread convolves q (ta) and k (tb) of its channel, an upper one v (ta).
   const int ch_a = lower ? kh * dk + ch : 2 * key_dim + head * dk + ch;
   const int ch_b = key_dim + kh * dk + ch;
+  const bool owner = !lower || head < hk;
   Taps ta, tb;
   // The first passes of the head's alpha and beta rows (weights as well).
   constexpr int kGateAhead = 2;
-  const DeltaNetGateRows& g = args.gate_rows;
+  const DeltaNetGateRows& g = a.gate_rows;
   const bool gate_rows = g.alpha_w != nullptr;
   const float4* wa = reinterpret_cast<const float4*>(g.alpha_w + static_cast<size_t>(head) * g.cols);
   const float4* wb = reinterpret_cast<const float4*>(g.beta_w + static_cast<size_t>(head) * g.cols);
+  const float4* norm = reinterpret_cast<const float4*>(g.norm_w);
+  const float4 one4 = make_float4(1.f, 1.f, 1.f, 1.f);
   float4 wa_ahead[kGateAhead], wb_ahead[kGateAhead], nw_ahead[kGateAhead];
   GridLaunchDependents();
-  if (args.early_state) {
-    LoadNarrowTile(state_tile, seq.ssm + state_at, dk, tid >> 5);
+  if (a.early_state) {
+    LoadNarrowTile(state_tile, seq.ssm_in + state_at, dk, warp);
     fetch_window(ch_a, ta);
     if (lower) {
       fetch_window(ch_b, tb);
@@ -378,131 +354,172 @@ DeltaNetLinearKernel(const __grid_constant__ LinearArgs args) {
       if (i < g.cols / 4) {
         wa_ahead[j] = wa[i];
         wb_ahead[j] = wb[i];
-        if (g.norm_w != nullptr) {
-          nw_ahead[j] = reinterpret_cast<const float4*>(g.norm_w)[i];
-        }
+        nw_ahead[j] = norm != nullptr ? norm[i] : one4;
       }
     }
   }
-  const float norm_w = lower ? args.ssm_norm[ch] : 0.f;
-  const float ssm_a = args.ssm_a[head], dt_bias = args.dt_bias[head];
+  const float norm_w = lower ? a.ssm_norm[ch] : 0.f;
+  const float ssm_a = a.ssm_a[head], dt_bias = a.dt_bias[head];
   GridDependencyWait();
-  if (!args.early_state) {
-    LoadNarrowTile(state_tile, seq.ssm + state_at, dk, tid >> 5);
+  if (!a.early_state) {
+    LoadNarrowTile(state_tile, seq.ssm_in + state_at, dk, warp);
     fetch_window(ch_a, ta);
     if (lower) {
       fetch_window(ch_b, tb);
     }
   }
-  // What the epilogue needs, requested now so that it has arrived by then.
-  const float z = lower ? x[channels + head * dk + ch] : 0.f;
-  ta.cur = x[ch_a];
-  if (lower) {
-    tb.cur = x[ch_b];
+  // What the tokens bring, the epilogue's z included, requested at once.
+  float cur_a[TOK], cur_b[TOK], z[TOK];
+#pragma unroll
+  for (int t = 0; t < TOK; ++t) {
+    cur_a[t] = cur_b[t] = z[t] = 0.f;
+    if (t < n) {
+      const float* in = seq.in + t * seq.in_stride;
+      cur_a[t] = in[ch_a];
+      if (lower) {
+        cur_b[t] = in[ch_b];
+        z[t] = in[channels + head * dk + ch];
+      }
+    }
+  }
+  // Five sums a token: the gate input's squares, the two gate dots, the q and k
+  // norms' squares; one block-wide reduction for all of them.
+  float sums[TOK][5];
+#pragma unroll
+  for (int t = 0; t < TOK; ++t) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      sums[t][i] = 0.f;
+    }
   }
   if (gate_rows) {
     // The head's alpha and beta rows against the normed input, one float4 per
     // thread and pass (GgufProjections serves these F32 rows through its own
     // dot, src/models/qwen35/gguf_projections.cpp:162-170). With norm weights
     // the input is the residual stream and the RMS norm is applied on the way
-    // (DeltaNetStep::Run, src/models/qwen35_2b/deltanet.cpp:358-392).
-    const float* gx = args.gate_x[blockIdx.y] != nullptr ? args.gate_x[blockIdx.y] : g.x;
-    const float4* xa = reinterpret_cast<const float4*>(gx);
-    // The input's first passes stay in registers between the norm's sum of
-    // squares and the dot products (one round trip to L2 for them, not two).
-    float4 x_ahead[kGateAhead];
+    // (DeltaNetStep::Run, src/models/qwen35_2b/deltanet.cpp:358-392): the dots are
+    // taken against x * w and scaled by the norm's 1 / rms afterwards (a scalar).
+    auto pass = [&](int i, const float4& nw, const float4& av, const float4& bv) {
+      float4 xv[TOK];
 #pragma unroll
-    for (int j = 0; j < kGateAhead; ++j) {
-      const int i = tid + j * threads;
-      x_ahead[j] = i < g.cols / 4 ? xa[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    // One pass and one block-wide reduction: with norm weights the dots are taken
-    // against x * w and scaled by the norm's 1 / rms afterwards (a scalar), so the
-    // sum of squares, both dots and the q / k norms below reduce together.
-    float sq = 0.f, pa = 0.f, pb = 0.f;
-    auto pass = [&](float4 xv, const float4& nw, const float4& av, const float4& bv) {
-      if (g.norm_w != nullptr) {
-        sq += xv.x * xv.x + xv.y * xv.y + xv.z * xv.z + xv.w * xv.w;
-        xv = make_float4(xv.x * nw.x, xv.y * nw.y, xv.z * nw.z, xv.w * nw.w);
+      for (int t = 0; t < TOK; ++t) {
+        xv[t] = t < n ? *(reinterpret_cast<const float4*>(seq.x + t * seq.x_stride) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      pa += av.x * xv.x + av.y * xv.y + av.z * xv.z + av.w * xv.w;
-      pb += bv.x * xv.x + bv.y * xv.y + bv.z * xv.z + bv.w * xv.w;
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) {
+        sums[t][0] += xv[t].x * xv[t].x + xv[t].y * xv[t].y + xv[t].z * xv[t].z + xv[t].w * xv[t].w;
+        const float4 x = make_float4(xv[t].x * nw.x, xv[t].y * nw.y, xv[t].z * nw.z, xv[t].w * nw.w);
+        sums[t][1] += av.x * x.x + av.y * x.y + av.z * x.z + av.w * x.w;
+        sums[t][2] += bv.x * x.x + bv.y * x.y + bv.z * x.z + bv.w * x.w;
+      }
     };
-    const float4 one4 = make_float4(1.f, 1.f, 1.f, 1.f);
 #pragma unroll
     for (int j = 0; j < kGateAhead; ++j) {
       const int i = tid + j * threads;
       if (i < g.cols / 4) {
-        pass(x_ahead[j], g.norm_w != nullptr ? nw_ahead[j] : one4, wa_ahead[j], wb_ahead[j]);
+        pass(i, nw_ahead[j], wa_ahead[j], wb_ahead[j]);
       }
     }
     for (int i = tid + kGateAhead * threads; i < g.cols / 4; i += threads) {
-      pass(xa[i], g.norm_w != nullptr ? reinterpret_cast<const float4*>(g.norm_w)[i] : one4, wa[i], wb[i]);
+      pass(i, norm != nullptr ? norm[i] : one4, wa[i], wb[i]);
     }
-    float qv = 0.f, kv = 0.f;
-    if (lower) {
-      qv = conv(ch_a, ta, head < hk);
-      kv = conv(ch_b, tb, head < hk);
-    } else {
-      sh.v[ch] = conv(ch_a, ta, true);
+  }
+  float qv[TOK], kv[TOK];
+#pragma unroll
+  for (int t = 0; t < TOK; ++t) {
+    qv[t] = kv[t] = 0.f;
+    if (t < n) {
+      const float first = conv(ta, cur_a[t]);
+      if (lower) {
+        qv[t] = first;
+        kv[t] = conv(tb, cur_b[t]);
+      } else {
+        sh.v[t][ch] = first;
+      }
+      if (owner && t >= n - 2) {
+        float* to = t == n - 1 ? seq.conv_out : seq.conv_saved;
+        store_window(to, ch_a, ta);
+        if (lower) {
+          store_window(to, ch_b, tb);
+        }
+      }
+      sums[t][3] = qv[t] * qv[t];
+      sums[t][4] = kv[t] * kv[t];
     }
-    float five[5] = {sq, pa, pb, qv * qv, kv * kv};
-    BlockSum5(five, sh, warps);
-    const float inv = g.norm_w != nullptr ? 1.0f / sqrtf(five[0] / static_cast<float>(g.cols) + g.eps) : 1.0f;
-    const float alpha = five[1] * inv, beta = five[2] * inv;
-    // The two gates by two threads of the upper half.
-    if (tid == dk) {
-      sh.gate[0] = expf(ssm_a * Softplus(alpha + dt_bias));
-    }
-    if (tid == (dk >= 64 ? dk + 32 : dk)) {
-      sh.gate[1] = Sigmoid(beta);
-    }
-    // L2 norms (+1e-6 under the root); q also takes 1/sqrt(dk).
-    if (lower) {
-      sh.q[ch] = qv * ((1.0f / sqrtf(five[3] + 1e-6f)) * (1.0f / sqrtf(static_cast<float>(dk))));
-      sh.k[ch] = kv * (1.0f / sqrtf(five[4] + 1e-6f));
-    }
-  } else {
-    const float* gates = x + channels + value_dim;  // alpha | beta follow z
-    const float alpha = gates[head];
-    const float beta = gates[hv + head];
-    if (tid == dk) {
-      sh.gate[0] = expf(ssm_a * Softplus(alpha + dt_bias));
-    }
-    if (tid == (dk >= 64 ? dk + 32 : dk)) {
-      sh.gate[1] = Sigmoid(beta);
-    }
-    float qq = 0.f, kk = 0.f, qv = 0.f, kv = 0.f;
-    if (lower) {
-      qv = conv(ch_a, ta, head < hk);
-      kv = conv(ch_b, tb, head < hk);
-      qq = qv * qv;
-      kk = kv * kv;
-    } else {
-      sh.v[ch] = conv(ch_a, ta, true);
-    }
-    BlockSum2(qq, kk, sh, warps);
-    if (lower) {
-      sh.q[ch] = qv * ((1.0f / sqrtf(qq + 1e-6f)) * (1.0f / sqrtf(static_cast<float>(dk))));
-      sh.k[ch] = kv * (1.0f / sqrtf(kk + 1e-6f));
+  }
+#pragma unroll
+  for (int t = 0; t < TOK; ++t) {
+    if (t < n) {
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const float total = WarpSum(sums[t][i]);
+        if (lane == 0) {
+          sh.scratch[(warp * TOK + t) * 5 + i] = total;
+        }
+      }
     }
   }
   __syncthreads();
-
-  float* dst = (seq.ssm_out != nullptr ? seq.ssm_out : seq.ssm) + state_at;
+#pragma unroll
+  for (int t = 0; t < TOK; ++t) {
+    if (t < n) {
+      // Every thread needs its token's q / k sums, the gates' lanes the others.
+      float qq = 0.f, kk = 0.f;
+      for (int w = 0; w < warps; ++w) {
+        qq += sh.scratch[(w * TOK + t) * 5 + 3];
+        kk += sh.scratch[(w * TOK + t) * 5 + 4];
+      }
+      // L2 norms (+1e-6 under the root); q also takes 1/sqrt(dk).
+      if (lower) {
+        sh.q[t][ch] = qv[t] * ((1.0f / sqrtf(qq + 1e-6f)) * (1.0f / sqrtf(static_cast<float>(dk))));
+        sh.k[t][ch] = kv[t] * (1.0f / sqrtf(kk + 1e-6f));
+      }
+    }
+  }
+  // The gates by lanes of the first upper warp: token tid / 2, decay and beta.
+  if (!lower && ch < 2 * n) {
+    const int t = ch >> 1, which = ch & 1;
+    float dot;
+    if (gate_rows) {
+      float sq = 0.f;
+      dot = 0.f;
+      for (int w = 0; w < warps; ++w) {
+        sq += sh.scratch[(w * TOK + t) * 5];
+        dot += sh.scratch[(w * TOK + t) * 5 + 1 + which];
+      }
+      if (norm != nullptr) {
+        dot *= 1.0f / sqrtf(sq / static_cast<float>(g.cols) + g.eps);
+      }
+    } else {
+      dot = seq.in[t * seq.in_stride + channels + value_dim + which * hv + head];   // alpha | beta follow z
+    }
+    sh.gate[t][which] = which == 0 ? expf(ssm_a * Softplus(dot + dt_bias)) : Sigmoid(dot);
+  }
+  __syncthreads();
   // (The scratch's last readers passed the barrier above.)
-  NarrowDeltaTile(state_tile, dst, dk, tid >> 5, sh, &sh.scratch[tid >> 5]);
+#pragma unroll
+  for (int t = 0; t < TOK; ++t) {
+    if (t < n) {
+      float* dst = t == n - 1 ? seq.ssm_last + state_at : (t == n - 2 ? seq.ssm + state_at : nullptr);
+      NarrowDeltaTile(state_tile, dst, dk, warp, sh.q[t], sh.k[t], sh.v[t], sh.gate[t][0], sh.gate[t][1], sh.y[t],
+                      &sh.scratch[t * warps + warp]);
+    }
+  }
   // Gated RMSNorm over the head's dk outputs: RMS(o) * w * silu(z); the warps'
   // tiles left their outputs' squares, so one barrier serves both.
   __syncthreads();
-  const float o = lower ? sh.y[ch] : 0.f;
-  float total = 0.f;
-  for (int w = 0; w < warps; ++w) {
-    total += sh.scratch[w];
-  }
   if (lower) {
-    const float inv = 1.0f / sqrtf(total / static_cast<float>(dk) + args.rms_eps);
-    seq.y[head * dk + ch] = o * inv * norm_w * Silu(z);
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) {
+      if (t < n) {
+        float total = 0.f;
+        for (int w = 0; w < warps; ++w) {
+          total += sh.scratch[t * warps + w];
+        }
+        const float inv = 1.0f / sqrtf(total / static_cast<float>(dk) + a.rms_eps);
+        seq.y[t * seq.y_stride + head * dk + ch] = sh.y[t][ch] * inv * norm_w * Silu(z[t]);
+      }
+    }
   }
 }
 
@@ -662,7 +679,12 @@ int gufo_cuda_deltanet_linear_device(gufo_cuda_ctx* ctx,
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "deltanet_linear: unknown layer handle");
   }
   GUFO_CUDA_TRY(cudaSetDevice(ctx->device));
-  return gufo::EnqueueDeltaNetLinear(ctx, it->second, seqs, nseq, ctx->early_state);
+  std::vector<gufo::DeltaNetSeq> step(nseq);
+  for (int s = 0; s < nseq; ++s) {
+    const gufo_cuda_linear_seq& q = seqs[s];
+    step[s] = gufo::OneTokenSeq(q.in, nullptr, q.conv_in, q.conv_out, q.ssm, q.ssm_out != nullptr ? q.ssm_out : q.ssm, q.y);
+  }
+  return gufo::EnqueueDeltaNetLinear(ctx, it->second, step.data(), nseq, ctx->early_state);
 }
 
 int gufo_cuda_deltanet_step_device(gufo_cuda_ctx* ctx, gufo_cuda_deltanet_layer layer, gufo_cuda_matrix ssm_alpha,
@@ -711,72 +733,82 @@ int gufo_cuda_deltanet_step_device(gufo_cuda_ctx* ctx, gufo_cuda_deltanet_layer 
   gates.cols = static_cast<int>(alpha->cols);
   gates.norm_w = attn_norm;
   gates.eps = rms_eps;
-  // Token t of every sequence that has one, in one launch per t. Windows
-  // alternate between conv_out and conv_saved so that the last token reads
-  // conv_saved and writes conv_out; the last of two or more tokens leaves ssm
-  // alone and writes ssm_spec.
-  std::vector<gufo_cuda_linear_seq> step;
-  std::vector<const float*> xs;
-  for (int t = 0; t < most; ++t) {
-    step.clear();
-    xs.clear();
+  // Sequences of the most tokens first: their blocks run longest.
+  std::vector<gufo::DeltaNetSeq> step;
+  step.reserve(nseq);
+  for (int n = most; n >= 1; --n) {
     for (int s = 0; s < nseq; ++s) {
       const gufo_cuda_deltanet_step_seq& q = seqs[s];
-      if (t >= q.n_tokens) {
-        continue;
+      if (q.n_tokens == n) {
+        step.push_back({q.in, q.h, q.conv_in, q.conv_saved, q.conv_out, q.ssm, q.ssm, n >= 2 ? q.ssm_spec : q.ssm, q.y,
+                        q.in_stride, q.h_stride, q.y_stride, n});
       }
-      const int from_end = q.n_tokens - 1 - t;   // 0 for the last token
-      float* dst = from_end % 2 == 0 ? q.conv_out : q.conv_saved;
-      const float* src = t == 0 ? q.conv_in : (from_end % 2 == 0 ? q.conv_saved : q.conv_out);
-      const bool speculative = q.n_tokens >= 2 && from_end == 0;
-      step.push_back({q.in + static_cast<size_t>(t) * q.in_stride, src, dst, q.ssm, speculative ? q.ssm_spec : nullptr,
-                      q.y + static_cast<size_t>(t) * q.y_stride});
-      xs.push_back(q.h + static_cast<size_t>(t) * q.h_stride);
-    }
-    gates.xs = xs.data();
-    // States are written by the launch before this one: no early state loads.
-    const int rc = gufo::EnqueueDeltaNetLinear(ctx, it->second, step.data(), static_cast<int>(step.size()), false,
-                                               &gates);
-    if (rc != GUFO_CUDA_OK) {
-      return rc;
     }
   }
-  return GUFO_CUDA_OK;
+  // States may be written by the launch before this one: no early state loads.
+  return gufo::EnqueueDeltaNetLinear(ctx, it->second, step.data(), nseq, false, &gates);
 }
 
 }  // extern "C"
 
 namespace gufo {
 
-int EnqueueDeltaNetLinear(gufo_cuda_ctx* ctx, const DeltaNetLayer& l,
-                          const gufo_cuda_linear_seq* seqs, int nseq, bool early_state,
-                          const DeltaNetGateRows* gate_rows) {
-  for (int s0 = 0; s0 < nseq; s0 += gufo::kMaxSeqs) {
-    const int n = nseq - s0 < gufo::kMaxSeqs ? nseq - s0 : gufo::kMaxSeqs;
-    gufo::LinearArgs args{};
-    for (int s = 0; s < n; ++s) {
-      args.seq[s] = seqs[s0 + s];
+namespace {
+
+template <int TOK, int WIN, int SEQS>
+int LaunchLinear(gufo_cuda_ctx* ctx, const LinearShape& shape, const DeltaNetSeq* seqs, int n) {
+  LinearArgs<SEQS> args;
+  args.shape = shape;
+  for (int s = 0; s < n; ++s) {
+    args.seq[s] = seqs[s];
+  }
+  GUFO_CUDA_TRY(LaunchOverlapped(DeltaNetLinearKernel<TOK, WIN, SEQS>, dim3(shape.value_heads, n), dim3(2 * shape.head_dim),
+                                 0, ctx->stream, 1, args));
+  ctx->launches.fetch_add(1);
+  return GUFO_CUDA_OK;
+}
+
+template <int TOK>
+int LaunchTokens(gufo_cuda_ctx* ctx, const LinearShape& shape, const DeltaNetSeq* seqs, int n) {
+  // One or two sequences (a decode step) in a small argument block; windows of
+  // up to three columns (four taps, the models' own) in few registers.
+  const bool narrow = shape.conv_kernel <= 4;
+  if (n <= 2) {
+    return narrow ? LaunchLinear<TOK, 3, 2>(ctx, shape, seqs, n) : LaunchLinear<TOK, 7, 2>(ctx, shape, seqs, n);
+  }
+  return narrow ? LaunchLinear<TOK, 3, kMaxSeqs>(ctx, shape, seqs, n) : LaunchLinear<TOK, 7, kMaxSeqs>(ctx, shape, seqs, n);
+}
+
+}  // namespace
+
+int EnqueueDeltaNetLinear(gufo_cuda_ctx* ctx, const DeltaNetLayer& l, const DeltaNetSeq* seqs, int nseq,
+                          bool early_state, const DeltaNetGateRows* gate_rows) {
+  LinearShape shape{};
+  shape.key_heads = l.key_heads;
+  shape.value_heads = l.value_heads;
+  shape.head_dim = l.head_dim;
+  shape.conv_kernel = l.conv_kernel;
+  shape.rms_eps = l.rms_eps;
+  shape.conv = l.conv;
+  shape.ssm_a = l.ssm_a;
+  shape.dt_bias = l.dt_bias;
+  shape.ssm_norm = l.ssm_norm;
+  shape.early_state = early_state ? 1 : 0;
+  if (gate_rows != nullptr) {
+    shape.gate_rows = *gate_rows;
+  }
+  for (int s0 = 0; s0 < nseq; s0 += kMaxSeqs) {
+    const int n = nseq - s0 < kMaxSeqs ? nseq - s0 : kMaxSeqs;
+    int most = 1;
+    for (int s = s0; s < s0 + n; ++s) {
+      most = seqs[s].tokens > most ? seqs[s].tokens : most;
     }
-    args.key_heads = l.key_heads;
-    args.value_heads = l.value_heads;
-    args.head_dim = l.head_dim;
-    args.conv_kernel = l.conv_kernel;
-    args.rms_eps = l.rms_eps;
-    args.conv = l.conv;
-    args.ssm_a = l.ssm_a;
-    args.dt_bias = l.dt_bias;
-    args.ssm_norm = l.ssm_norm;
-    args.early_state = early_state ? 1 : 0;
-    if (gate_rows != nullptr) {
-      args.gate_rows = *gate_rows;
-      for (int s = 0; s < n; ++s) {
-        args.gate_x[s] = gate_rows->xs != nullptr ? gate_rows->xs[s0 + s] : nullptr;
-      }
-      args.gate_rows.xs = nullptr;
+    const int rc = most == 1   ? LaunchTokens<1>(ctx, shape, seqs + s0, n)
+                   : most == 2 ? LaunchTokens<2>(ctx, shape, seqs + s0, n)
+                               : LaunchTokens<kMaxRunTokens>(ctx, shape, seqs + s0, n);
+    if (rc != GUFO_CUDA_OK) {
+      return rc;
     }
-    GUFO_CUDA_TRY(gufo::LaunchOverlapped(gufo::DeltaNetLinearKernel, dim3(l.value_heads, n),
-                                         dim3(2 * l.head_dim), 0, ctx->stream, 1, args));
-    ctx->launches.fetch_add(1);
   }
   return GUFO_CUDA_OK;
 }
