@@ -238,10 +238,11 @@ struct DeltaNetSeq {
   float* y;                // [tokens], y_stride apart
   int64_t in_stride, x_stride, y_stride;
   int tokens;
+  const float* gates;      // [tokens][2 value heads]: alpha | beta, or null (behind z in the input row)
 };
 inline DeltaNetSeq OneTokenSeq(const float* in, const float* x, const float* conv_in, float* conv_out, const float* ssm_in,
                                float* ssm_out, float* y) {
-  return {in, x, conv_in, nullptr, conv_out, ssm_in, nullptr, ssm_out, y, 0, 0, 0, 1};
+  return {in, x, conv_in, nullptr, conv_out, ssm_in, nullptr, ssm_out, y, 0, 0, 0, 1, nullptr};
 }
 // Mixer::Linear for every sequence (1 to 4 tokens each); the caller holds ctx->mu.
 // `early_state`: the states and conv windows were not written by the kernels
@@ -268,6 +269,9 @@ struct gufo_cuda_ctx {
   size_t stage_x_bytes = 0;
   float* stage_y = nullptr;
   size_t stage_y_bytes = 0;
+  // The gate dots of a DeltaNet step of several sequences.
+  uint8_t* gates = nullptr;
+  size_t gates_bytes = 0;
   // Fixed-point image of the activations of the product in flight.
   uint8_t* image = nullptr;
   size_t image_bytes = 0;

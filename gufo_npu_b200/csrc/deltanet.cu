@@ -62,109 +62,149 @@ struct LinearArgs {
 
 namespace {
 
+// Two fp32 values in a register pair and the packed instructions on them: half
+// the issue slots of the delta rule's arithmetic.
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair MakePair(float a, float b) {
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
+  return p;
+}
+__device__ __forceinline__ float2 Unpack(Pair p) {
+  float2 v;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ Pair Fma2(Pair a, Pair b, Pair c) {
+  Pair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ Pair Mul2(Pair a, Pair b) {
+  Pair d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // A warp's tile of COLS (8 or 16) adjacent columns of a head's state: a lane
 // holds rows ig, ig + 32 / G, ... (ig = lane / G, G = COLS / 4) of four adjacent
-// columns (4 * (lane % G)). Narrow tiles mean many warps per head.
+// columns (4 * (lane % G)), as two pairs. Narrow tiles mean many warps per head.
 template <int COLS>
 struct NarrowTile {
   static constexpr int kGroups = COLS / 4;                 // lanes across the columns
   static constexpr int kRowGroups = 32 / kGroups;
   static constexpr int kRowsPerLane = kMaxHeadDim / kRowGroups;
-  float4 s[kRowsPerLane];
+  ulonglong2 s[kRowsPerLane];
 };
 
-template <int COLS>
+template <int DK, int COLS>
 __device__ __forceinline__ void LoadNarrowTile(NarrowTile<COLS>& tile, const float* __restrict__ src, int dk,
                                                int tile_index) {
   using T = NarrowTile<COLS>;
   const int lane = threadIdx.x & 31;
   const int col = tile_index * COLS + 4 * (lane % T::kGroups);
   const int ig = lane / T::kGroups;
-  const int rows = dk / T::kRowGroups;
+  const int rows = (DK > 0 ? DK : dk) / T::kRowGroups;
+  if (DK > 0) {
+    dk = DK;
+  }
 #pragma unroll
   for (int r = 0; r < T::kRowsPerLane; ++r) {
     if (r < rows) {
-      tile.s[r] = *reinterpret_cast<const float4*>(src + static_cast<size_t>(r * T::kRowGroups + ig) * dk + col);
+      tile.s[r] = *reinterpret_cast<const ulonglong2*>(src + static_cast<size_t>(r * T::kRowGroups + ig) * dk + col);
     }
   }
 }
 
-// Sum over the warp's row groups; every lane gets its columns' totals.
-template <int COLS>
-__device__ __forceinline__ float4 NarrowColumnSum(float4 v) {
+// Scalars of one token's update, for raw k and q whose norms are factors.
+struct DeltaCoef {
+  float decay;
+  float beta;
+  float k;       // |k|^-1
+  float q;       // |q|^-1 dk^-1/2
+  float kq;      // k . q of the raw vectors
+};
+
+// The delta rule on this warp's column tile, which becomes S'. Per column j:
+//   u = decay (S^T k)_j,  delta = beta (v_j - u),  S' = decay S + k delta^T,
+//   y = (S'^T q)_j = decay (S^T q)_j + (k . q) delta:
+// both sums over the rows are taken in one pass over S (TileSums, which needs none
+// of the token's scalars), and the update (TileUpdate) needs no second reduction.
+// k2, q2: the head's raw vectors in shared memory, every value twice. DK: the head
+// dim where it is known at compile time (the models' 128), else 0.
+template <int DK, int COLS>
+__device__ __forceinline__ void TileSums(const NarrowTile<COLS>& tile, int dk, const Pair* q2, const Pair* k2,
+                                         float (&sum)[8]) {
+  using T = NarrowTile<COLS>;
+  const int ig = (threadIdx.x & 31) / T::kGroups;
+  const int rows = (DK > 0 ? DK : dk) / T::kRowGroups;
+  Pair u01 = 0, u23 = 0, w01 = 0, w23 = 0;
 #pragma unroll
-  for (int o = NarrowTile<COLS>::kGroups; o <= 16; o <<= 1) {
-    v.x += __shfl_xor_sync(0xFFFFFFFFu, v.x, o);
-    v.y += __shfl_xor_sync(0xFFFFFFFFu, v.y, o);
-    v.z += __shfl_xor_sync(0xFFFFFFFFu, v.z, o);
-    v.w += __shfl_xor_sync(0xFFFFFFFFu, v.w, o);
+  for (int r = 0; r < T::kRowsPerLane; ++r) {
+    if (r < rows) {
+      const Pair k = k2[r * T::kRowGroups + ig], q = q2[r * T::kRowGroups + ig];
+      u01 = Fma2(tile.s[r].x, k, u01);
+      u23 = Fma2(tile.s[r].y, k, u23);
+      w01 = Fma2(tile.s[r].x, q, w01);
+      w23 = Fma2(tile.s[r].y, q, w23);
+    }
   }
-  return v;
+  const float2 a = Unpack(u01), b = Unpack(u23), d = Unpack(w01), e = Unpack(w23);
+  sum[0] = a.x, sum[1] = a.y, sum[2] = b.x, sum[3] = b.y, sum[4] = d.x, sum[5] = d.y, sum[6] = e.x, sum[7] = e.y;
+  // Over the warp's row groups; every lane gets its columns' totals.
+#pragma unroll
+  for (int o = T::kGroups; o <= 16; o <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      sum[i] += __shfl_xor_sync(0xFFFFFFFFu, sum[i], o);
+    }
+  }
 }
 
-// The delta rule on this warp's column tile, which becomes S'. Writes S' to dst
-// (may be null) and the tile's outputs to out (no barrier); with `squares`, lane 0
-// also leaves the sum of the squares of the tile's outputs there. q, k, v: the
-// head's vectors in shared memory.
-template <int COLS>
-__device__ __forceinline__ void NarrowDeltaTile(NarrowTile<COLS>& tile, float* __restrict__ dst, int dk,
-                                                int tile_index, const float* q, const float* k, const float* v_in,
-                                                float decay, float beta, float* out, float* squares = nullptr) {
+// Writes S' to dst (may be null) and the tile's outputs to out (no barrier); with
+// `squares`, lane 0 also leaves the sum of their squares there.
+template <int DK, int COLS>
+__device__ __forceinline__ void TileUpdate(NarrowTile<COLS>& tile, const float (&sum)[8], float* __restrict__ dst, int dk,
+                                           int tile_index, const Pair* k2, const float* v_in, const DeltaCoef& c,
+                                           float* out, float* squares = nullptr) {
   using T = NarrowTile<COLS>;
   const int lane = threadIdx.x & 31;
   const int col = tile_index * COLS + 4 * (lane % T::kGroups);
   const int ig = lane / T::kGroups;
+  if (DK > 0) {
+    dk = DK;
+  }
   const int rows = dk / T::kRowGroups;
-  float4 (&s)[T::kRowsPerLane] = tile.s;
-  // Pass 1: u_j = sum_i S_ij * (k_i * decay).
-  float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 v4 = *reinterpret_cast<const float4*>(&v_in[col]);
+  const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+  float delta[4], y[4];
+  const float u_factor = c.decay * c.k, y_factor = c.decay * c.q, kq = c.kq * c.k * c.q;
 #pragma unroll
-  for (int r = 0; r < T::kRowsPerLane; ++r) {
-    if (r < rows) {
-      const float ki = k[r * T::kRowGroups + ig] * decay;
-      u.x = fmaf(s[r].x, ki, u.x);
-      u.y = fmaf(s[r].y, ki, u.y);
-      u.z = fmaf(s[r].z, ki, u.z);
-      u.w = fmaf(s[r].w, ki, u.w);
-    }
+  for (int i = 0; i < 4; ++i) {
+    delta[i] = c.beta * (v[i] - u_factor * sum[i]);
+    y[i] = fmaf(kq, delta[i], y_factor * sum[4 + i]);
+    delta[i] *= c.k;
   }
-  u = NarrowColumnSum<COLS>(u);
-  const float4 v = *reinterpret_cast<const float4*>(&v_in[col]);
-  float4 delta;
-  delta.x = beta * (v.x - u.x);
-  delta.y = beta * (v.y - u.y);
-  delta.z = beta * (v.z - u.z);
-  delta.w = beta * (v.w - u.w);
-  // Pass 2: S'_ij = S_ij * decay + k_i * delta_j; y_j = sum_i S'_ij * q_i.
-  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+  const Pair decay = MakePair(c.decay, c.decay);
+  const Pair d01 = MakePair(delta[0], delta[1]), d23 = MakePair(delta[2], delta[3]);
+  float* to = dst + static_cast<size_t>(ig) * dk + col;
 #pragma unroll
   for (int r = 0; r < T::kRowsPerLane; ++r) {
     if (r < rows) {
-      const int i = r * T::kRowGroups + ig;
-      const float ki = k[i];
-      const float qi = q[i];
-      float4 n;
-      n.x = fmaf(s[r].x, decay, ki * delta.x);
-      n.y = fmaf(s[r].y, decay, ki * delta.y);
-      n.z = fmaf(s[r].z, decay, ki * delta.z);
-      n.w = fmaf(s[r].w, decay, ki * delta.w);
+      const Pair k = k2[r * T::kRowGroups + ig];
+      tile.s[r].x = Fma2(tile.s[r].x, decay, Mul2(k, d01));
+      tile.s[r].y = Fma2(tile.s[r].y, decay, Mul2(k, d23));
       if (dst != nullptr) {
-        *reinterpret_cast<float4*>(dst + static_cast<size_t>(i) * dk + col) = n;
+        *reinterpret_cast<ulonglong2*>(to + r * T::kRowGroups * dk) = tile.s[r];
       }
-      s[r] = n;
-      y.x = fmaf(n.x, qi, y.x);
-      y.y = fmaf(n.y, qi, y.y);
-      y.z = fmaf(n.z, qi, y.z);
-      y.w = fmaf(n.w, qi, y.w);
     }
   }
-  y = NarrowColumnSum<COLS>(y);
   if (ig == 0) {
-    *reinterpret_cast<float4*>(&out[col]) = y;
+    *reinterpret_cast<float4*>(&out[col]) = make_float4(y[0], y[1], y[2], y[3]);
   }
   if (squares != nullptr) {
     // Lanes 0 .. kGroups - 1 hold the tile's COLS outputs.
-    float sq = ig == 0 ? y.x * y.x + y.y * y.y + y.z * y.z + y.w * y.w : 0.f;
+    float sq = ig == 0 ? y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3] : 0.f;
 #pragma unroll
     for (int o = T::kGroups / 2; o > 0; o >>= 1) {
       sq += __shfl_xor_sync(0xFFFFFFFFu, sq, o);
@@ -176,42 +216,50 @@ __device__ __forceinline__ void NarrowDeltaTile(NarrowTile<COLS>& tile, float* _
 }
 
 constexpr int kStepCols = 16;   // columns per warp in the decode step's kernel
-constexpr int kRuleCols = 16;   // and in the stand-alone delta rule (8: 4.9 us for config 3, 16: 4.1, 32: 4.6)
+constexpr int kRuleCols = 16;   // columns per warp in the stand-alone delta rule (8: 4.9 us for config 3, 16: 4.1, 32: 4.6)
 
 // Gates given: one warp per thread block, grid = (dk / 16, value_heads,
 // sequences). The tiles of a head need nothing from one another here, and
 // many small blocks per SM let one tile's stores overlap another's loads
 // (16-column tiles: 1024 warps for eight sequences of sixteen heads).
+template <int DK>
 __global__ void __launch_bounds__(32)
 DeltaRuleKernel(const __grid_constant__ DeltaRuleArgs args) {
-  __shared__ __align__(16) float q[kMaxHeadDim], k[kMaxHeadDim], v[kMaxHeadDim], y[kMaxHeadDim];
+  __shared__ __align__(16) Pair q2[kMaxHeadDim], k2[kMaxHeadDim];
+  __shared__ __align__(16) float v[kMaxHeadDim], y[kMaxHeadDim];
   const gufo_cuda_delta_seq& seq = args.seq[blockIdx.z];
   const int head = blockIdx.y;
   const int tile = blockIdx.x;
-  const int dk = args.head_dim;
+  const int dk = DK > 0 ? DK : args.head_dim;
   const int kh = head % args.key_heads;
   const int lane = threadIdx.x;
   const size_t state_at = static_cast<size_t>(head) * dk * dk;
   NarrowTile<kRuleCols> state;
   GridLaunchDependents();
   if (args.early_state) {
-    LoadNarrowTile(state, seq.state + state_at, dk, tile);
+    LoadNarrowTile<DK>(state, seq.state + state_at, dk, tile);
   }
   GridDependencyWait();
   if (!args.early_state) {
-    LoadNarrowTile(state, seq.state + state_at, dk, tile);
+    LoadNarrowTile<DK>(state, seq.state + state_at, dk, tile);
   }
+  float kq = 0.f;
   for (int i = lane; i < dk; i += 32) {
-    q[i] = seq.q[kh * dk + i];
-    k[i] = seq.k[kh * dk + i];
+    const float q = seq.q[kh * dk + i], k = seq.k[kh * dk + i];
+    q2[i] = MakePair(q, q);
+    k2[i] = MakePair(k, k);
+    kq = fmaf(k, q, kq);
   }
   if (lane < kRuleCols) {
     v[tile * kRuleCols + lane] = seq.v[head * dk + tile * kRuleCols + lane];
   }
   const float decay = seq.decay[head], beta = seq.beta[head];
+  const DeltaCoef coef{decay, beta, 1.0f, 1.0f, WarpSum(kq)};
   __syncwarp();
   float* dst = (seq.state_out != nullptr ? seq.state_out : seq.state) + state_at;
-  NarrowDeltaTile(state, dst, dk, tile, q, k, v, decay, beta, y);
+  float sums[8];
+  TileSums<DK>(state, dk, q2, k2, sums);
+  TileUpdate<DK>(state, sums, dst, dk, tile, k2, v, coef, y);
   __syncwarp();
   if (lane < kRuleCols) {
     seq.y[head * dk + tile * kRuleCols + lane] = y[tile * kRuleCols + lane];
@@ -219,46 +267,59 @@ DeltaRuleKernel(const __grid_constant__ DeltaRuleArgs args) {
 }
 
 __device__ __forceinline__ float Sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
+// The gates' arithmetic, spelled out: one sequence (in the mixer kernel) and several
+// (DeltaNetGatesKernel) get the same bits.
+__device__ __forceinline__ float Dot4(const float4& a, const float4& b, float sum) {
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, sum))));
+}
+__device__ __forceinline__ float4 Times4(const float4& a, const float4& b) {
+  return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
+}
+__device__ __forceinline__ float GateInverse(float squares, int cols, float eps) {
+  return 1.0f / sqrtf(squares / static_cast<float>(cols) + eps);
+}
 __device__ __forceinline__ float Silu(float x) { return x * Sigmoid(x); }
 __device__ __forceinline__ float Softplus(float x) {
   return x > 20.0f ? x : log1pf(expf(x));
 }
 
-// Mixer::Linear for one (sequence, value head), up to TOK tokens. grid =
+// Mixer::Linear for one (sequence, value head), one to four tokens. grid =
 // (value_heads, sequences), 2 * dk threads: thread t < dk owns channel t of the
 // head's q and k and output t of the epilogue, thread dk + t channel t of v; warp w
 // owns columns 16 w .. 16 w + 15 of the state. (With dk threads and 32 columns per
-// warp the kernel spent 6.5 us per layer of the decode step on four warps' worth of
-// dependent instructions.)
+// warp the decode step's kernel spent 6.5 us per layer on four warps' worth of
+// dependent instructions; 8 columns and 4 * dk threads gained it nothing and cost
+// 32 sequences of 32 heads 55 us instead of 48.)
 //
-// All that does not need the state - convolutions, gates, norms of every token -
-// is done first, for all tokens at once and under the state's load; the tokens then
-// follow one another on the state in registers with no block barrier between them
-// (a warp's columns need nothing from the others'), and the gated norms of all
-// tokens close the block. The state is read once and written once (a draft's once
-// more) whatever the tokens: as a launch per token index, 32 sequences of 32 heads
-// with one to four tokens took 110 us and moved the states up to eight times.
-template <int TOK>
+// All that does not need the state - convolutions, gate dots - is done first, token
+// after token under the state's load; then a warp each works out the tokens'
+// scalars, and the tokens follow one another on the state in registers with no
+// block barrier between them (a warp's columns need nothing from the others'); the
+// gated norms of all tokens close the block. The state is read once and written
+// once (a draft's once more) whatever the tokens. The token loops are not unrolled:
+// as straight code for four tokens the kernel ran out of the instruction cache.
 struct LinearShared {
-  float q[TOK][kMaxHeadDim];
-  float k[TOK][kMaxHeadDim];
-  float v[TOK][kMaxHeadDim];
-  float y[TOK][kMaxHeadDim];
-  float gate[TOK][2];                                  // decay, beta
-  float scratch[(2 * kDeltaThreads / 32) * 5 * TOK];   // five sums a token and warp
+  Pair q2[kMaxRunTokens][kMaxHeadDim];                 // every value twice
+  Pair k2[kMaxRunTokens][kMaxHeadDim];
+  float v[kMaxRunTokens][kMaxHeadDim];
+  float y[kMaxRunTokens][kMaxHeadDim];
+  float z[kMaxRunTokens][kMaxHeadDim];
+  DeltaCoef coef[kMaxRunTokens];
+  float gates[kMaxRunTokens][3][8];                   // a warp's part of the input's squares and the gate dots
+  float squares[kMaxRunTokens][8];                    // a warp's part of the outputs' squares
 };
 
-template <int TOK, int WIN, int SEQS>
+template <int DK, int WIN, int SEQS>
 __global__ void __launch_bounds__(2 * kDeltaThreads, SEQS > 2 ? 2 : 1)
 DeltaNetLinearKernel(const __grid_constant__ LinearArgs<SEQS> args) {
-  __shared__ __align__(16) LinearShared<TOK> sh;
+  __shared__ __align__(16) LinearShared sh;
   const LinearShape& a = args.shape;
   const DeltaNetSeq& seq = args.seq[blockIdx.y];
-  const int n = TOK == 1 ? 1 : seq.tokens;
+  const int n = seq.tokens;
   const int head = blockIdx.x;
   const int hk = a.key_heads;
   const int hv = a.value_heads;
-  const int dk = a.head_dim;
+  const int dk = DK > 0 ? DK : a.head_dim;
   const int threads = 2 * dk;
   const int warps = threads / 32;
   const int key_dim = hk * dk;
@@ -327,17 +388,18 @@ DeltaNetLinearKernel(const __grid_constant__ LinearArgs<SEQS> args) {
   const bool owner = !lower || head < hk;
   Taps ta, tb;
   // The first passes of the head's alpha and beta rows (weights as well).
+  // (Launches of several sequences find the dots done, DeltaNetGatesKernel.)
   constexpr int kGateAhead = 2;
   const DeltaNetGateRows& g = a.gate_rows;
-  const bool gate_rows = g.alpha_w != nullptr;
+  const bool gate_rows = SEQS <= 2 && g.alpha_w != nullptr;
   const float4* wa = reinterpret_cast<const float4*>(g.alpha_w + static_cast<size_t>(head) * g.cols);
   const float4* wb = reinterpret_cast<const float4*>(g.beta_w + static_cast<size_t>(head) * g.cols);
   const float4* norm = reinterpret_cast<const float4*>(g.norm_w);
-  const float4 one4 = make_float4(1.f, 1.f, 1.f, 1.f);
-  float4 wa_ahead[kGateAhead], wb_ahead[kGateAhead], nw_ahead[kGateAhead];
+  float4 wa_ahead[kGateAhead], wb_ahead[kGateAhead];   // times the norm's weights, where it has them
+  auto scaled = [&](const float4& w, int i) { return norm != nullptr ? Times4(w, norm[i]) : w; };
   GridLaunchDependents();
   if (a.early_state) {
-    LoadNarrowTile(state_tile, seq.ssm_in + state_at, dk, warp);
+    LoadNarrowTile<DK>(state_tile, seq.ssm_in + state_at, dk, warp);
     fetch_window(ch_a, ta);
     if (lower) {
       fetch_window(ch_b, tb);
@@ -352,9 +414,8 @@ DeltaNetLinearKernel(const __grid_constant__ LinearArgs<SEQS> args) {
     for (int j = 0; j < kGateAhead; ++j) {
       const int i = tid + j * threads;
       if (i < g.cols / 4) {
-        wa_ahead[j] = wa[i];
-        wb_ahead[j] = wb[i];
-        nw_ahead[j] = norm != nullptr ? norm[i] : one4;
+        wa_ahead[j] = scaled(wa[i], i);
+        wb_ahead[j] = scaled(wb[i], i);
       }
     }
   }
@@ -362,165 +423,259 @@ DeltaNetLinearKernel(const __grid_constant__ LinearArgs<SEQS> args) {
   const float ssm_a = a.ssm_a[head], dt_bias = a.dt_bias[head];
   GridDependencyWait();
   if (!a.early_state) {
-    LoadNarrowTile(state_tile, seq.ssm_in + state_at, dk, warp);
     fetch_window(ch_a, ta);
     if (lower) {
       fetch_window(ch_b, tb);
     }
   }
-  // What the tokens bring, the epilogue's z included, requested at once.
-  float cur_a[TOK], cur_b[TOK], z[TOK];
+  // What a token brings, requested a token ahead.
+  struct Row {
+    float a, b, z;
+    float4 x[kGateAhead];
+  };
+  auto fetch_row = [&](int t, Row& row) {
+    const float* in = seq.in + t * seq.in_stride;
+    row.a = in[ch_a];
+    row.b = lower ? in[ch_b] : 0.f;
+    row.z = lower ? in[channels + head * dk + ch] : 0.f;
+    if (gate_rows) {
+      const float4* x = reinterpret_cast<const float4*>(seq.x + t * seq.x_stride);
 #pragma unroll
-  for (int t = 0; t < TOK; ++t) {
-    cur_a[t] = cur_b[t] = z[t] = 0.f;
-    if (t < n) {
-      const float* in = seq.in + t * seq.in_stride;
-      cur_a[t] = in[ch_a];
-      if (lower) {
-        cur_b[t] = in[ch_b];
-        z[t] = in[channels + head * dk + ch];
+      for (int j = 0; j < kGateAhead; ++j) {
+        const int i = tid + j * threads;
+        row.x[j] = i < g.cols / 4 ? x[i] : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
+  };
+  Row next;
+  fetch_row(0, next);
+  // The state behind what is needed first: its 64 KB take their time.
+  if (!a.early_state) {
+    LoadNarrowTile<DK>(state_tile, seq.ssm_in + state_at, dk, warp);
   }
-  // Five sums a token: the gate input's squares, the two gate dots, the q and k
-  // norms' squares; one block-wide reduction for all of them.
-  float sums[TOK][5];
-#pragma unroll
-  for (int t = 0; t < TOK; ++t) {
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      sums[t][i] = 0.f;
+#pragma unroll 1
+  for (int t = 0; t < n; ++t) {
+    const Row row = next;
+    if (t + 1 < n) {
+      fetch_row(t + 1, next);
     }
-  }
-  if (gate_rows) {
-    // The head's alpha and beta rows against the normed input, one float4 per
-    // thread and pass (GgufProjections serves these F32 rows through its own
-    // dot, src/models/qwen35/gguf_projections.cpp:162-170). With norm weights
-    // the input is the residual stream and the RMS norm is applied on the way
-    // (DeltaNetStep::Run, src/models/qwen35_2b/deltanet.cpp:358-392): the dots are
-    // taken against x * w and scaled by the norm's 1 / rms afterwards (a scalar).
-    auto pass = [&](int i, const float4& nw, const float4& av, const float4& bv) {
-      float4 xv[TOK];
+    if (gate_rows) {
+      // The head's alpha and beta rows against the normed input, one float4 per
+      // thread and pass (GgufProjections serves these F32 rows through its own
+      // dot, src/models/qwen35/gguf_projections.cpp:162-170). With norm weights
+      // the input is the residual stream and the RMS norm is applied on the way
+      // (DeltaNetStep::Run, src/models/qwen35_2b/deltanet.cpp:358-392): the rows
+      // carry its weights and the dots are scaled by its 1 / rms afterwards.
+      float sums[3] = {};
+      auto pass = [&](const float4& x, const float4& av, const float4& bv) {
+        sums[0] = Dot4(x, x, sums[0]);
+        sums[1] = Dot4(av, x, sums[1]);
+        sums[2] = Dot4(bv, x, sums[2]);
+      };
 #pragma unroll
-      for (int t = 0; t < TOK; ++t) {
-        xv[t] = t < n ? *(reinterpret_cast<const float4*>(seq.x + t * seq.x_stride) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int t = 0; t < TOK; ++t) {
-        sums[t][0] += xv[t].x * xv[t].x + xv[t].y * xv[t].y + xv[t].z * xv[t].z + xv[t].w * xv[t].w;
-        const float4 x = make_float4(xv[t].x * nw.x, xv[t].y * nw.y, xv[t].z * nw.z, xv[t].w * nw.w);
-        sums[t][1] += av.x * x.x + av.y * x.y + av.z * x.z + av.w * x.w;
-        sums[t][2] += bv.x * x.x + bv.y * x.y + bv.z * x.z + bv.w * x.w;
-      }
-    };
-#pragma unroll
-    for (int j = 0; j < kGateAhead; ++j) {
-      const int i = tid + j * threads;
-      if (i < g.cols / 4) {
-        pass(i, nw_ahead[j], wa_ahead[j], wb_ahead[j]);
-      }
-    }
-    for (int i = tid + kGateAhead * threads; i < g.cols / 4; i += threads) {
-      pass(i, norm != nullptr ? norm[i] : one4, wa[i], wb[i]);
-    }
-  }
-  float qv[TOK], kv[TOK];
-#pragma unroll
-  for (int t = 0; t < TOK; ++t) {
-    qv[t] = kv[t] = 0.f;
-    if (t < n) {
-      const float first = conv(ta, cur_a[t]);
-      if (lower) {
-        qv[t] = first;
-        kv[t] = conv(tb, cur_b[t]);
-      } else {
-        sh.v[t][ch] = first;
-      }
-      if (owner && t >= n - 2) {
-        float* to = t == n - 1 ? seq.conv_out : seq.conv_saved;
-        store_window(to, ch_a, ta);
-        if (lower) {
-          store_window(to, ch_b, tb);
+      for (int j = 0; j < kGateAhead; ++j) {
+        if (tid + j * threads < g.cols / 4) {
+          pass(row.x[j], wa_ahead[j], wb_ahead[j]);
         }
       }
-      sums[t][3] = qv[t] * qv[t];
-      sums[t][4] = kv[t] * kv[t];
+      const float4* x = reinterpret_cast<const float4*>(seq.x + t * seq.x_stride);
+      for (int i = tid + kGateAhead * threads; i < g.cols / 4; i += threads) {
+        pass(x[i], scaled(wa[i], i), scaled(wb[i], i));
+      }
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        sums[i] = WarpSum(sums[i]);
+      }
+      if (lane < 3) {
+        sh.gates[t][lane][warp] = lane == 0 ? sums[0] : (lane == 1 ? sums[1] : sums[2]);
+      }
     }
-  }
-#pragma unroll
-  for (int t = 0; t < TOK; ++t) {
-    if (t < n) {
-#pragma unroll
-      for (int i = 0; i < 5; ++i) {
-        const float total = WarpSum(sums[t][i]);
-        if (lane == 0) {
-          sh.scratch[(warp * TOK + t) * 5 + i] = total;
-        }
+    const float value = conv(ta, row.a);
+    if (lower) {
+      const float k = conv(tb, row.b);
+      sh.q2[t][ch] = MakePair(value, value);
+      sh.k2[t][ch] = MakePair(k, k);
+      sh.z[t][ch] = row.z;
+    } else {
+      sh.v[t][ch] = value;
+    }
+    if (owner && t >= n - 2) {
+      float* to = t == n - 1 ? seq.conv_out : seq.conv_saved;
+      store_window(to, ch_a, ta);
+      if (lower) {
+        store_window(to, ch_b, tb);
       }
     }
   }
   __syncthreads();
+  // The tokens' scalars, a warp each: decay, beta, the norms of q and k.
+  for (int item = warp; item < 3 * n; item += warps) {
+    const int t = item / 3, which = item - 3 * t;
+    if (which < 2) {
+      float dot;
+      if (gate_rows) {
+        auto total = [&](int i) {
+          float part = lane < warps ? sh.gates[t][i][lane] : 0.f;
 #pragma unroll
-  for (int t = 0; t < TOK; ++t) {
-    if (t < n) {
-      // Every thread needs its token's q / k sums, the gates' lanes the others.
-      float qq = 0.f, kk = 0.f;
-      for (int w = 0; w < warps; ++w) {
-        qq += sh.scratch[(w * TOK + t) * 5 + 3];
-        kk += sh.scratch[(w * TOK + t) * 5 + 4];
+          for (int o = 4; o > 0; o >>= 1) {
+            part += __shfl_xor_sync(0xFFFFFFFFu, part, o);
+          }
+          return part;   // lanes 0 .. 7
+        };
+        const float inv = norm != nullptr ? GateInverse(total(0), g.cols, g.eps) : 1.0f;
+        dot = total(1 + which) * inv;
+      } else {
+        // Worked out before, or behind z in the input row.
+        const float* gates = seq.gates != nullptr ? seq.gates + t * 2 * hv : seq.in + t * seq.in_stride + channels + value_dim;
+        dot = gates[which * hv + head];   // alpha | beta
       }
-      // L2 norms (+1e-6 under the root); q also takes 1/sqrt(dk).
-      if (lower) {
-        sh.q[t][ch] = qv[t] * ((1.0f / sqrtf(qq + 1e-6f)) * (1.0f / sqrtf(static_cast<float>(dk))));
-        sh.k[t][ch] = kv[t] * (1.0f / sqrtf(kk + 1e-6f));
-      }
-    }
-  }
-  // The gates by lanes of the first upper warp: token tid / 2, decay and beta.
-  if (!lower && ch < 2 * n) {
-    const int t = ch >> 1, which = ch & 1;
-    float dot;
-    if (gate_rows) {
-      float sq = 0.f;
-      dot = 0.f;
-      for (int w = 0; w < warps; ++w) {
-        sq += sh.scratch[(w * TOK + t) * 5];
-        dot += sh.scratch[(w * TOK + t) * 5 + 1 + which];
-      }
-      if (norm != nullptr) {
-        dot *= 1.0f / sqrtf(sq / static_cast<float>(g.cols) + g.eps);
+      if (lane == 0 && which == 0) {
+        sh.coef[t].decay = expf(ssm_a * Softplus(dot + dt_bias));
+      } else if (lane == 0) {
+        sh.coef[t].beta = Sigmoid(dot);
       }
     } else {
-      dot = seq.in[t * seq.in_stride + channels + value_dim + which * hv + head];   // alpha | beta follow z
+      float qq = 0.f, kk = 0.f, kq = 0.f;
+      for (int i = lane; i < dk; i += 32) {
+        const float q = Unpack(sh.q2[t][i]).x, k = Unpack(sh.k2[t][i]).x;
+        qq = fmaf(q, q, qq);
+        kk = fmaf(k, k, kk);
+        kq = fmaf(k, q, kq);
+      }
+      qq = WarpSum(qq);
+      kk = WarpSum(kk);
+      kq = WarpSum(kq);
+      // L2 norms (+1e-6 under the root); q also takes 1/sqrt(dk).
+      if (lane < 2) {
+        const float inv = 1.0f / sqrtf((lane == 0 ? qq : kk) + 1e-6f);
+        (lane == 0 ? sh.coef[t].q : sh.coef[t].k) = lane == 0 ? inv * (1.0f / sqrtf(static_cast<float>(dk))) : inv;
+      }
+      if (lane == 0) {
+        sh.coef[t].kq = kq;
+      }
     }
-    sh.gate[t][which] = which == 0 ? expf(ssm_a * Softplus(dot + dt_bias)) : Sigmoid(dot);
   }
+  // (The first token's sums over the state, while others work the scalars out.)
+  float sums_of[8];
+  TileSums<DK>(state_tile, dk, sh.q2[0], sh.k2[0], sums_of);
   __syncthreads();
-  // (The scratch's last readers passed the barrier above.)
-#pragma unroll
-  for (int t = 0; t < TOK; ++t) {
-    if (t < n) {
-      float* dst = t == n - 1 ? seq.ssm_last + state_at : (t == n - 2 ? seq.ssm + state_at : nullptr);
-      NarrowDeltaTile(state_tile, dst, dk, warp, sh.q[t], sh.k[t], sh.v[t], sh.gate[t][0], sh.gate[t][1], sh.y[t],
-                      &sh.scratch[t * warps + warp]);
+#pragma unroll 1
+  for (int t = 0; t < n; ++t) {
+    float* dst = t == n - 1 ? seq.ssm_last + state_at : (t == n - 2 ? seq.ssm + state_at : nullptr);
+    const DeltaCoef coef = sh.coef[t];
+    TileUpdate<DK>(state_tile, sums_of, dst, dk, warp, sh.k2[t], sh.v[t], coef, sh.y[t], &sh.squares[t][warp]);
+    if (t + 1 < n) {
+      TileSums<DK>(state_tile, dk, sh.q2[t + 1], sh.k2[t + 1], sums_of);
     }
   }
   // Gated RMSNorm over the head's dk outputs: RMS(o) * w * silu(z); the warps'
   // tiles left their outputs' squares, so one barrier serves both.
   __syncthreads();
   if (lower) {
+#pragma unroll 1
+    for (int t = 0; t < n; ++t) {
+      float total = 0.f;
+      for (int w = 0; w < warps; ++w) {
+        total += sh.squares[t][w];
+      }
+      const float inv = 1.0f / sqrtf(total / static_cast<float>(dk) + a.rms_eps);
+      seq.y[t * seq.y_stride + head * dk + ch] = sh.y[t][ch] * inv * norm_w * Silu(sh.z[t][ch]);
+    }
+  }
+}
+
+// The gate dots of a step of several sequences: alpha = alpha_w[head] . x and beta
+// likewise, x = RMS(row) * norm_w where norm weights are given (DeltaNetStep::Run).
+// A block takes eight of the 2 * value_heads rows and eight tokens, its warps the
+// 128-value chunks of K round-robin, a lane four values of each. Inside the mixer
+// kernel every (sequence, head) block walked its two rows and the input once per
+// token, a chain of L2 round trips with nothing to hide it: 65 us for 32 sequences
+// of 32 heads, against 4 us here.
+constexpr int kGateTile = 8;
+constexpr int kGateRowsMax = kMaxSeqs * kMaxRunTokens;
+struct GatesArgs {
+  DeltaNetGateRows rows;
+  int value_heads;
+  int tokens;
+  float* out;                       // [tokens][2 * value_heads]
+  const float* x[kGateRowsMax];
+};
+
+__global__ void __launch_bounds__(2 * kDeltaThreads)
+DeltaNetGatesKernel(const __grid_constant__ GatesArgs a) {
+  __shared__ float partial[8][kGateTile * kGateTile + kGateTile];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r0 = blockIdx.x * kGateTile, t0 = blockIdx.y * kGateTile;
+  const int count = 2 * a.value_heads;
+  const float4* w[kGateTile];
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) {
-      if (t < n) {
-        float total = 0.f;
-        for (int w = 0; w < warps; ++w) {
-          total += sh.scratch[t * warps + w];
-        }
-        const float inv = 1.0f / sqrtf(total / static_cast<float>(dk) + a.rms_eps);
-        seq.y[t * seq.y_stride + head * dk + ch] = sh.y[t][ch] * inv * norm_w * Silu(z[t]);
+  for (int r = 0; r < kGateTile; ++r) {
+    const int row = min(r0 + r, count - 1);
+    w[r] = reinterpret_cast<const float4*>(row < a.value_heads ? a.rows.alpha_w + static_cast<size_t>(row) * a.rows.cols
+                                                               : a.rows.beta_w + static_cast<size_t>(row - a.value_heads) * a.rows.cols);
+  }
+  GridLaunchDependents();
+  GridDependencyWait();
+  float acc[kGateTile][kGateTile] = {}, sq[kGateTile] = {};
+  const float4* norm = reinterpret_cast<const float4*>(a.rows.norm_w);
+  for (int i = threadIdx.x; i < a.rows.cols / 4; i += blockDim.x) {
+    float4 x[kGateTile];
+#pragma unroll
+    for (int t = 0; t < kGateTile; ++t) {
+      x[t] = *(reinterpret_cast<const float4*>(a.x[min(t0 + t, a.tokens - 1)]) + i);
+      sq[t] = Dot4(x[t], x[t], sq[t]);
+    }
+    const float4 nw = norm != nullptr ? norm[i] : make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll
+    for (int r = 0; r < kGateTile; ++r) {
+      const float4 v = Times4(w[r][i], nw);
+#pragma unroll
+      for (int t = 0; t < kGateTile; ++t) {
+        acc[r][t] = Dot4(v, x[t], acc[r][t]);
       }
     }
   }
+#pragma unroll
+  for (int r = 0; r < kGateTile; ++r) {
+#pragma unroll
+    for (int t = 0; t < kGateTile; ++t) {
+      const float total = WarpSum(acc[r][t]);
+      if (lane == 0) {
+        partial[warp][r * kGateTile + t] = total;
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < kGateTile; ++t) {
+    const float total = WarpSum(sq[t]);
+    if (lane == 0) {
+      partial[warp][kGateTile * kGateTile + t] = total;
+    }
+  }
+  __syncthreads();
+  const int r = threadIdx.x / kGateTile, t = threadIdx.x % kGateTile;
+  if (r >= kGateTile || r0 + r >= count || t0 + t >= a.tokens) {
+    return;
+  }
+  // Over the warps in the order of the mixer kernel's shuffles.
+  auto total_of = [&](int i) {
+    float p[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      p[k] = 32 * k < static_cast<int>(blockDim.x) ? partial[k][i] : 0.f;
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+#pragma unroll
+      for (int k = 0; k < o; ++k) {
+        p[k] += p[k + o];
+      }
+    }
+    return p[0];
+  };
+  const float inv = norm != nullptr ? GateInverse(total_of(kGateTile * kGateTile + t), a.rows.cols, a.rows.eps) : 1.0f;
+  const float dot = total_of(r * kGateTile + t) * inv;
+  a.out[static_cast<size_t>(t0 + t) * count + r0 + r] = dot;
 }
 
 int CheckHeads(int key_heads, int value_heads, int head_dim) {
@@ -575,8 +730,8 @@ int gufo_cuda_delta_rule_device(gufo_cuda_ctx* ctx,
     args.head_dim = head_dim;
     args.early_state = ctx->early_state ? 1 : 0;
     const dim3 grid(head_dim / gufo::kRuleCols, value_heads, n);
-    GUFO_CUDA_TRY(gufo::LaunchOverlapped(gufo::DeltaRuleKernel, grid, dim3(32), 0,
-                                         ctx->stream, 1, args));
+    GUFO_CUDA_TRY(gufo::LaunchOverlapped(head_dim == 128 ? gufo::DeltaRuleKernel<128> : gufo::DeltaRuleKernel<0>, grid, dim3(32),
+                                         0, ctx->stream, 1, args));
     ctx->launches.fetch_add(1);
   }
   return GUFO_CUDA_OK;
@@ -741,7 +896,7 @@ int gufo_cuda_deltanet_step_device(gufo_cuda_ctx* ctx, gufo_cuda_deltanet_layer 
       const gufo_cuda_deltanet_step_seq& q = seqs[s];
       if (q.n_tokens == n) {
         step.push_back({q.in, q.h, q.conv_in, q.conv_saved, q.conv_out, q.ssm, q.ssm, n >= 2 ? q.ssm_spec : q.ssm, q.y,
-                        q.in_stride, q.h_stride, q.y_stride, n});
+                        q.in_stride, q.h_stride, q.y_stride, n, nullptr});
       }
     }
   }
@@ -755,28 +910,45 @@ namespace gufo {
 
 namespace {
 
-template <int TOK, int WIN, int SEQS>
+template <int DK, int WIN, int SEQS>
 int LaunchLinear(gufo_cuda_ctx* ctx, const LinearShape& shape, const DeltaNetSeq* seqs, int n) {
   LinearArgs<SEQS> args;
   args.shape = shape;
   for (int s = 0; s < n; ++s) {
     args.seq[s] = seqs[s];
   }
-  GUFO_CUDA_TRY(LaunchOverlapped(DeltaNetLinearKernel<TOK, WIN, SEQS>, dim3(shape.value_heads, n), dim3(2 * shape.head_dim),
-                                 0, ctx->stream, 1, args));
+  GUFO_CUDA_TRY(LaunchOverlapped(DeltaNetLinearKernel<DK, WIN, SEQS>, dim3(shape.value_heads, n), dim3(2 * shape.head_dim), 0,
+                                 ctx->stream, 1, args));
   ctx->launches.fetch_add(1);
   return GUFO_CUDA_OK;
 }
 
-template <int TOK>
-int LaunchTokens(gufo_cuda_ctx* ctx, const LinearShape& shape, const DeltaNetSeq* seqs, int n) {
-  // One or two sequences (a decode step) in a small argument block; windows of
-  // up to three columns (four taps, the models' own) in few registers.
-  const bool narrow = shape.conv_kernel <= 4;
-  if (n <= 2) {
-    return narrow ? LaunchLinear<TOK, 3, 2>(ctx, shape, seqs, n) : LaunchLinear<TOK, 7, 2>(ctx, shape, seqs, n);
+// Works out the sequences' gates into the context's scratch; `out` are the sequences
+// with their gates filled in.
+int EnqueueGates(gufo_cuda_ctx* ctx, const DeltaNetGateRows& rows, int value_heads, int head_dim, const DeltaNetSeq* seqs, int n,
+                 std::vector<DeltaNetSeq>* out) {
+  GatesArgs args;
+  args.rows = rows;
+  args.value_heads = value_heads;
+  args.tokens = 0;
+  const size_t want = static_cast<size_t>(kGateRowsMax) * 2 * value_heads * 4;
+  const int rc = ctx->GrowScratch(&ctx->gates, &ctx->gates_bytes, want, 128u << 10, "deltanet gates");
+  if (rc != GUFO_CUDA_OK) {
+    return rc;
   }
-  return narrow ? LaunchLinear<TOK, 3, kMaxSeqs>(ctx, shape, seqs, n) : LaunchLinear<TOK, 7, kMaxSeqs>(ctx, shape, seqs, n);
+  args.out = reinterpret_cast<float*>(ctx->gates);
+  out->assign(seqs, seqs + n);
+  for (DeltaNetSeq& seq : *out) {
+    seq.gates = args.out + static_cast<size_t>(args.tokens) * 2 * value_heads;
+    for (int t = 0; t < seq.tokens; ++t) {
+      args.x[args.tokens++] = seq.x + t * seq.x_stride;
+    }
+  }
+  GUFO_CUDA_TRY(LaunchOverlapped(DeltaNetGatesKernel,
+                                 dim3((2 * value_heads + kGateTile - 1) / kGateTile, (args.tokens + kGateTile - 1) / kGateTile),
+                                 dim3(2 * head_dim), 0, ctx->stream, 1, args));
+  ctx->launches.fetch_add(1);
+  return GUFO_CUDA_OK;
 }
 
 }  // namespace
@@ -799,13 +971,21 @@ int EnqueueDeltaNetLinear(gufo_cuda_ctx* ctx, const DeltaNetLayer& l, const Delt
   }
   for (int s0 = 0; s0 < nseq; s0 += kMaxSeqs) {
     const int n = nseq - s0 < kMaxSeqs ? nseq - s0 : kMaxSeqs;
-    int most = 1;
-    for (int s = s0; s < s0 + n; ++s) {
-      most = seqs[s].tokens > most ? seqs[s].tokens : most;
+    std::vector<DeltaNetSeq> with_gates;
+    const DeltaNetSeq* now = seqs + s0;
+    if (n > 2 && gate_rows != nullptr) {
+      const int rc = EnqueueGates(ctx, *gate_rows, l.value_heads, l.head_dim, now, n, &with_gates);
+      if (rc != GUFO_CUDA_OK) {
+        return rc;
+      }
+      now = with_gates.data();
     }
-    const int rc = most == 1   ? LaunchTokens<1>(ctx, shape, seqs + s0, n)
-                   : most == 2 ? LaunchTokens<2>(ctx, shape, seqs + s0, n)
-                               : LaunchTokens<kMaxRunTokens>(ctx, shape, seqs + s0, n);
+    // One or two sequences (a decode step) in a small argument block; the models' own
+    // shape (heads of 128, windows of up to three columns) with its loops unrolled.
+    const bool common = l.head_dim == 128 && shape.conv_kernel <= 4;
+    const int rc = n <= 2 ? (common ? LaunchLinear<128, 3, 2>(ctx, shape, now, n) : LaunchLinear<0, 7, 2>(ctx, shape, now, n))
+                          : (common ? LaunchLinear<128, 3, kMaxSeqs>(ctx, shape, now, n)
+                                    : LaunchLinear<0, 7, kMaxSeqs>(ctx, shape, now, n));
     if (rc != GUFO_CUDA_OK) {
       return rc;
     }

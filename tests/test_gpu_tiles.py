@@ -64,3 +64,59 @@ def test_f32_rows(ctx, tokens, rows, cols):
     got = ctx.matmul([(a, 0, rows), (a, rows, 2)], x, tokens, rows + 2)
     assert rel_l2(got, x.astype(np.float64) @ w.astype(np.float64).T) <= 1e-6
     ctx.matrix_free(a)
+
+
+@pytest.mark.parametrize("head_dim,conv_kernel,nseq", [(32, 2, 3), (64, 8, 5), (128, 4, 66), (128, 5, 3)])
+def test_mixer_run_of_many_sequences_equals_one_token_at_a_time(ctx, oracle, head_dim, conv_kernel, nseq):
+    """Sequences of one to four tokens together (more than one launch's worth in one case), bit for
+    bit against one sequence and token at a time; one of those against the oracle."""
+    from gufo_npu_b200 import synth
+    from gufo_npu_b200.backend import CudaMixer
+    from tests.test_oracle import _deltanet_cfg, _deltanet_weights
+    dev = torch.device("cuda:0")
+    cfg = synth.ModelConfig(layers=1, hidden=512, ffn=256, vocab=256, linear_key_heads=2, linear_value_heads=4,
+                            linear_head_dim=head_dim, conv_kernel=conv_kernel)
+    if cfg.value_dim % 256:
+        cfg.proj_type = Q.GGML_F32
+    tensors = synth.build_model(cfg, 5)
+    mixer = CudaMixer(ctx, cfg, tensors)
+    gen = torch.Generator(device=dev).manual_seed(11)
+    counts = [1 + i % 4 for i in range(nseq)]
+    width = cfg.conv_channels + cfg.value_dim + 2 * cfg.linear_value_heads
+
+    def rand(*shape):
+        return torch.randn(*shape, device=dev, generator=gen)
+    seqs = [{"n_tokens": n, "in": rand(n, width), "h": rand(n, cfg.hidden), "conv_in": rand(mixer.conv_values()),
+             "conv_out": rand(mixer.conv_values()), "conv_saved": rand(mixer.conv_values()),
+             "ssm": rand(mixer.ssm_values()) * 0.1, "ssm_spec": rand(mixer.ssm_values()),
+             "y": rand(n, cfg.value_dim)} for n in counts]
+    before = [(q["conv_in"].clone(), q["ssm"].clone()) for q in seqs]
+    torch.cuda.synchronize()
+    mixer.Run(0, seqs)
+    ctx.synchronize()
+    for i in sorted({0, 1, 2, nseq // 2, nseq - 1}):
+        q, n = seqs[i], counts[i]
+        conv, ssm = before[i]
+        for t in range(n):
+            one = {"n_tokens": 1, "in": q["in"][t:t + 1], "h": q["h"][t:t + 1], "conv_in": conv,
+                   "conv_out": torch.empty_like(conv), "ssm": ssm.clone(), "y": torch.empty(1, cfg.value_dim, device=dev)}
+            torch.cuda.synchronize()
+            mixer.Run(0, [one])
+            ctx.synchronize()
+            assert torch.equal(one["y"][0], q["y"][t]), (i, t)
+            if t == n - 1:
+                assert torch.equal(one["ssm"], q["ssm_spec"] if n > 1 else q["ssm"])
+                assert torch.equal(one["conv_out"], q["conv_out"])
+                assert n == 1 or (torch.equal(ssm, q["ssm"]) and torch.equal(conv, q["conv_saved"]))
+            conv, ssm = one["conv_out"], one["ssm"]
+    # Mixer::Linear (gates in the input row) of the same shape against the oracle.
+    x, conv, ssm = rand(3, width), rand(3, mixer.conv_values()), rand(3, mixer.ssm_values()) * 0.1
+    host = [(x[s].cpu().numpy(), conv[s].cpu().numpy().copy(), ssm[s].cpu().numpy().copy()) for s in range(3)]
+    out, y = torch.empty_like(conv), torch.empty(3, cfg.value_dim, device=dev)
+    torch.cuda.synchronize()
+    mixer.Linear(0, [{"in": x[s], "conv_in": conv[s], "conv_out": out[s], "ssm": ssm[s], "y": y[s]} for s in range(3)])
+    ctx.synchronize()
+    for s, (hx, hconv, hssm) in enumerate(host):
+        want, _ = oracle.deltanet_linear(_deltanet_cfg(cfg), _deltanet_weights(cfg, tensors, 0), hx, hconv, hssm)
+        assert rel_l2(y[s].cpu().numpy(), want) <= 1e-4
+        assert rel_l2(ssm[s].cpu().numpy(), hssm) <= 1e-4
