@@ -85,6 +85,7 @@ class Context:
         status = self.lib.gufo_cuda_ctx_create(device, C.c_void_p(stream or 0), C.byref(handle))
         _capi.check(self.lib, None, status)
         self.handle = handle
+        self._address = handle.value   # what the extension takes; 0 once closed
         self.device = device
         self.stream = stream or None
 
@@ -100,6 +101,7 @@ class Context:
         if getattr(self, "handle", None):
             self.lib.gufo_cuda_ctx_destroy(self.handle)
             self.handle = None
+            self._address = 0
 
     def __del__(self):
         try:
@@ -108,7 +110,8 @@ class Context:
             pass
 
     def _check(self, status: int) -> None:
-        _capi.check(self.lib, self.handle, status)
+        if status:
+            _capi.check(self.lib, self.handle, status)
 
     def set_stream(self, stream: int) -> None:
         self._check(self.lib.gufo_cuda_ctx_set_stream(self.handle, C.c_void_p(stream)))
@@ -181,8 +184,7 @@ class Context:
         """Host pointers: copies x up, runs, copies y down. parts: [(matrix, first, rows)]."""
         x = np.ascontiguousarray(x, dtype=np.float32)
         y = np.empty((tokens, out_width), dtype=np.float32)
-        self._check(self.lib.gufo_cuda_matmul(self.handle, self._parts(parts), len(parts),
-                                              C.c_void_p(x.ctypes.data), tokens, C.c_void_p(y.ctypes.data)))
+        self._check(_capi.native.matmul(self._address, parts, x, tokens, y))
         return y
 
     def matmul_host(self, parts_arr, nparts: int, x_ptr: int, tokens: int, y_ptr: int) -> None:
@@ -191,8 +193,7 @@ class Context:
                                               C.c_void_p(y_ptr)))
 
     def matmul_device(self, parts_arr, nparts: int, x, tokens: int, y) -> None:
-        self._check(self.lib.gufo_cuda_matmul_device(self.handle, parts_arr, nparts, C.c_void_p(_ptr(x)), tokens,
-                                                     C.c_void_p(_ptr(y))))
+        self._check(_capi.native.matmul_device(self._address, parts_arr, nparts, x, tokens, y))
 
     def matmul_fused_device(self, parts_arr, nparts: int, tokens: int, y, *, x=None, residual=None, delta=None,
                             norm_weight=None, rms_eps: float = 0.0, residual_out=None, scratch=None,
@@ -215,9 +216,8 @@ class Context:
     # -- routed experts -------------------------------------------------------
     def route_device(self, router, stride: int, tokens: int, experts: int, k: int, chosen, weights,
                      shared_scale=None) -> None:
-        self._check(self.lib.gufo_cuda_route_device(self.handle, C.c_void_p(_ptr(router)), stride, tokens, experts, k,
-                                                    C.c_void_p(_ptr(chosen)), C.c_void_p(_ptr(weights)),
-                                                    C.c_void_p(_ptr(shared_scale))))
+        self._check(_capi.native.route(self._address, router, stride, tokens, experts, k, chosen, weights,
+                                       shared_scale))
 
     def expert_ffn_device(self, bank: "_capi.ExpertBank", ids, pairs: int, x, x_stride: int, ffn, act, y,
                           pairs_per_input: int = 1) -> None:
@@ -230,10 +230,8 @@ class Context:
     def moe_ffn_device(self, bank: "_capi.ExpertBank", ids, weights, scale, tokens: int, k: int, x, x_stride: int,
                        shared, ffn, act, expert_out, out) -> None:
         """out[t] = shared[t] * scale[t] + the weighted sum of token t's k experts' FFN (device tensors)."""
-        self._check(self.lib.gufo_cuda_moe_ffn_device(
-            self.handle, C.byref(bank), C.c_void_p(_ptr(ids)), C.c_void_p(_ptr(weights)), C.c_void_p(_ptr(scale)),
-            tokens, k, C.c_void_p(_ptr(x)), x_stride, C.c_void_p(_ptr(shared)), C.c_void_p(_ptr(ffn)),
-            C.c_void_p(_ptr(act)), C.c_void_p(_ptr(expert_out)), C.c_void_p(_ptr(out))))
+        self._check(_capi.native.moe_ffn(self._address, bank, ids, weights, scale, tokens, k, x, x_stride, shared, ffn,
+                                         act, expert_out, out))
 
     def moe_combine_device(self, shared, scale, weights, expert_out, tokens: int, k: int, hidden: int, out) -> None:
         self._check(self.lib.gufo_cuda_moe_combine_device(self.handle, C.c_void_p(_ptr(shared)),
@@ -243,12 +241,7 @@ class Context:
 
     # -- DeltaNet -----------------------------------------------------------
     def delta_rule_device(self, seqs: List[dict], key_heads: int, value_heads: int, head_dim: int) -> None:
-        arr = (_capi.DeltaSeq * max(len(seqs), 1))()
-        for i, s in enumerate(seqs):
-            arr[i] = _capi.DeltaSeq(_ptr(s["state"]), _ptr(s.get("state_out")), _ptr(s["q"]), _ptr(s["k"]),
-                                    _ptr(s["v"]), _ptr(s["decay"]), _ptr(s["beta"]), _ptr(s["y"]))
-        self._check(self.lib.gufo_cuda_delta_rule_device(self.handle, arr, len(seqs), key_heads, value_heads,
-                                                         head_dim))
+        self._check(_capi.native.delta_rule(self._address, seqs, key_heads, value_heads, head_dim))
 
     def deltanet_layer_create(self, key_heads: int, value_heads: int, head_dim: int, conv_kernel: int,
                               rms_eps: float, conv, ssm_a, dt_bias, ssm_norm) -> int:
@@ -264,11 +257,7 @@ class Context:
         self._check(self.lib.gufo_cuda_deltanet_layer_free(self.handle, layer))
 
     def deltanet_linear_device(self, layer: int, seqs: List[dict]) -> None:
-        arr = (_capi.LinearSeq * max(len(seqs), 1))()
-        for i, s in enumerate(seqs):
-            arr[i] = _capi.LinearSeq(_ptr(s["in"]), _ptr(s["conv_in"]), _ptr(s["conv_out"]), _ptr(s["ssm"]),
-                                     _ptr(s.get("ssm_out")), _ptr(s["y"]))
-        self._check(self.lib.gufo_cuda_deltanet_linear_device(self.handle, layer, arr, len(seqs)))
+        self._check(_capi.native.deltanet_linear(self._address, layer, seqs))
 
 
 def _shape_error(name: str, shape, want) -> RuntimeError:
@@ -466,8 +455,7 @@ class CudaProjections:
         return self.ctx.matmul(parts, x, tokens, sum(p[2] for p in parts))
 
     def apply_device(self, stage: Stage, layer: int, x, tokens: int, y) -> None:
-        parts = self.parts(stage, layer)
-        self.ctx.matmul_device(Context._parts(parts), len(parts), x, tokens, y)
+        self.ctx.matmul_device(self.parts(stage, layer), None, x, tokens, y)
 
 
 class CudaMoe:
@@ -598,16 +586,10 @@ def _deltanet_run(self, layer: int, seqs: List[dict]) -> None:
     ssm_spec, y [n, y_stride] (device tensors; conv_saved / ssm_spec may be None for one token)."""
     if layer not in self.layers:
         raise ValueError(f"deltanet: layer {layer} is not a DeltaNet layer")
-    arr = (_capi.DeltaNetStepSeq * max(len(seqs), 1))()
-    for i, q in enumerate(seqs):
-        arr[i] = _capi.DeltaNetStepSeq(q["n_tokens"], _ptr(q["in"]), q["in"].stride(0), _ptr(q["h"]),
-                                       q["h"].stride(0), _ptr(q["conv_in"]), _ptr(q["conv_out"]),
-                                       _ptr(q.get("conv_saved")), _ptr(q["ssm"]), _ptr(q.get("ssm_spec")),
-                                       _ptr(q["y"]), q["y"].stride(0))
     alpha, beta, norm = self.gates[layer]
-    self.ctx._check(self.ctx.lib.gufo_cuda_deltanet_step_device(self.ctx.handle, self.layers[layer], alpha, beta,
-                                                                C.c_void_p(norm), self.config.rms_eps, arr,
-                                                                len(seqs)))
+    ctx = self.ctx
+    ctx._check(_capi.native.deltanet_step(ctx._address, self.layers[layer], alpha, beta, norm, self.config.rms_eps,
+                                          seqs))
 
 
 CudaMixer.Run = _deltanet_run
@@ -671,11 +653,13 @@ class CudaDecoder:
         _capi.check(lib, self.ctx.handle,
                     lib.gufo_cuda_decoder_create(self.ctx.handle, C.byref(config), C.byref(weights), C.byref(handle)))
         self.handle = handle
+        self._address = handle.value
 
     def close(self) -> None:
         if getattr(self, "handle", None):
             self.ctx.lib.gufo_cuda_decoder_destroy(self.handle)
             self.handle = None
+            self._address = 0
 
     def __del__(self):
         try:
@@ -690,7 +674,7 @@ class CudaDecoder:
         """Runs `token`; returns the logits (written into `logits` when given, e.g. pinned memory)."""
         if logits is None:
             logits = np.empty(self.config.vocab, dtype=np.float32)
-        self.ctx._check(self.ctx.lib.gufo_cuda_decoder_step(self.handle, token, C.c_void_p(_ptr(logits))))
+        self.ctx._check(_capi.native.decoder_step(self._address, token, logits))
         return logits
 
     def StepTokens(self, tokens: Sequence[int], logits: bool = True) -> Optional[np.ndarray]:

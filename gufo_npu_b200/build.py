@@ -1,14 +1,18 @@
-"""Builds libgufo_cuda.so (the C-ABI library) in-tree with nvcc for sm_100a."""
+"""Builds libgufo_cuda.so (the C-ABI library, nvcc for sm_100a) and _native.so (the Python side's
+per-call work, the host compiler) in-tree."""
 from __future__ import annotations
 
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgufo_cuda.so")
+NATIVE = os.path.join(HERE, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -20,16 +24,33 @@ def sources():
     return sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cu"))
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB):
+def _stale(target: str = LIB, suffixes=(".cu", ".cuh")) -> bool:
+    if not os.path.exists(target):
         return True
-    built = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(ROOT, "include", "gufo_cuda.h")]
-    return any(os.path.getmtime(d) > built for d in deps)
+    built = os.path.getmtime(target)
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(suffixes)]
+    return any(os.path.getmtime(d) > built for d in deps + [os.path.join(ROOT, "include", "gufo_cuda.h")])
+
+
+def build_native(force: bool = False) -> str:
+    """Compiles csrc/native.cpp against the interpreter's and torch's headers; returns its path."""
+    if not force and not _stale(NATIVE, (".cpp",)):
+        return NATIVE
+    torch = os.path.dirname(importlib.util.find_spec("torch").origin)
+    include = os.path.join(torch, "include")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-fvisibility=hidden",
+           "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"], "-isystem", include,
+           "-isystem", os.path.join(include, "torch", "csrc", "api", "include"), "-isystem", "/usr/local/cuda/include",
+           os.path.join(CSRC, "native.cpp"), "-o", NATIVE,
+           "-L", os.path.join(torch, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-ldl"]
+    subprocess.run(cmd, check=True)
+    return NATIVE
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compiles every .cu under csrc/ into one shared library; returns its path."""
+    """Compiles every .cu under csrc/ into one shared library; returns its path. The Python
+    extension is built beside it."""
+    build_native(force)
     if not force and not _stale():
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
