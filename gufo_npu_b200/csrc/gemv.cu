@@ -393,10 +393,18 @@ int LaunchGemv(gufo_cuda_ctx* ctx, const GemvArgs& base, int tokens) {
       args.y = y;
       args.y_stride = base.y_stride;
       args.tokens = m;
-      // One token: every thread block stages x itself, which saves the staging
-      // kernel (it reads x with 16-byte loads); more tokens share one staged image.
+      // Every thread block can stage x itself, or one staging kernel does it for all
+      // and the blocks copy the image. One token: always in the block (it reads x with
+      // 16-byte loads). More tokens, where the conversion is short beside a launch
+      // (2.8 us of host time, and one more step of the chain): two units per warp (a
+      // unit: 256 values of a row), or five where no block multiplies a second tile.
+      // Two rows through a layer of 2048 x 6144: 25.0 -> 20.5 us, eight of
+      // 1024 x 2048: 24.8 -> 17.3; beyond the line the conversions, repeated in every
+      // block, take longer than the launch (four rows of 2560 x 9728: 40.4 -> 45.8).
       const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-      args.prologue = m == 1 && aligned && !ctx->reuse_image ? kProloguePlain : kPrologueImage;
+      const int units = m * (base.cols / kSuperBlock);
+      const bool small = units <= 2 * kFastWarps || (units <= 5 * kFastWarps && base.total_rows <= 16 * 2 * ctx->sm_count);
+      args.prologue = (m == 1 || small) && aligned && !ctx->reuse_image ? kProloguePlain : kPrologueImage;
       args.x = x;
       bool staged = false;
       auto flush = [&]() -> int {

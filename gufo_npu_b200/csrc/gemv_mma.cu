@@ -88,6 +88,7 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   // Where the blocks of a cluster leave their sums for block 0: [2][8][16][TOKENS].
   __shared__ float peers[2 * 8 * 16 * TOKENS];
+  __shared__ float squares[kFastWarps * TOKENS];         // a fused norm's (FillImage)
   __shared__ __align__(8) uint64_t landed[kMaxStages];   // a slab's bytes have arrived
   // The barriers need no kernel argument: set up first, while the arguments' first
   // reads (constant-cache misses) are under way. A barrier takes eight arrivals.
@@ -245,8 +246,12 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
       *reinterpret_cast<uint4*>(zeros + i) = make_uint4(0u, 0u, 0u, 0u);
     }
   }
+  if (a.prologue != kPrologueImage) {
+    ZeroIdleColumns<TOKENS>(l, blocks, smem);
+  }
   float norm_ahead[8];
-  LoadNormAhead(a, norm_ahead);
+  LoadNormAhead<TOKENS>(a, norm_ahead);
+  const float inv_n = 1.0f / static_cast<float>(a.cols);
   GridLaunchDependents();
   // The weights above never depend on earlier kernels; the image and y do.
   GridDependencyWait();
@@ -263,8 +268,10 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   } else {
     FillImage<TOKENS>(a, l, smem, S::kExtra,
                       a.x + static_cast<size_t>(group / (a.x_group_div > 1 ? a.x_group_div : 1)) * a.x_group_stride,
-                      rank, ks, 8, norm_ahead);
+                      rank, ks, norm_ahead, squares, inv_n);
   }
+  // The norm's 1 / rms of the token whose row sums this thread stores.
+  const float row_scale = threadIdx.x < kTileFloats ? RowScale<TOKENS>(a, squares, threadIdx.x % TOKENS, inv_n) : 1.f;
 
   float out[kNB][4];
   float off[TOKENS];
@@ -317,7 +324,7 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     const int o = threadIdx.x;
     if (ks == 1) {
       if (o < kTileFloats) {
-        const float total = total_of(n % kExchange, o);
+        const float total = row_scale * total_of(n % kExchange, o);
         if (a.epilogue != kEpilogueSwiGlu) {
           store(n, o, total);
         } else if ((n & 1) == 0) {
@@ -341,7 +348,7 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     for (int p = 0; p < ks; ++p) {
       total += peers[((n & 1) * 8 + p) * kTileFloats + o];
     }
-    store(n, o, total);
+    store(n, o, row_scale * total);
   };
   clear();
   int n = 0, s = 0;   // tile and own-slab index being multiplied

@@ -162,10 +162,7 @@ __device__ __forceinline__ void StageBlock(const float (&v)[8], int lane, int to
   for (int i = 0; i < 8; ++i) {
     top = max(top, __float_as_uint(v[i]) & 0x7FFFFFFFu);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-  }
+  top = __reduce_max_sync(0xFFFFFFFFu, top);
   int e = static_cast<int>(top >> 23);  // biased exponent of the maximum
   const bool finite = e != 255;
   e = e < 22 ? 22 : e;
@@ -173,14 +170,17 @@ __device__ __forceinline__ void StageBlock(const float (&v)[8], int lane, int to
   const float up = __uint_as_float(static_cast<uint32_t>(275 - e) << 23);
   const float down = finite ? __uint_as_float(static_cast<uint32_t>(e - 21) << 23)
                             : __uint_as_float(0x7FC00000u);
-  // xi + 0x808080 has the balanced digits of xi, each offset by 128, in its
-  // three low bytes; flipping the offset bits leaves the signed bytes.
+  // Added to 1.5 * 2^23, x * up is rounded to its nearest integer xi in the low
+  // bits of the sum (one fused multiply-add where a conversion runs at a quarter
+  // of its rate). xi + 0x808080 has the balanced digits of xi, each offset by
+  // 128, in its three low bytes; flipping the offset bits leaves the signed
+  // bytes. (A block with an infinity or NaN: any digits, `down` is NaN.)
   uint32_t z[8];
   float sum = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int xi = finite ? __float2int_rn(v[i] * up) : 0;
-    z[i] = static_cast<uint32_t>(xi + 0x808080) ^ 0x808080u;
+    const uint32_t bits = __float_as_uint(fmaf(v[i], up, 12582912.0f));
+    z[i] = (bits + (0x808080u - 0x4B400000u)) ^ 0x808080u;
     sum += v[i];
   }
 #pragma unroll
@@ -210,46 +210,95 @@ __device__ __forceinline__ void StageBlock(const float (&v)[8], int lane, int to
 
 __device__ __forceinline__ float SiluFast(float x) { return x * (1.0f / (1.0f + expf(-x))); }
 
-// Builds the image of the launch's TOKENS rows in shared memory at `image` from
-// the launch's fused input (prologue != kPrologueImage). Warp w converts blocks
-// w, w + 8, ...; a lane holds eight adjacent values, so nothing is staged in
-// between. `x` is the plain / SwiGLU input (a.x, or a group's part of it). Rows
-// of several tokens follow one another: the residual, its pending add, the
-// normed vector and a plain x `cols` floats apart, a SwiGLU input [gate | up]
-// 2 * cols apart. A block that shares its tiles with a cluster (rank `rank` of
-// `ks`, slabs of `slab_blocks` blocks dealt round-robin) converts only the
-// blocks of its own slabs; the others are never read. Ends with a
-// __syncthreads. kFastThreads threads.
-// The norm weights of the calling warp's first block (values 8 * lane .. + 7 of
-// block `warp`), for FillImage: they never depend on an earlier kernel, so a
-// kernel asks for them before it waits for its predecessor (a layer's norm
-// vector is read once per step: the load goes all the way to HBM, about as long
-// as the whole conversion takes).
+// The image of a launch whose input is fused in (prologue != kPrologueImage) is
+// built by every thread block in its own shared memory, in units of one
+// 256-value block of one token: warp w converts units w, w + 8, ...; a lane holds
+// eight adjacent values. Rows of several tokens follow one another: the residual,
+// its pending add, the normed vector and a plain x `cols` floats apart, a SwiGLU
+// input [gate | up] 2 * cols apart.
+//
+// What bounds it: one L2 round trip for what the kernel before has just written
+// (0.8 us), then the issue slots of an SM whose resident blocks all convert at
+// once, and block-wide reductions that nothing hides. So a norm's 1 / rms is not
+// in the image: the planes are those of (h + delta) * w, and the kernel multiplies
+// its row sums by 1 / rms (RowScale) when it stores them. The sum of squares then
+// costs no barrier of its own, units are independent of one another, and with one
+// or two tokens the loads of two units (three of a plain row) are in flight
+// together; more tokens hold too many registers elsewhere in the kernel.
+// Eight tokens of the 24-layer, 2048-wide decoder: 6.35 -> 6.15 ms.
+
+// The norm weights of the calling warp's first unit, for FillImage: they never
+// depend on an earlier kernel, so a kernel asks for them before it waits for its
+// predecessor (a layer's norm vector is read once per step: the load goes all the
+// way to HBM, about as long as the whole conversion takes).
+template <int TOKENS>
 __device__ __forceinline__ void LoadNormAhead(const FastGemvArgs& a, float (&w)[8]) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int blocks = a.cols / kSuperBlock;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     w[i] = 0.f;
   }
-  if (a.prologue == kPrologueResNorm && warp < a.cols / kSuperBlock) {
-    const float4 v0 = *reinterpret_cast<const float4*>(a.norm_w + warp * kSuperBlock + lane * 8);
-    const float4 v1 = *reinterpret_cast<const float4*>(a.norm_w + warp * kSuperBlock + lane * 8 + 4);
+  if (a.prologue == kPrologueResNorm && warp < TOKENS * blocks) {
+    int b = warp;
+    while (TOKENS > 1 && b >= blocks) {
+      b -= blocks;
+    }
+    const float4 v0 = *reinterpret_cast<const float4*>(a.norm_w + b * kSuperBlock + lane * 8);
+    const float4 v1 = *reinterpret_cast<const float4*>(a.norm_w + b * kSuperBlock + lane * 8 + 4);
     w[0] = v0.x, w[1] = v0.y, w[2] = v0.z, w[3] = v0.w;
     w[4] = v1.x, w[5] = v1.y, w[6] = v1.z, w[7] = v1.w;
   }
 }
 
+// 1 / rms of token k after FillImage (1 without a norm): the warps' sums of
+// squares added in warp order. `inv_n` = 1 / cols.
+template <int TOKENS>
+__device__ __forceinline__ float RowScale(const FastGemvArgs& a, const float* squares, int k, float inv_n) {
+  if (a.prologue != kPrologueResNorm) {
+    return 1.f;
+  }
+  float total = 0.f;
+#pragma unroll
+  for (int w = 0; w < kFastWarps; ++w) {
+    total += squares[w * TOKENS + k];
+  }
+  return 1.0f / sqrtf(fmaf(total, inv_n, a.eps));
+}
+
+// Columns without a token keep a zero factor; independent of the input.
+template <int TOKENS>
+__device__ __forceinline__ void ZeroIdleColumns(const ImageLayout& l, int blocks, uint8_t* image) {
+  float* scale = reinterpret_cast<float*>(image + l.scale_at);
+  for (int i = threadIdx.x; i < blocks * l.kcols; i += kFastThreads) {
+    if (i % l.kcols >= kLimbs * TOKENS) {
+      scale[i] = 0.f;
+    }
+  }
+}
+
+// `x` is the plain / SwiGLU input (a.x, or a group's part of it). A block that
+// shares its tiles with a cluster (rank `rank` of `ks`, slabs of eight blocks
+// dealt round-robin) converts only the blocks of its own slabs; the others are
+// never read. keep_w: LoadNormAhead's. squares: [kFastWarps][TOKENS] in shared
+// memory, for RowScale. Ends with a __syncthreads. kFastThreads threads.
 template <int TOKENS>
 __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayout& l,
                                           uint8_t* image, float extra, const float* x,
-                                          int rank, int ks, int slab_blocks, const float (&keep_w)[8]) {
-  __shared__ float reduce[kFastWarps];
+                                          int rank, int ks, const float (&keep_w)[8],
+                                          float* squares, float inv_n) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int n = a.cols;
   const int blocks = n / kSuperBlock;
   const bool first = blockIdx.x == 0;
-  auto mine = [&](int b) { return ks == 1 || (b / slab_blocks) % ks == rank; };
+  auto mine = [&](int b) {
+    int s = ks == 1 ? rank : b >> 3;
+    while (s >= ks) {
+      s -= ks;
+    }
+    return s == rank;
+  };
   auto load8 = [&](const float* p, float (&v)[8]) {
     const float4 v0 = *reinterpret_cast<const float4*>(p);
     const float4 v1 = *reinterpret_cast<const float4*>(p + 4);
@@ -260,157 +309,163 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
     *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
   };
-  // Columns without a token keep a zero factor.
-  float* scale = reinterpret_cast<float*>(image + l.scale_at);
-  for (int i = threadIdx.x; i < blocks * l.kcols; i += kFastThreads) {
-    if (i % l.kcols >= kLimbs * TOKENS) {
-      scale[i] = 0.f;
+  // Unit (tok, b) of the calling warp and the next one, kFastWarps units on.
+  int tok = 0, b = warp;
+  auto settle = [&]() {
+    while (TOKENS > 1 && b >= blocks) {
+      b -= blocks;
+      ++tok;
     }
-  }
+  };
+  auto live = [&]() { return TOKENS > 1 ? tok < TOKENS : b < blocks; };
+  settle();
   if (a.prologue == kPrologueResNorm) {
     // vec::RmsNorm (src/core/vec.hpp:57-63) of the residual stream after its
-    // pending add (src/models/qwen35/decoder.cpp:493,504-508). The first pass
-    // sums the squares; the second reads the same values again (they sit in
-    // L2, and the warp's first block is still in registers).
-    // keep_w: the norm weights of the warp's first block, requested by the
-    // caller ahead of its dependency wait (LoadNormAhead).
+    // pending add (src/models/qwen35/decoder.cpp:493,504-508).
+    constexpr int kBatch = TOKENS <= 2 ? 2 : 1;
+    if (lane < TOKENS) {
+      squares[warp * TOKENS + lane] = 0.f;
+    }
+    __syncwarp();
+    float sq = 0.f;
+    bool first_unit = true;
 #pragma unroll 1
-    for (int tok = 0; tok < TOKENS; ++tok) {
-      const size_t row = static_cast<size_t>(tok) * n;
-      auto residual = [&](int at, float (&v)[8]) {
-        load8(a.h_in + row + at, v);
-        if (a.delta != nullptr) {
-          // Partial sums of several ranks are added in rank order.
-          const int parts = a.delta_parts > 1 ? a.delta_parts : 1;
-          for (int p = 0; p < parts; ++p) {
-            float d[8];
-            load8(a.delta + static_cast<size_t>(p) * a.delta_stride + row + at, d);
+    while (live()) {
+      float v[kBatch][8], d[kBatch][8], w[kBatch][8];
+      int at_tok[kBatch], at_b[kBatch];
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j) {
+        at_tok[j] = live() ? tok : -1;
+        at_b[j] = b;
+        if (live()) {
+          const int at = b * kSuperBlock + lane * 8;
+          const size_t row = static_cast<size_t>(tok) * n + at;
+          load8(a.h_in + row, v[j]);
+          if (a.delta != nullptr) {
+            load8(a.delta + row, d[j]);
+          }
+          if (j > 0 || !first_unit) {
+            load8(a.norm_w + at, w[j]);
+          } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              v[i] += d[i];
+              w[j][i] = keep_w[i];
             }
           }
         }
-      };
-      if (tok > 0) {
-        __syncthreads();   // the sums of the token before have been read
+        b += kFastWarps;
+        settle();
       }
-      float keep[8] = {};
-      float sq = 0.f;
-      for (int b = warp; b < blocks; b += kFastWarps) {
-        float v[8];
-        residual(b * kSuperBlock + lane * 8, v);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          sq = fmaf(v[i], v[i], sq);
-          if (b == warp) {
-            keep[i] = v[i];
-          }
-        }
-      }
-      sq = WarpSum(sq);
-      if (lane == 0) {
-        reduce[warp] = sq;
-      }
-      __syncthreads();
-      float total = 0.f;
-#pragma unroll
-      for (int w = 0; w < kFastWarps; ++w) {
-        total += reduce[w];
-      }
-      const float inv = 1.0f / sqrtf(total / static_cast<float>(n) + a.eps);
-      for (int b = warp; b < blocks; b += kFastWarps) {
-        // Block 0 writes the whole residual stream and normed vector.
-        if (!first && !mine(b)) {
+      for (int j = 0; j < kBatch; ++j) {
+        if (at_tok[j] < 0) {
           continue;
         }
-        const int at = b * kSuperBlock + lane * 8;
-        float v[8], w[8], out[8];
-        if (b == warp) {
+        const int at = at_b[j] * kSuperBlock + lane * 8;
+        const size_t row = static_cast<size_t>(at_tok[j]) * n + at;
+        if (a.delta != nullptr) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            v[i] = keep[i];
+            v[j][i] += d[j][i];
           }
-          for (int i = 0; i < 8; ++i) {
-            w[i] = keep_w[i];
+          // Partial sums of several ranks are added in rank order.
+#pragma unroll 1
+          for (int p = 1; p < a.delta_parts; ++p) {
+            load8(a.delta + static_cast<size_t>(p) * a.delta_stride + row, d[j]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              v[j][i] += d[j][i];
+            }
           }
-        } else {
-          residual(at, v);
-          load8(a.norm_w + at, w);
+        }
+        if (TOKENS > 1) {
+          sq = 0.f;
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          out[i] = v[i] * inv * w[i];
+          sq = fmaf(v[j][i], v[j][i], sq);
+          w[j][i] *= v[j][i];
         }
         if (first) {
-          store8(a.h_out + row + at, v);
-          if (a.normed_out != nullptr) {
-            store8(a.normed_out + row + at, out);
+          // Block 0 writes the whole residual stream (and normed vector, below).
+          store8(a.h_out + row, v[j]);
+        }
+        if (TOKENS > 1) {
+          const float sum = WarpSum(sq);
+          if (lane == 0) {
+            squares[warp * TOKENS + at_tok[j]] += sum;
           }
         }
-        StageBlock(out, lane, tok, b, l, image, extra);
+        if (mine(at_b[j])) {
+          StageBlock(w[j], lane, at_tok[j], at_b[j], l, image, extra);
+        }
+      }
+      first_unit = false;
+    }
+    if (TOKENS == 1) {
+      sq = WarpSum(sq);
+      if (lane == 0) {
+        squares[warp] = sq;
+      }
+    }
+    __syncthreads();
+    if (first && a.normed_out != nullptr) {
+      tok = 0, b = warp;
+      settle();
+#pragma unroll 1
+      for (; live(); b += kFastWarps, settle()) {
+        const float inv = RowScale<TOKENS>(a, squares, tok, inv_n);
+        const int at = b * kSuperBlock + lane * 8;
+        const size_t row = static_cast<size_t>(tok) * n + at;
+        float v[8], w[8];
+        load8(a.h_out + row, v);   // this lane's own stores
+        load8(a.norm_w + at, w);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          v[i] *= w[i] * inv;
+        }
+        store8(a.normed_out + row, v);
       }
     }
     if (first && threadIdx.x == 0 && a.advance != nullptr) {
       *a.advance += TOKENS;
     }
-  } else {
-    const size_t stride = a.prologue == kPrologueSwiGlu ? 2 * static_cast<size_t>(n) : static_cast<size_t>(n);
-    const bool act = a.prologue == kPrologueSwiGlu;
-    if constexpr (TOKENS == 1) {
-      // A warp's blocks in batches of kBatch: all loads of a batch are in flight
-      // before the first value is used (one round trip per batch, not per
-      // block; a 6144-value input is three blocks per warp).
-      constexpr int kBatch = 3;
-      for (int b0 = warp; b0 < blocks; b0 += kBatch * kFastWarps) {
-        float v[kBatch][8], up[kBatch][8];
+    return;
+  }
+  const bool act = a.prologue == kPrologueSwiGlu;
+  const size_t stride = act ? 2 * static_cast<size_t>(n) : static_cast<size_t>(n);
+  // All loads of a batch are in flight before the first value is used: one round
+  // trip per batch, not per block (a 6144-value input is three blocks per warp).
+  constexpr int kBatch = TOKENS == 1 ? 3 : TOKENS == 2 ? 2 : 1;
+#pragma unroll 1
+  while (live()) {
+    float v[kBatch][8], up[kBatch][8];
+    int at_tok[kBatch], at_b[kBatch];
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-          const int b = b0 + j * kFastWarps;
-          if (b < blocks && mine(b)) {
-            const int at = b * kSuperBlock + lane * 8;
-            load8(x + at, v[j]);
-            if (act) {
-              load8(x + n + at, up[j]);
-            }
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-          const int b = b0 + j * kFastWarps;
-          if (b < blocks && mine(b)) {
-            if (act) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                v[j][i] = SiluFast(v[j][i]) * up[j][i];
-              }
-            }
-            StageBlock(v[j], lane, 0, b, l, image, extra);
-          }
+    for (int j = 0; j < kBatch; ++j) {
+      const bool take = live() && mine(b);
+      at_tok[j] = take ? tok : -1;
+      at_b[j] = b;
+      if (take) {
+        const float* xt = x + tok * stride + b * kSuperBlock + lane * 8;
+        load8(xt, v[j]);
+        if (act) {
+          load8(xt + n, up[j]);
         }
       }
-    } else {
-      // More tokens hold more registers elsewhere in the kernel: block by block.
-#pragma unroll 1
-      for (int tok = 0; tok < TOKENS; ++tok) {
-        const float* xt = x + tok * stride;
-        for (int b = warp; b < blocks; b += kFastWarps) {
-          if (!mine(b)) {
-            continue;
-          }
-          const int at = b * kSuperBlock + lane * 8;
-          float v[8];
-          load8(xt + at, v);
-          if (act) {
-            float up[8];
-            load8(xt + n + at, up);
+      b += kFastWarps;
+      settle();
+    }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              v[i] = SiluFast(v[i]) * up[i];
-            }
+    for (int j = 0; j < kBatch; ++j) {
+      if (at_tok[j] >= 0) {
+        if (act) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            v[j][i] = SiluFast(v[j][i]) * up[j][i];
           }
-          StageBlock(v, lane, tok, b, l, image, extra);
         }
+        StageBlock(v[j], lane, at_tok[j], at_b[j], l, image, extra);
       }
     }
   }

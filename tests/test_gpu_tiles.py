@@ -54,6 +54,20 @@ def test_gemm_tiles_groups_and_cuts(ctx, ggml_type, tokens, rows, cols):
     ctx.matrix_free(m)
 
 
+@pytest.mark.parametrize("ggml_type", [Q.GGML_Q4_K, Q.GGML_Q6_K])
+@pytest.mark.parametrize("tokens,rows,cols", [
+    (2, 40, 2048), (3, 4752, 1280), (3, 33, 1536), (4, 4736, 2560), (5, 16, 2048), (8, 17, 256), (8, 4753, 1280), (6, 31, 1792),
+])
+def test_few_rows_converted_in_the_product_or_ahead_of_it(ctx, ggml_type, tokens, rows, cols):
+    """Either side of the line between the two (16 and 40 blocks of 256 values, 4736 rows)."""
+    m, w = _matrix(ctx, ggml_type, rows, cols, 60 + rows % 7)
+    x = G.normal(61 + tokens, tokens, cols)
+    got = ctx.matmul([(m, 0, rows)], x, tokens, rows)
+    want = x.astype(np.float64) @ w.T
+    assert rel_l2(got, want) <= 2e-6
+    ctx.matrix_free(m)
+
+
 @pytest.mark.parametrize("tokens", [1, 2, 3, 8, 9, 33])
 @pytest.mark.parametrize("rows,cols", [(1, 4), (7, 260), (8, 2048), (17, 1028)])
 def test_f32_rows(ctx, tokens, rows, cols):
