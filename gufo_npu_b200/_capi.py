@@ -117,6 +117,8 @@ SIGNATURES = {
     "gufo_cuda_free": (C.c_int, [C.c_void_p, C.c_void_p]),
     "gufo_cuda_upload": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t]),
     "gufo_cuda_download": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t]),
+    "gufo_cuda_host_take": (C.c_int, [C.c_void_p, C.c_size_t, C.POINTER(C.c_void_p)]),
+    "gufo_cuda_host_give": (C.c_int, [C.c_void_p]),
     "gufo_cuda_memset_zero": (C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t]),
     "gufo_cuda_matrix_upload": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int64, C.c_int64,
                                           C.POINTER(C.c_int64)]),

@@ -144,6 +144,18 @@ class Context:
         self._check(self.lib.gufo_cuda_download(self.handle, C.c_void_p(out.ctypes.data), C.c_void_p(src), out.nbytes))
         return out
 
+    def host_empty(self, shape) -> np.ndarray:
+        """An uninitialised float32 array for results. From 256 KB on it lies in pinned memory of a
+        bounded pool, which the GPU writes directly and which does not fault page by page."""
+        count = 1
+        for n in shape:
+            count *= n
+        if 4 * count >= 256 << 10:
+            buffer = _capi.native.host_buffer(self._address, 4 * count)
+            if buffer is not None:
+                return np.frombuffer(buffer, dtype=np.float32, count=count).reshape(shape)
+        return np.empty(shape, dtype=np.float32)
+
     def memset_zero(self, ptr: int, nbytes: int) -> None:
         self._check(self.lib.gufo_cuda_memset_zero(self.handle, C.c_void_p(ptr), nbytes))
 
@@ -183,7 +195,7 @@ class Context:
     def matmul(self, parts: Sequence, x: np.ndarray, tokens: int, out_width: int) -> np.ndarray:
         """Host pointers: copies x up, runs, copies y down. parts: [(matrix, first, rows)]."""
         x = np.ascontiguousarray(x, dtype=np.float32)
-        y = np.empty((tokens, out_width), dtype=np.float32)
+        y = self.host_empty((tokens, out_width))
         self._check(_capi.native.matmul(self._address, parts, x, tokens, y))
         return y
 
@@ -657,7 +669,8 @@ class CudaDecoder:
 
     def close(self) -> None:
         if getattr(self, "handle", None):
-            self.ctx.lib.gufo_cuda_decoder_destroy(self.handle)
+            if self.ctx.handle:   # a context closed first has taken its stream along
+                self.ctx.lib.gufo_cuda_decoder_destroy(self.handle)
             self.handle = None
             self._address = 0
 
@@ -673,7 +686,7 @@ class CudaDecoder:
     def Step(self, token: int, logits: Optional[np.ndarray] = None) -> np.ndarray:
         """Runs `token`; returns the logits (written into `logits` when given, e.g. pinned memory)."""
         if logits is None:
-            logits = np.empty(self.config.vocab, dtype=np.float32)
+            logits = self.ctx.host_empty((self.config.vocab,))
         self.ctx._check(_capi.native.decoder_step(self._address, token, logits))
         return logits
 
@@ -682,11 +695,8 @@ class CudaDecoder:
         one or two tokens from the current position in one pass; returns [count, vocab] logits, or
         None with `logits` off (prompt passes). After two tokens the second is a draft until
         `Resolve`."""
-        count = len(tokens)
-        ids = (C.c_int * max(count, 1))(*tokens)
-        out = np.empty((count, self.config.vocab), dtype=np.float32) if logits else None
-        self.ctx._check(self.ctx.lib.gufo_cuda_decoder_step_tokens(
-            self.handle, ids, count, int(logits), C.c_void_p(_ptr(out)) if logits else None))
+        out = self.ctx.host_empty((len(tokens), self.config.vocab)) if logits else None
+        self.ctx._check(_capi.native.decoder_step_tokens(self._address, tokens, int(logits), out))
         return out
 
     def step_tokens_device(self, tokens: Sequence[int]) -> int:

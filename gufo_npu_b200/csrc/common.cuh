@@ -175,6 +175,10 @@ struct FastGemvArgs {
   // every tile pair a block of its own.
   int epilogue;
   PeerOut peer_out;       // world == 0: an ordinary product
+  // Device word with the address of a second copy of y (mapped host memory; null
+  // where there is none): the same rows are stored there too. Read at run time, so
+  // a captured launch follows the caller's buffer.
+  float* const* mirror;
   PeerWait peer_wait;
 };
 
@@ -206,6 +210,8 @@ size_t DeviceRowBytes(int type, int64_t cols);
 
 struct gufo_cuda_ctx;
 namespace gufo {
+// The device's address of pinned host memory; null for pageable memory.
+void* DeviceAddress(const void* host);
 // Enqueues one Q4_K part on the int8 tensor-core kernel against a staged image.
 int LaunchGemvQ4KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
 // Whether the image of `tokens` rows of `cols` values fits in shared memory.
@@ -269,6 +275,11 @@ struct gufo_cuda_ctx {
   size_t stage_x_bytes = 0;
   float* stage_y = nullptr;
   size_t stage_y_bytes = 0;
+  // The same in pinned host memory.
+  float* host_x = nullptr;
+  size_t host_x_bytes = 0;
+  float* host_y = nullptr;
+  size_t host_y_bytes = 0;
   // The gate dots of a DeltaNet step of several sequences.
   uint8_t* gates = nullptr;
   size_t gates_bytes = 0;
@@ -311,6 +322,9 @@ struct gufo_cuda_ctx {
     return it == matrices.end() ? nullptr : &it->second;
   }
   int Reserve(float** buffer, size_t* have, size_t want);
+  // The same for host_x and host_y; GUFO_CUDA_OUT_OF_MEMORY (no error text) where
+  // no more memory is to be pinned: the caller copies pageable memory then.
+  int ReserveHost(float** buffer, size_t* have, size_t want);
   // Grows a device scratch block to `want` bytes (at least `floor`) without
   // freeing the old one and without waiting for the stream; refuses while the
   // stream is being captured (a capture cannot allocate). ctx->mu is held.

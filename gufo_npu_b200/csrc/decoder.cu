@@ -29,7 +29,7 @@ namespace {
 
 constexpr int kSmallThreads = kTeamThreads;
 constexpr int kStepTokens = 2;      // tokens of a pair step
-constexpr int kTokenSlots = 8;      // pinned token staging slots of a decoder
+constexpr int kStepSlots = 8;       // pinned staging slots of a decoder
 
 __device__ __forceinline__ float SigmoidF(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float SiluF(float x) { return x * SigmoidF(x); }
@@ -48,6 +48,31 @@ __device__ __forceinline__ float BlockSum256(float v, float* scratch) {
   }
   return total;
 }
+
+// What the host says to a step, copied into device memory ahead of it: the copy runs
+// while the host is still submitting the step's graph. (Measured against it, per step:
+// the words read from mapped memory by the step's first kernel, 2 us more; passed as
+// arguments of a launch in front of the graph, 3 to 16 us more, as a graph behind a
+// kernel starts later than one behind a copy.)
+struct StepWords {
+  int token[kStepTokens];
+  float* mirror;   // where the LM head stores its rows as well (mapped host memory), or null
+};
+
+// The embedding rows of a step's tokens. One thread block: the rows are a few kilobytes.
+__global__ void __launch_bounds__(kSmallThreads)
+EmbedStepKernel(const __grid_constant__ EmbedArgs embed, int tokens) {
+  GridLaunchDependents();
+  GridDependencyWait();
+  EmbedArgs a = embed;
+  for (int t = 0; t < tokens; ++t) {
+    EmbedBody(a, threadIdx.x);
+    ++a.token;
+    a.h += a.cols;
+  }
+}
+
+__global__ void SetWordKernel(int* word, int value) { *word = value; }
 
 // The embedding row (body in decode_device.cuh). One thread block.
 __global__ void __launch_bounds__(kSmallThreads)
@@ -247,14 +272,14 @@ struct gufo_cuda_decoder {
   float *expert_ffn = nullptr, *expert_act = nullptr, *expert_out = nullptr;
   int* chosen = nullptr;
   int* position_dev = nullptr;
-  int* token_dev = nullptr;      // [kStepTokens]
-  // Pinned staging for the token ids: a ring of slots, each reused only after
-  // the copy that read it has run (its event), so that steps enqueued without
-  // a wait in between never see one another's tokens. The last slot carries the
-  // position word Resolve uploads.
-  int* token_pinned = nullptr;   // [kTokenSlots + 1][kStepTokens]
-  cudaEvent_t token_read[gufo::kTokenSlots] = {};
-  unsigned token_slot = 0;
+  gufo::StepWords* words = nullptr;      // device
+  // Pinned staging for them: a slot is written again only after the copy that read
+  // it has run (its event, unless that step was waited for), so that steps
+  // enqueued without a wait in between never see one another's tokens.
+  gufo::StepWords* slots = nullptr;      // [kStepSlots]
+  cudaEvent_t slot_read[gufo::kStepSlots] = {};
+  bool slot_busy[gufo::kStepSlots] = {};
+  unsigned next_slot = 0;
   int position = 0;
   int conv_cur = 0;              // which of a layer's conv windows is current
   int pending = 0;               // tokens of the last step that await Resolve (0 or 2)
@@ -275,16 +300,13 @@ struct gufo_cuda_decoder {
   // One graph per (tokens - 1, current conv window, with logits); each kind of
   // step runs eagerly twice first (that sizes staging buffers and sets kernel
   // attributes, which a capture cannot).
-  // The last index: 0 no logits, 1 logits on the device, 2 logits on the device
-  // and mirrored into `host_mirror` by the LM head's own stores.
-  cudaGraphExec_t graph[2][2][3] = {};
-  int64_t graph_kernels[2][2][3] = {};
-  // A pinned, device-visible host buffer the caller reads logits from: the LM
-  // head writes its rows there as well (posted writes over PCIe while the
-  // kernel runs), so no copy follows the step. Null: logits are copied down.
-  float* host_mirror = nullptr;        // device-side address
-  const float* host_mirror_for = nullptr;   // the host pointer it belongs to
-  bool mirror_ok = false;              // the LM head is one tensor-core launch
+  cudaGraphExec_t graph[2][2][2] = {};
+  int64_t graph_kernels[2][2][2] = {};
+  // Whether the LM head is one tensor-core launch (for one and for two tokens):
+  // where the caller reads the logits from pinned memory, its stores put them
+  // there too (posted writes over PCIe while the kernel runs), and no copy
+  // follows the step.
+  bool mirror_ok[gufo::kStepTokens] = {};
   int eager_runs[2][2] = {};
   std::vector<void*> owned;   // every device allocation, for destroy
 
@@ -376,6 +398,7 @@ struct Input {
   const float* norm_w = nullptr;
   float* h_out = nullptr;
   int* advance = nullptr;
+  float* const* mirror = nullptr;  // FastGemvArgs::mirror
 };
 
 // One stage's product for `tokens` rows with its input fused into the GEMV
@@ -502,6 +525,7 @@ int FusedProduct(gufo_cuda_ctx* ctx, float rms_eps, const GemvArgs& stage, const
     }
     args.advance = first ? in.advance : nullptr;
     first = false;
+    args.mirror = in.mirror;
     if (peer_out != nullptr) {
       args.peer_out = *peer_out;
     }
@@ -564,20 +588,18 @@ void Mark(gufo_cuda_decoder* d, int kind) {
 // second token's go to ssm_spec and the other conv window (DeltaNetStep::Run,
 // src/models/qwen35_2b/deltanet.hpp:35-44). Token t's rows sit at t * width in
 // every activation buffer.
-int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens, bool mirror = false) {
+int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens) {
   gufo_cuda_ctx* ctx = d->ctx;
   const gufo_cuda_decoder_config& c = d->c;
   cudaStream_t st = ctx->stream;
   const dim3 one(1), block(kSmallThreads);
   const size_t hidden = static_cast<size_t>(c.hidden);
   int cur = 0;   // which residual buffer is current
-  for (int t = 0; t < tokens; ++t) {
-    EmbedArgs embed{d->embed.data, d->embed.type, static_cast<int>(d->embed.row_bytes), c.hidden,
-                    d->token_dev + t, d->h[0] + t * hidden};
-    GUFO_CUDA_TRY(LaunchOverlapped(EmbedKernel, one, block, 0, st, 1, embed));
-  }
-  ctx->launches.fetch_add(tokens);
+  const EmbedArgs embed{d->embed.data, d->embed.type, static_cast<int>(d->embed.row_bytes), c.hidden, d->words->token,
+                        d->h[0]};
   Mark(d, -1);
+  GUFO_CUDA_TRY(LaunchOverlapped(EmbedStepKernel, one, block, 0, st, 1, embed, tokens));
+  ctx->launches.fetch_add(1);
   Mark(d, GUFO_CUDA_TIMELINE_EMBED);
   const float* pending = nullptr;   // projection output not yet added to the residual
   for (int il = 0; il < c.layers; ++il) {
@@ -650,17 +672,8 @@ int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens, 
   last.h_out = d->h[cur ^ 1];
   last.advance = d->position_dev;
   d->final_h = last.h_out;
-  if (want_logits && mirror) {
-    // The logits go to the device buffer and, by the same stores, to the
-    // caller's pinned host buffer.
-    PeerOut both{};
-    both.world = 2;
-    both.rank = 0;
-    both.slot = -1;
-    both.y[0] = d->logits;
-    both.y[1] = d->host_mirror;
-    GUFO_STEP_TRY(FusedProduct(ctx, c.rms_eps, d->lm_head, last, d->normed, d->logits, tokens, &both, nullptr));
-  } else if (want_logits) {
+  if (want_logits) {
+    last.mirror = &d->words->mirror;
     GUFO_STEP_TRY(FusedProduct(d, d->lm_head, last, d->normed, d->logits, tokens));
   } else {
     // A prompt pass whose logits nobody reads: only the final residuals.
@@ -973,7 +986,7 @@ int EnqueueStepKernel(gufo_cuda_decoder* d, int parity, bool want_logits) {
   p.gemv = plan.gemv;
   p.delta = plan.delta;
   p.attn = plan.attn;
-  p.embed = EmbedArgs{d->embed.data, d->embed.type, static_cast<int>(d->embed.row_bytes), d->c.hidden, d->token_dev,
+  p.embed = EmbedArgs{d->embed.data, d->embed.type, static_cast<int>(d->embed.row_bytes), d->c.hidden, d->words->token,
                       d->h[0]};
   p.sync = plan.sync;
   p.stamps = plan.stamps;
@@ -1264,9 +1277,11 @@ int gufo_cuda_decoder_create(gufo_cuda_ctx* ctx, const gufo_cuda_decoder_config*
     }
     // One launch of the tensor-core GEMV: its stores can mirror the logits into host memory.
     const int type = d->lm_head.parts[0].type;
-    d->mirror_ok = d->lm_head.nparts == 1 &&
-                   ((type == GUFO_CUDA_Q4_K && gufo::Q4KFastFits(c.hidden, 1)) ||
-                    (type == GUFO_CUDA_Q6_K && gufo::Q6KFastFits(c.hidden, 1)));
+    for (int t = 0; t < gufo::kStepTokens; ++t) {
+      d->mirror_ok[t] = d->lm_head.nparts == 1 &&
+                        ((type == GUFO_CUDA_Q4_K && gufo::Q4KFastFits(c.hidden, t + 1)) ||
+                         (type == GUFO_CUDA_Q6_K && gufo::Q6KFastFits(c.hidden, t + 1)));
+    }
   }
   if ((rc = gufo::UploadVec(d, weights->output_norm, c.hidden, &d->output_norm, "output_norm")) != GUFO_CUDA_OK) {
     return fail(rc);
@@ -1427,14 +1442,14 @@ int gufo_cuda_decoder_create(gufo_cuda_ctx* ctx, const gufo_cuda_decoder_config*
   }
   if ((rc = gufo::Alloc(d, 4 * (two * c.experts_used + 1), reinterpret_cast<void**>(&d->chosen))) != GUFO_CUDA_OK ||
       (rc = gufo::Alloc(d, 4, reinterpret_cast<void**>(&d->position_dev))) != GUFO_CUDA_OK ||
-      (rc = gufo::Alloc(d, 4 * two, reinterpret_cast<void**>(&d->token_dev))) != GUFO_CUDA_OK) {
+      (rc = gufo::Alloc(d, sizeof(gufo::StepWords), reinterpret_cast<void**>(&d->words))) != GUFO_CUDA_OK) {
     return fail(rc);
   }
-  cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&d->token_pinned), 4 * two * (gufo::kTokenSlots + 1));
+  cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&d->slots), sizeof(gufo::StepWords) * gufo::kStepSlots);
   if (e != cudaSuccess) {
     return fail(gufo::CudaFail(e, "cudaMallocHost"));
   }
-  for (cudaEvent_t& read : d->token_read) {
+  for (cudaEvent_t& read : d->slot_read) {
     if ((e = cudaEventCreateWithFlags(&read, cudaEventDisableTiming)) != cudaSuccess) {
       return fail(gufo::CudaFail(e, "cudaEventCreate"));
     }
@@ -1475,16 +1490,16 @@ int gufo_cuda_decoder_destroy(gufo_cuda_decoder* d) {
   for (cudaEvent_t e : d->marks) {
     cudaEventDestroy(e);
   }
-  if (d->token_pinned != nullptr) {
-    cudaFreeHost(d->token_pinned);
+  if (d->slots != nullptr) {
+    cudaFreeHost(d->slots);
   }
-  if (d->plan.error_pinned != nullptr) {
-    cudaFreeHost(d->plan.error_pinned);
-  }
-  for (cudaEvent_t read : d->token_read) {
+  for (cudaEvent_t read : d->slot_read) {
     if (read != nullptr) {
       cudaEventDestroy(read);
     }
+  }
+  if (d->plan.error_pinned != nullptr) {
+    cudaFreeHost(d->plan.error_pinned);
   }
   delete d;
   return GUFO_CUDA_OK;
@@ -1534,56 +1549,40 @@ int gufo_cuda_decoder_step_tokens(gufo_cuda_decoder* d, const int* tokens, int c
   gufo_cuda_ctx* ctx = d->ctx;
   std::lock_guard<std::mutex> lock(ctx->mu);
   GUFO_CUDA_TRY(cudaSetDevice(ctx->device));
-  {
-    const unsigned slot = d->token_slot++ % gufo::kTokenSlots;
-    int* staged = d->token_pinned + slot * gufo::kStepTokens;
-    GUFO_CUDA_TRY(cudaEventSynchronize(d->token_read[slot]));   // returns at once for a slot never used
-    for (int t = 0; t < count; ++t) {
-      staged[t] = tokens[t];
-    }
-    GUFO_CUDA_TRY(cudaMemcpyAsync(d->token_dev, staged, 4 * count, cudaMemcpyHostToDevice, ctx->stream));
-    GUFO_CUDA_TRY(cudaEventRecord(d->token_read[slot], ctx->stream));
-  }
   const int parity = d->conv_cur;
   const int pair = count - 1;
-  int with = want_logits != 0 ? 1 : 0;
-  // One token into a pinned host buffer that the device can address: the LM
-  // head mirrors its rows there and no copy follows.
-  if (host_logits != nullptr && count == 1 && d->mirror_ok && d->c.use_graph && !d->timeline && !ctx->force_general &&
-      !ctx->step_kernel && d->eager_runs[pair][1] >= 2) {
-    if (host_logits != d->host_mirror_for) {
-      cudaPointerAttributes attr{};
-      float* device_side = nullptr;
-      if (cudaPointerGetAttributes(&attr, host_logits) == cudaSuccess && attr.type == cudaMemoryTypeHost &&
-          attr.devicePointer != nullptr && (reinterpret_cast<uintptr_t>(attr.devicePointer) & 15) == 0) {
-        device_side = static_cast<float*>(attr.devicePointer);
-      } else {
-        cudaGetLastError();   // pageable memory is not an error here
-      }
-      // The graphs of the old buffer hold its address.
-      for (int w = 0; w < 2; ++w) {
-        if (d->graph[0][w][2] != nullptr) {
-          cudaGraphExecDestroy(d->graph[0][w][2]);
-          d->graph[0][w][2] = nullptr;
-        }
-      }
-      d->host_mirror = device_side;
-      d->host_mirror_for = host_logits;
-    }
-    if (d->host_mirror != nullptr) {
-      with = 2;
-    }
-  }
-  const int ran = with == 2 ? 1 : with;   // which count of eager runs the step belongs to
-  auto enqueue = [&]() { return gufo::EnqueueStep(d, parity, with != 0, count, with == 2); };
+  const int with = want_logits != 0 ? 1 : 0;
   // One token: the whole step as one persistent kernel, where the model allows it.
   const bool kernel_step = count == 1 && d->plan.ok && ctx->step_kernel && !ctx->force_general && !d->timeline;
+  // Logits asked for in pinned memory that the device can address are stored there
+  // by the LM head itself. (Asked of the driver at every step, 0.3 us: the memory
+  // behind a pointer seen before may have been freed since.)
+  float* mirror = nullptr;
+  if (host_logits != nullptr && d->mirror_ok[pair] && !kernel_step && !d->timeline && !ctx->force_general) {
+    mirror = static_cast<float*>(gufo::DeviceAddress(host_logits));
+  }
+  {
+    const unsigned slot = d->next_slot++ % gufo::kStepSlots;
+    if (d->slot_busy[slot]) {
+      GUFO_CUDA_TRY(cudaEventSynchronize(d->slot_read[slot]));
+    }
+    for (int t = 0; t < count; ++t) {
+      d->slots[slot].token[t] = tokens[t];
+    }
+    d->slots[slot].mirror = mirror;
+    GUFO_CUDA_TRY(cudaMemcpyAsync(d->words, d->slots + slot, sizeof(gufo::StepWords), cudaMemcpyHostToDevice, ctx->stream));
+    d->slot_busy[slot] = host_logits == nullptr;   // else the stream is waited for below
+    if (d->slot_busy[slot]) {
+      GUFO_CUDA_TRY(cudaEventRecord(d->slot_read[slot], ctx->stream));
+    }
+  }
+  auto enqueue = [&]() { return gufo::EnqueueStep(d, parity, with != 0, count); };
   if (kernel_step) {
     const int rc = gufo::EnqueueStepKernel(d, parity, with != 0);
     if (rc != GUFO_CUDA_OK) {
       return rc;
     }
-  } else if (d->c.use_graph && d->eager_runs[pair][ran] >= 2 && !d->timeline) {
+  } else if (d->c.use_graph && d->eager_runs[pair][with] >= 2 && !d->timeline) {
     cudaGraphExec_t& exec = d->graph[pair][parity][with];
     if (exec == nullptr) {
       cudaGraph_t graph = nullptr;
@@ -1613,7 +1612,7 @@ int gufo_cuda_decoder_step_tokens(gufo_cuda_decoder* d, const int* tokens, int c
     if (rc != GUFO_CUDA_OK) {
       return rc;
     }
-    ++d->eager_runs[pair][ran];
+    ++d->eager_runs[pair][with];
   }
   d->position += count;
   d->conv_cur ^= 1;
@@ -1632,7 +1631,7 @@ int gufo_cuda_decoder_step_tokens(gufo_cuda_decoder* d, const int* tokens, int c
     d->mark_kind.clear();
     ++d->timeline_steps;
   }
-  if (host_logits != nullptr && with == 2) {
+  if (mirror != nullptr) {
     // The LM head wrote the caller's buffer itself; the step's end is all there is to wait for.
     GUFO_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   } else if (host_logits != nullptr) {
@@ -1718,12 +1717,9 @@ int gufo_cuda_decoder_resolve(gufo_cuda_decoder* d, int keep_second) {
                                     cudaMemcpyDeviceToDevice, ctx->stream));
     }
     --d->position;
-    int* word = d->token_pinned + gufo::kTokenSlots * gufo::kStepTokens;
-    *word = d->position;
-    GUFO_CUDA_TRY(cudaMemcpyAsync(d->position_dev, word, 4, cudaMemcpyHostToDevice, ctx->stream));
-    // The pinned word is read when the copy runs: wait, so that a later
-    // Resolve cannot overwrite it first.
-    GUFO_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    gufo::SetWordKernel<<<1, 1, 0, ctx->stream>>>(d->position_dev, d->position);
+    GUFO_CUDA_TRY(cudaGetLastError());
+    ctx->launches.fetch_add(1);
   }
   d->pending = 0;
   return GUFO_CUDA_OK;

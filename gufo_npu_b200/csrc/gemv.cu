@@ -2,8 +2,9 @@
 // Projections::Apply (GgufProjections::MatMul,
 // src/models/qwen35/gguf_projections.cpp:239-286 in the reference).
 //
-// This file holds the general kernel: any row count, any mix of Q4_K, Q6_K and
-// F32 parts in one launch, 1..8 tokens per weight read. One warp owns one
+// This file holds the kernels for F32 (GemvRowsF32), Q5_K and Q8_0 (GemvSplit) rows
+// and the general kernel: any row count, any mix of types in one launch, 1..8
+// tokens per weight read. There one warp owns one
 // output row; lanes split the row's blocks so that a warp reads whole 128-byte
 // lines, codes are turned into fp32 once and reused for every token, and the
 // sub-block scale and min are applied per 32 (Q4_K) or 16 (Q6_K) values:
@@ -11,6 +12,8 @@
 //   Q6_K:  d * sum_g sc_g * ((q - 32) . x)_g
 // fp32 accumulation throughout; lanes are combined with warp shuffles.
 // HBM-bound: algorithmic bytes are the GGUF row bytes plus x and y.
+#include <cstring>
+
 #include "gemv.cuh"
 #include "gemm_tc.cuh"
 
@@ -20,7 +23,7 @@ namespace {
 
 template <int M>
 __device__ __forceinline__ void RowQ4K(const uint8_t* __restrict__ row, int cols,
-                                       const float* __restrict__ x, int lane,
+                                       const float* x, int lane,
                                        float (&acc)[M]) {
   const int p = lane >> 3;        // sub-block pair of this lane's word
   const int c = (lane & 7) * 4;   // first value inside the sub-blocks
@@ -44,8 +47,8 @@ __device__ __forceinline__ void RowQ4K(const uint8_t* __restrict__ row, int cols
     const int at = b * kSuperBlock + 64 * p + c;
 #pragma unroll
     for (int t = 0; t < M; ++t) {
-      const float4 xl = __ldg(reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols + at));
-      const float4 xh = __ldg(reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols + at + 32));
+      const float4 xl = *reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols + at);
+      const float4 xh = *reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols + at + 32);
       const float dot_lo = l0 * xl.x + l1 * xl.y + l2 * xl.z + l3 * xl.w;
       const float dot_hi = h0 * xh.x + h1 * xh.y + h2 * xh.z + h3 * xh.w;
       const float sum_lo = (xl.x + xl.y) + (xl.z + xl.w);
@@ -58,7 +61,7 @@ __device__ __forceinline__ void RowQ4K(const uint8_t* __restrict__ row, int cols
 
 template <int M>
 __device__ __forceinline__ void RowQ6K(const uint8_t* __restrict__ row, int cols,
-                                       const float* __restrict__ x, int lane,
+                                       const float* x, int lane,
                                        float (&acc)[M]) {
   const int blocks = cols / kSuperBlock;
   for (int b = 0; b < blocks; ++b) {
@@ -87,7 +90,7 @@ __device__ __forceinline__ void RowQ6K(const uint8_t* __restrict__ row, int cols
 #pragma unroll
       for (int t = 0; t < M; ++t) {
         const float* xt = x + static_cast<size_t>(t) * cols + at;
-        part[t] += w0 * __ldg(xt) + w1 * __ldg(xt + 32) + w2 * __ldg(xt + 64) + w3 * __ldg(xt + 96);
+        part[t] += w0 * xt[0] + w1 * xt[32] + w2 * xt[64] + w3 * xt[96];
       }
     }
 #pragma unroll
@@ -101,7 +104,7 @@ __device__ __forceinline__ void RowQ6K(const uint8_t* __restrict__ row, int cols
 // (gguf_dot::DotK4<true>, src/models/qwen35/gguf_dot.hpp:115-193).
 template <int M>
 __device__ __forceinline__ void RowQ5K(const uint8_t* __restrict__ row, int cols,
-                                       const float* __restrict__ x, int lane,
+                                       const float* x, int lane,
                                        float (&acc)[M]) {
   const int p = lane >> 3;        // sub-block pair of this lane's word
   const int c = (lane & 7) * 4;   // first value inside the sub-blocks
@@ -130,8 +133,8 @@ __device__ __forceinline__ void RowQ5K(const uint8_t* __restrict__ row, int cols
     const int at = b * kSuperBlock + 64 * p + c;
 #pragma unroll
     for (int t = 0; t < M; ++t) {
-      const float4 xl = __ldg(reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols + at));
-      const float4 xh = __ldg(reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols + at + 32));
+      const float4 xl = *reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols + at);
+      const float4 xh = *reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols + at + 32);
       const float dot_lo = l0 * xl.x + l1 * xl.y + l2 * xl.z + l3 * xl.w;
       const float dot_hi = h0 * xh.x + h1 * xh.y + h2 * xh.z + h3 * xh.w;
       const float sum_lo = (xl.x + xl.y) + (xl.z + xl.w);
@@ -146,7 +149,7 @@ __device__ __forceinline__ void RowQ5K(const uint8_t* __restrict__ row, int cols
 // of every block (gguf_dot::DotQ8_0, gguf_dot.hpp:31-69).
 template <int M>
 __device__ __forceinline__ void RowQ8_0(const uint8_t* __restrict__ row, int cols,
-                                        const float* __restrict__ x, int lane,
+                                        const float* x, int lane,
                                         float (&acc)[M]) {
   const int blocks = cols / kQ8Block;
   for (int b = 0; b < blocks; ++b) {
@@ -155,21 +158,21 @@ __device__ __forceinline__ void RowQ8_0(const uint8_t* __restrict__ row, int col
     const float w = d * static_cast<float>(static_cast<int>(static_cast<int8_t>(__ldg(block + 2 + lane))));
 #pragma unroll
     for (int t = 0; t < M; ++t) {
-      acc[t] = fmaf(w, __ldg(x + static_cast<size_t>(t) * cols + b * kQ8Block + lane), acc[t]);
+      acc[t] = fmaf(w, x[static_cast<size_t>(t) * cols + b * kQ8Block + lane], acc[t]);
     }
   }
 }
 
 template <int M>
 __device__ __forceinline__ void RowF32(const uint8_t* __restrict__ row, int cols,
-                                       const float* __restrict__ x, int lane,
+                                       const float* x, int lane,
                                        float (&acc)[M]) {
   const float4* w = reinterpret_cast<const float4*>(row);
   for (int i = lane; i < cols / 4; i += 32) {
     const float4 v = __ldg(w + i);
 #pragma unroll
     for (int t = 0; t < M; ++t) {
-      const float4 xv = __ldg(reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols) + i);
+      const float4 xv = *(reinterpret_cast<const float4*>(x + static_cast<size_t>(t) * cols) + i);
       acc[t] += v.x * xv.x + v.y * xv.y + v.z * xv.z + v.w * xv.w;
     }
   }
@@ -191,8 +194,10 @@ GemvRows(const __grid_constant__ GemvArgs args) {
   }
   const GemvPart& part = args.parts[p];
   const uint8_t* data = part.data + static_cast<size_t>(local) * part.row_bytes;
-  const float* x = args.x;
+  const float* x = args.x;   // read with coherent loads: written while this kernel may already be resident
   float* y = args.y;
+  GridLaunchDependents();
+  GridDependencyWait();
   if (args.group_ids != nullptr) {
     const int id = args.group_ids[blockIdx.y];
     if (id < 0) {
@@ -323,11 +328,200 @@ int LaunchRowsF32(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
   return GUFO_CUDA_OK;
 }
 
+// Q5_K and Q8_0 rows of whole 256-value blocks, up to M tokens: a thread block takes
+// kSplitRows rows, its warps the 256-value blocks of K round-robin, a lane eight
+// values of each. The rows' loads of a block are in flight together and a row of
+// 2048 values is one round trip deep, where one warp per row walks eight (Q8_0:
+// sixty-four, a byte a lane); a token's inputs are read once for the rows.
+constexpr int kSplitRows = 4;
+
+// Eight weights of a Q5_K block: values 64 p + c .. + 3 and the same 32 further on
+// (p = lane / 8, c = 4 (lane % 8)).
+__device__ __forceinline__ void SplitWeights5(const uint4& head, uint32_t h, uint32_t q, int p, float (&w)[8]) {
+  const float d = HalfBitsToFloat(static_cast<uint16_t>(head.x & 0xFFFF));
+  const float dmin = HalfBitsToFloat(static_cast<uint16_t>(head.x >> 16));
+  int sc_lo, m_lo, sc_hi, m_hi;
+  ScaleMinK4(2 * p, head.y, head.z, head.w, &sc_lo, &m_lo);
+  ScaleMinK4(2 * p + 1, head.y, head.z, head.w, &sc_hi, &m_hi);
+  const float d_lo = d * static_cast<float>(sc_lo), o_lo = dmin * static_cast<float>(m_lo);
+  const float d_hi = d * static_cast<float>(sc_hi), o_hi = dmin * static_cast<float>(m_hi);
+  h >>= 2 * p;   // the fifth bits of this pair of sub-blocks
+  const uint32_t lo = (q & 0x0F0F0F0Fu) | ((h << 4) & 0x10101010u);
+  const uint32_t hi = ((q >> 4) & 0x0F0F0F0Fu) | ((h << 3) & 0x10101010u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    // A byte under the exponent of 2^23, the bias taken off: no conversion.
+    const float l = __uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7440u | i)) - 8388608.0f;
+    const float g = __uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7440u | i)) - 8388608.0f;
+    w[i] = fmaf(d_lo, l, -o_lo);
+    w[4 + i] = fmaf(d_hi, g, -o_hi);
+  }
+}
+
+template <int TYPE, int M>
+__global__ void __launch_bounds__(256)
+GemvSplit(const __grid_constant__ GemvArgs args, int tokens) {
+  constexpr bool kQ5 = TYPE == GUFO_CUDA_Q5_K;
+  constexpr int kBlockBytes = kQ5 ? kQ5KBytes : kSuperBlock / kQ8Block * kQ8Bytes;
+  __shared__ float partial[8][kSplitRows * M];
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  // Rows past the end repeat the last one, tokens past the end the last token.
+  const uint8_t* row[kSplitRows];
+#pragma unroll
+  for (int r = 0; r < kSplitRows; ++r) {
+    int local = min(static_cast<int>(blockIdx.x) * kSplitRows + r, args.total_rows - 1);
+    int p = 0;
+    while (p + 1 < args.nparts && local >= args.parts[p].rows) {
+      local -= args.parts[p].rows;
+      ++p;
+    }
+    row[r] = args.parts[p].data + static_cast<size_t>(local) * args.parts[p].row_bytes;
+  }
+  // Where this lane's eight inputs sit: two groups of four.
+  const int at = kQ5 ? 64 * (lane >> 3) + 4 * (lane & 7) : 8 * lane;
+  constexpr int kApart = kQ5 ? 32 : 4;
+  // Q8_0: eight codes at a 2-byte boundary, out of aligned words.
+  const int code = 34 * (lane >> 2) + 2 + 8 * (lane & 3);
+  const bool odd = (code & 2) != 0;
+  GridLaunchDependents();
+  GridDependencyWait();
+  float acc[kSplitRows][M];
+#pragma unroll
+  for (int r = 0; r < kSplitRows; ++r) {
+#pragma unroll
+    for (int t = 0; t < M; ++t) {
+      acc[r][t] = 0.f;
+    }
+  }
+  for (int b = warp; b < args.cols / kSuperBlock; b += 8) {
+    float w[kSplitRows][8];
+    if constexpr (kQ5) {
+      uint4 head[kSplitRows];
+      uint32_t h[kSplitRows], q[kSplitRows];
+#pragma unroll
+      for (int r = 0; r < kSplitRows; ++r) {
+        const uint8_t* block = row[r] + static_cast<size_t>(b) * kBlockBytes;
+        head[r] = __ldg(reinterpret_cast<const uint4*>(block));
+        h[r] = __ldg(reinterpret_cast<const uint32_t*>(block + 16) + (lane & 7));
+        q[r] = __ldg(reinterpret_cast<const uint32_t*>(block + 48) + lane);
+      }
+#pragma unroll
+      for (int r = 0; r < kSplitRows; ++r) {
+        SplitWeights5(head[r], h[r], q[r], lane >> 3, w[r]);
+      }
+    } else {
+      uint32_t q[kSplitRows][3];
+      uint16_t d[kSplitRows];
+#pragma unroll
+      for (int r = 0; r < kSplitRows; ++r) {
+        const uint8_t* block = row[r] + static_cast<size_t>(b) * kBlockBytes;
+        const uint32_t* words = reinterpret_cast<const uint32_t*>(block + (code & ~3));
+        q[r][0] = __ldg(words);
+        q[r][1] = __ldg(words + 1);
+        q[r][2] = odd ? __ldg(words + 2) : 0u;
+        d[r] = __ldg(reinterpret_cast<const uint16_t*>(block + 34 * (lane >> 2)));
+      }
+#pragma unroll
+      for (int r = 0; r < kSplitRows; ++r) {
+        const uint32_t pick = odd ? 0x5432u : 0x3210u;
+        // Codes + 128 as bytes under the exponent of 2^23.
+        const uint32_t lo = __byte_perm(q[r][0], q[r][1], pick) ^ 0x80808080u;
+        const uint32_t hi = __byte_perm(q[r][1], q[r][2], pick) ^ 0x80808080u;
+        const float scale = HalfBitsToFloat(d[r]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          w[r][i] = scale * (__uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7440u | i)) - 8388736.0f);
+          w[r][4 + i] = scale * (__uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7440u | i)) - 8388736.0f);
+        }
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < M; ++t) {
+      const float* x = args.x + static_cast<size_t>(min(t, tokens - 1)) * args.cols + b * kSuperBlock + at;
+      const float4 x0 = *reinterpret_cast<const float4*>(x);
+      const float4 x1 = *reinterpret_cast<const float4*>(x + kApart);
+#pragma unroll
+      for (int r = 0; r < kSplitRows; ++r) {
+        float sum = fmaf(w[r][0], x0.x, fmaf(w[r][1], x0.y, fmaf(w[r][2], x0.z, w[r][3] * x0.w)));
+        sum = fmaf(w[r][4], x1.x, fmaf(w[r][5], x1.y, fmaf(w[r][6], x1.z, fmaf(w[r][7], x1.w, sum))));
+        acc[r][t] += sum;
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kSplitRows; ++r) {
+#pragma unroll
+    for (int t = 0; t < M; ++t) {
+      const float total = WarpSum(acc[r][t]);
+      if (lane == 0) {
+        partial[warp][r * M + t] = total;
+      }
+    }
+  }
+  __syncthreads();
+  const int r = threadIdx.x / M, t = threadIdx.x % M;
+  int local = static_cast<int>(blockIdx.x) * kSplitRows + r;
+  if (threadIdx.x >= kSplitRows * M || local >= args.total_rows || t >= tokens) {
+    return;
+  }
+  float total = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    total += partial[k][threadIdx.x];
+  }
+  int p = 0;
+  while (p + 1 < args.nparts && local >= args.parts[p].rows) {
+    local -= args.parts[p].rows;
+    ++p;
+  }
+  args.y[static_cast<size_t>(t) * args.y_stride + args.parts[p].out_offset + local] = total;
+}
+
+// Whether GemvSplit runs a part: whole 256-value blocks at the alignment of its loads.
+bool SplitRuns(const GemvPart& part, int cols) {
+  const uintptr_t align = part.type == GUFO_CUDA_Q5_K ? 16 : 4;
+  return (part.type == GUFO_CUDA_Q5_K || part.type == GUFO_CUDA_Q8_0) && cols % kSuperBlock == 0 &&
+         reinterpret_cast<uintptr_t>(part.data) % align == 0 && part.row_bytes % align == 0;
+}
+
+template <int TYPE>
+int LaunchSplit(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
+  const dim3 grid((args.total_rows + kSplitRows - 1) / kSplitRows);
+  auto launch = [&](auto kernel) { return LaunchOverlapped(kernel, grid, dim3(256), 0, ctx->stream, 1, args, tokens); };
+  GUFO_CUDA_TRY(tokens == 1   ? launch(GemvSplit<TYPE, 1>)
+                : tokens == 2 ? launch(GemvSplit<TYPE, 2>)
+                : tokens <= 4 ? launch(GemvSplit<TYPE, 4>)
+                              : launch(GemvSplit<TYPE, 8>));
+  ctx->launches.fetch_add(1);
+  return GUFO_CUDA_OK;
+}
+
 template <int M>
-void LaunchRows(const GemvArgs& args, cudaStream_t stream) {
+int LaunchRows(gufo_cuda_ctx* ctx, const GemvArgs& args) {
   const int warps = 8;
   const dim3 grid((args.total_rows + warps - 1) / warps, args.group_ids != nullptr ? args.groups : 1);
-  GemvRows<M><<<grid, warps * 32, 0, stream>>>(args);
+  GUFO_CUDA_TRY(LaunchOverlapped(GemvRows<M>, grid, dim3(warps * 32), 0, ctx->stream, 1, args));
+  ctx->launches.fetch_add(1);
+  return GUFO_CUDA_OK;
+}
+
+// Host rows into device memory, read straight from mapped pinned memory: a launch
+// and a PCIe round trip, where a copy costs the copy engine's start and its
+// hand-over to the next kernel (8 KB: 3 us against 10).
+__global__ void __launch_bounds__(256)
+FetchKernel(const float* __restrict__ src, float* __restrict__ dst, int64_t n) {
+  GridLaunchDependents();
+  GridDependencyWait();   // dst may still be read by the product before
+  for (int64_t i = 4 * (blockIdx.x * static_cast<int64_t>(256) + threadIdx.x); i < n; i += 4 * 256 * static_cast<int64_t>(gridDim.x)) {
+    if (i + 4 <= n) {
+      *reinterpret_cast<float4*>(dst + i) = __ldcv(reinterpret_cast<const float4*>(src + i));
+    } else {
+      for (int64_t j = i; j < n; ++j) {
+        dst[j] = __ldcv(src + j);
+      }
+    }
+  }
 }
 
 }  // namespace
@@ -444,29 +638,47 @@ int LaunchGemv(gufo_cuda_ctx* ctx, const GemvArgs& base, int tokens) {
         return rc;
       }
     }
+    GemvArgs split5 = rest, split8 = rest;
     for (int p = 0; p < base.nparts; ++p) {
       const GemvPart& part = base.parts[p];
       if ((fast4 && part.type == GUFO_CUDA_Q4_K) || (fast6 && part.type == GUFO_CUDA_Q6_K)) {
         continue;
       }
-      rest.parts[rest.nparts++] = part;
-      rest.total_rows += part.rows;
+      GemvArgs& to = ctx->force_general || !SplitRuns(part, base.cols) ? rest
+                     : part.type == GUFO_CUDA_Q5_K                     ? split5
+                                                                       : split8;
+      to.parts[to.nparts++] = part;
+      to.total_rows += part.rows;
+    }
+    if (split5.nparts > 0) {
+      const int rc = LaunchSplit<GUFO_CUDA_Q5_K>(ctx, split5, m);
+      if (rc != GUFO_CUDA_OK) {
+        return rc;
+      }
+    }
+    if (split8.nparts > 0) {
+      const int rc = LaunchSplit<GUFO_CUDA_Q8_0>(ctx, split8, m);
+      if (rc != GUFO_CUDA_OK) {
+        return rc;
+      }
     }
     if (rest.nparts == 0) {
       continue;
     }
+    int rc = GUFO_CUDA_OK;
     switch (m) {
-      case 1: LaunchRows<1>(rest, ctx->stream); break;
-      case 2: LaunchRows<2>(rest, ctx->stream); break;
-      case 3: LaunchRows<3>(rest, ctx->stream); break;
-      case 4: LaunchRows<4>(rest, ctx->stream); break;
-      case 5: LaunchRows<5>(rest, ctx->stream); break;
-      case 6: LaunchRows<6>(rest, ctx->stream); break;
-      case 7: LaunchRows<7>(rest, ctx->stream); break;
-      default: LaunchRows<8>(rest, ctx->stream); break;
+      case 1: rc = LaunchRows<1>(ctx, rest); break;
+      case 2: rc = LaunchRows<2>(ctx, rest); break;
+      case 3: rc = LaunchRows<3>(ctx, rest); break;
+      case 4: rc = LaunchRows<4>(ctx, rest); break;
+      case 5: rc = LaunchRows<5>(ctx, rest); break;
+      case 6: rc = LaunchRows<6>(ctx, rest); break;
+      case 7: rc = LaunchRows<7>(ctx, rest); break;
+      default: rc = LaunchRows<8>(ctx, rest); break;
     }
-    ctx->launches.fetch_add(1);
-    GUFO_CUDA_TRY(cudaGetLastError());
+    if (rc != GUFO_CUDA_OK) {
+      return rc;
+    }
   }
   return GUFO_CUDA_OK;
 }
@@ -561,9 +773,7 @@ int LaunchGemvGrouped(gufo_cuda_ctx* ctx, const GemvArgs& base, int prologue, fl
       rest.x_group_stride = base.cols;
       rest.x_group_div = 1;
     }
-    LaunchRows<1>(rest, ctx->stream);
-    ctx->launches.fetch_add(1);
-    GUFO_CUDA_TRY(cudaGetLastError());
+    return LaunchRows<1>(ctx, rest);
   }
   return GUFO_CUDA_OK;
 }
@@ -660,24 +870,65 @@ int gufo_cuda_matmul(gufo_cuda_ctx* ctx, const gufo_cuda_rows* parts, int nparts
     return rc;
   }
   GUFO_CUDA_TRY(cudaSetDevice(ctx->device));
-  const size_t x_bytes = static_cast<size_t>(tokens) * args.cols * 4;
-  const size_t y_bytes = static_cast<size_t>(tokens) * args.total_rows * 4;
+  const size_t x_values = static_cast<size_t>(tokens) * args.cols, x_bytes = 4 * x_values;
+  const size_t y_values = static_cast<size_t>(tokens) * args.total_rows, y_bytes = 4 * y_values;
   rc = ctx->Reserve(&ctx->stage_x, &ctx->stage_x_bytes, x_bytes);
-  if (rc == GUFO_CUDA_OK) {
-    rc = ctx->Reserve(&ctx->stage_y, &ctx->stage_y_bytes, y_bytes);
-  }
   if (rc != GUFO_CUDA_OK) {
     return rc;
   }
-  GUFO_CUDA_TRY(cudaMemcpyAsync(ctx->stage_x, host_x, x_bytes, cudaMemcpyHostToDevice, ctx->stream));
+  // x: from pinned memory (the caller's, or the context's after a copy by this
+  // thread) a kernel fetches it; more than kStagedBytes of pageable memory are left
+  // to the driver's copy, whose fixed cost no longer counts there.
+  constexpr size_t kStagedBytes = 1u << 20;
+  const float* from = static_cast<const float*>(gufo::DeviceAddress(host_x));
+  if (from == nullptr && x_bytes <= kStagedBytes &&
+      ctx->ReserveHost(&ctx->host_x, &ctx->host_x_bytes, x_bytes) == GUFO_CUDA_OK) {
+    std::memcpy(ctx->host_x, host_x, x_bytes);
+    from = static_cast<const float*>(gufo::DeviceAddress(ctx->host_x));
+  }
+  if (from != nullptr && reinterpret_cast<uintptr_t>(from) % 16 == 0 && x_bytes <= kStagedBytes) {
+    const int blocks = static_cast<int>((x_values + 1023) / 1024);
+    GUFO_CUDA_TRY(gufo::LaunchOverlapped(gufo::FetchKernel, dim3(blocks), dim3(256), 0, ctx->stream, 1, from,
+                                         ctx->stage_x, static_cast<int64_t>(x_values)));
+    ctx->launches.fetch_add(1);
+  } else {
+    GUFO_CUDA_TRY(cudaMemcpyAsync(ctx->stage_x, host_x, x_bytes, cudaMemcpyHostToDevice, ctx->stream));
+  }
+  // y: the GEMV kernels store up to kDirectValues straight into pinned memory
+  // (posted writes, hidden behind the weights); more go through device memory and a
+  // copy, as single rows are a poor fit for PCIe.
+  constexpr size_t kDirectValues = 16384;
+  float* to = static_cast<float*>(gufo::DeviceAddress(host_y));
+  float* stage = nullptr;   // pinned memory that stands for a pageable y
+  if (to == nullptr && y_bytes <= kStagedBytes &&
+      ctx->ReserveHost(&ctx->host_y, &ctx->host_y_bytes, y_bytes) == GUFO_CUDA_OK) {
+    stage = ctx->host_y;
+    to = static_cast<float*>(gufo::DeviceAddress(stage));
+  }
   args.x = ctx->stage_x;
-  args.y = ctx->stage_y;
-  rc = gufo::LaunchGemv(ctx, args, tokens);
-  if (rc != GUFO_CUDA_OK) {
-    return rc;
+  if (to != nullptr && tokens <= gufo::kMaxTokens && y_values <= kDirectValues) {
+    args.y = to;
+    rc = gufo::LaunchGemv(ctx, args, tokens);
+    if (rc != GUFO_CUDA_OK) {
+      return rc;
+    }
+  } else {
+    rc = ctx->Reserve(&ctx->stage_y, &ctx->stage_y_bytes, y_bytes);
+    if (rc != GUFO_CUDA_OK) {
+      return rc;
+    }
+    args.y = ctx->stage_y;
+    rc = gufo::LaunchGemv(ctx, args, tokens);
+    if (rc != GUFO_CUDA_OK) {
+      return rc;
+    }
+    GUFO_CUDA_TRY(cudaMemcpyAsync(stage != nullptr ? stage : host_y, ctx->stage_y, y_bytes, cudaMemcpyDeviceToHost,
+                                  ctx->stream));
   }
-  GUFO_CUDA_TRY(cudaMemcpyAsync(host_y, ctx->stage_y, y_bytes, cudaMemcpyDeviceToHost, ctx->stream));
   GUFO_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (stage != nullptr) {
+    std::memcpy(host_y, stage, y_bytes);
+  }
   return GUFO_CUDA_OK;
 }
 

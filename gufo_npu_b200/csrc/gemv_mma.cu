@@ -89,6 +89,7 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   // Where the blocks of a cluster leave their sums for block 0: [2][8][16][TOKENS].
   __shared__ float peers[2 * 8 * 16 * TOKENS];
   __shared__ float squares[kFastWarps * TOKENS];         // a fused norm's (FillImage)
+  __shared__ float* mirror;                              // the second copy of y, if any
   __shared__ __align__(8) uint64_t landed[kMaxStages];   // a slab's bytes have arrived
   // The barriers need no kernel argument: set up first, while the arguments' first
   // reads (constant-cache misses) are under way. A barrier takes eight arrivals.
@@ -257,6 +258,9 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   GridDependencyWait();
   // Row-split ranks: the input vector may still be on its way from the peers.
   PeerWaitBlock(a.peer_wait);
+  if (threadIdx.x == 0) {   // read behind the image's barrier
+    mirror = a.mirror != nullptr ? *a.mirror : nullptr;
+  }
   if (a.prologue == kPrologueImage) {
     const uint32_t base = SharedAddress(smem);
     for (int at = threadIdx.x * 16; at < l.bytes; at += kFastThreads * 16) {
@@ -313,6 +317,9 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
         }
       } else {
         a.y[at] = total;
+        if (mirror != nullptr) {
+          mirror[at] = total;
+        }
       }
     }
   };
@@ -486,8 +493,8 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     __syncthreads();
     gather(my_tiles - 1);
   }
-  if (a.peer_out.world > 0 && a.peer_out.slot >= 0) {
-    PeerSignal(a.peer_out);   // slot < 0: copies that nobody waits on by flag (a host mirror)
+  if (a.peer_out.world > 0) {
+    PeerSignal(a.peer_out);
   }
 }
 

@@ -30,6 +30,9 @@ struct Api {
   decltype(&gufo_cuda_route_device) route;
   decltype(&gufo_cuda_moe_ffn_device) moe_ffn;
   decltype(&gufo_cuda_decoder_step) decoder_step;
+  decltype(&gufo_cuda_decoder_step_tokens) decoder_step_tokens;
+  decltype(&gufo_cuda_host_take) host_take;
+  decltype(&gufo_cuda_host_give) host_give;
 } api;
 
 // Raised to the interpreter as whatever exception is already set.
@@ -374,6 +377,67 @@ PyObject* DecoderStep(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// decoder_step_tokens(decoder address, tokens, want_logits, logits)
+PyObject* DecoderStepTokens(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return Guarded(n, 4, [&] {
+    auto* decoder = static_cast<gufo_cuda_decoder*>(PyLong_AsVoidPtr(a[0]));
+    Ref list(PySequence_Fast(a[1], "gufo_cuda: tokens must be a sequence"));
+    const int count = static_cast<int>(PySequence_Fast_GET_SIZE(list.o));
+    std::vector<int> tokens(count > 0 ? count : 1);
+    for (int i = 0; i < count; ++i) {
+      tokens[i] = SmallInt(PySequence_Fast_GET_ITEM(list.o, i));
+    }
+    const int want = SmallInt(a[2]);
+    float* logits = Ptr<float>(a[3]);
+    return Unlocked([&] { return api.decoder_step_tokens(decoder, tokens.data(), count, want, logits); });
+  });
+}
+
+// A block of the library's pinned memory, exposed through the buffer protocol and
+// given back when the last array over it has gone.
+struct HostBuffer {
+  PyObject_HEAD
+  void* data;
+  Py_ssize_t bytes;
+};
+
+void HostBufferDealloc(PyObject* self) {
+  api.host_give(reinterpret_cast<HostBuffer*>(self)->data);
+  Py_TYPE(self)->tp_free(self);
+}
+
+int HostBufferGet(PyObject* self, Py_buffer* view, int flags) {
+  auto* b = reinterpret_cast<HostBuffer*>(self);
+  return PyBuffer_FillInfo(view, self, b->data, b->bytes, 0, flags);
+}
+
+PyBufferProcs host_buffer_procs = {HostBufferGet, nullptr};
+PyTypeObject host_buffer_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+// host_buffer(ctx, bytes): a HostBuffer, or None where the pool is at its bound.
+PyObject* NewHostBuffer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return Guarded(n, 2, [&]() -> PyObject* {
+    gufo_cuda_ctx* ctx = Context(a[0]);
+    const long long bytes = Int(a[1]);
+    void* data = nullptr;
+    int status;
+    Py_BEGIN_ALLOW_THREADS
+    status = api.host_take(ctx, static_cast<size_t>(bytes), &data);
+    Py_END_ALLOW_THREADS
+    if (status != GUFO_CUDA_OK || data == nullptr) {
+      Py_RETURN_NONE;
+    }
+    auto* b = PyObject_New(HostBuffer, &host_buffer_type);
+    if (b == nullptr) {
+      api.host_give(data);
+      throw Failed();
+    }
+    b->data = data;
+    b->bytes = bytes;
+    return reinterpret_cast<PyObject*>(b);
+  });
+}
+
 // bind(library handle): looks the entry points up in the loaded library.
 PyObject* Bind(PyObject*, PyObject* handle) {
   void* lib = PyLong_AsVoidPtr(handle);
@@ -396,6 +460,9 @@ PyObject* Bind(PyObject*, PyObject* handle) {
   find(&api.route, "gufo_cuda_route_device");
   find(&api.moe_ffn, "gufo_cuda_moe_ffn_device");
   find(&api.decoder_step, "gufo_cuda_decoder_step");
+  find(&api.decoder_step_tokens, "gufo_cuda_decoder_step_tokens");
+  find(&api.host_take, "gufo_cuda_host_take");
+  find(&api.host_give, "gufo_cuda_host_give");
   if (missing != nullptr) {
     return PyErr_Format(PyExc_ImportError, "libgufo_cuda.so has no %s", missing);
   }
@@ -413,6 +480,8 @@ PyMethodDef methods[] = {
     FAST("route", Route),
     FAST("moe_ffn", MoeFfn),
     FAST("decoder_step", DecoderStep),
+    FAST("decoder_step_tokens", DecoderStepTokens),
+    FAST("host_buffer", NewHostBuffer),
     {nullptr, nullptr, 0, nullptr},
 };
 #undef FAST
@@ -435,6 +504,14 @@ PyMODINIT_FUNC PyInit__native() {
     if ((*n.key = PyUnicode_InternFromString(n.name)) == nullptr) {
       return nullptr;
     }
+  }
+  host_buffer_type.tp_name = "gufo_npu_b200._native.HostBuffer";
+  host_buffer_type.tp_basicsize = sizeof(HostBuffer);
+  host_buffer_type.tp_dealloc = HostBufferDealloc;
+  host_buffer_type.tp_as_buffer = &host_buffer_procs;
+  host_buffer_type.tp_flags = Py_TPFLAGS_DEFAULT;
+  if (PyType_Ready(&host_buffer_type) != 0) {
+    return nullptr;
   }
   return PyModule_Create(&module);
 }

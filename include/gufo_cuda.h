@@ -108,6 +108,12 @@ int gufo_cuda_upload(gufo_cuda_ctx* ctx, void* device_dst, const void* host_src,
 int gufo_cuda_download(gufo_cuda_ctx* ctx, void* host_dst,
                        const void* device_src, size_t bytes);
 int gufo_cuda_memset_zero(gufo_cuda_ctx* ctx, void* device_ptr, size_t bytes);
+/* Pinned host memory for results, from a pool of the process (bounded; kept
+ * blocks are freed with the last context). *host is NULL where the pool is at
+ * its bound: use pageable memory then. Give a block back with
+ * gufo_cuda_host_give, also after the context has gone. */
+int gufo_cuda_host_take(gufo_cuda_ctx* ctx, size_t bytes, void** host);
+int gufo_cuda_host_give(void* host);
 
 /* ---- weights ---------------------------------------------------------- */
 
@@ -625,9 +631,8 @@ int gufo_cuda_decoder_reset(gufo_cuda_decoder* decoder);
  * current position, advances the state, and leaves the vocab logits in
  * host_logits (may be NULL to leave them on the device only). Pageable memory
  * gets a copy after the step. Pinned memory that the device can address
- * (cudaHostAlloc, cudaHostRegister; 16-byte aligned) is written by the LM
- * head's own stores while that kernel runs, once the step replays as a graph:
- * pass the same buffer step after step (a new buffer costs a graph capture).
+ * (cudaHostAlloc, cudaHostRegister, gufo_cuda_host_take) is written by the LM
+ * head's own stores while that kernel runs.
  * Returns GUFO_CUDA_BAD_ARGUMENT for a token outside [0, vocab) and
  * GUFO_CUDA_TOO_LARGE when the attention cache is full. */
 int gufo_cuda_decoder_step(gufo_cuda_decoder* decoder, int token,

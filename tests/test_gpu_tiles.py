@@ -134,3 +134,95 @@ def test_mixer_run_of_many_sequences_equals_one_token_at_a_time(ctx, oracle, hea
         want, _ = oracle.deltanet_linear(_deltanet_cfg(cfg), _deltanet_weights(cfg, tensors, 0), hx, hconv, hssm)
         assert rel_l2(y[s].cpu().numpy(), want) <= 1e-4
         assert rel_l2(ssm[s].cpu().numpy(), hssm) <= 1e-4
+
+
+def _random_rows(ctx, ggml_type, rows, cols, seed):
+    """Any code bytes beside small fp16 scales: a matrix handle and its values in float64."""
+    rng = np.random.default_rng(seed)
+    per, size = Q.BLOCK_ELEMENTS[ggml_type], Q.BLOCK_BYTES[ggml_type]
+    raw = rng.integers(0, 256, (rows * cols // per, size), dtype=np.uint8)
+    for at in ((0, 2) if ggml_type == Q.GGML_Q5_K else (0,)):
+        raw[:, at:at + 2] = (1e-3 * (1.0 + rng.random(raw.shape[0]))).astype(np.float16).view(np.uint8).reshape(-1, 2)
+    m = ctx.matrix_upload(ggml_type, raw.reshape(rows, -1), rows, cols)
+    return m, ctx.dequantize(m, 0, rows, cols).astype(np.float64)
+
+
+@pytest.mark.parametrize("ggml_type", [Q.GGML_Q5_K, Q.GGML_Q8_0])
+@pytest.mark.parametrize("tokens", [1, 2, 3, 5, 8, 9])
+@pytest.mark.parametrize("rows,cols", [(1, 256), (7, 2048), (133, 2304), (6, 9728)])
+def test_q5_and_q8_rows_split_over_warps(ctx, ggml_type, tokens, rows, cols):
+    """Row and token counts off the tile, K shorter and longer than a round of the warps; two parts
+    with a cut inside one."""
+    m, w = _random_rows(ctx, ggml_type, rows + 2, cols, 50 + rows)
+    x = G.normal(51 + tokens, tokens, cols)
+    got = ctx.matmul([(m, 0, rows), (m, rows, 2)], x, tokens, rows + 2)
+    want = x.astype(np.float64) @ w.T
+    assert rel_l2(got, want) <= 1e-6
+    ctx.matrix_free(m)
+
+
+@pytest.mark.parametrize("tokens,rows,cols", [(1, 16384, 256), (1, 16385, 256), (8, 9000, 512), (40, 7000, 8192), (3, 5, 768)])
+def test_host_rows_pinned_and_pageable(ctx, tokens, rows, cols):
+    """Host inputs and results on either side of the sizes that are staged, stored directly or left to
+    the driver's copy, in pageable and in pinned memory: the same bytes."""
+    m, w = _matrix(ctx, Q.GGML_Q4_K, rows, cols, 41)
+    x = G.normal(42, tokens, cols).astype(np.float32)
+    got = ctx.matmul([(m, 0, rows)], x, tokens, rows)
+    assert rel_l2(got, x.astype(np.float64) @ w.T) <= 1e-3
+    kept = got.copy()
+    parts = Context._parts([(m, 0, rows)])
+    px, py = torch.from_numpy(x).pin_memory(), torch.empty(tokens, rows).pin_memory()
+    y = np.empty((tokens, rows), dtype=np.float32)
+    for xa, ya, out in ((px.data_ptr(), y.ctypes.data, y), (px.data_ptr(), py.data_ptr(), py.numpy()),
+                        (x.ctypes.data, py.data_ptr(), py.numpy())):
+        out[:] = 0
+        ctx.matmul_host(parts, 1, xa, tokens, ya)
+        assert np.array_equal(out, kept)
+    other = ctx.matmul([(m, 0, rows)], 2 * x, tokens, rows)
+    assert np.array_equal(got, kept) and not np.shares_memory(got, other)
+    ctx.matrix_free(m)
+
+
+@pytest.mark.parametrize("vocab", [512, 40000])
+def test_step_logits_in_any_memory(ctx, vocab):
+    """Logits left on the device (many steps, none waited for), in pageable, pooled
+    and alternating pinned memory: the same bits; pairs to the rounding of another order of sums."""
+    from gufo_npu_b200 import synth
+    from gufo_npu_b200.backend import CudaDecoder, CudaProjections
+    cfg = synth.ModelConfig(layers=4, hidden=256, ffn=512, vocab=vocab, heads=2, kv_heads=1, head_dim=128, rope_dim=32,
+                            linear_key_heads=2, linear_value_heads=4, linear_head_dim=128)
+    tensors = synth.build_model(cfg, 3)
+    dec = CudaDecoder(CudaProjections(ctx, cfg, tensors), tensors, max_positions=64, use_graph=True)
+    tokens = [(37 * i + 11) % vocab for i in range(24)]
+    want = []
+    for t in tokens:
+        at = dec.step_device(t)
+        want.append(ctx.download(at, vocab))
+    dec.Reset()
+    for t in tokens:
+        at = dec.step_device(t)
+    assert np.array_equal(ctx.download(at, vocab), want[-1])
+    dec.Reset()
+    pinned = [torch.empty(vocab).pin_memory() for _ in range(2)]
+    held = []
+    for i, t in enumerate(tokens):
+        if i % 4 == 3:
+            got = dec.Step(t)
+        elif i % 4 == 2:
+            got = dec.Step(t, np.empty(vocab, dtype=np.float32))
+        else:
+            got = dec.Step(t, pinned[i % 2]).numpy().copy()
+        held.append(got)
+    for got, w in zip(held, want):
+        assert np.array_equal(got, w)
+    dec.Reset()
+    for i in range(0, 16, 2):
+        got = dec.StepTokens(tokens[i:i + 2])
+        assert rel_l2(got[0], want[i]) <= 5e-4 and rel_l2(got[1], want[i + 1]) <= 5e-4
+        dec.Resolve(True)
+    dec.Reset()
+    for i in range(8):
+        got = dec.StepTokens([tokens[i], tokens[(i + 5) % 8]])
+        assert rel_l2(got[0], want[i]) <= 5e-4
+        dec.Resolve(False)
+    dec.close()
