@@ -238,8 +238,9 @@ GemvRows(const __grid_constant__ GemvArgs args) {
 // flight together and a row of 2560 values is three chunks deep, where one warp
 // per row walks twenty; the inputs are read once per eight rows. 64 rows x 2560
 // values: 512 tokens were 64 launches of the kernel above (1.2 ms with the gaps).
-constexpr int kF32Rows = 8;
-template <int TOK>
+// Where eight rows a block would leave SMs without one (a router: 257 rows, 33
+// blocks) a block takes two.
+template <int kF32Rows, int TOK>
 __global__ void __launch_bounds__(256)
 GemvRowsF32(const __grid_constant__ GemvArgs args, int tokens) {
   __shared__ float partial[8][kF32Rows * TOK];
@@ -315,15 +316,16 @@ GemvRowsF32(const __grid_constant__ GemvArgs args, int tokens) {
   args.y[static_cast<size_t>(t0 + t) * args.y_stride + args.parts[p].out_offset + local] = total;
 }
 
+template <int ROWS>
 int LaunchRowsF32(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
-  const unsigned rows = (args.total_rows + kF32Rows - 1) / kF32Rows;
+  const unsigned rows = (args.total_rows + ROWS - 1) / ROWS;
   auto launch = [&](auto kernel, int tok) {
     return LaunchOverlapped(kernel, dim3(rows, (tokens + tok - 1) / tok), dim3(256), 0, ctx->stream, 1, args, tokens);
   };
-  GUFO_CUDA_TRY(tokens == 1   ? launch(GemvRowsF32<1>, 1)
-                : tokens == 2 ? launch(GemvRowsF32<2>, 2)
-                : tokens <= 4 ? launch(GemvRowsF32<4>, 4)
-                              : launch(GemvRowsF32<8>, 8));
+  GUFO_CUDA_TRY(tokens == 1   ? launch(GemvRowsF32<ROWS, 1>, 1)
+                : tokens == 2 ? launch(GemvRowsF32<ROWS, 2>, 2)
+                : tokens <= 4 ? launch(GemvRowsF32<ROWS, 4>, 4)
+                              : launch(GemvRowsF32<ROWS, 8>, 8));
   ctx->launches.fetch_add(1);
   return GUFO_CUDA_OK;
 }
@@ -559,7 +561,8 @@ int LaunchGemv(gufo_cuda_ctx* ctx, const GemvArgs& base, int tokens) {
       to.total_rows += base.parts[p].rows;
     }
     if (f32.nparts > 0) {
-      const int rc = LaunchRowsF32(ctx, f32, tokens);
+      const int blocks = (f32.total_rows + 7) / 8 * ((tokens + 7) / 8);
+      const int rc = blocks < ctx->sm_count ? LaunchRowsF32<2>(ctx, f32, tokens) : LaunchRowsF32<8>(ctx, f32, tokens);
       if (rc != GUFO_CUDA_OK || other.nparts == 0) {
         return rc;
       }
@@ -731,6 +734,7 @@ int LaunchGemvGrouped(gufo_cuda_ctx* ctx, const GemvArgs& base, int prologue, fl
   args.groups = base.groups;
   args.x_group_stride = base.x_group_stride;
   args.x_group_div = base.x_group_div;
+  args.early_input = base.early_input;
   args.y_group_stride = base.y_group_stride;
   if (activate) {
     if (!GroupedSwiGluInProduct(ctx, base)) {

@@ -31,6 +31,7 @@ struct GemvArgs {
   int x_group_stride = 0;
   int x_group_div = 1;
   int y_group_stride = 0;
+  int early_input = 0;
 };
 
 // Enqueues, for every group g with group_ids[g] >= 0 (device memory), the

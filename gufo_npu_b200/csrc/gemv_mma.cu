@@ -76,7 +76,8 @@ size_t SharedBytes(int cols) {
          static_cast<size_t>(ONE ? 1 : Slab<TYPE>::kStages) * Slab<TYPE>::kBytes;
 }
 
-template <int TYPE, int TOKENS, int PER_SM, bool ONE = false>
+// GROUPED: the routed experts' products, one token a group (FastGemvArgs).
+template <int TYPE, int TOKENS, int PER_SM, bool ONE = false, bool GROUPED = false>
 __global__ void __launch_bounds__(kFastThreads, PER_SM)
 GemvMma(const __grid_constant__ FastGemvArgs a) {
   using S = Slab<TYPE>;
@@ -126,8 +127,7 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
                                           : (t < 2 ? lane_plane : none);
   const uint8_t* lane_second = t < 2 ? none : lane_plane;
   const int tiles_per_group = TotalTiles(a);
-  const bool grouped = a.group_ids != nullptr;
-  const int row_tiles = grouped ? tiles_per_group * a.groups : tiles_per_group;
+  const int row_tiles = GROUPED ? tiles_per_group * a.groups : tiles_per_group;
   // With ksplit > 1 a cluster of ksplit blocks shares each tile.
   // (No division here: a block's first slabs cannot be requested before these
   // are known, and nothing hides a chain of integer divisions at a kernel's start.
@@ -156,17 +156,26 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   // Grouped launches give a block one tile of its group, or (SwiGLU epilogue) one
   // gate tile and the up tile of the same rows.
   const int units_per_group = a.epilogue == kEpilogueSwiGlu ? tiles_per_group / 2 : tiles_per_group;
-  if (grouped) {
-    GridDependencyWait();   // the ids come from an earlier kernel
-    group = slot / units_per_group;
+  // The ids come from an earlier kernel. Where that one lets this grid start only
+  // after it has itself waited for everything before it (early_input: the router's
+  // top-k), the inputs are complete already, and the image is built while the ids
+  // are still being found. The dependents (the down product) start behind this
+  // wait: they may read the ids and the weights ahead of their own.
+  auto choose = [&]() {
+    GridDependencyWait();
+    GridLaunchDependents();
     const int id = a.group_ids[group];
-    if (id < 0) {
+    matrix = static_cast<size_t>(id);
+    return id >= 0;
+  };
+  if constexpr (GROUPED) {
+    group = slot / units_per_group;
+    if (!a.early_input && !choose()) {
       return;
     }
-    matrix = static_cast<size_t>(id);
   }
   auto locate = [&](int n, int* part, int* local) {
-    LocateTile(a, grouped ? slot - group * units_per_group + (n & 1) * units_per_group : slot + n * stride, part,
+    LocateTile(a, GROUPED ? slot - group * units_per_group + (n & 1) * units_per_group : slot + n * stride, part,
                local);
   };
   __syncthreads();
@@ -234,12 +243,12 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   // before, for the slab kStages - 1 on.
   constexpr bool kEarly = TOKENS == 1;
   constexpr int kAhead = kEarly || ONE ? kStages : kStages - 1;
-  {
-    const int first = min(kAhead, my_slabs);
-    issue_first(first);
-    for (int q = 0; q < first; ++q) {
-      advance();
-    }
+  const int requested = min(kAhead, my_slabs);
+  for (int q = 0; q < requested; ++q) {
+    advance();
+  }
+  if (!GROUPED || !a.early_input) {
+    issue_first(requested);
   }
   if constexpr (S::kZeros) {
     // Read only after the image's barrier below.
@@ -253,9 +262,11 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   float norm_ahead[8];
   LoadNormAhead<TOKENS>(a, norm_ahead);
   const float inv_n = 1.0f / static_cast<float>(a.cols);
-  GridLaunchDependents();
-  // The weights above never depend on earlier kernels; the image and y do.
-  GridDependencyWait();
+  if constexpr (!GROUPED) {
+    GridLaunchDependents();
+    // The weights above never depend on earlier kernels; the image and y do.
+    GridDependencyWait();
+  }
   // Row-split ranks: the input vector may still be on its way from the peers.
   PeerWaitBlock(a.peer_wait);
   if (threadIdx.x == 0) {   // read behind the image's barrier
@@ -273,6 +284,12 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     FillImage<TOKENS>(a, l, smem, S::kExtra,
                       a.x + static_cast<size_t>(group / (a.x_group_div > 1 ? a.x_group_div : 1)) * a.x_group_stride,
                       rank, ks, norm_ahead, squares, inv_n);
+  }
+  if (GROUPED && a.early_input) {
+    if (!choose()) {
+      return;
+    }
+    issue_first(requested);
   }
   // The norm's 1 / rms of the token whose row sums this thread stores.
   const float row_scale = threadIdx.x < kTileFloats ? RowScale<TOKENS>(a, squares, threadIdx.x % TOKENS, inv_n) : 1.f;
@@ -499,11 +516,11 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
 }
 
 // Lets the kernel use all the shared memory a block may have (once per device).
-template <int TYPE, int TOKENS, int PER_SM, bool ONE = false>
+template <int TYPE, int TOKENS, int PER_SM, bool ONE = false, bool GROUPED = false>
 int Configure(const gufo_cuda_ctx* ctx) {
   static bool configured[16] = {};
   if (!configured[ctx->device & 15]) {
-    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemvMma<TYPE, TOKENS, PER_SM, ONE>,
+    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemvMma<TYPE, TOKENS, PER_SM, ONE, GROUPED>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kFastMaxShared));
     configured[ctx->device & 15] = true;
   }
@@ -548,7 +565,7 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
     if (TYPE != GUFO_CUDA_Q4_K) {
       return Fail(GUFO_CUDA_UNSUPPORTED_TYPE, "fast gemv: grouped launches run Q4_K only");
     }
-    if (args.groups <= 0 || args.tokens != 1 || args.prologue == kPrologueImage) {
+    if (args.groups <= 0 || TOKENS != 1 || args.prologue == kPrologueImage || args.prologue == kPrologueResNorm) {
       return Fail(GUFO_CUDA_BAD_ARGUMENT, "fast gemv: a grouped launch takes one token and a fused input");
     }
     launch.ksplit = 1;
@@ -598,11 +615,24 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
       }
     }
   }
+  if constexpr (TYPE == GUFO_CUDA_Q4_K && TOKENS == 1) {
+    if (args.group_ids != nullptr) {
+      const int rc = Configure<TYPE, TOKENS, PER_SM, false, true>(ctx);
+      if (rc != GUFO_CUDA_OK) {
+        return rc;
+      }
+      launch.tiles_each = args.epilogue == kEpilogueSwiGlu ? 2 : 1;
+      launch.tiles_more = 0;
+      GUFO_CUDA_TRY(LaunchOverlapped(GemvMma<TYPE, TOKENS, PER_SM, false, true>, dim3(grid), dim3(kFastThreads), smem,
+                                     ctx->stream, 1, launch));
+      ctx->launches.fetch_add(1);
+      return GUFO_CUDA_OK;
+    }
+  }
   {
     // Tiles per block (ksplit == 1): block b takes tiles b, b + grid, ...
-    const int total = row_tiles * (args.group_ids != nullptr ? args.groups : 1);
-    launch.tiles_each = total / grid;
-    launch.tiles_more = total % grid;
+    launch.tiles_each = row_tiles / grid;
+    launch.tiles_more = row_tiles % grid;
   }
   GUFO_CUDA_TRY(LaunchOverlapped(GemvMma<TYPE, TOKENS, PER_SM>, dim3(grid), dim3(kFastThreads), smem, ctx->stream,
                                  launch.ksplit, launch));

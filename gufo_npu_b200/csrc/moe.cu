@@ -17,94 +17,118 @@ namespace gufo {
 
 namespace {
 
-constexpr int kRouteThreads = 32;
+constexpr int kRouteThreads = 256;
 constexpr int kRouteMaxExperts = 1024;
 // The smallest positive normal fp16: the floor of the top-k probability mass
 // (moe.cpp:12).
 constexpr double kWeightSumFloor = 6.103515625e-5;
 
-// One warp per token; lane l holds experts l, l + 32, ... (PER_LANE of them) in
-// registers. Probabilities are exp(logit - max) in double as in the reference;
-// their sum is a shuffle tree instead of the reference's index-order loop,
-// which can move a weight by the last bit of its fp32 value. The arg-max rounds
-// order (probability, id) exactly as the reference does (moe.cpp:28-32).
+// One block per token. Probabilities are exp(logit - max) in double as in the
+// reference, computed by all threads; warp 0 then holds experts l, l + 32, ...
+// (PER_LANE of them) in lane l. Their sum is a shuffle tree instead of the
+// reference's index-order loop, which can move a weight by the last bit of its fp32
+// value. The arg-max rounds order (probability, id) exactly as the reference does
+// (moe.cpp:28-32): the bits of positive doubles order as integers, so a round is
+// three warp-wide integer reductions (high words, low words, ids) where doubles
+// passed through shuffles took fifteen dependent steps. Bound by latency: an L2
+// round trip, then dependent steps.
+// The dependents may start once the wait has returned: they find every kernel
+// before this one complete (EnqueueMoeFfn relies on it).
 template <int PER_LANE>
 __global__ void __launch_bounds__(kRouteThreads)
 RouteKernel(const float* __restrict__ logits, int stride, int experts, int k,
             int* __restrict__ chosen, float* __restrict__ weights, float* __restrict__ shared_scale) {
-  extern __shared__ double picked[];   // [k]: the chosen probabilities in slot order
-  GridDependencyWait();
+  constexpr int kEach = PER_LANE * 32 / kRouteThreads;
+  extern __shared__ double shared_prob[];   // [experts], then [k] the chosen ones in slot order
+  __shared__ float warp_top[kRouteThreads / 32];
+  double* picked = shared_prob + experts;
   const int token = blockIdx.x;
   const float* row = logits + static_cast<size_t>(token) * stride;
-  const int lane = threadIdx.x;
-  double prob[PER_LANE];
+  const int lane = threadIdx.x & 31;
+  GridDependencyWait();
+  GridLaunchDependents();
+  float v[kEach];
   float top = -FLT_MAX;
 #pragma unroll
-  for (int j = 0; j < PER_LANE; ++j) {
-    const int e = lane + 32 * j;
-    if (e < experts) {
-      top = fmaxf(top, row[e]);
-    }
+  for (int j = 0; j < kEach; ++j) {
+    const int e = threadIdx.x + kRouteThreads * j;
+    v[j] = e < experts ? row[e] : -FLT_MAX;
+    top = fmaxf(top, v[j]);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
   }
+  if (lane == 0) {
+    warp_top[threadIdx.x >> 5] = top;
+  }
+  if (threadIdx.x == kRouteThreads - 32 && shared_scale != nullptr) {
+    shared_scale[token] = static_cast<float>(1.0 / (1.0 + exp(-static_cast<double>(row[experts]))));
+  }
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kRouteThreads / 32; ++w) {
+    top = fmaxf(top, warp_top[w]);
+  }
   const double max_logit = static_cast<double>(top);
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) {
+    const int e = threadIdx.x + kRouteThreads * j;
+    if (e < experts) {
+      shared_prob[e] = exp(static_cast<double>(v[j]) - max_logit);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) {
+    return;
+  }
+  unsigned long long key[PER_LANE];
+  unsigned left = 0;   // which of the lane's entries can still win a round
   double total = 0;
 #pragma unroll
   for (int j = 0; j < PER_LANE; ++j) {
     const int e = lane + 32 * j;
-    // Entries past the end never win a round.
-    prob[j] = e < experts ? exp(static_cast<double>(row[e]) - max_logit) : -1.0;
-    total += e < experts ? prob[j] : 0.0;
+    const double prob = e < experts ? shared_prob[e] : -1.0;
+    total += e < experts ? prob : 0.0;
+    key[j] = static_cast<unsigned long long>(__double_as_longlong(prob));
+    left |= prob >= 0.0 ? 1u << j : 0u;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     total += __shfl_xor_sync(0xFFFFFFFFu, total, o);
   }
-  if (lane == 0 && shared_scale != nullptr) {
-    shared_scale[token] = static_cast<float>(1.0 / (1.0 + exp(-static_cast<double>(row[experts]))));
-  }
-  // k rounds: every lane offers its best remaining entry, the warp keeps the
-  // larger probability and the lower id on ties; the winner drops to -1.
-  double mass = 0;
   for (int slot = 0; slot < k; ++slot) {
-    double best = -2.0;
+    unsigned long long best = 0;
     int at = 0x7FFFFFFF;
 #pragma unroll
     for (int j = 0; j < PER_LANE; ++j) {
       // Ascending j is ascending id, so a strict compare keeps the lower id.
-      if (prob[j] > best) {
-        best = prob[j];
+      if ((left >> j & 1u) != 0 && (at == 0x7FFFFFFF || key[j] > best)) {
+        best = key[j];
         at = lane + 32 * j;
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double other = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-      const int other_at = __shfl_xor_sync(0xFFFFFFFFu, at, o);
-      if (other > best || (other == best && other_at < at)) {
-        best = other;
-        at = other_at;
-      }
-    }
-    if ((at & 31) == lane) {
-#pragma unroll
-      for (int j = 0; j < PER_LANE; ++j) {
-        if (j == (at >> 5)) {
-          prob[j] = -1.0;
-        }
-      }
+    const unsigned high = static_cast<unsigned>(best >> 32), low = static_cast<unsigned>(best);
+    const unsigned top_high = __reduce_max_sync(0xFFFFFFFFu, high);
+    const unsigned top_low = __reduce_max_sync(0xFFFFFFFFu, high == top_high ? low : 0u);
+    const int winner = __reduce_min_sync(0xFFFFFFFFu, high == top_high && low == top_low ? at : 0x7FFFFFFF);
+    if (winner == at && at != 0x7FFFFFFF) {
+      left &= ~(1u << (at >> 5));
     }
     if (lane == 0) {
-      picked[slot] = best;
-      chosen[static_cast<size_t>(token) * k + slot] = at;
+      picked[slot] = __longlong_as_double(static_cast<long long>(static_cast<unsigned long long>(top_high) << 32 | top_low));
+      chosen[static_cast<size_t>(token) * k + slot] = winner;
     }
-    // The slot-order sum of the chosen probabilities (moe.cpp:33-36).
-    mass += best / total;
   }
   __syncwarp();
+  // The slot-order sum of the chosen probabilities (moe.cpp:33-36).
+  double mass = 0;
+  for (int first = 0; first < k; first += 32) {
+    const double mine = first + lane < k ? picked[first + lane] / total : 0.0;
+    for (int s = 0; s < 32 && first + s < k; ++s) {
+      mass += __shfl_sync(0xFFFFFFFFu, mine, s);
+    }
+  }
   mass = mass > kWeightSumFloor ? mass : kWeightSumFloor;
   for (int slot = lane; slot < k; slot += 32) {
     weights[static_cast<size_t>(token) * k + slot] = static_cast<float>(picked[slot] / total / mass);
@@ -139,7 +163,7 @@ int EnqueueRoute(gufo_cuda_ctx* ctx, const float* logits, int stride, int tokens
   if (tokens <= 0 || experts <= 0 || k <= 0 || k > experts || experts > kRouteMaxExperts || stride < experts) {
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "route: 1 <= k <= experts <= 1024, stride >= experts");
   }
-  const size_t smem = static_cast<size_t>(k) * sizeof(double);
+  const size_t smem = static_cast<size_t>(experts + k) * sizeof(double);
   if (experts <= 256) {
     GUFO_CUDA_TRY(LaunchOverlapped(RouteKernel<8>, dim3(tokens), dim3(kRouteThreads), smem, ctx->stream, 1, logits,
                                    stride, experts, k, chosen, weights, shared_scale));
@@ -148,6 +172,8 @@ int EnqueueRoute(gufo_cuda_ctx* ctx, const float* logits, int stride, int tokens
                                    stride, experts, k, chosen, weights, shared_scale));
   }
   ctx->launches.fetch_add(1);
+  ctx->route_launch = LaunchCount().load();
+  ctx->route_stream = ctx->stream;
   return GUFO_CUDA_OK;
 }
 
@@ -387,7 +413,6 @@ NarrowCombineQ4K(const __grid_constant__ NarrowCombineArgs a) {
   constexpr int kCols = 256 * BLOCKS;
   __shared__ __align__(16) float xs[kCombineSlots][kCols];
   GridLaunchDependents();
-  GridDependencyWait();
   const int token = blockIdx.y;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -406,7 +431,8 @@ NarrowCombineQ4K(const __grid_constant__ NarrowCombineArgs a) {
     pair[j] = c;
     col[j] = 256 * b + 64 * c + 8 * p;
   }
-  // The k rows first (they come from HBM), then the inputs.
+  // The k rows first, ahead of the wait: the gate / up product lets this grid start
+  // only once the ids are complete, and the rows come from HBM.
   uint4 head[kCombineSlots][kPer];
   uint2 codes[kCombineSlots][kPer];
   int id[kCombineSlots];
@@ -422,6 +448,7 @@ NarrowCombineQ4K(const __grid_constant__ NarrowCombineArgs a) {
       }
     }
   }
+  GridDependencyWait();
   for (int i = threadIdx.x * 4; i < a.k * kCols; i += 256 * 4) {
     const int s = i / kCols;
     *reinterpret_cast<float4*>(&xs[s][i - s * kCols]) =
@@ -564,7 +591,11 @@ int EnqueueMoeFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids, co
   const int blocks = down.cols / kSuperBlock;
   if (k <= kCombineSlots && NarrowFits(down) && blocks <= 2 && GroupedSwiGluInProduct(ctx, in)) {
     // Two launches: gate / up with the SwiGLU in its epilogue, then the down rows
-    // of a token's experts with the weighted sum.
+    // of a token's experts with the weighted sum. Directly behind the router's top-k
+    // (nothing else has been launched since, from any context) the inputs are
+    // complete once the first of them runs; its image is built while the top-k is
+    // being found.
+    in.early_input = ctx->route_launch == LaunchCount().load() && ctx->route_stream == ctx->stream ? 1 : 0;
     const int rc = LaunchGemvGrouped(ctx, in, kProloguePlain, nullptr, true);
     if (rc != GUFO_CUDA_OK) {
       return rc;

@@ -226,3 +226,26 @@ def test_step_logits_in_any_memory(ctx, vocab):
         assert rel_l2(got[0], want[i]) <= 5e-4
         dec.Resolve(False)
     dec.close()
+
+
+@pytest.mark.parametrize("experts,k", [(8, 8), (33, 4), (256, 8), (257, 3), (1024, 40)])
+def test_route_ties_and_counts(ctx, oracle, experts, k):
+    """Expert counts off the warp and block widths, equal logits among the best, more slots than lanes."""
+    dev = torch.device("cuda:0")
+    tokens = 3
+    logits = G.normal(31 + experts, tokens, experts + 1).astype(np.float32)
+    logits[1, : experts // 2] = 2.5          # ties: the lower id first
+    logits[2, experts // 3] = 1e4            # every other probability underflows
+    x = torch.from_numpy(logits).to(dev)
+    chosen = torch.empty(tokens, k, dtype=torch.int32, device=dev)
+    weights = torch.empty(tokens, k, device=dev)
+    scale = torch.empty(tokens, device=dev)
+    torch.cuda.synchronize()
+    ctx.route_device(x, experts + 1, tokens, experts, k, chosen, weights, scale)
+    ctx.synchronize()
+    for t in range(tokens):
+        p = np.exp(logits[t, :experts].astype(np.float64) - float(logits[t, :experts].max()))
+        order = np.lexsort((np.arange(experts), -p))[:k]
+        assert chosen[t].cpu().numpy().tolist() == order.tolist()
+        picked = p[order] / p.sum()
+        assert rel_l2(weights[t].cpu().numpy(), picked / max(picked.sum(), 6.103515625e-5)) <= 1e-6
