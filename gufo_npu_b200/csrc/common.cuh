@@ -284,6 +284,9 @@ struct gufo_cuda_ctx {
   // The gate dots of a DeltaNet step of several sequences.
   uint8_t* gates = nullptr;
   size_t gates_bytes = 0;
+  // Attention: arrival counters (zero between launches), then partial sums.
+  uint8_t* attn = nullptr;
+  size_t attn_bytes = 0;
   // Fixed-point image of the activations of the product in flight.
   uint8_t* image = nullptr;
   size_t image_bytes = 0;

@@ -440,6 +440,7 @@ int gufo_cuda_ctx_destroy(gufo_cuda_ctx* ctx) {
   cudaFree(ctx->stage_x);
   cudaFree(ctx->stage_y);
   ctx->retired.emplace_back(ctx->gates, ctx->gates_bytes);
+  ctx->retired.emplace_back(ctx->attn, ctx->attn_bytes);
   ctx->retired.emplace_back(ctx->image, ctx->image_bytes);
   ctx->retired.emplace_back(ctx->tc_scratch, ctx->tc_scratch_bytes);
   for (const auto& block : ctx->retired) {

@@ -50,6 +50,11 @@ struct AttnArgs {
   int offset = 0;           // the token sits at *position + offset
 };
 
+// The one-launch attention kernel (attention.cu): whether it runs a shape, and its
+// launch. The caller holds ctx->mu.
+bool AttentionFits(const AttnArgs& a);
+int LaunchAttention(gufo_cuda_ctx* ctx, const AttnArgs& a);
+
 // Shared memory of one team running the attention bodies.
 struct AttnScratch {
   float reduce[kTeamWarps];

@@ -157,7 +157,11 @@ int Upload(gufo_cuda_ctx* ctx, const T* host, size_t n, T** dev) {
   return GUFO_CUDA_OK;
 }
 
+// Other head dimensions (and the cross-check of the one-launch kernel): three launches.
 int EnqueueAttention(gufo_cuda_ctx* ctx, const AttnArgs& a) {
+  if (!ctx->force_general && AttentionFits(a)) {
+    return LaunchAttention(ctx, a);
+  }
   const dim3 block(kSmallThreads);
   GUFO_CUDA_TRY(LaunchOverlapped(AttnPrepKernel, dim3(a.heads + a.kv_heads), block, 0, ctx->stream, 1, a));
   GUFO_CUDA_TRY(LaunchOverlapped(AttnSliceKernel, dim3(kAttnSplits, a.kv_heads), block, 0, ctx->stream, 1, a));

@@ -249,3 +249,59 @@ def test_route_ties_and_counts(ctx, oracle, experts, k):
         assert chosen[t].cpu().numpy().tolist() == order.tolist()
         picked = p[order] / p.sum()
         assert rel_l2(weights[t].cpu().numpy(), picked / max(picked.sum(), 6.103515625e-5)) <= 1e-6
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,rope_dim", [(8, 1, 64, 64), (3, 3, 128, 32), (16, 4, 256, 64),
+                                                              (2, 1, 256, 0), (5, 1, 128, 128)])
+@pytest.mark.parametrize("positions", [1, 2, 17, 64, 65, 128, 129, 193, 1000, 4099, 9001])
+def test_attention_chunks_and_splits(ctx, heads, kv_heads, head_dim, rope_dim, positions):
+    """Lengths around a chunk, around what one block takes and with a ragged last slice, in float64;
+    a later call finds the arrival counters as it needs them."""
+    import ctypes as C
+    from gufo_npu_b200 import _capi
+    dev = torch.device("cuda:0")
+    hd, group, pos = head_dim, heads // kv_heads, positions - 1
+    gen = torch.Generator(device=dev).manual_seed(positions)
+
+    def rand(*shape):
+        return torch.randn(*shape, device=dev, generator=gen)
+    keys, values = rand(positions + 3, kv_heads * hd).half(), rand(positions + 3, kv_heads * hd).half()
+    row, wq, wk = rand(2 * heads * hd + 2 * kv_heads * hd), 1 + 0.1 * rand(hd), 1 + 0.1 * rand(hd)
+    row[:2 * hd] *= 1e-3   # a head far smaller than the others
+    freq = (1.0 / 1e4 ** (2.0 * torch.arange(max(rope_dim // 2, 1), device=dev, dtype=torch.float64) / max(rope_dim, 1))).float()
+    position = torch.tensor([pos], dtype=torch.int32, device=dev)
+    queries, partials = torch.empty(heads * hd, device=dev), torch.empty(kv_heads * 32 * group * (hd + 2), device=dev)
+    out = torch.empty(heads * hd, device=dev)
+    args = _capi.AttentionArgs(heads, kv_heads, hd, rope_dim, positions + 3, 1e-6,
+                               *[t.data_ptr() for t in (position, row, wq, wk, freq, keys, values, queries, partials, out)])
+    torch.cuda.synchronize()
+    for _ in range(2):
+        out.zero_()
+        torch.cuda.synchronize()
+        ctx._check(ctx.lib.gufo_cuda_attention_device(ctx.handle, C.byref(args)))
+        ctx.synchronize()
+
+    def head(x, w):
+        x = x.double()
+        x = x / torch.sqrt((x * x).mean() + 1e-6) * w.double()
+        half = rope_dim // 2
+        if half:
+            angle = pos * freq[:half].double()
+            lo, hi = x[:half].clone(), x[half:2 * half].clone()
+            x[:half] = lo * torch.cos(angle) - hi * torch.sin(angle)
+            x[half:2 * half] = lo * torch.sin(angle) + hi * torch.cos(angle)
+        return x
+    q_gate = row[:2 * heads * hd].reshape(heads, 2, hd)
+    k_new = row[2 * heads * hd:][:kv_heads * hd].reshape(kv_heads, hd)
+    v_new = row[2 * heads * hd + kv_heads * hd:].reshape(kv_heads, hd)
+    K, V = keys.double().reshape(-1, kv_heads, hd), values.double().reshape(-1, kv_heads, hd)
+    want = torch.empty(heads, hd, dtype=torch.float64, device=dev)
+    for h in range(heads):
+        kh = h // group
+        assert (K[pos, kh] - head(k_new[kh], wk)).abs().max() <= 2e-3 * K[pos, kh].abs().max()
+        assert torch.equal(V[pos, kh], v_new[kh].half().double())
+        p = torch.softmax(K[:positions, kh] @ head(q_gate[h, 0], wq) / hd ** 0.5, 0)
+        want[h] = (p @ V[:positions, kh]) * torch.sigmoid(q_gate[h, 1].double())
+    assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 2e-6
+    for h in range(heads):
+        assert rel_l2(out.reshape(heads, hd)[h].cpu().numpy(), want[h].cpu().numpy()) <= 5e-6, h
