@@ -155,7 +155,8 @@ struct FastGemvArgs {
   // memory. Set by the launcher for matrices with few rows.
   int ksplit;
   int tiles_each;         // set by the launcher: with ksplit == 1 block b multiplies tiles_each tiles,
-  int tiles_more;         //   one more if b < tiles_more
+  int tiles_more;         //   one more if b < tiles_more (gemv_units.cu, kEpilogueSwiGlu: two more)
+  int depth;              // set by the launcher: units in a warp's ring (gemv_units.cu)
   // Grouped launches (the routed experts of a MoE layer): the parts are stacks
   // of `rows`-row matrices, group g multiplies matrix group_ids[g] of every
   // part (a negative id skips the group) with its own input and output. The
@@ -215,9 +216,11 @@ namespace gufo {
 void* DeviceAddress(const void* host);
 // Enqueues one Q4_K part on the int8 tensor-core kernel against a staged image.
 int LaunchGemvQ4KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
+// The launch of gemv_units.cu, and whether its shared memory holds `tokens` rows.
+int LaunchGemvUnits(gufo_cuda_ctx* ctx, int type, const FastGemvArgs& args);
+bool UnitsFit(int type, int cols, int tokens);
 // Whether the image of `tokens` rows of `cols` values fits in shared memory.
 bool Q4KFastFits(int cols, int tokens);
-bool FastSwiGluPairsFit(const gufo_cuda_ctx* ctx, int type, int cols, int tokens, int pairs);
 // The F32 alpha / beta rows of a DeltaNet layer's input product, for a step
 // that computes the two gates inside the mixer kernel instead of reading them
 // from the product's output: a = alpha_w[head] . x, b = beta_w[head] . x.
@@ -396,14 +399,16 @@ int ResidentBlocks(Kernel kernel, int device, int threads, size_t smem, int clus
     int device;
     size_t smem;
     int cluster;
+    Kernel kernel;
     int blocks;
   };
-  static Entry cache[32];
+  static Entry cache[256];
   static int cached = 0;
   static std::mutex mutex;
   std::lock_guard<std::mutex> lock(mutex);
   for (int i = 0; i < cached; ++i) {
-    if (cache[i].device == device && cache[i].smem == smem && cache[i].cluster == cluster_x) {
+    if (cache[i].device == device && cache[i].smem == smem && cache[i].cluster == cluster_x &&
+        cache[i].kernel == kernel) {
       return cache[i].blocks;
     }
   }
@@ -435,31 +440,10 @@ int ResidentBlocks(Kernel kernel, int device, int threads, size_t smem, int clus
     }
     blocks = per_sm * sms;
   }
-  if (cached < 32) {
-    cache[cached++] = Entry{device, smem, cluster_x, blocks};
+  if (cached < 256) {
+    cache[cached++] = Entry{device, smem, cluster_x, kernel, blocks};
   }
   return blocks;
-}
-
-// Picks how many blocks share a tile's slabs (1, 2, 3 or 4: the largest that
-// still lets every tile run at once) and the grid for it.
-template <typename Kernel>
-void PlanFastGrid(Kernel kernel, int device, int threads, size_t smem, int row_tiles, int slabs,
-                  int* ksplit, int* grid) {
-  for (int ks = slabs < 4 ? slabs : 4; ks >= 2; --ks) {
-    const int resident = ResidentBlocks(kernel, device, threads, smem, ks);
-    if (row_tiles * ks <= resident) {
-      *ksplit = ks;
-      *grid = row_tiles * ks;
-      return;
-    }
-  }
-  int resident = ResidentBlocks(kernel, device, threads, smem, 1);
-  if (resident <= 0) {
-    resident = 1;
-  }
-  *ksplit = 1;
-  *grid = row_tiles < resident ? row_tiles : resident;
 }
 
 // ---- device helpers ------------------------------------------------------

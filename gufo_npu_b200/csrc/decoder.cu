@@ -562,12 +562,12 @@ int FusedProduct(gufo_cuda_decoder* d, const GemvArgs& stage, const Input& in, f
 }
 
 // Whether the gate / up product `stage` can leave silu(gate) * up by itself for
-// `tokens` rows: two parts of one tensor-core format with equal whole tiles, and
-// a resident thread block for every tile pair.
+// `tokens` rows: two parts of one tensor-core format with equal whole tiles.
 bool SwiGluInProduct(const gufo_cuda_ctx* ctx, const GemvArgs& stage, int tokens) {
   return !ctx->force_general && stage.nparts == 2 && stage.parts[0].rows == stage.parts[1].rows &&
          stage.parts[0].rows % 16 == 0 && stage.parts[0].type == stage.parts[1].type &&
-         FastSwiGluPairsFit(ctx, stage.parts[0].type, stage.cols, tokens, static_cast<int>(stage.parts[0].rows / 16));
+         ((stage.parts[0].type == GUFO_CUDA_Q4_K && Q4KFastFits(stage.cols, tokens)) ||
+          (stage.parts[0].type == GUFO_CUDA_Q6_K && Q6KFastFits(stage.cols, tokens)));
 }
 
 // Records an event that closes a stage of kind `kind` (timeline mode only).

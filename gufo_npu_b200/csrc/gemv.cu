@@ -569,8 +569,25 @@ int LaunchGemv(gufo_cuda_ctx* ctx, const GemvArgs& base, int tokens) {
       return LaunchGemv(ctx, other, tokens);
     }
   }
-  for (int t0 = 0; t0 < tokens; t0 += kMaxTokens) {
-    const int m = tokens - t0 < kMaxTokens ? tokens - t0 : kMaxTokens;
+  // Tokens per pass: as many as the images of the tensor-core kernels hold (eight rows
+  // of 9728 values do not fit, four do: two passes, 33 us at 2560 rows of Q6_K, instead
+  // of the general kernel's one, 87 us).
+  int most = kMaxTokens;
+  for (int p = 0; p < base.nparts && !ctx->force_general; ++p) {
+    const int type = base.parts[p].type;
+    if (type == GUFO_CUDA_Q4_K || type == GUFO_CUDA_Q6_K) {
+      auto* fits = type == GUFO_CUDA_Q4_K ? Q4KFastFits : Q6KFastFits;
+      while (fits(base.cols, 1) && !fits(base.cols, most)) {
+        --most;
+      }
+    }
+  }
+  if (most < tokens) {
+    const int passes = (tokens + most - 1) / most;
+    most = (tokens + passes - 1) / passes;   // of one size
+  }
+  for (int t0 = 0; t0 < tokens; t0 += most) {
+    const int m = tokens - t0 < most ? tokens - t0 : most;
     const float* x = base.x + static_cast<size_t>(t0) * base.cols;
     float* y = base.y + static_cast<size_t>(t0) * base.y_stride;
     GemvArgs rest = base;

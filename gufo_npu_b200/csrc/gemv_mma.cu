@@ -1,4 +1,4 @@
-// Q4_K and Q6_K GEMV / small-M GEMM (1..8 tokens) on the int8 tensor-core
+// Q4_K and Q6_K GEMV (one token; more in gemv_units.cu) on the int8 tensor-core
 // path: the reference's fused row dots (gguf_dot::DotK4 and DotQ6_K,
 // src/models/qwen35/gguf_dot.hpp:115-188,203-290) with the code dots taken
 // exactly by mma.sync (arithmetic in mma_common.cuh, the per-unit math and the
@@ -527,25 +527,35 @@ int Configure(const gufo_cuda_ctx* ctx) {
   return GUFO_CUDA_OK;
 }
 
-// One token needs few enough registers for three resident blocks per SM.
-template <int TOKENS>
-constexpr int PerSm() { return TOKENS == 1 ? 3 : 2; }
-
-// Whether `pairs` (gate tile, up tile) pairs each get a resident block.
-template <int TYPE, int TOKENS>
-bool PairsFit(const gufo_cuda_ctx* ctx, int cols, int pairs) {
-  const size_t smem = SharedBytes<TYPE, TOKENS>(cols);
-  if (smem > static_cast<size_t>(kFastMaxShared) || Configure<TYPE, TOKENS, PerSm<TOKENS>()>(ctx) != GUFO_CUDA_OK) {
-    return false;
+// Picks how many blocks share a tile's slabs (1, 2, 3 or 4: the largest that
+// still lets every tile run at once) and the grid for it.
+template <typename Kernel>
+void PlanFastGrid(Kernel kernel, int device, int threads, size_t smem, int row_tiles, int slabs,
+                  int* ksplit, int* grid) {
+  for (int ks = slabs < 4 ? slabs : 4; ks >= 2; --ks) {
+    const int resident = ResidentBlocks(kernel, device, threads, smem, ks);
+    if (row_tiles * ks <= resident) {
+      *ksplit = ks;
+      *grid = row_tiles * ks;
+      return;
+    }
   }
-  return pairs <= ResidentBlocks(GemvMma<TYPE, TOKENS, PerSm<TOKENS>()>, ctx->device, kFastThreads, smem, 1);
+  int resident = ResidentBlocks(kernel, device, threads, smem, 1);
+  if (resident <= 0) {
+    resident = 1;
+  }
+  *ksplit = 1;
+  *grid = row_tiles < resident ? row_tiles : resident;
 }
+
+// LaunchVariant leaves the launch to gemv_units.cu.
+constexpr int kNotTaken = -1;
 
 template <int TYPE, int TOKENS, int PER_SM>
 int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
   const size_t smem = SharedBytes<TYPE, TOKENS>(args.cols);
   if (smem > static_cast<size_t>(kFastMaxShared)) {
-    return GUFO_CUDA_TOO_LARGE;
+    return kNotTaken;
   }
   {
     const int rc = Configure<TYPE, TOKENS, PER_SM>(ctx);
@@ -585,13 +595,16 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
     launch.ksplit = 1;
     grid = row_tiles / 2;
     if (grid > ResidentBlocks(GemvMma<TYPE, TOKENS, PER_SM>, ctx->device, kFastThreads, smem, 1)) {
-      return GUFO_CUDA_TOO_LARGE;   // more tile pairs than resident blocks: the caller activates by itself
+      return kNotTaken;   // more tile pairs than resident blocks
     }
   } else {
     // Few rows and several slabs per tile: split the tiles' slabs over a cluster.
     PlanFastGrid(GemvMma<TYPE, TOKENS, PER_SM>, ctx->device, kFastThreads, smem, row_tiles, slabs, &launch.ksplit,
                  &grid);
-    if constexpr (TOKENS <= 2) {
+    if (launch.ksplit == 1 && slabs > 1 && args.cols % (8 * kSuperBlock) != 0) {
+      return kNotTaken;
+    }
+    {
       // Rows of two to four slabs whose (tile, slab) pairs do not all get a block
       // above: the one-slab form is smaller and may hold them (a 2048 x 6144 Q6_K
       // product: clusters of three blocks with one slab each instead of two blocks
@@ -640,68 +653,20 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
   return GUFO_CUDA_OK;
 }
 
-template <int TYPE, int TOKENS>
-int Launch(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
-  return LaunchVariant<TYPE, TOKENS, PerSm<TOKENS>()>(ctx, args);
-}
-
-template <int TYPE>
-bool Fits(int cols, int tokens) {
-  switch (tokens) {
-    case 1: return SharedBytes<TYPE, 1>(cols) <= static_cast<size_t>(kFastMaxShared);
-    case 2: return SharedBytes<TYPE, 2>(cols) <= static_cast<size_t>(kFastMaxShared);
-    case 3: return SharedBytes<TYPE, 3>(cols) <= static_cast<size_t>(kFastMaxShared);
-    case 4: return SharedBytes<TYPE, 4>(cols) <= static_cast<size_t>(kFastMaxShared);
-    case 5: return SharedBytes<TYPE, 5>(cols) <= static_cast<size_t>(kFastMaxShared);
-    case 6: return SharedBytes<TYPE, 6>(cols) <= static_cast<size_t>(kFastMaxShared);
-    case 7: return SharedBytes<TYPE, 7>(cols) <= static_cast<size_t>(kFastMaxShared);
-    case 8: return SharedBytes<TYPE, 8>(cols) <= static_cast<size_t>(kFastMaxShared);
-    default: return false;
-  }
-}
-
+// One token runs here, but for launches of several slabs a row of which the last is
+// ragged and which no cluster shares; the rest in gemv_units.cu (the figures that draw
+// the line stand there).
 template <int TYPE>
 int LaunchTokens(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
-  switch (args.tokens) {
-    case 1: return Launch<TYPE, 1>(ctx, args);
-    case 2: return Launch<TYPE, 2>(ctx, args);
-    case 3: return Launch<TYPE, 3>(ctx, args);
-    case 4: return Launch<TYPE, 4>(ctx, args);
-    case 5: return Launch<TYPE, 5>(ctx, args);
-    case 6: return Launch<TYPE, 6>(ctx, args);
-    case 7: return Launch<TYPE, 7>(ctx, args);
-    case 8: return Launch<TYPE, 8>(ctx, args);
-    default: return Fail(GUFO_CUDA_BAD_ARGUMENT, "fast gemv: 1 to 8 tokens per launch");
-  }
-}
-
-template <int TYPE>
-bool PairsFitTokens(const gufo_cuda_ctx* ctx, int cols, int tokens, int pairs) {
-  switch (tokens) {
-    case 1: return PairsFit<TYPE, 1>(ctx, cols, pairs);
-    case 2: return PairsFit<TYPE, 2>(ctx, cols, pairs);
-    case 3: return PairsFit<TYPE, 3>(ctx, cols, pairs);
-    case 4: return PairsFit<TYPE, 4>(ctx, cols, pairs);
-    case 5: return PairsFit<TYPE, 5>(ctx, cols, pairs);
-    case 6: return PairsFit<TYPE, 6>(ctx, cols, pairs);
-    case 7: return PairsFit<TYPE, 7>(ctx, cols, pairs);
-    case 8: return PairsFit<TYPE, 8>(ctx, cols, pairs);
-    default: return false;
-  }
+  const int rc = args.tokens == 1 ? LaunchVariant<TYPE, 1, 3>(ctx, args) : kNotTaken;   // three blocks per SM
+  return rc == kNotTaken ? LaunchGemvUnits(ctx, TYPE, args) : rc;
 }
 
 }  // namespace
 
-// Whether a launch with the SwiGLU epilogue can give each of `pairs` tile pairs
-// (rows of one part / 16) a resident thread block.
-bool FastSwiGluPairsFit(const gufo_cuda_ctx* ctx, int type, int cols, int tokens, int pairs) {
-  return type == GUFO_CUDA_Q4_K ? PairsFitTokens<GUFO_CUDA_Q4_K>(ctx, cols, tokens, pairs)
-                                : type == GUFO_CUDA_Q6_K && PairsFitTokens<GUFO_CUDA_Q6_K>(ctx, cols, tokens, pairs);
-}
-
 // Whether `tokens` rows of `cols` values fit the shared-memory image.
-bool Q4KFastFits(int cols, int tokens) { return Fits<GUFO_CUDA_Q4_K>(cols, tokens); }
-bool Q6KFastFits(int cols, int tokens) { return Fits<GUFO_CUDA_Q6_K>(cols, tokens); }
+bool Q4KFastFits(int cols, int tokens) { return UnitsFit(GUFO_CUDA_Q4_K, cols, tokens); }
+bool Q6KFastFits(int cols, int tokens) { return UnitsFit(GUFO_CUDA_Q6_K, cols, tokens); }
 
 // Enqueues the Q4_K / Q6_K parts of one launch (a staged image or a fused input).
 int LaunchGemvQ4KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args) { return LaunchTokens<GUFO_CUDA_Q4_K>(ctx, args); }

@@ -30,11 +30,8 @@ struct Q4KUnit {
   uint2 code[8];   // index 2 * pair + (0: row g, 1: row g + 8)
 };
 
-// Reads this lane's fragments of block `block` of a slab in shared memory.
-__device__ __forceinline__ void LoadUnit(Q4KUnit& u, const uint8_t* slab, int block,
-                                         int g, int t) {
-  const uint8_t* b0 = slab + g * kSlabRowBytes + block * kQ4KBytes;
-  const uint8_t* b1 = b0 + 8 * kSlabRowBytes;
+// Reads this lane's fragments: b0 and b1 are the block's bytes of rows g and g + 8.
+__device__ __forceinline__ void LoadFragments(Q4KUnit& u, const uint8_t* b0, const uint8_t* b1, int t) {
   u.head[0] = *reinterpret_cast<const uint4*>(b0);
   u.head[1] = *reinterpret_cast<const uint4*>(b1);
 #pragma unroll
@@ -42,6 +39,13 @@ __device__ __forceinline__ void LoadUnit(Q4KUnit& u, const uint8_t* slab, int bl
     u.code[2 * p] = *reinterpret_cast<const uint2*>(b0 + 16 + 32 * p + 8 * t);
     u.code[2 * p + 1] = *reinterpret_cast<const uint2*>(b1 + 16 + 32 * p + 8 * t);
   }
+}
+
+// The same from block `block` of a slab in shared memory.
+__device__ __forceinline__ void LoadUnit(Q4KUnit& u, const uint8_t* slab, int block,
+                                         int g, int t) {
+  const uint8_t* b0 = slab + g * kSlabRowBytes + block * kQ4KBytes;
+  LoadFragments(u, b0, b0 + 8 * kSlabRowBytes, t);
 }
 
 // The eight 6-bit scales and mins of a block as bytes of two words each

@@ -34,6 +34,23 @@ struct Q6KUnit {
   uint32_t d[2];       // [row]: fp16 bits
 };
 
+// Reads this lane's fragments of a unit that lies by itself: row0 and row1 are rows g
+// and g + 8, each ql | qh | scales | the d of its slab's blocks, of which it is the jth.
+__device__ __forceinline__ void LoadFragments(Q6KUnit& u, const uint8_t* row0, const uint8_t* row1, int j, int t) {
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const uint8_t* row = r == 0 ? row0 : row1;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      u.ql[r][half][0] = *reinterpret_cast<const uint2*>(row + 8 * t + 64 * half);
+      u.ql[r][half][1] = *reinterpret_cast<const uint2*>(row + 8 * t + 64 * half + 32);
+      u.qh[r][half] = *reinterpret_cast<const uint2*>(row + 128 + 8 * t + 32 * half);
+    }
+    u.sc[r] = *reinterpret_cast<const uint4*>(row + 192);
+    u.d[r] = *reinterpret_cast<const uint16_t*>(row + 208 + 2 * j);
+  }
+}
+
 // Reads this lane's fragments of block `j` of a slab of `n` blocks.
 __device__ __forceinline__ void LoadUnit(Q6KUnit& u, const uint8_t* slab, int j, int n,
                                          int g, int t) {

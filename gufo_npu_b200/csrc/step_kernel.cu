@@ -53,9 +53,6 @@ struct TeamSync {
   __device__ __forceinline__ void operator()() const { NamedSync(id, kTeamThreads); }
 };
 
-__device__ __forceinline__ void MbarArrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ unsigned LoadAcquireGpu(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -305,3 +305,37 @@ def test_attention_chunks_and_splits(ctx, heads, kv_heads, head_dim, rope_dim, p
     assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 2e-6
     for h in range(heads):
         assert rel_l2(out.reshape(heads, hd)[h].cpu().numpy(), want[h].cpu().numpy()) <= 5e-6, h
+
+
+@pytest.mark.parametrize("ggml_type", [Q.GGML_Q4_K, Q.GGML_Q6_K])
+@pytest.mark.parametrize("tokens,rows,cols", [
+    (1, 20000, 2560), (2, 33, 256), (2, 20011, 768), (3, 16, 9728), (5, 9001, 2304), (8, 40, 2816), (8, 1500, 9728),
+    (4, 12000, 512), (7, 2560, 4096),
+])
+def test_units_of_ragged_rows(ctx, ggml_type, tokens, rows, cols):
+    """Fewer blocks a row than warps, rounds that end inside a tile, rows off the tile, several tiles
+    a thread block, clusters, and more tokens than fit one pass."""
+    m, w = _matrix(ctx, ggml_type, rows, cols, 20 + cols % 13)
+    x = G.normal(21 + tokens, tokens, cols)
+    got = ctx.matmul([(m, 0, rows)], x, tokens, rows)
+    want = x.astype(np.float64) @ w.T
+    assert rel_l2(got, want) <= 2e-6
+    for t in range(tokens):
+        assert rel_l2(got[t], want[t]) <= 4e-6, t
+    ctx.matrix_free(m)
+
+
+@pytest.mark.parametrize("tokens,rows,cols", [(1, 9728, 2560), (2, 9728, 2560), (2, 16, 512), (2, 6144, 2048)])
+def test_activating_product_with_more_tile_pairs_than_blocks(ctx, tokens, rows, cols):
+    dev = torch.device("cuda:0")
+    (mg, wg), (mu, wu) = (_matrix(ctx, Q.GGML_Q4_K, rows, cols, s) for s in (14, 15))
+    x = torch.from_numpy(G.normal(16, tokens, cols).astype(np.float32)).to(dev)
+    act = torch.empty(tokens, rows, device=dev)
+    torch.cuda.synchronize()
+    ctx.matmul_fused_device(Context._parts([(mg, 0, rows), (mu, 0, rows)]), 2, tokens, act, x=x, activate=True)
+    ctx.synchronize()
+    x64 = x.cpu().numpy().astype(np.float64)
+    g, u = x64 @ wg.T, x64 @ wu.T
+    assert rel_l2(act.cpu().numpy(), g / (1.0 + np.exp(-g)) * u) <= 5e-6
+    ctx.matrix_free(mg)
+    ctx.matrix_free(mu)
