@@ -356,9 +356,11 @@ int gufo_cuda_ctx_create(int device, void* stream, gufo_cuda_ctx** out) {
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "ctx_create: no such device");
   }
   GUFO_CUDA_TRY(cudaSetDevice(device));
-  cudaDeviceProp prop;
-  GUFO_CUDA_TRY(cudaGetDeviceProperties(&prop, device));
-  if (prop.major != 10) {
+  // Single attributes: cudaGetDeviceProperties asks the driver for all of them, 2.5 ms.
+  int major = 0, sm_count = 0;
+  GUFO_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+  GUFO_CUDA_TRY(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+  if (major != 10) {
     return Fail(GUFO_CUDA_RUNTIME,
                 "device is not sm_100: the kernels are built for sm_100a only");
   }
@@ -367,7 +369,7 @@ int gufo_cuda_ctx_create(int device, void* stream, gufo_cuda_ctx** out) {
     return Fail(GUFO_CUDA_OUT_OF_MEMORY, "ctx_create: host allocation failed");
   }
   ctx->device = device;
-  ctx->sm_count = prop.multiProcessorCount;
+  ctx->sm_count = sm_count;
   if (stream != nullptr) {
     ctx->stream = static_cast<cudaStream_t>(stream);
   } else {
