@@ -163,9 +163,20 @@ struct FastGemvArgs {
   // ids live on the device, so a router kernel can feed the launch directly.
   const int* group_ids;   // null: one ungrouped product
   int groups;
+  int group_blocks;       // set by the launcher: thread blocks per group
   int x_group_stride;     // floats between the inputs (0: shared)
   int x_group_div;        // groups per input: group g reads input g / x_group_div (0 counts as 1)
   int early_input;        // the inputs are complete as soon as this grid runs, ahead of its dependency wait
+  // A mixture (LaunchGemvMixture): the rows of `mix_experts` matrices of parts[0] side
+  // by side, `mix_blocks` 256-value blocks of each, `groups` inputs; input g uses the
+  // matrices mix_ids[g][..] (< 0: none), its values times mix_weights[g][..], and
+  // adds mix_base[g] (rows values) times mix_scale[g].
+  const int* mix_ids;
+  const float* mix_weights;
+  int mix_experts;
+  int mix_blocks;
+  const float* mix_base;
+  const float* mix_scale;
   // Timing experiments (context option "gemv_variant"; wrong results): 1 skips
   // the multiplies and leaves only the data movement.
   int variant;
@@ -218,6 +229,12 @@ void* DeviceAddress(const void* host);
 int LaunchGemvQ4KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
 // The launch of gemv_units.cu, and whether its shared memory holds `tokens` rows.
 int LaunchGemvUnits(gufo_cuda_ctx* ctx, int type, const FastGemvArgs& args);
+// y[g] = mix_base[g] * mix_scale[g] + the weighted sum over the experts e of input g of
+// W_e x[g][e] (Q4_K; FastGemvArgs). The ids and weights have to be complete once this
+// grid runs. MixtureFits: whether its shared memory holds `cols` = experts * blocks * 256
+// values.
+int LaunchGemvMixture(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
+bool MixtureFits(int cols);
 bool UnitsFit(int type, int cols, int tokens);
 // Whether the image of `tokens` rows of `cols` values fits in shared memory.
 bool Q4KFastFits(int cols, int tokens);

@@ -30,6 +30,7 @@
 // ran 20 % slower on the 262144 x 2048 product.)
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "peer.cuh"
@@ -126,8 +127,7 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   const uint8_t* lane_first = TOKENS == 1 ? (one_live ? smem + (g & 3) * l.plane_stride + 8 * t : none)
                                           : (t < 2 ? lane_plane : none);
   const uint8_t* lane_second = t < 2 ? none : lane_plane;
-  const int tiles_per_group = TotalTiles(a);
-  const int row_tiles = GROUPED ? tiles_per_group * a.groups : tiles_per_group;
+  const int row_tiles = TotalTiles(a);
   // With ksplit > 1 a cluster of ksplit blocks shares each tile.
   // (No division here: a block's first slabs cannot be requested before these
   // are known, and nothing hides a chain of integer divisions at a kernel's start.
@@ -136,7 +136,14 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   int rank = 0;
   int slot = static_cast<int>(blockIdx.x);
   int stride = static_cast<int>(gridDim.x);
-  int my_tiles = a.tiles_each + (slot < a.tiles_more ? 1 : 0);
+  int group = 0;   // GROUPED: picks the matrix of each part, the input and the output
+  if constexpr (GROUPED) {
+    group = slot / a.group_blocks;
+    slot -= group * a.group_blocks;
+    stride = a.group_blocks;
+  }
+  const bool pairs = GROUPED && a.epilogue == kEpilogueSwiGlu;
+  int my_tiles = (a.tiles_each + (slot < a.tiles_more ? 1 : 0)) * (pairs ? 2 : 1);
   int slabs_mine = slabs_per_tile;
   if (ks > 1) {
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -149,13 +156,9 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     }
   }
   const int my_slabs = my_tiles * slabs_mine;
-  // A grouped launch has one block per tile; the block's group picks the
-  // matrix of each part, the input and the output.
-  int group = 0;
+  // A block of a grouped launch takes tiles slot, slot + stride, ... of its group, or
+  // (SwiGLU epilogue) those gate tiles, each followed by the up tile of the same rows.
   size_t matrix = 0;
-  // Grouped launches give a block one tile of its group, or (SwiGLU epilogue) one
-  // gate tile and the up tile of the same rows.
-  const int units_per_group = a.epilogue == kEpilogueSwiGlu ? tiles_per_group / 2 : tiles_per_group;
   // The ids come from an earlier kernel. Where that one lets this grid start only
   // after it has itself waited for everything before it (early_input: the router's
   // top-k), the inputs are complete already, and the image is built while the ids
@@ -169,14 +172,12 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     return id >= 0;
   };
   if constexpr (GROUPED) {
-    group = slot / units_per_group;
     if (!a.early_input && !choose()) {
       return;
     }
   }
   auto locate = [&](int n, int* part, int* local) {
-    LocateTile(a, GROUPED ? slot - group * units_per_group + (n & 1) * units_per_group : slot + n * stride, part,
-               local);
+    LocateTile(a, pairs ? slot + (n >> 1) * stride + (n & 1) * (row_tiles / 2) : slot + n * stride, part, local);
   };
   __syncthreads();
 
@@ -579,12 +580,9 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
       return Fail(GUFO_CUDA_BAD_ARGUMENT, "fast gemv: a grouped launch takes one token and a fused input");
     }
     launch.ksplit = 1;
-    grid = row_tiles * args.groups;   // one block per tile
-    if (args.epilogue == kEpilogueSwiGlu) {
-      if (args.nparts != 2 || args.parts[0].rows != args.parts[1].rows || args.parts[0].rows % 16 != 0) {
-        return Fail(GUFO_CUDA_BAD_ARGUMENT, "fast gemv: the SwiGLU epilogue takes two parts of equal whole tiles");
-      }
-      grid /= 2;                      // one block per (gate tile, up tile) pair
+    if (args.epilogue == kEpilogueSwiGlu &&
+        (args.nparts != 2 || args.parts[0].rows != args.parts[1].rows || args.parts[0].rows % 16 != 0)) {
+      return Fail(GUFO_CUDA_BAD_ARGUMENT, "fast gemv: the SwiGLU epilogue takes two parts of equal whole tiles");
     }
   } else if (args.epilogue == kEpilogueSwiGlu) {
     // One block per (gate tile, up tile) pair: block t takes tiles t and t + grid.
@@ -634,9 +632,19 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
       if (rc != GUFO_CUDA_OK) {
         return rc;
       }
-      launch.tiles_each = args.epilogue == kEpilogueSwiGlu ? 2 : 1;
-      launch.tiles_more = 0;
-      GUFO_CUDA_TRY(LaunchOverlapped(GemvMma<TYPE, TOKENS, PER_SM, false, true>, dim3(grid), dim3(kFastThreads), smem,
+      // As many blocks a group as let the whole launch be resident in the fewest rounds
+      // of tiles (pairs): a block converts its group's input once for all of its tiles
+      // and streams their weights through its ring (one block per pair: 1024 blocks
+      // for 32 experts of 512 rows, each with a start and a conversion of its own).
+      auto* kernel = GemvMma<TYPE, TOKENS, PER_SM, false, true>;
+      const int resident = std::max(1, ResidentBlocks(kernel, ctx->device, kFastThreads, smem, 1));
+      const int items = args.epilogue == kEpilogueSwiGlu ? row_tiles / 2 : row_tiles;
+      const int64_t all = static_cast<int64_t>(items) * args.groups;
+      const int rounds = static_cast<int>((all + resident - 1) / resident);
+      launch.group_blocks = (items + rounds - 1) / rounds;
+      launch.tiles_each = items / launch.group_blocks;
+      launch.tiles_more = items % launch.group_blocks;
+      GUFO_CUDA_TRY(LaunchOverlapped(kernel, dim3(launch.group_blocks * args.groups), dim3(kFastThreads), smem,
                                      ctx->stream, 1, launch));
       ctx->launches.fetch_add(1);
       return GUFO_CUDA_OK;

@@ -285,11 +285,14 @@ __device__ __forceinline__ void ZeroIdleColumns(const ImageLayout& l, int blocks
 // dealt round-robin) converts only the blocks of its own slabs; the others are
 // never read. keep_w: LoadNormAhead's. squares: [kFastWarps][TOKENS] in shared
 // memory, for RowScale. Ends with a __syncthreads. kFastThreads threads.
-template <int TOKENS>
+// MIX: a.x holds the experts' inputs of a mixture one after the other; every value is
+// multiplied by its expert's weight (`mix`: the input's weights, `mix_ids` its ids).
+template <int TOKENS, bool MIX = false>
 __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayout& l,
                                           uint8_t* image, float extra, const float* x,
                                           int rank, int ks, const float (&keep_w)[8],
-                                          float* squares, float inv_n) {
+                                          float* squares, float inv_n,
+                                          const int* mix_ids = nullptr, const float* mix = nullptr) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int n = a.cols;
@@ -466,6 +469,14 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             v[j][i] = SiluFast(v[j][i]) * up[j][i];
+          }
+        }
+        if constexpr (MIX) {
+          const int e = at_b[j] / a.mix_blocks;
+          const float w = mix_ids[e] >= 0 ? mix[e] : 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            v[j][i] = mix_ids[e] >= 0 ? w * v[j][i] : 0.f;
           }
         }
         StageBlock(v[j], lane, at_tok[j], at_b[j], l, image, extra);

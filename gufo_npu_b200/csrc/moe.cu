@@ -383,140 +383,6 @@ int LaunchNarrowGrouped(gufo_cuda_ctx* ctx, const GemvArgs& g, bool swiglu) {
   }
 }
 
-// The down product of a token's k (<= 8) chosen experts and Decoder::MoeFfn's
-// weighted sum in one launch (decoder.cpp:541-556): out[t][row] = shared[t][row] *
-// scale[t] + the sum, in slot order, of weights[t][s] * (row of expert ids[t][s]
-// times act[t][s]). A warp takes a row (BLOCKS = 1: two rows) of all k experts at
-// once: k row loads in flight, the k activated inputs of the token in shared
-// memory. A slot with ids < 0 adds nothing.
-struct NarrowCombineArgs {
-  const uint8_t* w;
-  int rows;
-  int row_bytes;
-  const int* ids;          // [tokens][k]
-  const float* weights;    // [tokens][k]
-  const float* scale;      // [tokens]
-  const float* shared;     // [tokens][rows]
-  const float* act;        // [tokens][k][256 * BLOCKS]
-  int k;
-  float* out;              // [tokens][rows]; may be shared
-};
-
-constexpr int kCombineSlots = 8;
-
-template <int BLOCKS>
-__global__ void __launch_bounds__(256)
-NarrowCombineQ4K(const __grid_constant__ NarrowCombineArgs a) {
-  constexpr int kSlots = 16 * BLOCKS;
-  constexpr int kPer = kSlots > 32 ? kSlots / 32 : 1;
-  constexpr int kRowsAtOnce = kSlots < 32 ? 32 / kSlots : 1;
-  constexpr int kCols = 256 * BLOCKS;
-  __shared__ __align__(16) float xs[kCombineSlots][kCols];
-  GridLaunchDependents();
-  const int token = blockIdx.y;
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int sub = kRowsAtOnce > 1 ? lane / kSlots : 0;
-  const int row = (blockIdx.x * 8 + warp) * kRowsAtOnce + sub;
-  const int load_row = min(row, a.rows - 1);
-  int at[kPer], part[kPer], pair[kPer], col[kPer];
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int slot = (lane + 32 * j) % kSlots;
-    const int b = slot >> 4;
-    const int c = (slot >> 2) & 3;
-    const int p = slot & 3;
-    at[j] = b * kQ4KBytes;
-    part[j] = 32 * c + 8 * p;
-    pair[j] = c;
-    col[j] = 256 * b + 64 * c + 8 * p;
-  }
-  // The k rows first, ahead of the wait: the gate / up product lets this grid start
-  // only once the ids are complete, and the rows come from HBM.
-  uint4 head[kCombineSlots][kPer];
-  uint2 codes[kCombineSlots][kPer];
-  int id[kCombineSlots];
-#pragma unroll
-  for (int s = 0; s < kCombineSlots; ++s) {
-    id[s] = s < a.k ? a.ids[token * a.k + s] : -1;
-    if (id[s] >= 0) {
-      const uint8_t* from = a.w + (static_cast<size_t>(id[s]) * a.rows + load_row) * a.row_bytes;
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) {
-        head[s][j] = *reinterpret_cast<const uint4*>(from + at[j]);
-        codes[s][j] = *reinterpret_cast<const uint2*>(from + at[j] + 16 + part[j]);
-      }
-    }
-  }
-  GridDependencyWait();
-  for (int i = threadIdx.x * 4; i < a.k * kCols; i += 256 * 4) {
-    const int s = i / kCols;
-    *reinterpret_cast<float4*>(&xs[s][i - s * kCols]) =
-        *reinterpret_cast<const float4*>(a.act + (static_cast<size_t>(token) * a.k + s) * kCols + (i - s * kCols));
-  }
-  __syncthreads();
-  float sum[kCombineSlots];
-#pragma unroll
-  for (int s = 0; s < kCombineSlots; ++s) {
-    sum[s] = 0.f;
-    if (id[s] >= 0) {
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) {
-        const float4 l0 = *reinterpret_cast<const float4*>(&xs[s][col[j]]);
-        const float4 l1 = *reinterpret_cast<const float4*>(&xs[s][col[j] + 4]);
-        const float4 h0 = *reinterpret_cast<const float4*>(&xs[s][col[j] + 32]);
-        const float4 h1 = *reinterpret_cast<const float4*>(&xs[s][col[j] + 36]);
-        const float lo[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-        const float hi[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-        const float d = HalfBitsToFloat(static_cast<uint16_t>(head[s][j].x & 0xFFFF));
-        const float dmin = HalfBitsToFloat(static_cast<uint16_t>(head[s][j].x >> 16));
-        int sc_lo, m_lo, sc_hi, m_hi;
-        ScaleMinK4(2 * pair[j], head[s][j].y, head[s][j].z, head[s][j].w, &sc_lo, &m_lo);
-        ScaleMinK4(2 * pair[j] + 1, head[s][j].y, head[s][j].z, head[s][j].w, &sc_hi, &m_hi);
-        float dot_lo = 0.f, dot_hi = 0.f, lo_sum = 0.f, hi_sum = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint32_t word = i < 4 ? codes[s][j].x : codes[s][j].y;
-          const uint32_t byte = (word >> (8 * (i & 3))) & 0xFFu;
-          dot_lo = fmaf(static_cast<float>(byte & 15u), lo[i], dot_lo);
-          dot_hi = fmaf(static_cast<float>(byte >> 4), hi[i], dot_hi);
-          lo_sum += lo[i];
-          hi_sum += hi[i];
-        }
-        sum[s] += d * (static_cast<float>(sc_lo) * dot_lo + static_cast<float>(sc_hi) * dot_hi) -
-                  dmin * (static_cast<float>(m_lo) * lo_sum + static_cast<float>(m_hi) * hi_sum);
-      }
-    }
-  }
-#pragma unroll
-  for (int o = kSlots < 32 ? kSlots / 2 : 16; o > 0; o >>= 1) {
-#pragma unroll
-    for (int s = 0; s < kCombineSlots; ++s) {
-      sum[s] += __shfl_xor_sync(0xFFFFFFFFu, sum[s], o);
-    }
-  }
-  if ((lane % (kSlots < 32 ? kSlots : 32)) == 0 && row < a.rows) {
-    const size_t at_out = static_cast<size_t>(token) * a.rows + row;
-    float v = a.shared[at_out] * a.scale[token];
-#pragma unroll
-    for (int s = 0; s < kCombineSlots; ++s) {
-      if (s < a.k && id[s] >= 0) {
-        v = fmaf(a.weights[token * a.k + s], sum[s], v);
-      }
-    }
-    a.out[at_out] = v;
-  }
-}
-
-template <int BLOCKS>
-int LaunchNarrowCombine(gufo_cuda_ctx* ctx, const NarrowCombineArgs& args, int tokens) {
-  constexpr int kBlockRows = 8 * (16 * BLOCKS < 32 ? 32 / (16 * BLOCKS) : 1);
-  GUFO_CUDA_TRY(LaunchOverlapped(NarrowCombineQ4K<BLOCKS>, dim3((args.rows + kBlockRows - 1) / kBlockRows, tokens),
-                                 dim3(256), 0, ctx->stream, 1, args));
-  ctx->launches.fetch_add(1);
-  return GUFO_CUDA_OK;
-}
-
 }  // namespace
 
 int EnqueueExpertFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids, int pairs, const float* x,
@@ -588,30 +454,34 @@ int EnqueueMoeFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids, co
   in.x_group_div = k;
   in.y_group_stride = bank.expert_ffn;
   GemvArgs down = bank.down;
-  const int blocks = down.cols / kSuperBlock;
-  if (k <= kCombineSlots && NarrowFits(down) && blocks <= 2 && GroupedSwiGluInProduct(ctx, in)) {
-    // Two launches: gate / up with the SwiGLU in its epilogue, then the down rows
-    // of a token's experts with the weighted sum. Directly behind the router's top-k
-    // (nothing else has been launched since, from any context) the inputs are
+  if (down.parts[0].type == GUFO_CUDA_Q4_K && down.cols % kSuperBlock == 0 && MixtureFits(k * down.cols) &&
+      (reinterpret_cast<uintptr_t>(act) & 15) == 0 && GroupedSwiGluInProduct(ctx, in)) {
+    // Two launches: gate / up with the SwiGLU in its epilogue, then the down rows of a
+    // token's experts side by side with the weighted sum. Directly behind the router's
+    // top-k (nothing else has been launched since, from any context) the inputs are
     // complete once the first of them runs; its image is built while the top-k is
-    // being found.
+    // being found. It lets the second start only once the ids are complete.
     in.early_input = ctx->route_launch == LaunchCount().load() && ctx->route_stream == ctx->stream ? 1 : 0;
     const int rc = LaunchGemvGrouped(ctx, in, kProloguePlain, nullptr, true);
     if (rc != GUFO_CUDA_OK) {
       return rc;
     }
-    NarrowCombineArgs args{};
-    args.w = down.parts[0].data;
-    args.rows = down.parts[0].rows;
+    FastGemvArgs args{};
+    args.parts[0] = {down.parts[0].data, down.parts[0].rows, 0};
+    args.cols = k * down.cols;
     args.row_bytes = down.parts[0].row_bytes;
-    args.ids = ids;
-    args.weights = weights;
-    args.scale = scale;
-    args.shared = shared;
-    args.act = act;
-    args.k = k;
-    args.out = out;
-    return blocks == 1 ? LaunchNarrowCombine<1>(ctx, args, tokens) : LaunchNarrowCombine<2>(ctx, args, tokens);
+    args.x = act;
+    args.y = out;
+    args.y_stride = bank.hidden;
+    args.tokens = 1;
+    args.groups = tokens;
+    args.mix_ids = ids;
+    args.mix_weights = weights;
+    args.mix_experts = k;
+    args.mix_blocks = down.cols / kSuperBlock;
+    args.mix_base = shared;
+    args.mix_scale = scale;
+    return LaunchGemvMixture(ctx, args);
   }
   const int rc = EnqueueExpertFfn(ctx, bank, ids, tokens * k, x, x_stride, k, ffn, act, expert_out);
   if (rc != GUFO_CUDA_OK) {

@@ -339,3 +339,42 @@ def test_activating_product_with_more_tile_pairs_than_blocks(ctx, tokens, rows, 
     assert rel_l2(act.cpu().numpy(), g / (1.0 + np.exp(-g)) * u) <= 5e-6
     ctx.matrix_free(mg)
     ctx.matrix_free(mu)
+
+
+@pytest.mark.parametrize("tokens,k,hidden,ffn,experts", [(1, 1, 256, 256, 4), (3, 3, 1280, 768, 7), (5, 8, 2048, 512, 16),
+                                                         (16, 4, 1536, 256, 64)])
+def test_mixture_of_given_experts(ctx, tokens, k, hidden, ffn, experts):
+    """The FFN of chosen experts and their weighted sum, with experts left out and chosen twice, one
+    to three blocks a row and one to several tiles a thread block, in float64."""
+    from gufo_npu_b200 import _capi
+    dev = torch.device("cuda:0")
+    mats, w = [], []
+    for seed, rows, cols in ((1, ffn, hidden), (2, ffn, hidden), (3, hidden, ffn)):
+        m, v = _matrix(ctx, Q.GGML_Q4_K, rows * experts, cols, seed)
+        mats.append(m)
+        w.append(v.reshape(experts, rows, cols))
+    bank = _capi.ExpertBank(*mats, experts, ffn, hidden)
+    rng = np.random.default_rng(tokens)
+    ids = rng.integers(0, experts, (tokens, k)).astype(np.int32)
+    if k > 1:
+        ids[0, 1] = -1
+        ids[-1, 0] = ids[-1, k - 1]
+    wt, sc = rng.random((tokens, k)).astype(np.float32), rng.random(tokens).astype(np.float32)
+    x, shared = (G.normal(s, tokens, hidden).astype(np.float32) for s in (4, 5))
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+    t_ids, t_wt, t_sc, t_x, t_sh = map(up, (ids, wt, sc, x, shared))
+    nan = lambda *s: torch.full(s, float("nan"), device=dev)
+    buf, act, eo = nan(tokens * k, 2 * ffn), nan(tokens * k, ffn), nan(tokens, k, hidden)
+    torch.cuda.synchronize()
+    ctx.moe_ffn_device(bank, t_ids, t_wt, t_sc, tokens, k, t_x, hidden, t_sh, buf, act, eo, t_sh)
+    ctx.synchronize()
+    want = shared.astype(np.float64) * sc[:, None]
+    for t in range(tokens):
+        for s in range(k):
+            e = ids[t, s]
+            if e >= 0:
+                g, u = w[0][e] @ x[t], w[1][e] @ x[t]
+                want[t] += float(wt[t, s]) * (w[2][e] @ (g / (1 + np.exp(-g)) * u))
+    assert rel_l2(t_sh.cpu().numpy(), want) <= 5e-6
+    for m in mats:
+        ctx.matrix_free(m)
