@@ -78,7 +78,9 @@ size_t SharedBytes(int cols) {
 }
 
 // GROUPED: the routed experts' products, one token a group (FastGemvArgs).
-template <int TYPE, int TOKENS, int PER_SM, bool ONE = false, bool GROUPED = false>
+// PAIRS: a block may take several (gate tile, up tile) pairs; else one, tiles blockIdx.x
+// and blockIdx.x + gridDim.x (the decode step's kernel stays 1 % faster without).
+template <int TYPE, int TOKENS, int PER_SM, bool ONE = false, bool GROUPED = false, bool PAIRS = GROUPED>
 __global__ void __launch_bounds__(kFastThreads, PER_SM)
 GemvMma(const __grid_constant__ FastGemvArgs a) {
   using S = Slab<TYPE>;
@@ -142,7 +144,7 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     slot -= group * a.group_blocks;
     stride = a.group_blocks;
   }
-  const bool pairs = GROUPED && a.epilogue == kEpilogueSwiGlu;
+  const bool pairs = PAIRS && a.epilogue == kEpilogueSwiGlu;
   int my_tiles = (a.tiles_each + (slot < a.tiles_more ? 1 : 0)) * (pairs ? 2 : 1);
   int slabs_mine = slabs_per_tile;
   if (ks > 1) {
@@ -156,8 +158,8 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     }
   }
   const int my_slabs = my_tiles * slabs_mine;
-  // A block of a grouped launch takes tiles slot, slot + stride, ... of its group, or
-  // (SwiGLU epilogue) those gate tiles, each followed by the up tile of the same rows.
+  // A block takes tiles slot, slot + stride, ... (of its group), or (SwiGLU epilogue)
+  // those gate tiles, each followed by the up tile of the same rows.
   size_t matrix = 0;
   // The ids come from an earlier kernel. Where that one lets this grid start only
   // after it has itself waited for everything before it (early_input: the router's
@@ -517,11 +519,11 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
 }
 
 // Lets the kernel use all the shared memory a block may have (once per device).
-template <int TYPE, int TOKENS, int PER_SM, bool ONE = false, bool GROUPED = false>
+template <int TYPE, int TOKENS, int PER_SM, bool ONE = false, bool GROUPED = false, bool PAIRS = GROUPED>
 int Configure(const gufo_cuda_ctx* ctx) {
   static bool configured[16] = {};
   if (!configured[ctx->device & 15]) {
-    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemvMma<TYPE, TOKENS, PER_SM, ONE, GROUPED>,
+    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemvMma<TYPE, TOKENS, PER_SM, ONE, GROUPED, PAIRS>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kFastMaxShared));
     configured[ctx->device & 15] = true;
   }
@@ -585,7 +587,6 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
       return Fail(GUFO_CUDA_BAD_ARGUMENT, "fast gemv: the SwiGLU epilogue takes two parts of equal whole tiles");
     }
   } else if (args.epilogue == kEpilogueSwiGlu) {
-    // One block per (gate tile, up tile) pair: block t takes tiles t and t + grid.
     if (args.nparts != 2 || args.parts[0].rows != args.parts[1].rows || args.parts[0].rows % 16 != 0 ||
         args.peer_out.world > 0) {
       return Fail(GUFO_CUDA_BAD_ARGUMENT, "fast gemv: the SwiGLU epilogue takes two parts of equal whole tiles");
@@ -593,7 +594,23 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
     launch.ksplit = 1;
     grid = row_tiles / 2;
     if (grid > ResidentBlocks(GemvMma<TYPE, TOKENS, PER_SM>, ctx->device, kFastThreads, smem, 1)) {
-      return kNotTaken;   // more tile pairs than resident blocks
+      // More tile pairs than resident blocks: several a block (2 x 8192 x 2048: a step of
+      // twelve layers 387 -> 349 us against the unit kernel).
+      if (slabs > 1 && args.cols % (8 * kSuperBlock) != 0) {
+        return kNotTaken;
+      }
+      const int rc = Configure<TYPE, TOKENS, PER_SM, false, false, true>(ctx);
+      if (rc != GUFO_CUDA_OK) {
+        return rc;
+      }
+      auto* many = GemvMma<TYPE, TOKENS, PER_SM, false, false, true>;
+      const int items = grid;
+      grid = std::max(1, std::min(items, ResidentBlocks(many, ctx->device, kFastThreads, smem, 1)));
+      launch.tiles_each = items / grid;
+      launch.tiles_more = items % grid;
+      GUFO_CUDA_TRY(LaunchOverlapped(many, dim3(grid), dim3(kFastThreads), smem, ctx->stream, 1, launch));
+      ctx->launches.fetch_add(1);
+      return GUFO_CUDA_OK;
     }
   } else {
     // Few rows and several slabs per tile: split the tiles' slabs over a cluster.

@@ -325,7 +325,7 @@ def test_units_of_ragged_rows(ctx, ggml_type, tokens, rows, cols):
     ctx.matrix_free(m)
 
 
-@pytest.mark.parametrize("tokens,rows,cols", [(1, 9728, 2560), (2, 9728, 2560), (2, 16, 512), (2, 6144, 2048)])
+@pytest.mark.parametrize("tokens,rows,cols", [(1, 9728, 2560), (1, 8192, 2048), (1, 7120, 512), (2, 9728, 2560), (2, 16, 512), (2, 6144, 2048)])
 def test_activating_product_with_more_tile_pairs_than_blocks(ctx, tokens, rows, cols):
     dev = torch.device("cuda:0")
     (mg, wg), (mu, wu) = (_matrix(ctx, Q.GGML_Q4_K, rows, cols, s) for s in (14, 15))
