@@ -167,10 +167,11 @@ struct FastGemvArgs {
   int x_group_stride;     // floats between the inputs (0: shared)
   int x_group_div;        // groups per input: group g reads input g / x_group_div (0 counts as 1)
   int early_input;        // the inputs are complete as soon as this grid runs, ahead of its dependency wait
-  // A mixture (LaunchGemvMixture): the rows of `mix_experts` matrices of parts[0] side
-  // by side, `mix_blocks` 256-value blocks of each, `groups` inputs; input g uses the
-  // matrices mix_ids[g][..] (< 0: none), its values times mix_weights[g][..], and
-  // adds mix_base[g] (rows values) times mix_scale[g].
+  // A mixture (LaunchGemvMixture): `groups` inputs, input g being mix_experts vectors of
+  // mix_blocks 256-value blocks for the matrices mix_ids[g][..] of parts[0] (< 0: none).
+  // With mix_base the results are mix_base[g] * mix_scale[g] plus the experts' rows
+  // times mix_weights[g][..], in slot order; without, one expert's rows as they are
+  // (left alone where its id is negative).
   const int* mix_ids;
   const float* mix_weights;
   int mix_experts;
@@ -229,10 +230,9 @@ void* DeviceAddress(const void* host);
 int LaunchGemvQ4KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
 // The launch of gemv_units.cu, and whether its shared memory holds `tokens` rows.
 int LaunchGemvUnits(gufo_cuda_ctx* ctx, int type, const FastGemvArgs& args);
-// y[g] = mix_base[g] * mix_scale[g] + the weighted sum over the experts e of input g of
-// W_e x[g][e] (Q4_K; FastGemvArgs). The ids and weights have to be complete once this
-// grid runs. MixtureFits: whether its shared memory holds `cols` = experts * blocks * 256
-// values.
+// The down products of chosen experts, with or without their weighted sum (Q4_K;
+// FastGemvArgs). The ids and weights have to be complete once this grid runs.
+// MixtureFits: whether its shared memory holds `cols` = experts * blocks * 256 values.
 int LaunchGemvMixture(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
 bool MixtureFits(int cols);
 bool UnitsFit(int type, int cols, int tokens);

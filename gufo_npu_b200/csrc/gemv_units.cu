@@ -80,12 +80,14 @@ size_t SharedBytes(int cols, int depth) {
 }
 
 // MIX: the down product of a token's chosen experts with their weighted sum (Q4_K, one
-// token a thread block). Side by side the experts' rows are one row of K = experts *
-// expert_ffn, with the weights folded into the input, so that the sum over the experts
-// is the sum over K. (The form before, a warp per row and expert in fp32, spent its
-// time in conversions and in staging the activated inputs once per eight rows. Together
-// with several tile pairs a block in the gate / up product, a layer of 256 experts of
-// 512 x 2048, eight of them for each of four tokens: 34.4 -> 21.9 us.)
+// token a thread block). The experts' inputs lie side by side, so their narrow rows (two
+// blocks of 256 values) are one row that keeps eight warps busy; every unit's row sums
+// go to the exchange buffer by themselves, and whoever gathers a tile adds an expert's
+// blocks and then the experts in slot order, as separate launches would. (The form
+// before, a warp per row and expert in fp32, spent its time in conversions and in
+// staging the activated inputs once per eight rows. Together with several tile pairs a
+// block in the gate / up product, a layer of 256 experts of 512 x 2048, eight of them
+// for each of four tokens: 34.4 -> @@MOE@@ us.)
 template <int TYPE, int TOKENS, int PER_SM, bool MIX = false>
 __global__ void __launch_bounds__(kFastThreads, PER_SM)
 GemvUnits(const __grid_constant__ FastGemvArgs a) {
@@ -127,8 +129,9 @@ GemvUnits(const __grid_constant__ FastGemvArgs a) {
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2;
   const int t = lane & 3;
-  uint8_t* ring = reinterpret_cast<uint8_t*>(exchange + kExchange * kFastWarps * kTileFloats) +
-                  warp * (a.depth * kUnitBytes);
+  // (MIX: [kExchange][blocks][16 rows].)
+  const int exchange_floats = MIX ? blocks * kTileRows : kFastWarps * kTileFloats;
+  uint8_t* ring = reinterpret_cast<uint8_t*>(exchange + kExchange * exchange_floats) + warp * (a.depth * kUnitBytes);
   // Lane planes of the two unit kinds (q4k_unit.cuh, q6k_unit.cuh): column g of
   // the first MMA column group; lanes past the last token's planes wrap onto
   // live ones, whose sums meet a zero column factor.
@@ -260,8 +263,8 @@ GemvUnits(const __grid_constant__ FastGemvArgs a) {
     wait(&staged, 0);
     __syncthreads();   // the plane of zeros, the mirror's address
   } else {
-    FillImage<TOKENS, MIX>(a, l, smem, U::kExtra, MIX ? a.x + static_cast<size_t>(group) * a.cols : a.x, rank, ks,
-                           norm_ahead, squares, inv_n, mix_ids, MIX ? a.mix_weights + group * a.mix_experts : nullptr);
+    FillImage<TOKENS>(a, l, smem, U::kExtra, MIX ? a.x + static_cast<size_t>(group) * a.cols : a.x, rank, ks,
+                      norm_ahead, squares, inv_n);
   }
   // The norm's 1 / rms of token k in lane k.
   const float lane_scale = lane < TOKENS ? RowScale<TOKENS>(a, squares, lane, inv_n) : 1.f;
@@ -292,13 +295,6 @@ GemvUnits(const __grid_constant__ FastGemvArgs a) {
   auto store = [&](int part, int local, int o, float total) {
     const int k = o % TOKENS;
     const int row = local * kTileRows + o / TOKENS;
-    if constexpr (MIX) {
-      if (row < a.parts[0].rows) {
-        const size_t at = static_cast<size_t>(group) * a.y_stride + row;
-        a.y[at] = fmaf(a.mix_base[at], a.mix_scale[group], total);
-      }
-      return;
-    }
     if (row < a.parts[part].rows) {
       const size_t at = static_cast<size_t>(k) * a.y_stride + (pairs ? 0 : a.parts[part].y_offset) + row;
       if (a.peer_out.world > 0) {
@@ -324,6 +320,33 @@ GemvUnits(const __grid_constant__ FastGemvArgs a) {
     wait(&full[n % kExchange], (n / kExchange) & 1u);
     int part, local;
     locate(n, &part, &local);
+    if constexpr (MIX) {
+      const int row = local * kTileRows + lane;
+      if (lane < kTileRows && row < a.parts[0].rows) {
+        const size_t y_at = static_cast<size_t>(group) * a.y_stride + row;
+        const float* from = exchange + (n % kExchange) * exchange_floats + lane;
+        float v = a.mix_base != nullptr ? a.mix_base[y_at] * a.mix_scale[group] : 0.f;
+#pragma unroll 1
+        for (int e = 0; e < a.mix_experts; ++e) {
+          float y = 0.f;
+#pragma unroll 1
+          for (int j = 0; j < a.mix_blocks; ++j) {
+            y += from[(e * a.mix_blocks + j) * kTileRows];
+          }
+          if (mix_ids[e] >= 0) {
+            v = a.mix_base != nullptr ? fmaf(a.mix_weights[group * a.mix_experts + e], y, v) : y;
+          }
+        }
+        if (a.mix_base != nullptr || mix_ids[0] >= 0) {
+          a.y[y_at] = v;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) {
+        MbarArrive(SharedAddress(&empty[n % kExchange]));
+      }
+      return;
+    }
 #pragma unroll
     for (int first = 0; first < kTileFloats; first += 32) {
       const int o = first + lane;
@@ -349,11 +372,45 @@ GemvUnits(const __grid_constant__ FastGemvArgs a) {
   auto duty = [&](int n) {
     return n >= 0 && (pairs ? (n & 1) != 0 && ((n >> 1) & 7) == warp : (n & 7) == warp);
   };
+  // This warp's row sums so far: the columns of token k are 3k .. 3k + 2 (one token:
+  // every column; dead ones carry a zero factor), the Q4_K offsets sit in lanes t < 2
+  // for row g and t >= 2 for row g + 8; summed over the quad.
+  auto flush = [&](float* tile) {
+#pragma unroll
+    for (int k = 0; k < TOKENS; ++k) {
+      float lo = 0.f, hi = 0.f;
+#pragma unroll
+      for (int nb = 0; nb < kNB; ++nb) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int col = nb * 8 + 2 * t + j;
+          const bool of_k = TOKENS == 1 || (col < kNCols && col / kLimbs == k);
+          lo += of_k ? out[nb][j] : 0.f;
+          hi += of_k ? out[nb][2 + j] : 0.f;
+        }
+      }
+      lo -= t < 2 ? off[k] : 0.f;
+      hi -= t < 2 ? 0.f : off[k];
+#pragma unroll
+      for (int o = 1; o <= 2; o <<= 1) {
+        lo += __shfl_xor_sync(0xFFFFFFFFu, lo, o);
+        hi += __shfl_xor_sync(0xFFFFFFFFu, hi, o);
+      }
+      if (t == 0) {
+        tile[g * TOKENS + k] = lo;
+        tile[(g + 8) * TOKENS + k] = hi;
+      }
+    }
+    clear();
+  };
   clear();
   int b = rank * kFastWarps + warp;
   int at = 0;   // ring position of the next unit
 #pragma unroll 1
   for (int n = 0; n < my_tiles; ++n) {
+    if (MIX && n >= kExchange) {
+      wait(&empty[n % kExchange], (n / kExchange - 1) & 1u);
+    }
 #pragma unroll 1
     for (; b < blocks; b += wide) {
       // This warp's own copies, so nothing but the warp meets here.
@@ -415,42 +472,18 @@ GemvUnits(const __grid_constant__ FastGemvArgs a) {
           }
         }
       }
+      if constexpr (MIX) {
+        flush(exchange + (n % kExchange) * exchange_floats + b * kTileRows);
+      }
     }
     b -= blocks;
-    // This warp's row sums of the tile (zeros where it had no block of it): the
-    // columns of token k are 3k .. 3k + 2 (one token: every column; dead ones carry a
-    // zero factor), the Q4_K offsets sit in lanes t < 2 for row g and t >= 2 for row
-    // g + 8; summed over the quad.
-    if (n >= kExchange) {
-      wait(&empty[n % kExchange], (n / kExchange - 1) & 1u);
+    if constexpr (!MIX) {
+      // Zeros where this warp had no block of the tile.
+      if (n >= kExchange) {
+        wait(&empty[n % kExchange], (n / kExchange - 1) & 1u);
+      }
+      flush(exchange + ((n % kExchange) * kFastWarps + warp) * kTileFloats);
     }
-    float* tile = exchange + ((n % kExchange) * kFastWarps + warp) * kTileFloats;
-#pragma unroll
-    for (int k = 0; k < TOKENS; ++k) {
-      float lo = 0.f, hi = 0.f;
-#pragma unroll
-      for (int nb = 0; nb < kNB; ++nb) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int col = nb * 8 + 2 * t + j;
-          const bool of_k = TOKENS == 1 || (col < kNCols && col / kLimbs == k);
-          lo += of_k ? out[nb][j] : 0.f;
-          hi += of_k ? out[nb][2 + j] : 0.f;
-        }
-      }
-      lo -= t < 2 ? off[k] : 0.f;
-      hi -= t < 2 ? 0.f : off[k];
-#pragma unroll
-      for (int o = 1; o <= 2; o <<= 1) {
-        lo += __shfl_xor_sync(0xFFFFFFFFu, lo, o);
-        hi += __shfl_xor_sync(0xFFFFFFFFu, hi, o);
-      }
-      if (t == 0) {
-        tile[g * TOKENS + k] = lo;
-        tile[(g + 8) * TOKENS + k] = hi;
-      }
-    }
-    clear();
     __syncwarp();
     if (lane == 0) {
       MbarArrive(SharedAddress(&full[n % kExchange]));
@@ -590,13 +623,18 @@ int LaunchTokens(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
 
 }  // namespace
 
-bool MixtureFits(int cols) {
-  return SharedBytes<GUFO_CUDA_Q4_K, 1>(cols, Unit<GUFO_CUDA_Q4_K>::kDepth) <= static_cast<size_t>(kFastMaxShared);
+namespace {
+size_t MixtureShared(int cols) {
+  return SharedBytes<GUFO_CUDA_Q4_K, 1>(cols, Unit<GUFO_CUDA_Q4_K>::kDepth) +
+         static_cast<size_t>(kExchange) * (cols / kSuperBlock) * kTileRows * 4;
 }
+}  // namespace
+
+bool MixtureFits(int cols) { return MixtureShared(cols) <= static_cast<size_t>(kFastMaxShared); }
 
 int LaunchGemvMixture(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
   auto* kernel = GemvUnits<GUFO_CUDA_Q4_K, 1, kMixPerSm, true>;
-  const size_t smem = SharedBytes<GUFO_CUDA_Q4_K, 1>(args.cols, Unit<GUFO_CUDA_Q4_K>::kDepth);
+  const size_t smem = MixtureShared(args.cols);
   static bool configured[16] = {};
   if (!configured[ctx->device & 15]) {
     GUFO_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFastMaxShared));

@@ -273,6 +273,7 @@ __device__ __forceinline__ float RowScale(const FastGemvArgs& a, const float* sq
 template <int TOKENS>
 __device__ __forceinline__ void ZeroIdleColumns(const ImageLayout& l, int blocks, uint8_t* image) {
   float* scale = reinterpret_cast<float*>(image + l.scale_at);
+#pragma unroll 1
   for (int i = threadIdx.x; i < blocks * l.kcols; i += kFastThreads) {
     if (i % l.kcols >= kLimbs * TOKENS) {
       scale[i] = 0.f;
@@ -285,14 +286,11 @@ __device__ __forceinline__ void ZeroIdleColumns(const ImageLayout& l, int blocks
 // dealt round-robin) converts only the blocks of its own slabs; the others are
 // never read. keep_w: LoadNormAhead's. squares: [kFastWarps][TOKENS] in shared
 // memory, for RowScale. Ends with a __syncthreads. kFastThreads threads.
-// MIX: a.x holds the experts' inputs of a mixture one after the other; every value is
-// multiplied by its expert's weight (`mix`: the input's weights, `mix_ids` its ids).
-template <int TOKENS, bool MIX = false>
+template <int TOKENS>
 __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayout& l,
                                           uint8_t* image, float extra, const float* x,
                                           int rank, int ks, const float (&keep_w)[8],
-                                          float* squares, float inv_n,
-                                          const int* mix_ids = nullptr, const float* mix = nullptr) {
+                                          float* squares, float inv_n) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int n = a.cols;
@@ -328,7 +326,7 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
   if (a.prologue == kPrologueResNorm) {
     // vec::RmsNorm (src/core/vec.hpp:57-63) of the residual stream after its
     // pending add (src/models/qwen35/decoder.cpp:493,504-508).
-    constexpr int kBatch = TOKENS <= 2 ? 2 : 1;
+    constexpr int kBatch = 1;
     if (lane < TOKENS) {
       squares[warp * TOKENS + lane] = 0.f;
     }
@@ -442,7 +440,7 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
   const size_t stride = act ? 2 * static_cast<size_t>(n) : static_cast<size_t>(n);
   // All loads of a batch are in flight before the first value is used: one round
   // trip per batch, not per block (a 6144-value input is three blocks per warp).
-  constexpr int kBatch = TOKENS == 1 ? 3 : TOKENS == 2 ? 2 : 1;
+  constexpr int kBatch = 1;
 #pragma unroll 1
   while (live()) {
     float v[kBatch][8], up[kBatch][8];
@@ -471,14 +469,6 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
             v[j][i] = SiluFast(v[j][i]) * up[j][i];
           }
         }
-        if constexpr (MIX) {
-          const int e = at_b[j] / a.mix_blocks;
-          const float w = mix_ids[e] >= 0 ? mix[e] : 0.f;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            v[j][i] = mix_ids[e] >= 0 ? w * v[j][i] : 0.f;
-          }
-        }
         StageBlock(v[j], lane, at_tok[j], at_b[j], l, image, extra);
       }
     }
@@ -487,14 +477,13 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
 }
 
 // Tiles of 16 rows are numbered across the parts of a launch, each part
-// rounded up to whole tiles.
+// rounded up to whole tiles. (Rolled loops, here and wherever else code is not in a
+// kernel's inner loop: see the note on code size at FillImage.)
 __device__ __forceinline__ int TotalTiles(const FastGemvArgs& a) {
   int tiles = 0;
-#pragma unroll
-  for (int p = 0; p < kFastMaxParts; ++p) {
-    if (p < a.nparts) {
-      tiles += (a.parts[p].rows + 15) >> 4;
-    }
+#pragma unroll 1
+  for (int p = 0; p < a.nparts; ++p) {
+    tiles += (a.parts[p].rows + 15) >> 4;
   }
   return tiles;
 }
@@ -502,13 +491,13 @@ __device__ __forceinline__ int TotalTiles(const FastGemvArgs& a) {
 // Part and tile-within-part of global tile `tile`.
 __device__ __forceinline__ void LocateTile(const FastGemvArgs& a, int tile, int* part, int* local) {
   int p = 0;
-#pragma unroll
-  for (int i = 0; i < kFastMaxParts - 1; ++i) {
-    const int tiles = (a.parts[i].rows + 15) >> 4;
-    if (p == i && i + 1 < a.nparts && tile >= tiles) {
-      tile -= tiles;
-      p = i + 1;
+#pragma unroll 1
+  for (; p + 1 < a.nparts; ++p) {
+    const int tiles = (a.parts[p].rows + 15) >> 4;
+    if (tile < tiles) {
+      break;
     }
+    tile -= tiles;
   }
   *part = p;
   *local = tile;

@@ -226,161 +226,31 @@ int BuildExpertBank(gufo_cuda_ctx* ctx, const gufo_cuda_expert_bank& bank, Exper
 
 namespace {
 
-// The grouped product of narrow Q4_K matrices (1, 2 or 4 blocks of 256 values a
-// row: an expert's down projection, 2048 x 512 here) with one fp32 input per
-// group. The 16-row x 8-block tiles of the fast GEMV leave six of eight warps
-// idle on such rows and pay an input conversion per tile; here sixteen lanes
-// take a block of a row (a lane: eight bytes of codes, i.e. eight values each of
-// the sub-blocks 2c and 2c + 1, with the sixteen inputs they meet held in
-// registers for all of the warp's rows), dequantize as the reference does
-// (w = d * sc * q - dmin * m, DequantQ4_K, src/core/quant.cpp:64-96) and reduce
-// over the row's lanes. `x` is plain, or [gate | up] per group when `swiglu`.
-struct NarrowArgs {
-  const uint8_t* w;      // experts stacked along the rows
-  int rows;              // of one expert
-  int row_bytes;
-  const int* ids;        // [groups], < 0: nothing to do
-  const float* x;
-  int x_stride;          // floats between the groups' inputs
-  int x_div;             // groups per input
-  int swiglu;
-  float* y;
-  int y_stride;          // floats between the groups' outputs
-};
-
-constexpr int kNarrowPasses = 8;   // rows (or row pairs) a warp multiplies, loads issued together
-
-__device__ __forceinline__ float NarrowSilu(float v) { return v * (1.0f / (1.0f + expf(-v))); }
-
-template <int BLOCKS>
-__global__ void __launch_bounds__(256)
-NarrowGroupedQ4K(const __grid_constant__ NarrowArgs a) {
-  constexpr int kSlots = 16 * BLOCKS;                       // lane slots a row
-  constexpr int kPer = kSlots > 32 ? kSlots / 32 : 1;       // slots a lane
-  constexpr int kRowsAtOnce = kSlots < 32 ? 32 / kSlots : 1;
-  constexpr int kWarpRows = kNarrowPasses * kRowsAtOnce;
-  GridLaunchDependents();
-  GridDependencyWait();   // the ids and the inputs come from earlier kernels
-  const int group = blockIdx.y;
-  const int id = a.ids[group];
-  if (id < 0) {
-    return;
-  }
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int first = (blockIdx.x * 8 + warp) * kWarpRows;
-  const uint8_t* matrix = a.w + static_cast<size_t>(id) * a.rows * a.row_bytes;
-  const float* x = a.x + static_cast<size_t>(group / (a.x_div > 1 ? a.x_div : 1)) * a.x_stride;
-  const int cols = 256 * BLOCKS;
-  // This lane's slots: block b, 32-byte chunk c of its codes, eight-byte part p.
-  int at[kPer];       // byte offset of the block in the row
-  int part[kPer];     // offset of the eight code bytes behind the block's 16-byte head
-  int pair[kPer];     // c: sub-blocks 2c (low nibbles) and 2c + 1 (high)
-  float lo[kPer][8], hi[kPer][8], lo_sum[kPer], hi_sum[kPer];
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int slot = (lane + 32 * j) % kSlots;
-    const int b = slot >> 4;
-    const int c = (slot >> 2) & 3;
-    const int p = slot & 3;
-    at[j] = b * kQ4KBytes;
-    part[j] = 32 * c + 8 * p;
-    pair[j] = c;
-    const int col = 256 * b + 64 * c + 8 * p;
-    lo_sum[j] = hi_sum[j] = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (a.swiglu) {
-        lo[j][i] = NarrowSilu(x[col + i]) * x[cols + col + i];
-        hi[j][i] = NarrowSilu(x[col + 32 + i]) * x[cols + col + 32 + i];
-      } else {
-        lo[j][i] = x[col + i];
-        hi[j][i] = x[col + 32 + i];
-      }
-      lo_sum[j] += lo[j][i];
-      hi_sum[j] += hi[j][i];
-    }
-  }
-  const int sub = kRowsAtOnce > 1 ? lane / kSlots : 0;   // which of the rows taken at once
-  uint4 head[kNarrowPasses][kPer];
-  uint2 codes[kNarrowPasses][kPer];
-#pragma unroll
-  for (int r = 0; r < kNarrowPasses; ++r) {
-    // Rows past the end repeat the last row; their sums are not stored.
-    const int row = min(first + r * kRowsAtOnce + sub, a.rows - 1);
-    const uint8_t* from = matrix + static_cast<size_t>(row) * a.row_bytes;
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      head[r][j] = *reinterpret_cast<const uint4*>(from + at[j]);
-      codes[r][j] = *reinterpret_cast<const uint2*>(from + at[j] + 16 + part[j]);
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < kNarrowPasses; ++r) {
-    float sum = 0.f;
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const float d = HalfBitsToFloat(static_cast<uint16_t>(head[r][j].x & 0xFFFF));
-      const float dmin = HalfBitsToFloat(static_cast<uint16_t>(head[r][j].x >> 16));
-      int sc_lo, m_lo, sc_hi, m_hi;
-      ScaleMinK4(2 * pair[j], head[r][j].y, head[r][j].z, head[r][j].w, &sc_lo, &m_lo);
-      ScaleMinK4(2 * pair[j] + 1, head[r][j].y, head[r][j].z, head[r][j].w, &sc_hi, &m_hi);
-      float dot_lo = 0.f, dot_hi = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t word = i < 4 ? codes[r][j].x : codes[r][j].y;
-        const uint32_t byte = (word >> (8 * (i & 3))) & 0xFFu;
-        dot_lo = fmaf(static_cast<float>(byte & 15u), lo[j][i], dot_lo);
-        dot_hi = fmaf(static_cast<float>(byte >> 4), hi[j][i], dot_hi);
-      }
-      sum += d * (static_cast<float>(sc_lo) * dot_lo + static_cast<float>(sc_hi) * dot_hi) -
-             dmin * (static_cast<float>(m_lo) * lo_sum[j] + static_cast<float>(m_hi) * hi_sum[j]);
-    }
-#pragma unroll
-    for (int o = kSlots < 32 ? kSlots / 2 : 16; o > 0; o >>= 1) {
-      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    }
-    const int row = first + r * kRowsAtOnce + sub;
-    if ((lane % (kSlots < 32 ? kSlots : 32)) == 0 && row < a.rows) {
-      a.y[static_cast<size_t>(group) * a.y_stride + row] = sum;
-    }
-  }
+// The down rows of `groups` inputs, each with k chosen experts (FastGemvArgs::mix_*).
+int LaunchDown(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids, const float* weights, const float* scale,
+               const float* shared, int groups, int k, const float* act, float* out) {
+  FastGemvArgs args{};
+  args.parts[0] = {bank.down.parts[0].data, bank.down.parts[0].rows, 0};
+  args.cols = k * bank.down.cols;
+  args.row_bytes = bank.down.parts[0].row_bytes;
+  args.x = act;
+  args.y = out;
+  args.y_stride = bank.hidden;
+  args.tokens = 1;
+  args.groups = groups;
+  args.mix_ids = ids;
+  args.mix_weights = weights;
+  args.mix_experts = k;
+  args.mix_blocks = bank.down.cols / kSuperBlock;
+  args.mix_base = shared;
+  args.mix_scale = scale;
+  return LaunchGemvMixture(ctx, args);
 }
 
-template <int BLOCKS>
-int LaunchNarrow(gufo_cuda_ctx* ctx, const NarrowArgs& args, int groups) {
-  constexpr int kSlots = 16 * BLOCKS;
-  constexpr int kBlockRows = 8 * kNarrowPasses * (kSlots < 32 ? 32 / kSlots : 1);
-  GUFO_CUDA_TRY(LaunchOverlapped(NarrowGroupedQ4K<BLOCKS>, dim3((args.rows + kBlockRows - 1) / kBlockRows, groups),
-                                 dim3(256), 0, ctx->stream, 1, args));
-  ctx->launches.fetch_add(1);
-  return GUFO_CUDA_OK;
-}
-
-// Whether the narrow kernel takes a grouped product of one Q4_K part.
-bool NarrowFits(const GemvArgs& g) {
-  const int blocks = g.cols / kSuperBlock;
-  return g.nparts == 1 && g.parts[0].type == GUFO_CUDA_Q4_K && g.cols % kSuperBlock == 0 &&
-         (blocks == 1 || blocks == 2 || blocks == 4);
-}
-
-int LaunchNarrowGrouped(gufo_cuda_ctx* ctx, const GemvArgs& g, bool swiglu) {
-  NarrowArgs args{};
-  args.w = g.parts[0].data;
-  args.rows = g.parts[0].rows;
-  args.row_bytes = g.parts[0].row_bytes;
-  args.ids = g.group_ids;
-  args.x = g.x;
-  args.x_stride = g.x_group_stride;
-  args.x_div = g.x_group_div;
-  args.swiglu = swiglu ? 1 : 0;
-  args.y = g.y + g.parts[0].out_offset;
-  args.y_stride = g.y_group_stride;
-  switch (g.cols / kSuperBlock) {
-    case 1: return LaunchNarrow<1>(ctx, args, g.groups);
-    case 2: return LaunchNarrow<2>(ctx, args, g.groups);
-    default: return LaunchNarrow<4>(ctx, args, g.groups);
-  }
+// Whether the mixture kernel takes the down rows of k experts at a time.
+bool DownFits(const gufo_cuda_ctx* ctx, const ExpertBank& bank, int k, const float* act) {
+  return !ctx->force_general && bank.down.parts[0].type == GUFO_CUDA_Q4_K && bank.down.cols % kSuperBlock == 0 &&
+         MixtureFits(k * bank.down.cols) && (reinterpret_cast<uintptr_t>(act) & 15) == 0;
 }
 
 }  // namespace
@@ -414,8 +284,8 @@ int EnqueueExpertFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids,
     }
     down.x = act;
     down.x_group_stride = bank.expert_ffn;
-    return NarrowFits(down) ? LaunchNarrowGrouped(ctx, down, false)
-                            : LaunchGemvGrouped(ctx, down, kProloguePlain, nullptr);
+    return DownFits(ctx, bank, 1, act) ? LaunchDown(ctx, bank, ids, nullptr, nullptr, nullptr, pairs, 1, act, y)
+                                       : LaunchGemvGrouped(ctx, down, kProloguePlain, nullptr);
   }
   int rc = LaunchGemvGrouped(ctx, in, kProloguePlain, nullptr);
   if (rc != GUFO_CUDA_OK) {
@@ -423,8 +293,7 @@ int EnqueueExpertFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids,
   }
   down.x = ffn;
   down.x_group_stride = 2 * bank.expert_ffn;
-  return NarrowFits(down) ? LaunchNarrowGrouped(ctx, down, true)
-                          : LaunchGemvGrouped(ctx, down, kPrologueSwiGlu, act);
+  return LaunchGemvGrouped(ctx, down, kPrologueSwiGlu, act);
 }
 
 int EnqueueMoeCombine(gufo_cuda_ctx* ctx, const float* shared, const float* scale, const float* weights,
@@ -453,9 +322,7 @@ int EnqueueMoeFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids, co
   in.x_group_stride = x_stride;
   in.x_group_div = k;
   in.y_group_stride = bank.expert_ffn;
-  GemvArgs down = bank.down;
-  if (down.parts[0].type == GUFO_CUDA_Q4_K && down.cols % kSuperBlock == 0 && MixtureFits(k * down.cols) &&
-      (reinterpret_cast<uintptr_t>(act) & 15) == 0 && GroupedSwiGluInProduct(ctx, in)) {
+  if (DownFits(ctx, bank, k, act) && GroupedSwiGluInProduct(ctx, in)) {
     // Two launches: gate / up with the SwiGLU in its epilogue, then the down rows of a
     // token's experts side by side with the weighted sum. Directly behind the router's
     // top-k (nothing else has been launched since, from any context) the inputs are
@@ -466,22 +333,7 @@ int EnqueueMoeFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids, co
     if (rc != GUFO_CUDA_OK) {
       return rc;
     }
-    FastGemvArgs args{};
-    args.parts[0] = {down.parts[0].data, down.parts[0].rows, 0};
-    args.cols = k * down.cols;
-    args.row_bytes = down.parts[0].row_bytes;
-    args.x = act;
-    args.y = out;
-    args.y_stride = bank.hidden;
-    args.tokens = 1;
-    args.groups = tokens;
-    args.mix_ids = ids;
-    args.mix_weights = weights;
-    args.mix_experts = k;
-    args.mix_blocks = down.cols / kSuperBlock;
-    args.mix_base = shared;
-    args.mix_scale = scale;
-    return LaunchGemvMixture(ctx, args);
+    return LaunchDown(ctx, bank, ids, weights, scale, shared, tokens, k, act, out);
   }
   const int rc = EnqueueExpertFfn(ctx, bank, ids, tokens * k, x, x_stride, k, ffn, act, expert_out);
   if (rc != GUFO_CUDA_OK) {

@@ -45,6 +45,7 @@ __device__ __forceinline__ void PeerSignal(const PeerOut& out) {
       mine[kSentWord + out.slot] = turn;
       mine[kTurnWord + out.slot] = turn;
       __threadfence_system();
+#pragma unroll 1
       for (int p = 0; p < out.world; ++p) {
         StoreReleaseSys(out.header[p] + kSlotFlags + 64 * out.slot + 8 * out.rank, turn);
       }
@@ -65,6 +66,7 @@ __device__ __forceinline__ void PeerWaitBlock(const PeerWait& w) {
     const unsigned turn = *reinterpret_cast<const volatile unsigned*>(w.header + kTurnWord + w.slot);
     const long long limit = *reinterpret_cast<const volatile unsigned*>(w.header + kErrorWord) != 0 ? 0 : w.limit;
     const long long start = clock64();
+#pragma unroll 1
     for (int p = 0; p < w.world; ++p) {
       const unsigned* flag = w.header + kSlotFlags + 64 * w.slot + 8 * p;
       // Flags only grow; the difference copes with the counter wrapping.
