@@ -239,9 +239,14 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
       ++req_n;
     }
   };
-  // A warp reads its fragments ahead of the block's barrier, so the slot is free for
-  // the slab kStages on as soon as the barrier has passed.
-  const int requested = min(kStages, my_slabs);
+  // One token: a warp reads its fragments ahead of the block's barrier, so the
+  // slot is free for the slab kStages on as soon as the barrier has passed.
+  // More tokens hold too many registers for that to pay (the two-token step ran
+  // 7 % slower with it): the barrier comes first and frees the slot of the slab
+  // before, for the slab kStages - 1 on.
+  constexpr bool kEarly = TOKENS == 1;
+  constexpr int kAhead = kEarly || ONE ? kStages : kStages - 1;
+  const int requested = min(kAhead, my_slabs);
   for (int q = 0; q < requested; ++q) {
     advance();
   }
@@ -328,7 +333,7 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
       if (a.peer_out.world > 0) {
         // Row-split ranks: this rank's rows go straight into every rank's copy
         // of the full vector (plain stores over NVLink for the peers).
-#pragma unroll 1
+#pragma unroll 1   // not in the decode step's way: unrolled it costs 4-layer steps 2 %
         for (int p = 0; p < a.peer_out.world; ++p) {
           a.peer_out.y[p][at] = total;
         }
@@ -346,47 +351,40 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   float held_gate = 0.f;
   auto gather = [&](int n) {
     const int o = threadIdx.x;
-    float total = o < kTileFloats ? total_of(n % kExchange, o) : 0.f;
-    if (ks > 1) {
-      float* slot_in_leader = cluster.map_shared_rank(peers, 0) + ((n & 1) * 8 + rank) * kTileFloats;
+    if (ks == 1) {
       if (o < kTileFloats) {
-        slot_in_leader[o] = total;
+        const float total = row_scale * total_of(n % kExchange, o);
+        if (a.epilogue != kEpilogueSwiGlu) {
+          store(n, o, total);
+        } else if ((n & 1) == 0) {
+          held_gate = total;
+        } else {
+          store(n, o, SiluFast(held_gate) * total);
+        }
       }
-      cluster.sync();
-      total = 0.f;
-#pragma unroll 1
-      for (int p = 0; p < ks && o < kTileFloats; ++p) {
-        total += peers[((n & 1) * 8 + p) * kTileFloats + o];
-      }
+      return;
     }
-    total *= row_scale;
-    bool mine = rank == 0 && o < kTileFloats;
-    if (a.epilogue == kEpilogueSwiGlu) {
-      if ((n & 1) == 0) {
-        held_gate = total;
-        mine = false;
-      } else {
-        total *= SiluFast(held_gate);
-      }
+    float total = o < kTileFloats ? total_of(n % kExchange, o) : 0.f;
+    float* slot_in_leader = cluster.map_shared_rank(peers, 0) + ((n & 1) * 8 + rank) * kTileFloats;
+    if (o < kTileFloats) {
+      slot_in_leader[o] = total;
     }
-    if (mine) {
-      store(n, o, total);
+    cluster.sync();
+    if (rank != 0 || o >= kTileFloats) {
+      return;
     }
+    total = 0.f;
+    for (int p = 0; p < ks; ++p) {
+      total += peers[((n & 1) * 8 + p) * kTileFloats + o];
+    }
+    store(n, o, row_scale * total);
   };
   clear();
   int n = 0, s = 0;   // tile and own-slab index being multiplied
-  // One turn more than there are slabs: behind the last, its tile's row sums are left.
-#pragma unroll 1
-  for (int q = 0; q <= my_slabs; ++q) {
-    const bool last = q == my_slabs;
-    const int slab = rank + s * ks;
-    const int nblk = min(8, blocks - slab * 8);
-    const int b = slab * 8 + warp;
-    const bool mine = !last && warp < nblk && a.variant != 1;
-    typename std::conditional<kQ4, q4k::Q4KUnit, q6k::Q6KUnit>::type unit;
-    if (!last) {
-      // Slab q has landed when its barrier's phase completes (bounded: the copies
-      // were issued by this block; a wait that runs out gives the slab up).
+  for (int q = 0; q < my_slabs; ++q) {
+    // Slab q has landed when its barrier's phase completes (bounded: the copies
+    // were issued by this block; a wait that runs out gives the slab up).
+    {
       const uint32_t bar = SharedAddress(&landed[q % kStages]);
       const uint32_t parity = (q / kStages) & 1u;
       if (!MbarTryWait(bar, parity)) {
@@ -394,30 +392,40 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
         while (!MbarTryWait(bar, parity) && clock64() - start < kLandLimit) {
         }
       }
-      const uint8_t* data = ring + (q % kStages) * S::kBytes;
-      if (mine) {
-        if constexpr (kQ4) {
-          q4k::LoadUnit(unit, data, warp, g, t);
-        } else {
-          q6k::LoadUnit(unit, data, warp, nblk, g, t);
+    }
+    const int slab = rank + s * ks;
+    const int nblk = min(8, blocks - slab * 8);
+    const int b = slab * 8 + warp;
+    const bool mine = warp < nblk && a.variant != 1;
+    const uint8_t* data = ring + (q % kStages) * S::kBytes;
+    typename std::conditional<kQ4, q4k::Q4KUnit, q6k::Q6KUnit>::type unit;
+    // The block's barrier: behind it a ring slot is free (every warp is done with
+    // its slab: read into registers, or multiplied) and the row sums of the tile
+    // before are in the exchange buffer. Warp q % 8 requests the next slab.
+    auto meet = [&]() {
+      __syncthreads();
+      if (q + kAhead < my_slabs) {
+        if (warp == (q & 7)) {
+          issue(q + kAhead, req_n, req_s);
         }
+        advance();
+      }
+      if (s == 0 && n > 0) {
+        gather(n - 1);
+      }
+    };
+    if constexpr (!kEarly) {
+      meet();
+    }
+    if (mine) {
+      if constexpr (kQ4) {
+        q4k::LoadUnit(unit, data, warp, g, t);
+      } else {
+        q6k::LoadUnit(unit, data, warp, nblk, g, t);
       }
     }
-    // The block's barrier: behind it the ring slot is free (every warp has read its
-    // fragments) and the row sums of the tile before are in the exchange buffer. Warp
-    // q % 8 requests the next slab.
-    __syncthreads();
-    if (q + kStages < my_slabs) {
-      if (warp == (q & 7)) {
-        issue(q + kStages, req_n, req_s);
-      }
-      advance();
-    }
-    if (s == 0 && n > 0) {
-      gather(n - 1);
-    }
-    if (last) {
-      break;
+    if constexpr (kEarly) {
+      meet();
     }
     if (mine) {
       if constexpr (kQ4) {
@@ -502,6 +510,10 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     } else {
       ++s;
     }
+  }
+  if (my_tiles > 0) {
+    __syncthreads();
+    gather(my_tiles - 1);
   }
   if (a.peer_out.world > 0) {
     PeerSignal(a.peer_out);

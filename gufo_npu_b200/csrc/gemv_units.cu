@@ -87,7 +87,7 @@ size_t SharedBytes(int cols, int depth) {
 // before, a warp per row and expert in fp32, spent its time in conversions and in
 // staging the activated inputs once per eight rows. Together with several tile pairs a
 // block in the gate / up product, a layer of 256 experts of 512 x 2048, eight of them
-// for each of four tokens: 34.4 -> @@MOE@@ us.)
+// for each of four tokens: 34.4 -> 21.7 us.)
 template <int TYPE, int TOKENS, int PER_SM, bool MIX = false>
 __global__ void __launch_bounds__(kFastThreads, PER_SM)
 GemvUnits(const __grid_constant__ FastGemvArgs a) {

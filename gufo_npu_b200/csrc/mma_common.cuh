@@ -225,10 +225,17 @@ __device__ __forceinline__ float SiluFast(float x) { return x * (1.0f / (1.0f + 
 // once, and block-wide reductions that nothing hides. So a norm's 1 / rms is not
 // in the image: the planes are those of (h + delta) * w, and the kernel multiplies
 // its row sums by 1 / rms (RowScale) when it stores them. The sum of squares then
-// costs no barrier of its own, units are independent of one another, and with one
-// or two tokens the loads of two units (three of a plain row) are in flight
-// together; more tokens hold too many registers elsewhere in the kernel.
-// Eight tokens of the 24-layer, 2048-wide decoder: 6.35 -> 6.15 ms.
+// costs no barrier of its own, and units are independent of one another. Eight
+// tokens of the 24-layer, 2048-wide decoder: 6.35 -> 6.15 ms.
+//
+// And the size of the code: in a step whose kernels alternate, what runs once is
+// fetched through the instruction caches at every start. With two tokens the loads of
+// two units are in flight together, at the price of two copies of the conversion; with
+// one token, where a row of 2048 values is one unit a warp, the copies (two, and three
+// for a plain row) made the kernel 100 KB instead of 72: the decoder's eight tokens
+// took 5.85 instead of 5.6 ms, the 4-layer one's 760 instead of 700 us. (One loop for
+// both kinds of input, a single conversion: slower again, 5.98 ms, as the norm's path
+// then jumps over the activation's code.)
 
 // The norm weights of the calling warp's first unit, for FillImage: they never
 // depend on an earlier kernel, so a kernel asks for them before it waits for its
@@ -326,7 +333,7 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
   if (a.prologue == kPrologueResNorm) {
     // vec::RmsNorm (src/core/vec.hpp:57-63) of the residual stream after its
     // pending add (src/models/qwen35/decoder.cpp:493,504-508).
-    constexpr int kBatch = 1;
+    constexpr int kBatch = TOKENS == 2 ? 2 : 1;
     if (lane < TOKENS) {
       squares[warp * TOKENS + lane] = 0.f;
     }
@@ -438,9 +445,7 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
   }
   const bool act = a.prologue == kPrologueSwiGlu;
   const size_t stride = act ? 2 * static_cast<size_t>(n) : static_cast<size_t>(n);
-  // All loads of a batch are in flight before the first value is used: one round
-  // trip per batch, not per block (a 6144-value input is three blocks per warp).
-  constexpr int kBatch = 1;
+  constexpr int kBatch = TOKENS == 2 ? 2 : 1;
 #pragma unroll 1
   while (live()) {
     float v[kBatch][8], up[kBatch][8];
@@ -477,13 +482,14 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
 }
 
 // Tiles of 16 rows are numbered across the parts of a launch, each part
-// rounded up to whole tiles. (Rolled loops, here and wherever else code is not in a
-// kernel's inner loop: see the note on code size at FillImage.)
+// rounded up to whole tiles.
 __device__ __forceinline__ int TotalTiles(const FastGemvArgs& a) {
   int tiles = 0;
-#pragma unroll 1
-  for (int p = 0; p < a.nparts; ++p) {
-    tiles += (a.parts[p].rows + 15) >> 4;
+#pragma unroll
+  for (int p = 0; p < kFastMaxParts; ++p) {
+    if (p < a.nparts) {
+      tiles += (a.parts[p].rows + 15) >> 4;
+    }
   }
   return tiles;
 }
@@ -491,13 +497,13 @@ __device__ __forceinline__ int TotalTiles(const FastGemvArgs& a) {
 // Part and tile-within-part of global tile `tile`.
 __device__ __forceinline__ void LocateTile(const FastGemvArgs& a, int tile, int* part, int* local) {
   int p = 0;
-#pragma unroll 1
-  for (; p + 1 < a.nparts; ++p) {
-    const int tiles = (a.parts[p].rows + 15) >> 4;
-    if (tile < tiles) {
-      break;
+#pragma unroll
+  for (int i = 0; i < kFastMaxParts - 1; ++i) {
+    const int tiles = (a.parts[i].rows + 15) >> 4;
+    if (p == i && i + 1 < a.nparts && tile >= tiles) {
+      tile -= tiles;
+      p = i + 1;
     }
-    tile -= tiles;
   }
   *part = p;
   *local = tile;
