@@ -8,15 +8,14 @@
 // algorithmic traffic is 2 * dk * dk * 4 bytes per head, the HBM roofline of
 // this kernel. Columns of S evolve independently
 // (src/models/qwen35/prefill_mixer.cpp:662-667), so one thread block takes one
-// (sequence, value head) and each of its warps one tile of 32 columns.
+// (sequence, value head) and each of its eight warps one tile of 16 columns.
 //
-// Warp layout: lane = 8 * ig + jq; jq owns four adjacent columns (one float4),
-// ig owns rows ig, ig + 4, ..., so one load instruction of a warp covers four
-// 128-byte row segments. A lane keeps its dk / 4 float4 of S (128 registers at
-// dk = 128) from the loads to the stores: all of a tile's state is requested
-// from HBM at once, the column sums of the two passes need only two shuffle
-// steps, and the block meets just once, for the gated RMSNorm over the head's
-// dk outputs.
+// Warp layout: lane = 4 * ig + jq; jq owns four adjacent columns (one float4), ig
+// owns rows ig, ig + 8, ..., so one load instruction of a warp covers eight 64-byte
+// row segments. A lane keeps its dk / 8 float4 of S (64 registers at dk = 128) from
+// the loads to the stores: all of a tile's state is requested from HBM at once, the
+// column sums need three shuffle steps, and the block meets just once more, for the
+// gated RMSNorm over the head's dk outputs.
 #include "common.cuh"
 
 #include <vector>

@@ -5,8 +5,9 @@
 // A decode batch hands over dozens of tensors per call, and through ctypes each
 // of them cost an attribute lookup, a method call and a wrapped integer: 100 us
 // of Python for a mixer step of 32 sequences whose kernels take 44 us, 19 us for
-// an 8-sequence DeltaNet update of 4 us; here both are hidden behind the kernels. Only the
-// calls of the per-token path come through this file; set-up stays with ctypes.
+// an 8-sequence DeltaNet update of 4 us; here both are hidden behind the kernels.
+// Only the calls of the per-token path come through this file; set-up stays with
+// ctypes.
 // Every function returns the C ABI's status, which the caller turns into an
 // exception, and runs the call itself without the interpreter lock, as ctypes
 // does. bind() takes the handle of the already loaded library, so nothing here
