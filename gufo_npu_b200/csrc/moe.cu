@@ -88,10 +88,13 @@ RouteKernel(const float* __restrict__ logits, int stride, int experts, int k,
 #pragma unroll
   for (int j = 0; j < PER_LANE; ++j) {
     const int e = lane + 32 * j;
-    const double prob = e < experts ? shared_prob[e] : -1.0;
-    total += e < experts ? prob : 0.0;
-    key[j] = static_cast<unsigned long long>(__double_as_longlong(prob));
-    left |= prob >= 0.0 ? 1u << j : 0u;
+    const double prob = e < experts ? shared_prob[e] : 0.0;
+    total += prob;
+    // A NaN (of a NaN or an infinite logit) ranks with the zeros: the ids stay below
+    // `experts` whatever the logits, as the products that follow address by them. The
+    // row's total is NaN then, and so is every weight.
+    key[j] = prob >= 0.0 ? static_cast<unsigned long long>(__double_as_longlong(prob)) : 0ull;
+    left |= e < experts ? 1u << j : 0u;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {

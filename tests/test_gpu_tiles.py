@@ -251,6 +251,27 @@ def test_route_ties_and_counts(ctx, oracle, experts, k):
         assert rel_l2(weights[t].cpu().numpy(), picked / max(picked.sum(), 6.103515625e-5)) <= 1e-6
 
 
+@pytest.mark.parametrize("experts,k", [(7, 7), (64, 8), (300, 8)])
+def test_route_of_logits_that_are_not_finite(ctx, experts, k):
+    """The ids stay distinct and below `experts` (the products address by them); the weights are NaN."""
+    dev = torch.device("cuda:0")
+    nan, inf = float("nan"), float("inf")
+    logits = torch.randn(6, experts + 1, device=dev, generator=torch.Generator(device=dev).manual_seed(experts))
+    logits[0, :experts] = nan
+    logits[1, 3] = nan
+    logits[2, 5] = inf
+    logits[3, :experts - 2] = nan
+    logits[4, :experts] = -inf
+    chosen = torch.full((6, k), -7, dtype=torch.int32, device=dev)
+    weights, scale = torch.zeros(6, k, device=dev), torch.zeros(6, device=dev)
+    torch.cuda.synchronize()
+    ctx.route_device(logits, experts + 1, 6, experts, k, chosen, weights, scale)
+    ctx.synchronize()
+    for row in chosen.cpu().tolist():
+        assert min(row) >= 0 and max(row) < experts and len(set(row)) == k
+    assert weights[:5].isnan().all() and torch.isfinite(weights[5]).all() and torch.isfinite(scale).all()
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim,rope_dim", [(8, 1, 64, 64), (3, 3, 128, 32), (16, 4, 256, 64),
                                                               (2, 1, 256, 0), (5, 1, 128, 128)])
 @pytest.mark.parametrize("positions", [1, 2, 17, 64, 65, 128, 129, 193, 1000, 4099, 9001])
