@@ -245,6 +245,12 @@ class Context:
         self._check(_capi.native.moe_ffn(self._address, bank, ids, weights, scale, tokens, k, x, x_stride, shared, ffn,
                                          act, expert_out, out))
 
+    def moe_layer_device(self, bank: "_capi.ExpertBank", router, stride: int, tokens: int, k: int, chosen, weights,
+                         scale, x, x_stride: int, shared, ffn, act, expert_out, out) -> None:
+        """route_device and moe_ffn_device on what it chose, in one call (device tensors)."""
+        self._check(_capi.native.moe_layer(self._address, bank, router, stride, tokens, k, chosen, weights, scale, x,
+                                           x_stride, shared, ffn, act, expert_out, out))
+
     def moe_combine_device(self, shared, scale, weights, expert_out, tokens: int, k: int, hidden: int, out) -> None:
         self._check(self.lib.gufo_cuda_moe_combine_device(self.handle, C.c_void_p(_ptr(shared)),
                                                           C.c_void_p(_ptr(scale)), C.c_void_p(_ptr(weights)),
@@ -538,12 +544,14 @@ class CudaMoe:
         """out[t] = shared[t] * scale + sum of the routed experts' outputs (device tensors)."""
         if tokens > self.max_tokens:
             raise ValueError("CudaMoe: more tokens than max_tokens")
-        self.route(layer, normed, tokens)
         if self.expert_range is None:
             c = self.config
-            self.ctx.moe_ffn_device(self.banks[layer], self.chosen, self.weights, self.scale, tokens, c.experts_used,
-                                    normed, c.hidden, shared, self.ffn, self.act, self.expert_out, out)
+            self.projections.apply_device(Stage.kRouter, layer, normed, tokens, self.router)
+            self.ctx.moe_layer_device(self.banks[layer], self.router, c.experts + 1, tokens, c.experts_used, self.chosen,
+                                      self.weights, self.scale, normed, c.hidden, shared, self.ffn, self.act,
+                                      self.expert_out, out)
             return
+        self.route(layer, normed, tokens)
         self.experts(layer, normed, tokens)
         self.combine(shared, tokens, out)
 

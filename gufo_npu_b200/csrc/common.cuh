@@ -327,9 +327,6 @@ struct gufo_cuda_ctx {
   // previous product (wrong results unless x is unchanged).
   bool reuse_image = false;
   int gemv_variant = 0;
-  // LaunchCount and the stream right after the last router top-k.
-  uint64_t route_launch = ~0ull;
-  cudaStream_t route_stream = nullptr;
   // The caller's promise that DeltaNet states passed to this context were not
   // written by the two kernels enqueued just before the call.
   bool early_state = false;
@@ -368,13 +365,6 @@ struct gufo_cuda_ctx {
 
 namespace gufo {
 
-// Launches that may overlap their predecessor, over all contexts: two equal readings
-// say that none has come in between.
-inline std::atomic<uint64_t>& LaunchCount() {
-  static std::atomic<uint64_t> count{0};
-  return count;
-}
-
 // Launches `kernel` so that it may begin while the previous kernel in the
 // stream is still draining (programmatic dependent launch). Such a kernel must
 // execute GridDependencyWait() before it reads anything an earlier kernel
@@ -403,7 +393,6 @@ cudaError_t LaunchOverlapped(void (*kernel)(KernelArgs...), dim3 grid, dim3 bloc
   }
   config.attrs = attr;
   config.numAttrs = n;
-  LaunchCount().fetch_add(1);
   return cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
 }
 

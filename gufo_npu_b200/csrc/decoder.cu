@@ -664,7 +664,7 @@ int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens) 
       GUFO_STEP_TRY(EnqueueRoute(ctx, d->router, c.experts + 1, tokens, c.experts, c.experts_used, d->chosen,
                                  d->route_weights, d->shared_scale));
       GUFO_STEP_TRY(EnqueueMoeFfn(ctx, l.bank, d->chosen, d->route_weights, d->shared_scale, tokens, c.experts_used,
-                                  d->normed, c.hidden, d->out, d->expert_ffn, d->expert_act, d->expert_out, d->out));
+                                  d->normed, c.hidden, d->out, d->expert_ffn, d->expert_act, d->expert_out, d->out, true));
     }
     Mark(d, GUFO_CUDA_TIMELINE_FFN_DOWN);
     pending = d->out;

@@ -163,7 +163,7 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   size_t matrix = 0;
   // The ids come from an earlier kernel. Where that one lets this grid start only
   // after it has itself waited for everything before it (early_input: the router's
-  // top-k), the inputs are complete already, and the image is built while the ids
+  // top-k, enqueued in the same call), the inputs are complete already, and the image is built while the ids
   // are still being found. The dependents (the down product) start behind this
   // wait: they may read the ids and the weights ahead of their own.
   auto choose = [&]() {

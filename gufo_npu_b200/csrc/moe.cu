@@ -175,8 +175,6 @@ int EnqueueRoute(gufo_cuda_ctx* ctx, const float* logits, int stride, int tokens
                                    stride, experts, k, chosen, weights, shared_scale));
   }
   ctx->launches.fetch_add(1);
-  ctx->route_launch = LaunchCount().load();
-  ctx->route_stream = ctx->stream;
   return GUFO_CUDA_OK;
 }
 
@@ -312,7 +310,7 @@ int EnqueueMoeCombine(gufo_cuda_ctx* ctx, const float* shared, const float* scal
 
 int EnqueueMoeFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids, const float* weights,
                   const float* scale, int tokens, int k, const float* x, int x_stride, const float* shared,
-                  float* ffn, float* act, float* expert_out, float* out) {
+                  float* ffn, float* act, float* expert_out, float* out, bool behind_route) {
   if (tokens <= 0 || k <= 0 || ids == nullptr || weights == nullptr || scale == nullptr || x == nullptr ||
       shared == nullptr || ffn == nullptr || act == nullptr || expert_out == nullptr || out == nullptr) {
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "moe ffn: null pointer or no tokens");
@@ -328,10 +326,10 @@ int EnqueueMoeFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids, co
   if (DownFits(ctx, bank, k, act) && GroupedSwiGluInProduct(ctx, in)) {
     // Two launches: gate / up with the SwiGLU in its epilogue, then the down rows of a
     // token's experts side by side with the weighted sum. Directly behind the router's
-    // top-k (nothing else has been launched since, from any context) the inputs are
-    // complete once the first of them runs; its image is built while the top-k is
-    // being found. It lets the second start only once the ids are complete.
-    in.early_input = ctx->route_launch == LaunchCount().load() && ctx->route_stream == ctx->stream ? 1 : 0;
+    // top-k the inputs are complete once the first of them runs (RouteKernel), and its
+    // image is built while the top-k is being found. It lets the second start only once
+    // the ids are complete.
+    in.early_input = behind_route ? 1 : 0;
     const int rc = LaunchGemvGrouped(ctx, in, kProloguePlain, nullptr, true);
     if (rc != GUFO_CUDA_OK) {
       return rc;
@@ -407,7 +405,37 @@ int gufo_cuda_moe_ffn_device(gufo_cuda_ctx* ctx, const gufo_cuda_expert_bank* ba
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "moe ffn: x_stride is 0 (shared input) or at least hidden");
   }
   return gufo::EnqueueMoeFfn(ctx, built, ids, weights, scale, tokens, k, x, static_cast<int>(x_stride), shared, ffn,
-                             act, expert_out, out);
+                             act, expert_out, out, false);
+}
+
+int gufo_cuda_moe_layer_device(gufo_cuda_ctx* ctx, const gufo_cuda_expert_bank* bank, const float* router, int stride,
+                               int tokens, int k, int* chosen, float* weights, float* scale, const float* x,
+                               int64_t x_stride, const float* shared, float* ffn, float* act, float* expert_out,
+                               float* out) {
+  if (ctx == nullptr || bank == nullptr || router == nullptr || chosen == nullptr || weights == nullptr ||
+      scale == nullptr || x == nullptr || shared == nullptr || ffn == nullptr || act == nullptr ||
+      expert_out == nullptr || out == nullptr) {
+    return Fail(GUFO_CUDA_BAD_ARGUMENT, "moe layer: null pointer");
+  }
+  std::lock_guard<std::mutex> lock(ctx->mu);
+  GUFO_CUDA_TRY(cudaSetDevice(ctx->device));
+  gufo::ExpertBank built;
+  int rc = gufo::BuildExpertBank(ctx, *bank, &built);
+  if (rc != GUFO_CUDA_OK) {
+    return rc;
+  }
+  if (stride < bank->experts + 1) {
+    return Fail(GUFO_CUDA_BAD_ARGUMENT, "moe layer: the shared expert's logit follows the experts'");
+  }
+  if (x_stride != 0 && x_stride < bank->hidden) {
+    return Fail(GUFO_CUDA_BAD_ARGUMENT, "moe layer: x_stride is 0 (shared input) or at least hidden");
+  }
+  rc = gufo::EnqueueRoute(ctx, router, stride, tokens, bank->experts, k, chosen, weights, scale);
+  if (rc != GUFO_CUDA_OK) {
+    return rc;
+  }
+  return gufo::EnqueueMoeFfn(ctx, built, chosen, weights, scale, tokens, k, x, static_cast<int>(x_stride), shared, ffn,
+                             act, expert_out, out, true);
 }
 
 int gufo_cuda_moe_combine_device(gufo_cuda_ctx* ctx, const float* shared, const float* scale, const float* weights,

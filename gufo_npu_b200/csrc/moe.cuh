@@ -34,10 +34,11 @@ int EnqueueMoeCombine(gufo_cuda_ctx* ctx, const float* shared, const float* scal
 // sum of the k chosen experts' FFN of x_t (x_t = x + t * x_stride). Two launches
 // where the bank's shapes allow (Q4_K, and k * expert_ffn values fit a thread block's
 // image): the gate / up product with its SwiGLU, and the down rows with the weighted
-// sum; otherwise
-// EnqueueExpertFfn and EnqueueMoeCombine through `ffn` and `expert_out`.
+// sum; otherwise EnqueueExpertFfn and EnqueueMoeCombine through `ffn` and `expert_out`.
+// `behind_route`: the caller enqueued EnqueueRoute for these ids just before, in the
+// same call, with nothing in between.
 int EnqueueMoeFfn(gufo_cuda_ctx* ctx, const ExpertBank& bank, const int* ids, const float* weights,
                   const float* scale, int tokens, int k, const float* x, int x_stride, const float* shared,
-                  float* ffn, float* act, float* expert_out, float* out);
+                  float* ffn, float* act, float* expert_out, float* out, bool behind_route);
 
 }  // namespace gufo

@@ -30,6 +30,7 @@ struct Api {
   decltype(&gufo_cuda_deltanet_step_device) deltanet_step;
   decltype(&gufo_cuda_route_device) route;
   decltype(&gufo_cuda_moe_ffn_device) moe_ffn;
+  decltype(&gufo_cuda_moe_layer_device) moe_layer;
   decltype(&gufo_cuda_decoder_step) decoder_step;
   decltype(&gufo_cuda_decoder_step_tokens) decoder_step_tokens;
   decltype(&gufo_cuda_host_take) host_take;
@@ -337,24 +338,29 @@ PyObject* Route(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+gufo_cuda_expert_bank Bank(PyObject* o) {
+  gufo_cuda_expert_bank bank;
+  Py_buffer view;
+  if (PyObject_GetBuffer(o, &view, PyBUF_SIMPLE) != 0) {
+    throw Failed();
+  }
+  const bool fits = view.len == static_cast<Py_ssize_t>(sizeof(bank));
+  if (fits) {
+    bank = *static_cast<const gufo_cuda_expert_bank*>(view.buf);
+  }
+  PyBuffer_Release(&view);
+  if (!fits) {
+    PyErr_SetString(PyExc_TypeError, "gufo_cuda: an ExpertBank is needed");
+    throw Failed();
+  }
+  return bank;
+}
+
 // moe_ffn(ctx, bank, ids, weights, scale, tokens, k, x, x_stride, shared, ffn, act, expert_out, out)
 PyObject* MoeFfn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return Guarded(n, 14, [&] {
     gufo_cuda_ctx* ctx = Context(a[0]);
-    gufo_cuda_expert_bank bank;
-    Py_buffer view;
-    if (PyObject_GetBuffer(a[1], &view, PyBUF_SIMPLE) != 0) {
-      throw Failed();
-    }
-    const bool fits = view.len == static_cast<Py_ssize_t>(sizeof(bank));
-    if (fits) {
-      bank = *static_cast<const gufo_cuda_expert_bank*>(view.buf);
-    }
-    PyBuffer_Release(&view);
-    if (!fits) {
-      PyErr_SetString(PyExc_TypeError, "gufo_cuda: an ExpertBank is needed");
-      throw Failed();
-    }
+    const gufo_cuda_expert_bank bank = Bank(a[1]);
     const int* ids = Ptr<const int>(a[2]);
     const float *weights = Ptr<const float>(a[3]), *scale = Ptr<const float>(a[4]);
     const int tokens = SmallInt(a[5]), k = SmallInt(a[6]);
@@ -364,6 +370,26 @@ PyObject* MoeFfn(PyObject*, PyObject* const* a, Py_ssize_t n) {
     float *ffn = Ptr<float>(a[10]), *act = Ptr<float>(a[11]), *expert_out = Ptr<float>(a[12]), *out = Ptr<float>(a[13]);
     return Unlocked([&] {
       return api.moe_ffn(ctx, &bank, ids, weights, scale, tokens, k, x, x_stride, shared, ffn, act, expert_out, out);
+    });
+  });
+}
+
+// moe_layer(ctx, bank, router, stride, tokens, k, chosen, weights, scale, x, x_stride, shared, ffn, act, expert_out, out)
+PyObject* MoeLayer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return Guarded(n, 16, [&] {
+    gufo_cuda_ctx* ctx = Context(a[0]);
+    const gufo_cuda_expert_bank bank = Bank(a[1]);
+    const float* router = Ptr<const float>(a[2]);
+    const int stride = SmallInt(a[3]), tokens = SmallInt(a[4]), k = SmallInt(a[5]);
+    int* chosen = Ptr<int>(a[6]);
+    float *weights = Ptr<float>(a[7]), *scale = Ptr<float>(a[8]);
+    const float* x = Ptr<const float>(a[9]);
+    const long long x_stride = Int(a[10]);
+    const float* shared = Ptr<const float>(a[11]);
+    float *ffn = Ptr<float>(a[12]), *act = Ptr<float>(a[13]), *expert_out = Ptr<float>(a[14]), *out = Ptr<float>(a[15]);
+    return Unlocked([&] {
+      return api.moe_layer(ctx, &bank, router, stride, tokens, k, chosen, weights, scale, x, x_stride, shared, ffn, act,
+                           expert_out, out);
     });
   });
 }
@@ -460,6 +486,7 @@ PyObject* Bind(PyObject*, PyObject* handle) {
   find(&api.deltanet_step, "gufo_cuda_deltanet_step_device");
   find(&api.route, "gufo_cuda_route_device");
   find(&api.moe_ffn, "gufo_cuda_moe_ffn_device");
+  find(&api.moe_layer, "gufo_cuda_moe_layer_device");
   find(&api.decoder_step, "gufo_cuda_decoder_step");
   find(&api.decoder_step_tokens, "gufo_cuda_decoder_step_tokens");
   find(&api.host_take, "gufo_cuda_host_take");
@@ -480,6 +507,7 @@ PyMethodDef methods[] = {
     FAST("deltanet_step", DeltaNetStep),
     FAST("route", Route),
     FAST("moe_ffn", MoeFfn),
+    FAST("moe_layer", MoeLayer),
     FAST("decoder_step", DecoderStep),
     FAST("decoder_step_tokens", DecoderStepTokens),
     FAST("host_buffer", NewHostBuffer),

@@ -462,6 +462,18 @@ int gufo_cuda_moe_ffn_device(gufo_cuda_ctx* ctx,
                              const float* shared, float* ffn, float* act,
                              float* expert_out, float* out);
 
+/* gufo_cuda_route_device (bank->experts experts; stride at least one more) and
+ * gufo_cuda_moe_ffn_device on what it chose, in one call: the same results. As
+ * nothing can come between the two, the products start on x while the top-k is
+ * still being found. */
+int gufo_cuda_moe_layer_device(gufo_cuda_ctx* ctx,
+                               const gufo_cuda_expert_bank* bank,
+                               const float* router, int stride, int tokens, int k,
+                               int* chosen, float* weights, float* scale,
+                               const float* x, int64_t x_stride,
+                               const float* shared, float* ffn, float* act,
+                               float* expert_out, float* out);
+
 /* out[t] = shared[t] * scale[t] + sum over slots, in slot order, of
  * weights[t][slot] * expert_out[t][slot] (decoder.cpp:541-556). out may be
  * shared. */

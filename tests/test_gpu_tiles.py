@@ -362,6 +362,50 @@ def test_activating_product_with_more_tile_pairs_than_blocks(ctx, tokens, rows, 
     ctx.matrix_free(mu)
 
 
+def test_experts_read_what_the_caller_wrote_behind_the_route():
+    """The caller's own kernels write x between the route and the products, on one stream; and the
+    two in one call: the same bits as with everything in place beforehand."""
+    from gufo_npu_b200 import _capi
+    dev = torch.device("cuda:0")
+    tokens, k, hidden, ffn, experts = 4, 8, 2048, 512, 16
+    stream = torch.cuda.Stream()
+    own = Context(0, stream.cuda_stream)
+    bank = _capi.ExpertBank(*[_matrix(own, Q.GGML_Q4_K, rows * experts, cols, seed)[0]
+                              for seed, rows, cols in ((1, ffn, hidden), (2, ffn, hidden), (3, hidden, ffn))],
+                            experts, ffn, hidden)
+    gen = torch.Generator(device=dev).manual_seed(3)
+    rounds = 24
+    logits, xs = (torch.randn(rounds, tokens, w, device=dev, generator=gen) for w in (experts + 1, hidden))
+    shared = torch.randn(tokens, hidden, device=dev, generator=gen)
+    chosen, weights = torch.empty(tokens, k, dtype=torch.int32, device=dev), torch.empty(tokens, k, device=dev)
+    scale = torch.empty(tokens, device=dev)
+    buf, act, eo = (torch.empty(tokens * k, w, device=dev) for w in (2 * ffn, ffn, hidden))
+    got, one, want = (torch.empty(rounds, tokens, hidden, device=dev) for _ in range(3))
+    x = torch.zeros(tokens, hidden, device=dev)
+    torch.cuda.synchronize()
+
+    def experts_of(x, out):
+        own.moe_ffn_device(bank, chosen, weights, scale, tokens, k, x, hidden, shared, buf, act, eo, out)
+    with torch.cuda.stream(stream):
+        for r in range(rounds):
+            own.route_device(logits[r], experts + 1, tokens, experts, k, chosen, weights, scale)
+            stream.synchronize()
+            experts_of(xs[r], want[r])
+        for r in range(rounds):
+            own.route_device(logits[r], experts + 1, tokens, experts, k, chosen, weights, scale)
+            torch.mul(xs[r], 1.0, out=x)
+            experts_of(x, got[r])
+            x.zero_()
+        for r in range(rounds):
+            torch.mul(xs[r], 1.0, out=x)
+            own.moe_layer_device(bank, logits[r], experts + 1, tokens, k, chosen, weights, scale, x, hidden, shared, buf,
+                                 act, eo, one[r])
+            x.zero_()
+    stream.synchronize()
+    assert torch.equal(got, want) and torch.equal(one, want)
+    own.close()
+
+
 @pytest.mark.parametrize("tokens,k,hidden,ffn,experts", [(1, 1, 256, 256, 4), (3, 3, 1280, 768, 7), (5, 8, 2048, 512, 16),
                                                          (16, 4, 1536, 256, 64)])
 def test_mixture_of_given_experts(ctx, tokens, k, hidden, ffn, experts):
