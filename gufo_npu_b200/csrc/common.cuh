@@ -265,17 +265,18 @@ struct DeltaNetSeq {
   float* y;                // [tokens], y_stride apart
   int64_t in_stride, x_stride, y_stride;
   int tokens;
-  const float* gates;      // [tokens][2 value heads]: alpha | beta, or null (behind z in the input row)
+  const float* gates;      // where its tokens' gate dots are given, gates_stride apart (set by the launcher)
+  int64_t gates_stride;
 };
 inline DeltaNetSeq OneTokenSeq(const float* in, const float* x, const float* conv_in, float* conv_out, const float* ssm_in,
                                float* ssm_out, float* y) {
-  return {in, x, conv_in, nullptr, conv_out, ssm_in, nullptr, ssm_out, y, 0, 0, 0, 1, nullptr};
+  return {in, x, conv_in, nullptr, conv_out, ssm_in, nullptr, ssm_out, y, 0, 0, 0, 1, nullptr, 0};
 }
 // Mixer::Linear for every sequence (1 to 4 tokens each); the caller holds ctx->mu.
 // `early_state`: the states and conv windows were not written by the kernels
 // shortly before this one in the stream (several may be in flight at once), so
 // their loads may run ahead of the dependency wait.
-int EnqueueDeltaNetLinear(gufo_cuda_ctx* ctx, const DeltaNetLayer& layer, const DeltaNetSeq* seqs, int nseq,
+int EnqueueDeltaNetLinear(gufo_cuda_ctx* ctx, const DeltaNetLayer& layer, DeltaNetSeq* seqs, int nseq,
                           bool early_state, const DeltaNetGateRows* gate_rows = nullptr);
 // The same for Q6_K parts (image with group sums of 16).
 int LaunchGemvQ6KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
@@ -301,12 +302,24 @@ struct gufo_cuda_ctx {
   size_t host_x_bytes = 0;
   float* host_y = nullptr;
   size_t host_y_bytes = 0;
-  // The gate dots of a DeltaNet step of several sequences.
-  uint8_t* gates = nullptr;
-  size_t gates_bytes = 0;
   // Attention: arrival counters (zero between launches), then partial sums.
   uint8_t* attn = nullptr;
   size_t attn_bytes = 0;
+  // Scratch of kernels that calls on different streams of this context may have in
+  // flight at once: a block per kind and stream (by the id the runtime never gives out
+  // twice), never handed to a captured launch.
+  enum ScratchKind { kGatesScratch, kAttnScratch };
+  struct StreamBlock {
+    ScratchKind kind;
+    unsigned long long stream;
+    uint8_t* data;
+    size_t bytes;
+  };
+  static constexpr size_t kStreamBlocks = 32;
+  std::vector<StreamBlock> stream_blocks;
+  unsigned long long stream_id = 0;   // of `stream`, where the runtime knows it
+  bool stream_named = false;
+  void NameStream();
   // Fixed-point image of the activations of the product in flight.
   uint8_t* image = nullptr;
   size_t image_bytes = 0;
@@ -349,6 +362,10 @@ struct gufo_cuda_ctx {
   // The same for host_x and host_y; GUFO_CUDA_OUT_OF_MEMORY (no error text) where
   // no more memory is to be pinned: the caller copies pageable memory then.
   int ReserveHost(float** buffer, size_t* have, size_t want);
+  // At least `want` bytes (allocated `floor` at a time) of the current stream's block of
+  // a kind, or null while the stream is being captured or where kStreamBlocks exist
+  // already: the caller then does without. `fresh`: its content is new. ctx->mu is held.
+  int StreamScratch(ScratchKind kind, size_t want, size_t floor, uint8_t** data, bool* fresh);
   // Grows a device scratch block to `want` bytes (at least `floor`) without
   // freeing the old one and without waiting for the stream; refuses while the
   // stream is being captured (a capture cannot allocate). ctx->mu is held.

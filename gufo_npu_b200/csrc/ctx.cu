@@ -380,6 +380,7 @@ int gufo_cuda_ctx_create(int device, void* stream, gufo_cuda_ctx** out) {
     }
     ctx->own_stream = true;
   }
+  ctx->NameStream();
   gufo::Pool().Enter(device);
   gufo::Pinned().Enter();
   *out = ctx;
@@ -397,6 +398,41 @@ int gufo_cuda_ctx::ReserveHost(float** buffer, size_t* have, size_t want) {
   gufo::Pinned().Give(*buffer);   // every call that used it has waited for its work
   *buffer = static_cast<float*>(fresh);
   return GUFO_CUDA_OK;
+}
+
+void gufo_cuda_ctx::NameStream() {
+  stream_named = cudaStreamGetId(stream, &stream_id) == cudaSuccess;
+  if (!stream_named) {
+    cudaGetLastError();   // whoever enqueues on it finds out
+  }
+}
+
+int gufo_cuda_ctx::StreamScratch(ScratchKind kind, size_t want, size_t floor, uint8_t** data, bool* fresh) {
+  *data = nullptr;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+  if (!stream_named || cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();   // the legacy stream beside a capture: no block either
+    return GUFO_CUDA_OK;
+  }
+  StreamBlock* block = nullptr;
+  for (StreamBlock& b : stream_blocks) {
+    if (b.kind == kind && b.stream == stream_id) {
+      block = &b;
+    }
+  }
+  if (block == nullptr) {
+    if (stream_blocks.size() == kStreamBlocks) {
+      return GUFO_CUDA_OK;
+    }
+    stream_blocks.push_back({kind, stream_id, nullptr, 0});
+    block = &stream_blocks.back();
+  }
+  if (fresh != nullptr) {
+    *fresh = block->bytes < want;
+  }
+  const int rc = GrowScratch(&block->data, &block->bytes, want, floor, "stream scratch");
+  *data = block->data;
+  return rc;
 }
 
 int gufo_cuda_ctx::GrowScratch(uint8_t** block, size_t* have, size_t want, size_t floor, const char* what) {
@@ -441,8 +477,10 @@ int gufo_cuda_ctx_destroy(gufo_cuda_ctx* ctx) {
   }
   cudaFree(ctx->stage_x);
   cudaFree(ctx->stage_y);
-  ctx->retired.emplace_back(ctx->gates, ctx->gates_bytes);
   ctx->retired.emplace_back(ctx->attn, ctx->attn_bytes);
+  for (const auto& block : ctx->stream_blocks) {
+    ctx->retired.emplace_back(block.data, block.bytes);
+  }
   ctx->retired.emplace_back(ctx->image, ctx->image_bytes);
   ctx->retired.emplace_back(ctx->tc_scratch, ctx->tc_scratch_bytes);
   for (const auto& block : ctx->retired) {
@@ -489,6 +527,7 @@ int gufo_cuda_ctx_set_stream(gufo_cuda_ctx* ctx, void* stream) {
     ctx->own_stream = false;
   }
   ctx->stream = static_cast<cudaStream_t>(stream);
+  ctx->NameStream();
   return GUFO_CUDA_OK;
 }
 

@@ -628,9 +628,9 @@ int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens) 
       // One token: window to window, state in place. Two: the window and the state
       // after the first stay in conv_saved and ssm, the second's go to the other
       // window and ssm_spec.
-      const DeltaNetSeq seq{d->in, d->normed, l.conv[parity], l.conv_saved, l.conv[parity ^ 1], l.ssm, l.ssm,
+      DeltaNetSeq seq{d->in, d->normed, l.conv[parity], l.conv_saved, l.conv[parity ^ 1], l.ssm, l.ssm,
                             tokens == 2 ? l.ssm_spec : l.ssm, d->mixed, static_cast<int64_t>(in_width),
-                            static_cast<int64_t>(hidden), static_cast<int64_t>(mixed_width), tokens, nullptr};
+                            static_cast<int64_t>(hidden), static_cast<int64_t>(mixed_width), tokens, nullptr, 0};
       GUFO_STEP_TRY(EnqueueDeltaNetLinear(ctx, l.linear, &seq, 1, true,
                                           l.gate_rows.alpha_w != nullptr ? &l.gate_rows : nullptr));
     }

@@ -333,7 +333,7 @@ int gufo_cuda_deltanet_linear_device(gufo_cuda_ctx* ctx,
  * reference's two-token form; accepting the draft is ssm <- ssm_spec, rejecting
  * it conv <- conv_saved). With one token: ssm in place, conv_in -> conv_out,
  * conv_saved / ssm_spec unused (may be NULL). conv_in, conv_out and conv_saved
- * are distinct buffers. One launch per token index over all sequences. */
+ * are distinct buffers. One launch, or two from three sequences on. */
 typedef struct gufo_cuda_deltanet_step_seq {
   int n_tokens;          /* 1 .. 4 */
   const float* in;       /* [n_tokens] rows, in_stride floats apart */

@@ -136,6 +136,51 @@ def test_mixer_run_of_many_sequences_equals_one_token_at_a_time(ctx, oracle, hea
         assert rel_l2(ssm[s].cpu().numpy(), hssm) <= 1e-4
 
 
+@pytest.mark.parametrize("inplace", [False, True])
+def test_mixer_run_inside_a_first_capture_and_over_its_own_input(inplace):
+    """Three sequences captured by a context that has run nothing, and outputs laid over z: the bits of
+    a plain call."""
+    from gufo_npu_b200 import synth
+    from gufo_npu_b200.backend import CudaMixer
+    dev = torch.device("cuda:0")
+    cfg = synth.ModelConfig(layers=1, hidden=512, ffn=256, vocab=256, linear_key_heads=2, linear_value_heads=4)
+    tensors = synth.build_model(cfg, 5)
+    width, z_at = cfg.conv_channels + cfg.value_dim + 2 * cfg.linear_value_heads, cfg.conv_channels
+    gen = torch.Generator(device=dev).manual_seed(2)
+
+    def rand(*shape):
+        return torch.randn(*shape, device=dev, generator=gen)
+    results = []
+    first = [(rand(2, width), rand(2, cfg.hidden)) for _ in range(3)]
+    for captured in (False, True):
+        stream = torch.cuda.Stream()
+        own = Context(0, stream.cuda_stream)
+        mixer = CudaMixer(own, cfg, tensors)
+        gen.manual_seed(7)
+        seqs = []
+        for row, h in first:
+            row = row.clone()
+            seqs.append({"n_tokens": 2, "in": row, "h": h, "conv_in": rand(mixer.conv_values()),
+                         "conv_out": rand(mixer.conv_values()), "conv_saved": rand(mixer.conv_values()),
+                         "ssm": rand(mixer.ssm_values()) * 0.1, "ssm_spec": rand(mixer.ssm_values()),
+                         "y": row[:, z_at:z_at + cfg.value_dim] if inplace and captured else
+                         torch.empty(2, cfg.value_dim, device=dev)})
+        torch.cuda.synchronize()
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                mixer.Run(0, seqs)
+            graph.replay()
+        else:
+            mixer.Run(0, seqs)
+        torch.cuda.synchronize()
+        results.append([torch.cat([q[key].reshape(-1) for q in seqs]) for key in ("y", "ssm", "ssm_spec", "conv_out")])
+        del mixer
+        own.close()
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
 def _random_rows(ctx, ggml_type, rows, cols, seed):
     """Any code bytes beside small fp16 scales: a matrix handle and its values in float64."""
     rng = np.random.default_rng(seed)
