@@ -38,10 +38,8 @@ constexpr int kWarps = 8;
 constexpr int kChunk = 64;          // positions per stage
 constexpr int kStages = 2;
 constexpr int kAlone = 128;         // positions one block takes by itself
-constexpr int kMaxSplits = 64;
 constexpr int kPadHalves = 8;       // row padding: ldmatrix rows fall in distinct banks
 constexpr float kProbScale = 16384.0f;
-constexpr size_t kCounterBytes = 4096;
 
 struct FastAttnArgs {
   AttnArgs a;
@@ -63,7 +61,7 @@ struct Smem {
   float q_scale[8];                                    // score factor of a head
   float keep[8];                                       // rescaling of the sums so far
   float top[8], total[8];
-  float weight[8][kMaxSplits];                         // merge: a split's factor
+  float weight[8][kAttnMaxSplits];                       // merge: a split's factor
   int last;
 };
 
@@ -455,7 +453,6 @@ int Launch(gufo_cuda_ctx* ctx, const FastAttnArgs& f) {
 
 bool AttentionFits(const AttnArgs& a) {
   return (a.head_dim == 64 || a.head_dim == 128 || a.head_dim == 256) && a.heads / a.kv_heads <= 8 &&
-         a.kv_heads <= static_cast<int>(kCounterBytes / sizeof(unsigned)) &&
          ((reinterpret_cast<uintptr_t>(a.keys) | reinterpret_cast<uintptr_t>(a.values)) & 15) == 0;
 }
 
@@ -463,21 +460,37 @@ int LaunchAttention(gufo_cuda_ctx* ctx, const AttnArgs& a) {
   FastAttnArgs f{a};
   // One resident block per SM, and no more than a warp's lanes hold twice.
   f.splits = ctx->sm_count / a.kv_heads;
-  f.splits = f.splits < 1 ? 1 : f.splits > kMaxSplits ? kMaxSplits : f.splits;
-  const size_t parts = static_cast<size_t>(f.splits) * a.heads;
-  const size_t sums = parts * a.head_dim * 4;   // a multiple of 256
-  const size_t want = kCounterBytes + sums + parts * 8;
-  const bool fresh = ctx->attn_bytes < want;
-  const int rc = ctx->GrowScratch(&ctx->attn, &ctx->attn_bytes, want, 1u << 20, "attention");
-  if (rc != GUFO_CUDA_OK) {
-    return rc;
+  f.splits = f.splits < 1 ? 1 : f.splits > kAttnMaxSplits ? kAttnMaxSplits : f.splits;
+  // Counters and partial sums: a decoder's own, else the stream's, so that calls on
+  // several streams share none. A captured call has to do with what the caller gave it,
+  // as its graph may run beside any other: kAttnSplits slices of partials less one (for
+  // the alignment), and counters in the queries' place, cleared ahead of every launch
+  // (a second node of the graph).
+  if (a.arrived != nullptr) {
+    f.arrived = a.arrived;
+    f.sums = a.partials;
+  } else if (f.splits > 1) {
+    const size_t counters = (static_cast<size_t>(a.kv_heads) * 4 + 255) / 256 * 256;
+    const size_t want = counters + static_cast<size_t>(f.splits) * a.heads * (a.head_dim + 2) * 4;
+    uint8_t* scratch = nullptr;
+    bool fresh = false;
+    const int rc = ctx->StreamScratch(gufo_cuda_ctx::kAttnScratch, want, 256u << 10, &scratch, &fresh);
+    if (rc != GUFO_CUDA_OK) {
+      return rc;
+    }
+    if (scratch == nullptr) {
+      f.splits = f.splits < kAttnSplits ? f.splits : kAttnSplits - 1;
+      f.arrived = reinterpret_cast<unsigned*>(a.queries);
+      f.sums = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(a.partials) + 15) & ~static_cast<uintptr_t>(15));
+    } else {
+      f.arrived = reinterpret_cast<unsigned*>(scratch);
+      f.sums = reinterpret_cast<float*>(scratch + counters);
+    }
+    if (scratch == nullptr || fresh) {
+      GUFO_CUDA_TRY(cudaMemsetAsync(f.arrived, 0, static_cast<size_t>(a.kv_heads) * 4, ctx->stream));
+    }
   }
-  if (fresh) {
-    GUFO_CUDA_TRY(cudaMemsetAsync(ctx->attn, 0, kCounterBytes, ctx->stream));
-  }
-  f.arrived = reinterpret_cast<unsigned*>(ctx->attn);
-  f.sums = reinterpret_cast<float*>(ctx->attn + kCounterBytes);
-  f.stats = reinterpret_cast<float*>(ctx->attn + kCounterBytes + sums);
+  f.stats = f.sums + static_cast<size_t>(f.splits) * a.heads * a.head_dim;
   switch (a.head_dim) {
     case 64: return Launch<64>(ctx, f);
     case 128: return Launch<128>(ctx, f);

@@ -302,9 +302,6 @@ struct gufo_cuda_ctx {
   size_t host_x_bytes = 0;
   float* host_y = nullptr;
   size_t host_y_bytes = 0;
-  // Attention: arrival counters (zero between launches), then partial sums.
-  uint8_t* attn = nullptr;
-  size_t attn_bytes = 0;
   // Scratch of kernels that calls on different streams of this context may have in
   // flight at once: a block per kind and stream (by the id the runtime never gives out
   // twice), never handed to a captured launch.

@@ -477,7 +477,6 @@ int gufo_cuda_ctx_destroy(gufo_cuda_ctx* ctx) {
   }
   cudaFree(ctx->stage_x);
   cudaFree(ctx->stage_y);
-  ctx->retired.emplace_back(ctx->attn, ctx->attn_bytes);
   for (const auto& block : ctx->stream_blocks) {
     ctx->retired.emplace_back(block.data, block.bytes);
   }

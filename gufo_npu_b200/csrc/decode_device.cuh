@@ -15,6 +15,7 @@ namespace gufo {
 constexpr int kTeamThreads = 256;
 constexpr int kTeamWarps = kTeamThreads / 32;
 constexpr int kAttnSplits = 32;     // position slices per KV head
+constexpr int kAttnMaxSplits = 64;  // of the one-launch kernel, where the scratch has room for them
 constexpr int kMaxGroup = 8;        // query heads per KV head
 constexpr int kMaxPerLane = 8;      // head_dim / 32
 
@@ -48,6 +49,10 @@ struct AttnArgs {
   float* partials;          // [kv_heads][splits][group][hd + 2]
   float* ctx;               // [heads][hd]
   int offset = 0;           // the token sits at *position + offset
+  // One-launch kernel: arrival counters [kv_heads], zero between launches, that belong
+  // to these launches alone, as do partials (room for kAttnMaxSplits slices then). Null:
+  // LaunchAttention finds some.
+  unsigned* arrived = nullptr;
 };
 
 // The one-launch attention kernel (attention.cu): whether it runs a shape, and its

@@ -276,6 +276,7 @@ struct gufo_cuda_decoder {
   float *expert_ffn = nullptr, *expert_act = nullptr, *expert_out = nullptr;
   int* chosen = nullptr;
   int* position_dev = nullptr;
+  unsigned* attn_arrived = nullptr;   // AttnArgs::arrived
   gufo::StepWords* words = nullptr;      // device
   // Pinned staging for them: a slot is written again only after the copy that read
   // it has run (its event, unless that step was waited for), so that steps
@@ -621,7 +622,7 @@ int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens) 
     for (int t = 0; l.attention && t < tokens; ++t) {
       AttnArgs a{c.heads, c.kv_heads, c.head_dim, c.rope_dim, c.max_positions, c.rms_eps,
                  d->position_dev, d->in + t * in_width, l.q_norm, l.k_norm, d->inv_freq, l.keys, l.values,
-                 d->queries, d->partials, d->mixed + t * mixed_width, t};
+                 d->queries, d->partials, d->mixed + t * mixed_width, t, d->attn_arrived};
       GUFO_STEP_TRY(EnqueueAttention(ctx, a));
     }
     if (!l.attention) {
@@ -1431,7 +1432,7 @@ int gufo_cuda_decoder_create(gufo_cuda_ctx* ctx, const gufo_cuda_decoder_config*
               {&d->out, two * c.hidden},
               {&d->ffn, two * 2 * c.ffn}, {&d->act, two * c.ffn},
               {&d->logits, two * c.vocab}, {&d->queries, static_cast<size_t>(attn_dim)},
-              {&d->partials, static_cast<size_t>(c.kv_heads) * gufo::kAttnSplits * group * (c.head_dim + 2)},
+              {&d->partials, static_cast<size_t>(c.kv_heads) * gufo::kAttnMaxSplits * group * (c.head_dim + 2)},
               // MoE scratch (a few floats for a dense model).
               {&d->router, two * (static_cast<size_t>(c.experts) + 1)},
               {&d->route_weights, two * c.experts_used + 1},
@@ -1446,6 +1447,8 @@ int gufo_cuda_decoder_create(gufo_cuda_ctx* ctx, const gufo_cuda_decoder_config*
   }
   if ((rc = gufo::Alloc(d, 4 * (two * c.experts_used + 1), reinterpret_cast<void**>(&d->chosen))) != GUFO_CUDA_OK ||
       (rc = gufo::Alloc(d, 4, reinterpret_cast<void**>(&d->position_dev))) != GUFO_CUDA_OK ||
+      (rc = gufo::Alloc(d, 4 * static_cast<size_t>(c.kv_heads > 0 ? c.kv_heads : 1),
+                        reinterpret_cast<void**>(&d->attn_arrived))) != GUFO_CUDA_OK ||
       (rc = gufo::Alloc(d, sizeof(gufo::StepWords), reinterpret_cast<void**>(&d->words))) != GUFO_CUDA_OK) {
     return fail(rc);
   }
@@ -1469,6 +1472,7 @@ int gufo_cuda_decoder_create(gufo_cuda_ctx* ctx, const gufo_cuda_decoder_config*
     cudaMemsetAsync(d->ssm_all[0], 0, d->ssm_all_bytes, ctx->stream);
   }
   cudaMemsetAsync(d->position_dev, 0, 4, ctx->stream);
+  cudaMemsetAsync(d->attn_arrived, 0, 4 * static_cast<size_t>(c.kv_heads > 0 ? c.kv_heads : 1), ctx->stream);
   GUFO_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return GUFO_CUDA_OK;
 }

@@ -381,7 +381,11 @@ int gufo_cuda_swiglu_device(gufo_cuda_ctx* ctx, const float* ffn, int f,
 /* Mixer::Attention for one token (src/models/qwen35/decoder.cpp:267-412): q/k
  * RMSNorm and RoPE, the fp16 cache append at *position, softmax over positions
  * 0..*position in slices, the output gate. `in` is the kAttentionIn row
- * [q and gate | k | v]; `ctx_out` gets heads * head_dim values. */
+ * [q and gate | k | v]; `ctx_out` gets heads * head_dim values. Scratch of this
+ * call alone: queries and partials (while the stream is being captured, and for
+ * head dims other than 64, 128 and 256), else a block the context keeps per
+ * stream. So calls on different streams, and captured graphs, with scratch of
+ * their own may be in flight together. */
 typedef struct gufo_cuda_attention_args {
   int heads, kv_heads, head_dim, rope_dim, max_positions;
   float rms_eps;

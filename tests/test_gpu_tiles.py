@@ -373,6 +373,66 @@ def test_attention_chunks_and_splits(ctx, heads, kv_heads, head_dim, rope_dim, p
         assert rel_l2(out.reshape(heads, hd)[h].cpu().numpy(), want[h].cpu().numpy()) <= 5e-6, h
 
 
+def _attention_call(positions, heads, kv_heads, hd, seed):
+    """Tensors of one attention call on random rows, the last of them its output, and its arguments."""
+    from gufo_npu_b200 import _capi
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(seed)
+
+    def rand(*shape):
+        return torch.randn(*shape, device=dev, generator=gen)
+    tensors = [torch.tensor([positions - 1], dtype=torch.int32, device=dev), rand(2 * (heads + kv_heads) * hd),
+               1 + 0.1 * rand(hd), 1 + 0.1 * rand(hd), 0.1 + rand(16).abs(), rand(positions, kv_heads * hd).half(),
+               rand(positions, kv_heads * hd).half(), torch.empty(heads * hd, device=dev),
+               torch.empty(32 * heads * (hd + 2), device=dev), torch.empty(heads * hd, device=dev)]
+    return tensors, _capi.AttentionArgs(heads, kv_heads, hd, 32, positions, 1e-6, *[t.data_ptr() for t in tensors])
+
+
+def test_attention_on_two_streams_and_in_concurrent_graphs():
+    """Calls of one context that may be in flight together, on two streams and in two graphs captured
+    by a context that has run none: each has the bits of a call by itself."""
+    import ctypes as C
+    shapes = [(9001, 8, 2, 256), (3000, 8, 2, 256), (700, 2, 1, 128), (16000, 16, 4, 64)]
+    calls = [_attention_call(*shapes[i % 4], i) for i in range(16)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+
+    def run(own, args):
+        own._check(own.lib.gufo_cuda_attention_device(own.handle, C.byref(args)))
+    own = Context(0)
+    want = []
+    for tensors, args in calls:
+        torch.cuda.synchronize()
+        run(own, args)
+        own.synchronize()
+        want.append(tensors[-1].clone())
+        tensors[-1].zero_()
+    torch.cuda.synchronize()
+    for _ in range(4):
+        for i, (_, args) in enumerate(calls):
+            own.set_stream(streams[i % 2].cuda_stream)
+            run(own, args)
+    torch.cuda.synchronize()
+    for (tensors, _), w in zip(calls, want):
+        assert torch.equal(tensors[-1], w)
+        tensors[-1].zero_()
+    own.close()
+    own = Context(0, streams[0].cuda_stream)
+    graphs = []
+    for half in range(2):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], stream=streams[0]):
+            for _, args in calls[half::2]:
+                run(own, args)
+    for _ in range(4):
+        for graph, stream in zip(graphs, streams):
+            with torch.cuda.stream(stream):
+                graph.replay()
+    torch.cuda.synchronize()
+    for (tensors, _), w in zip(calls, want):
+        assert rel_l2(tensors[-1].cpu().numpy(), w.cpu().numpy()) <= 2e-6   # other slices in a graph
+    own.close()
+
+
 @pytest.mark.parametrize("ggml_type", [Q.GGML_Q4_K, Q.GGML_Q6_K])
 @pytest.mark.parametrize("tokens,rows,cols", [
     (1, 20000, 2560), (2, 33, 256), (2, 20011, 768), (3, 16, 9728), (5, 9001, 2304), (8, 40, 2816), (8, 1500, 9728),
