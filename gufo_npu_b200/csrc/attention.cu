@@ -40,6 +40,7 @@ constexpr int kStages = 2;
 constexpr int kAlone = 128;         // positions one block takes by itself
 constexpr int kPadHalves = 8;       // row padding: ldmatrix rows fall in distinct banks
 constexpr float kProbScale = 16384.0f;
+constexpr size_t kCounterBytes = 1024;   // of the stream's scratch: counters of up to 256 KV heads
 
 struct FastAttnArgs {
   AttnArgs a;
@@ -460,7 +461,7 @@ int LaunchAttention(gufo_cuda_ctx* ctx, const AttnArgs& a) {
   FastAttnArgs f{a};
   // One resident block per SM, and no more than a warp's lanes hold twice.
   f.splits = ctx->sm_count / a.kv_heads;
-  f.splits = f.splits < 1 ? 1 : f.splits > kAttnMaxSplits ? kAttnMaxSplits : f.splits;
+  f.splits = f.splits < 1 || a.kv_heads * sizeof(unsigned) > kCounterBytes ? 1 : f.splits > kAttnMaxSplits ? kAttnMaxSplits : f.splits;
   // Counters and partial sums: a decoder's own, else the stream's, so that calls on
   // several streams share none. A captured call has to do with what the caller gave it,
   // as its graph may run beside any other: kAttnSplits slices of partials less one (for
@@ -470,8 +471,7 @@ int LaunchAttention(gufo_cuda_ctx* ctx, const AttnArgs& a) {
     f.arrived = a.arrived;
     f.sums = a.partials;
   } else if (f.splits > 1) {
-    const size_t counters = (static_cast<size_t>(a.kv_heads) * 4 + 255) / 256 * 256;
-    const size_t want = counters + static_cast<size_t>(f.splits) * a.heads * (a.head_dim + 2) * 4;
+    const size_t want = kCounterBytes + static_cast<size_t>(f.splits) * a.heads * (a.head_dim + 2) * 4;
     uint8_t* scratch = nullptr;
     bool fresh = false;
     const int rc = ctx->StreamScratch(gufo_cuda_ctx::kAttnScratch, want, 256u << 10, &scratch, &fresh);
@@ -484,10 +484,12 @@ int LaunchAttention(gufo_cuda_ctx* ctx, const AttnArgs& a) {
       f.sums = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(a.partials) + 15) & ~static_cast<uintptr_t>(15));
     } else {
       f.arrived = reinterpret_cast<unsigned*>(scratch);
-      f.sums = reinterpret_cast<float*>(scratch + counters);
+      f.sums = reinterpret_cast<float*>(scratch + kCounterBytes);
     }
     if (scratch == nullptr || fresh) {
-      GUFO_CUDA_TRY(cudaMemsetAsync(f.arrived, 0, static_cast<size_t>(a.kv_heads) * 4, ctx->stream));
+      // All counters of a block that stays: the next call may have more KV heads.
+      const size_t bytes = scratch == nullptr ? static_cast<size_t>(a.kv_heads) * 4 : kCounterBytes;
+      GUFO_CUDA_TRY(cudaMemsetAsync(f.arrived, 0, bytes, ctx->stream));
     }
   }
   f.stats = f.sums + static_cast<size_t>(f.splits) * a.heads * a.head_dim;

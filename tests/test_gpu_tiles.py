@@ -388,6 +388,29 @@ def _attention_call(positions, heads, kv_heads, hd, seed):
     return tensors, _capi.AttentionArgs(heads, kv_heads, hd, 32, positions, 1e-6, *[t.data_ptr() for t in tensors])
 
 
+def test_attention_in_used_scratch_with_more_kv_heads_than_before(ctx):
+    """A context that takes over another's scratch, its first call on one KV head, the next on four."""
+    import ctypes as C
+    other = Context(0)
+    m, _ = _matrix(other, Q.GGML_Q4_K, 4752, 1280, 3)
+    other.matmul([(m, 0, 4752)], G.normal(4, 8, 1280), 8, 4752)   # leaves bytes in a block of 256 KB
+    other.close()
+    own = Context(0)
+    outs = []
+    for heads, kv_heads, hd in ((2, 1, 128), (4, 4, 64)):
+        for use in (own, ctx):
+            tensors, args = _attention_call(300, heads, kv_heads, hd, 1)
+            torch.cuda.synchronize()
+            for general in (0, 1):
+                use.set_option("general_gemv", general)
+                use._check(use.lib.gufo_cuda_attention_device(use.handle, C.byref(args)))
+                use.synchronize()
+                outs.append(tensors[-1].clone())
+            use.set_option("general_gemv", 0)
+            assert rel_l2(outs[-2].cpu().numpy(), outs[-1].cpu().numpy()) <= 2e-6
+    own.close()
+
+
 def test_attention_on_two_streams_and_in_concurrent_graphs():
     """Calls of one context that may be in flight together, on two streams and in two graphs captured
     by a context that has run none: each has the bits of a call by itself."""
