@@ -22,9 +22,10 @@
 // the group's (at most eight) query heads as the rows and the fp16 cache rows as they
 // are. The fp32 operands (queries; probabilities) are split into two halves, rows
 // 0-7 and 8-15 of the same instruction, so that 22 bits of them count, scaled by a
-// power of two ahead of the split so that small ones keep their bits as well; fp32
-// accumulation. Warps take the chunk's positions for the scores, the query heads for
-// the softmax, the head's dimensions for the sums.
+// power of two ahead of the split so that small ones keep their bits as well; each
+// instruction's sixteen products are added up in fp32 (MmaF16). Warps take the chunk's
+// positions for the scores, the query heads for the softmax, the head's dimensions for
+// the sums.
 //
 // 8 query heads on 2 KV heads of 256: 4096 positions 12.3 -> 4.8 us, 16384 positions
 // 51 -> 10.5 us; a few positions of one KV head of 128: 7.2 -> 3.1 us.
@@ -81,11 +82,18 @@ __device__ __forceinline__ void Ldmatrix2Trans(uint32_t& r0, uint32_t& r1, const
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
                : "=r"(r0), "=r"(r1) : "r"(Address(p)));
 }
+// d = a b of sixteen values. The tensor core cuts off what does not fit its adder, so
+// sums over more than that are taken with fp32 adds, which round: accumulated by the
+// instruction, the outputs were up to three times as far from a float64 result as with
+// fp32 arithmetic throughout (16384 positions: 7.7e-7 against 2.6e-7; now 2.4e-7).
 __device__ __forceinline__ void MmaF16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void Add4(float (&d)[4], const float (&x)[4]) {
+  d[0] += x[0], d[1] += x[1], d[2] += x[2], d[3] += x[3];
 }
 
 // RMSNorm and RoPE of one head by a warp: lane l ends with elements l, l + 32, ...
@@ -264,19 +272,25 @@ AttnKernel(const __grid_constant__ FastAttnArgs f) {
     }
     // Scores: warp w takes positions 8w .. 8w + 7.
     if (8 * warp < count) {
-      float d[4] = {0.f, 0.f, 0.f, 0.f}, d2[4] = {0.f, 0.f, 0.f, 0.f};
+      float d[4][4] = {};
 #pragma unroll
       for (int k0 = 0; k0 < HD; k0 += 32) {
         uint32_t b[4], q0[4], q1[4];
         Ldmatrix4(b, &s.k[st][8 * warp + (lane & 7)][k0 + 8 * (lane >> 3)]);
         Ldmatrix4(q0, &s.q[lane & 15][k0 + 8 * (lane >> 4)]);
         Ldmatrix4(q1, &s.q[lane & 15][k0 + 16 + 8 * (lane >> 4)]);
-        MmaF16(d, q0, b[0], b[1]);
-        MmaF16(d2, q1, b[2], b[3]);
+        float p0[4], p1[4];
+        MmaF16(p0, q0, b[0], b[1]);
+        MmaF16(p1, q1, b[2], b[3]);
+        Add4(p0, p1);
+        Add4(d[(k0 / 32) % 4], p0);
       }
+      Add4(d[0], d[1]);
+      Add4(d[2], d[3]);
+      Add4(d[0], d[2]);
       const float factor = s.q_scale[g];
-      s.score[g][8 * warp + 2 * t] = ((d[0] + d2[0]) + (d[2] + d2[2])) * factor;
-      s.score[g][8 * warp + 2 * t + 1] = ((d[1] + d2[1]) + (d[3] + d2[3])) * factor;
+      s.score[g][8 * warp + 2 * t] = (d[0][0] + d[0][2]) * factor;
+      s.score[g][8 * warp + 2 * t + 1] = (d[0][1] + d[0][3]) * factor;
     }
     __syncthreads();
     if (warp < group) {
@@ -309,13 +323,12 @@ AttnKernel(const __grid_constant__ FastAttnArgs f) {
     // Weighted sums: warp w takes HD / 8 dimensions.
     {
       const float keep = g < group ? s.keep[g] : 0.f;
-#pragma unroll
-      for (int n = 0; n < kTiles; ++n) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          acc[n][i] *= keep;
-        }
-      }
+      float part[kTiles][4] = {};
+      auto add = [&](int n, const uint32_t (&p)[4], uint32_t b0, uint32_t b1) {
+        float x[4];
+        MmaF16(x, p, b0, b1);
+        Add4(part[n], x);
+      };
 #pragma unroll
       for (int k0 = 0; k0 < kChunk; k0 += 16) {
         if (k0 < count) {
@@ -324,16 +337,23 @@ AttnKernel(const __grid_constant__ FastAttnArgs f) {
           if constexpr (kTiles == 1) {
             uint32_t b0, b1;
             Ldmatrix2Trans(b0, b1, &s.v[st][k0 + (lane & 15)][dim0]);
-            MmaF16(acc[0], p, b0, b1);
+            add(0, p, b0, b1);
           } else {
 #pragma unroll
             for (int n = 0; n < kTiles; n += 2) {
               uint32_t b[4];
               Ldmatrix4Trans(b, &s.v[st][k0 + (lane & 15)][dim0 + 8 * n + 8 * (lane >> 4)]);
-              MmaF16(acc[n], p, b[0], b[1]);
-              MmaF16(acc[n + 1], p, b[2], b[3]);
+              add(n, p, b[0], b[1]);
+              add(n + 1, p, b[2], b[3]);
             }
           }
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < kTiles; ++n) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          acc[n][i] = fmaf(acc[n][i], keep, part[n][i]);
         }
       }
     }
