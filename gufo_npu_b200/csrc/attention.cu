@@ -29,6 +29,8 @@
 //
 // 8 query heads on 2 KV heads of 256: 4096 positions 12.3 -> 4.8 us, 16384 positions
 // 51 -> 10.5 us; a few positions of one KV head of 128: 7.2 -> 3.1 us.
+#include <cfloat>
+
 #include "decode_device.cuh"
 
 namespace gufo {
@@ -129,6 +131,54 @@ __device__ __forceinline__ void NormRope(const AttnArgs& a, const float* x, cons
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
     out[i] = row[lane + 32 * i];
+  }
+}
+
+// A block's slice once more, for one warp's dimensions, in plain fp32: where something
+// is not finite. A product of two halves turns an infinite cache value into NaN (one half
+// may be zero, or of the other sign) where the fp32 product is infinite, and a score of
+// minus infinity weighs nothing. out: [group][HD / 8 sums | maximum, sum of weights].
+template <int HD>
+__device__ __noinline__ void SliceInFp32(const AttnArgs& a, const float* in_q, int kh, int group, int pos, int begin,
+                                         int end, float* row, float* out) {
+  constexpr int kPer = HD / 32, kDims = HD / kWarps;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t stride = static_cast<size_t>(a.kv_heads) * HD;
+  const float scale = 1.0f / sqrtf(static_cast<float>(HD));
+  for (int head = 0; head < group; ++head) {
+    float q[kPer];
+    NormRope<HD>(a, in_q + static_cast<size_t>(head) * 2 * HD, a.q_norm, pos, lane, row, q);
+    auto score = [&](int j) {
+      const __half* k = a.keys + static_cast<size_t>(j) * stride + static_cast<size_t>(kh) * HD;
+      float dot = 0.f;
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        dot = fmaf(q[i], __half2float(k[lane + 32 * i]), dot);
+      }
+      return WarpSum(dot) * scale;
+    };
+    float top = -INFINITY, total = 0.f, value = 0.f;
+    for (int j = begin; j < end; ++j) {
+      const float s = score(j);
+      top = fmaxf(top, s);
+      total = s != s ? s : total;   // a NaN is the result
+    }
+    for (int j = begin; j < end && (top > -INFINITY || total != total); ++j) {
+      const float p = expf(score(j) - top);
+      total += p;
+      if (lane < kDims) {
+        value = fmaf(p, __half2float(a.values[static_cast<size_t>(j) * stride + static_cast<size_t>(kh) * HD + warp * kDims + lane]),
+                     value);
+      }
+    }
+    if (lane < kDims) {
+      out[head * (kDims + 2) + lane] = value * kProbScale;
+    }
+    if (lane == 0) {
+      out[head * (kDims + 2) + kDims] = top;
+      out[head * (kDims + 2) + kDims + 1] = total;
+    }
+    __syncwarp();
   }
 }
 
@@ -361,6 +411,29 @@ AttnKernel(const __grid_constant__ FastAttnArgs f) {
     load(c + kStages);
   }
 
+  float top = g < group ? s.top[g] : 0.f, total = g < group ? s.total[g] : 0.f;
+  float sum = total;
+#pragma unroll
+  for (int n = 0; n < kTiles; ++n) {
+    sum += (acc[n][0] + acc[n][1]) + (acc[n][2] + acc[n][3]);
+  }
+  if (__any_sync(0xFFFFFFFFu, !(fabsf(sum) <= FLT_MAX))) {
+    constexpr int kDims = HD / kWarps;
+    // (The chunks' buffers are free behind the loop's last barrier.)
+    float* exact = reinterpret_cast<float*>(s.k) + warp * 8 * (kDims + 2);
+    SliceInFp32<HD>(a, in_q, kh, group, pos, begin, end, rows[warp], exact);
+    if (g < group) {
+      exact += g * (kDims + 2);
+#pragma unroll
+      for (int n = 0; n < kTiles; ++n) {
+        acc[n][0] = exact[8 * n + 2 * t];
+        acc[n][1] = exact[8 * n + 2 * t + 1];
+        acc[n][2] = acc[n][3] = 0.f;
+      }
+      top = exact[kDims];
+      total = exact[kDims + 1];
+    }
+  }
   // Head g's sums: the two halves' rows added; dimensions dim0 + 8n + 2t, + 1.
   auto finish = [&](int head, int e, float value, float inv_total) {
     const float gate = __ldcg(in_q + static_cast<size_t>(head) * 2 * HD + HD + e);
@@ -368,7 +441,7 @@ AttnKernel(const __grid_constant__ FastAttnArgs f) {
   };
   if (active == 1) {
     if (g < group) {
-      const float inv_total = 1.0f / (s.total[g] * kProbScale);
+      const float inv_total = 1.0f / (total * kProbScale);
 #pragma unroll
       for (int n = 0; n < kTiles; ++n) {
         finish(g, dim0 + 8 * n + 2 * t, acc[n][0] + acc[n][2], inv_total);
@@ -385,9 +458,9 @@ AttnKernel(const __grid_constant__ FastAttnArgs f) {
       *to = make_float2(acc[n][0] + acc[n][2], acc[n][1] + acc[n][3]);
     }
   }
-  if (threadIdx.x < group) {
-    f.stats[(part * group + threadIdx.x) * 2] = s.top[threadIdx.x];
-    f.stats[(part * group + threadIdx.x) * 2 + 1] = s.total[threadIdx.x];
+  if (warp == 0 && t == 0 && g < group) {
+    f.stats[(part * group + g) * 2] = top;
+    f.stats[(part * group + g) * 2 + 1] = total;
   }
   __threadfence();
   __syncthreads();
@@ -438,6 +511,11 @@ AttnKernel(const __grid_constant__ FastAttnArgs f) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         v[i] = __ldcg(reinterpret_cast<const float4*>(from + static_cast<size_t>(min(p0 + i, active - 1)) * values));
+      }
+      // (Past the end a zero, not a zero weight: the last slice may hold an infinity.)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        v[i] = p0 + i < active ? v[i] : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int i = 0; i < 16; ++i) {

@@ -444,6 +444,38 @@ def test_attention_is_as_close_to_float64_as_fp32_arithmetic(ctx, heads, kv_head
     assert np.mean(errors) <= 3.5e-7, errors
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 2, 256), (2, 1, 128), (4, 4, 64)])
+@pytest.mark.parametrize("positions", [1, 60, 700])
+@pytest.mark.parametrize("what", ["value", "own value", "key", "keys", "own key", "query"])
+def test_attention_over_cache_rows_that_are_not_finite(ctx, heads, kv_heads, head_dim, positions, what):
+    """An infinite cache element (an fp16 overflow) reaches what it reaches in exact arithmetic, and no
+    more."""
+    import ctypes as C
+    tensors, args = _attention_call(positions, heads, kv_heads, head_dim, 3)
+    row, keys, values = tensors[1], tensors[5], tensors[6]
+    at = positions // 2
+    if what == "value":
+        values[at, 5] = float("inf")
+    elif what == "own value":
+        row[2 * heads * head_dim + kv_heads * head_dim + 7] = -1e9
+    elif what == "key":
+        keys[at, 40] = float("inf")
+    elif what == "keys":     # the first half of the slices
+        keys[:at + 1, 40] = -float("inf")
+    elif what == "own key":
+        tensors[3][40] = 1e9
+    else:
+        row[3] = float("inf")
+    torch.cuda.synchronize()
+    ctx._check(ctx.lib.gufo_cuda_attention_device(ctx.handle, C.byref(args)))
+    ctx.synchronize()
+    got, want = tensors[-1].double(), _attention_in_float64(tensors, args).reshape(-1)
+    assert torch.equal(want.isnan(), got.isnan())
+    assert torch.equal(want[want.isinf()], got[want.isinf()])
+    finite = torch.isfinite(want)
+    assert torch.isfinite(got[finite]).all() and rel_l2(got[finite].cpu().numpy(), want[finite].cpu().numpy()) <= 2e-6
+
+
 def test_attention_on_two_streams_and_in_concurrent_graphs():
     """Calls of one context that may be in flight together, on two streams and in two graphs captured
     by a context that has run none: each has the bits of a call by itself."""
