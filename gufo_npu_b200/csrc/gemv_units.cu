@@ -72,8 +72,8 @@ constexpr int kExchange = 4;
 constexpr int kTileRows = 16;
 
 template <int TYPE, int TOKENS>
-size_t SharedBytes(int cols, int depth) {
-  const ImageLayout l = MakeImageLayout(TOKENS, cols, Unit<TYPE>::kGroup);
+size_t SharedBytes(int cols, int depth, int limbs = kLimbs) {
+  const ImageLayout l = MakeImageLayout(TOKENS, cols, Unit<TYPE>::kGroup, limbs);
   return static_cast<size_t>(l.bytes) + (Unit<TYPE>::kZeros ? l.plane_stride : 0) +
          static_cast<size_t>(kExchange) * kFastWarps * kTileRows * TOKENS * 4 +
          static_cast<size_t>(depth) * kFastWarps * kTileRows * Unit<TYPE>::kRow;
@@ -87,13 +87,16 @@ size_t SharedBytes(int cols, int depth) {
 // before, a warp per row and expert in fp32, spent its time in conversions and in
 // staging the activated inputs once per eight rows. Together with several tile pairs a
 // block in the gate / up product, a layer of 256 experts of 512 x 2048, eight of them
-// for each of four tokens: 34.4 -> 21.7 us.)
+// for each of four tokens: 34.4 -> 21.7 us. The inputs have a fourth byte plane, which
+// costs the products no instruction: with 24 bits, as elsewhere, the rows were up to
+// three times as far from a float64 result as the fp32 ones.)
 template <int TYPE, int TOKENS, int PER_SM, bool MIX = false>
 __global__ void __launch_bounds__(kFastThreads, PER_SM)
 GemvUnits(const __grid_constant__ FastGemvArgs a) {
   using U = Unit<TYPE>;
   constexpr bool kQ4 = TYPE == GUFO_CUDA_Q4_K;
-  constexpr int kNCols = TOKENS * kLimbs;
+  constexpr int kLimbsHere = MIX ? kMixLimbs : kLimbs;
+  constexpr int kNCols = TOKENS * kLimbsHere;
   constexpr int kNB = (kNCols + 7) / 8;
   constexpr int kTileFloats = kTileRows * TOKENS;   // per warp in an exchange buffer: row sums per token
   constexpr int kUnitBytes = kTileRows * U::kRow;
@@ -117,7 +120,7 @@ GemvUnits(const __grid_constant__ FastGemvArgs a) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  const ImageLayout l = MakeImageLayout(TOKENS, a.cols, U::kGroup);
+  const ImageLayout l = MakeImageLayout(TOKENS, a.cols, U::kGroup, kLimbsHere);
   const int blocks = a.cols / kSuperBlock;
   const float* col_scale = reinterpret_cast<const float*>(smem + l.scale_at);
   const float* sums = reinterpret_cast<const float*>(smem + l.sums_at);
@@ -242,7 +245,7 @@ GemvUnits(const __grid_constant__ FastGemvArgs a) {
     }
   }
   if (a.prologue != kPrologueImage) {
-    ZeroIdleColumns<TOKENS>(l, blocks, smem);
+    ZeroIdleColumns<TOKENS, kLimbsHere>(l, blocks, smem);
   }
   float norm_ahead[8];
   LoadNormAhead<TOKENS>(a, norm_ahead);
@@ -263,7 +266,7 @@ GemvUnits(const __grid_constant__ FastGemvArgs a) {
     wait(&staged, 0);
     __syncthreads();   // the plane of zeros, the mirror's address
   } else {
-    FillImage<TOKENS>(a, l, smem, U::kExtra, MIX ? a.x + static_cast<size_t>(group) * a.cols : a.x, rank, ks,
+    FillImage<TOKENS, kLimbsHere>(a, l, smem, U::kExtra, MIX ? a.x + static_cast<size_t>(group) * a.cols : a.x, rank, ks,
                       norm_ahead, squares, inv_n);
   }
   // The norm's 1 / rms of token k in lane k.
@@ -625,7 +628,7 @@ int LaunchTokens(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
 
 namespace {
 size_t MixtureShared(int cols) {
-  return SharedBytes<GUFO_CUDA_Q4_K, 1>(cols, Unit<GUFO_CUDA_Q4_K>::kDepth) +
+  return SharedBytes<GUFO_CUDA_Q4_K, 1>(cols, Unit<GUFO_CUDA_Q4_K>::kDepth, kMixLimbs) +
          static_cast<size_t>(kExchange) * (cols / kSuperBlock) * kTileRows * 4;
 }
 }  // namespace

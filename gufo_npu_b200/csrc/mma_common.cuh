@@ -24,6 +24,7 @@
 namespace gufo {
 
 constexpr int kLimbs = 3;            // byte planes per token
+constexpr int kMixLimbs = 4;         // of a mixture's input (one token): the fourth holds what rounding xi took off
 constexpr int kPlanePad = 32;        // bytes: plane stride = cols + 32 keeps the
                                      // 64-bit fragment reads free of bank conflicts
 constexpr int kFastWarps = 8;
@@ -44,14 +45,14 @@ struct ImageLayout {
   int bytes;
 };
 
-__host__ __device__ inline ImageLayout MakeImageLayout(int tokens, int cols, int group) {
+__host__ __device__ inline ImageLayout MakeImageLayout(int tokens, int cols, int group, int limbs = kLimbs) {
   ImageLayout l;
   l.tokens = tokens;
   l.cols = cols;
   l.group = group;
-  l.kcols = (tokens * kLimbs + 7) / 8 * 8;
+  l.kcols = (tokens * limbs + 7) / 8 * 8;
   l.plane_stride = cols + kPlanePad;
-  l.scale_at = tokens * kLimbs * l.plane_stride;
+  l.scale_at = tokens * limbs * l.plane_stride;
   l.sums_at = l.scale_at + (cols / kSuperBlock) * l.kcols * 4;
   l.bytes = l.sums_at + tokens * (cols / group) * 4;
   return l;
@@ -156,6 +157,7 @@ __device__ __forceinline__ void CopyImageToShared(uint8_t* dst, const uint8_t* s
 // or global memory): the calling warp's lane holds values 8 * lane .. + 7 of the
 // block in v. Writes the three byte planes, the group sums and the column
 // factors of block `b`.
+template <int LIMBS = kLimbs>
 __device__ __forceinline__ void StageBlock(const float (&v)[8], int lane, int tok, int b,
                                            const ImageLayout& l, uint8_t* image, float extra) {
   // Largest magnitude by integer compare of the bit patterns, so that a NaN
@@ -179,10 +181,16 @@ __device__ __forceinline__ void StageBlock(const float (&v)[8], int lane, int to
   // 128, in its three low bytes; flipping the offset bits leaves the signed
   // bytes. (A block with an infinity or NaN: any digits, `down` is NaN.)
   uint32_t z[8];
+  uint32_t rest[8];   // low bytes: the fourth limbs
   float sum = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const uint32_t bits = __float_as_uint(fmaf(v[i], up, 12582912.0f));
+    if constexpr (LIMBS == kMixLimbs) {
+      // What the rounding took off (exact, at most a half), in 254ths: -127 .. 127.
+      const float off = fmaf(v[i], up, 12582912.0f - __uint_as_float(bits));
+      rest[i] = __float_as_uint(fmaf(off, 254.0f, 12582912.0f));
+    }
     z[i] = (bits + (0x808080u - 0x4B400000u)) ^ 0x808080u;
     sum += v[i];
   }
@@ -191,8 +199,14 @@ __device__ __forceinline__ void StageBlock(const float (&v)[8], int lane, int to
     const uint32_t pick = 0x0040u + 0x11u * limb;  // byte `limb` of both operands
     const uint32_t w0 = __byte_perm(__byte_perm(z[0], z[1], pick), __byte_perm(z[2], z[3], pick), 0x5410u);
     const uint32_t w1 = __byte_perm(__byte_perm(z[4], z[5], pick), __byte_perm(z[6], z[7], pick), 0x5410u);
-    uint8_t* plane = image + static_cast<size_t>(tok * kLimbs + limb) * l.plane_stride;
+    uint8_t* plane = image + static_cast<size_t>(tok * LIMBS + limb) * l.plane_stride;
     *reinterpret_cast<uint2*>(plane + b * kSuperBlock + lane * 8) = make_uint2(w0, w1);
+  }
+  if constexpr (LIMBS == kMixLimbs) {
+    uint8_t* plane = image + static_cast<size_t>(tok * LIMBS + kLimbs) * l.plane_stride;
+    *reinterpret_cast<uint2*>(plane + b * kSuperBlock + lane * 8) =
+        make_uint2(__byte_perm(__byte_perm(rest[0], rest[1], 0x0040u), __byte_perm(rest[2], rest[3], 0x0040u), 0x5410u),
+                   __byte_perm(__byte_perm(rest[4], rest[5], 0x0040u), __byte_perm(rest[6], rest[7], 0x0040u), 0x5410u));
   }
   // Group sums of the fp32 values: the lanes of one group are adjacent.
   const int lanes_per_group = l.group / 8;  // 4 (groups of 32) or 2 (of 16)
@@ -204,10 +218,10 @@ __device__ __forceinline__ void StageBlock(const float (&v)[8], int lane, int to
     sums[static_cast<size_t>(tok) * (l.cols / l.group) + b * (kSuperBlock / l.group) +
          lane / lanes_per_group] = sum;
   }
-  if (lane < kLimbs) {
-    const float limb = lane == 0 ? 1.f : (lane == 1 ? 256.f : 65536.f);
+  if (lane < LIMBS) {
+    const float limb = lane == 0 ? 1.f : (lane == 1 ? 256.f : (lane == 2 ? 65536.f : 1.f / 254.f));
     float* scale = reinterpret_cast<float*>(image + l.scale_at);
-    scale[b * l.kcols + tok * kLimbs + lane] = down * limb * extra;
+    scale[b * l.kcols + tok * LIMBS + lane] = down * limb * extra;
   }
 }
 
@@ -277,12 +291,12 @@ __device__ __forceinline__ float RowScale(const FastGemvArgs& a, const float* sq
 }
 
 // Columns without a token keep a zero factor; independent of the input.
-template <int TOKENS>
+template <int TOKENS, int LIMBS = kLimbs>
 __device__ __forceinline__ void ZeroIdleColumns(const ImageLayout& l, int blocks, uint8_t* image) {
   float* scale = reinterpret_cast<float*>(image + l.scale_at);
 #pragma unroll 1
   for (int i = threadIdx.x; i < blocks * l.kcols; i += kFastThreads) {
-    if (i % l.kcols >= kLimbs * TOKENS) {
+    if (i % l.kcols >= LIMBS * TOKENS) {
       scale[i] = 0.f;
     }
   }
@@ -293,7 +307,7 @@ __device__ __forceinline__ void ZeroIdleColumns(const ImageLayout& l, int blocks
 // dealt round-robin) converts only the blocks of its own slabs; the others are
 // never read. keep_w: LoadNormAhead's. squares: [kFastWarps][TOKENS] in shared
 // memory, for RowScale. Ends with a __syncthreads. kFastThreads threads.
-template <int TOKENS>
+template <int TOKENS, int LIMBS = kLimbs>
 __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayout& l,
                                           uint8_t* image, float extra, const float* x,
                                           int rank, int ks, const float (&keep_w)[8],
@@ -408,7 +422,7 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
           }
         }
         if (mine(at_b[j])) {
-          StageBlock(w[j], lane, at_tok[j], at_b[j], l, image, extra);
+          StageBlock<LIMBS>(w[j], lane, at_tok[j], at_b[j], l, image, extra);
         }
       }
       first_unit = false;
@@ -474,7 +488,7 @@ __device__ __forceinline__ void FillImage(const FastGemvArgs& a, const ImageLayo
             v[j][i] = SiluFast(v[j][i]) * up[j][i];
           }
         }
-        StageBlock(v[j], lane, at_tok[j], at_b[j], l, image, extra);
+        StageBlock<LIMBS>(v[j], lane, at_tok[j], at_b[j], l, image, extra);
       }
     }
   }
