@@ -30,7 +30,10 @@ constexpr int kPlanePad = 32;        // bytes: plane stride = cols + 32 keeps th
 constexpr int kFastWarps = 8;
 constexpr int kFastThreads = kFastWarps * 32;
 constexpr int kMaxTokensFast = 8;    // tokens per launch (three MMA column groups)
-constexpr int kFastMaxShared = 200 * 1024;
+// Of dynamic shared memory; the kernels' own arrays (up to 4.5 KB) come on top. The line
+// decides how many rows one pass over the weights takes: at 200 KB eight rows of 5120
+// values went in two passes (Q6_K, 2560 rows: 20.8 us, in one 14.0).
+constexpr int kFastMaxShared = 220 * 1024;
 
 // Byte layout of the staged activations of `tokens` rows of `cols` values,
 // identical in global and shared memory. Every offset is a multiple of 16.

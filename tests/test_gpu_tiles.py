@@ -539,6 +539,22 @@ def test_units_of_ragged_rows(ctx, ggml_type, tokens, rows, cols):
     ctx.matrix_free(m)
 
 
+@pytest.mark.parametrize("ggml_type,tokens,cols", [(Q.GGML_Q4_K, 8, 5376), (Q.GGML_Q4_K, 7, 6144), (Q.GGML_Q4_K, 5, 8960),
+                                                  (Q.GGML_Q6_K, 8, 5120), (Q.GGML_Q6_K, 7, 5888), (Q.GGML_Q6_K, 5, 8192)])
+def test_widest_rows_of_one_pass(ctx, ggml_type, tokens, cols):
+    """The rows go over the weights once: a launch that converts them and one that multiplies."""
+    m, w = _matrix(ctx, ggml_type, 4800, cols, 9)
+    x = torch.from_numpy(G.normal(10, tokens, cols).astype(np.float32)).to("cuda:0")
+    y = torch.empty(tokens, 4800, device="cuda:0")
+    torch.cuda.synchronize()
+    before = ctx.launch_count()
+    ctx.matmul_device([(m, 0, 4800)], None, x, tokens, y)
+    assert ctx.launch_count() - before == 2
+    ctx.synchronize()
+    assert rel_l2(y.cpu().numpy(), x.cpu().numpy().astype(np.float64) @ w.T) <= 2e-6
+    ctx.matrix_free(m)
+
+
 @pytest.mark.parametrize("tokens,rows,cols", [(1, 9728, 2560), (1, 8192, 2048), (1, 7120, 512), (2, 9728, 2560), (2, 16, 512), (2, 6144, 2048)])
 def test_activating_product_with_more_tile_pairs_than_blocks(ctx, tokens, rows, cols):
     dev = torch.device("cuda:0")
