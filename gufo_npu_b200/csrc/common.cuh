@@ -224,8 +224,9 @@ size_t DeviceRowBytes(int type, int64_t cols);
 
 struct gufo_cuda_ctx;
 namespace gufo {
-// The device's address of pinned host memory; null for pageable memory.
-void* DeviceAddress(const void* host);
+// The device's address of `bytes` of pinned host memory at a float boundary; null for
+// memory that is not, or not all of it, pinned and the device's to address.
+void* DeviceAddress(const void* host, size_t bytes);
 // Enqueues one Q4_K part on the int8 tensor-core kernel against a staged image.
 int LaunchGemvQ4KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
 // The launch of gemv_units.cu, and whether its shared memory holds `tokens` rows.

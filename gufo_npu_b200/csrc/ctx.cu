@@ -2,6 +2,7 @@
 #include "common.cuh"
 #include "gemm_tc.cuh"
 
+#include <cuda.h>
 #include <sys/mman.h>
 
 #include <cstdlib>
@@ -300,14 +301,42 @@ HostPool& Pinned() {
 
 }  // namespace
 
-// The device's address of pinned host memory; null for pageable memory.
-void* DeviceAddress(const void* host) {
-  cudaPointerAttributes attr{};
-  if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) {
-    cudaGetLastError();   // memory CUDA does not know is not an error here
+namespace {
+// cuPointerGetAttributes, a host function of the driver (looked up once): several
+// attributes in one call, and no error for memory that CUDA does not know.
+using PointerAttributes = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+PointerAttributes PointerQuery() {
+  static const PointerAttributes query = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<PointerAttributes>(fn);
+  }();
+  return query;
+}
+}  // namespace
+
+void* DeviceAddress(const void* host, size_t bytes) {
+  const PointerAttributes query = PointerQuery();
+  if (query == nullptr || bytes == 0) {
     return nullptr;
   }
-  return attr.type == cudaMemoryTypeHost ? attr.devicePointer : nullptr;
+  unsigned type = 0;
+  CUdeviceptr device = 0, start = 0;
+  size_t size = 0;
+  CUpointer_attribute names[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* values[] = {&type, &device, &start, &size};
+  if (query(4, names, values, reinterpret_cast<CUdeviceptr>(host)) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST ||
+      device == 0 || device % sizeof(float) != 0) {
+    return nullptr;
+  }
+  // (The range is given by its device address.)
+  return device >= start && device + bytes <= start + size ? reinterpret_cast<void*>(device) : nullptr;
 }
 
 }  // namespace gufo

@@ -1532,6 +1532,8 @@ int gufo_cuda_decoder_reset(gufo_cuda_decoder* d) {
   return GUFO_CUDA_OK;
 }
 
+static int StepTokens(gufo_cuda_decoder* d, const int* tokens, int count, int want_logits, float* host_logits);
+
 int gufo_cuda_decoder_step_tokens(gufo_cuda_decoder* d, const int* tokens, int count, int want_logits,
                                   float* host_logits) {
   if (d == nullptr || tokens == nullptr) {
@@ -1557,6 +1559,16 @@ int gufo_cuda_decoder_step_tokens(gufo_cuda_decoder* d, const int* tokens, int c
   gufo_cuda_ctx* ctx = d->ctx;
   std::lock_guard<std::mutex> lock(ctx->mu);
   GUFO_CUDA_TRY(cudaSetDevice(ctx->device));
+  const int rc = StepTokens(d, tokens, count, want_logits, host_logits);
+  if (rc != GUFO_CUDA_OK && host_logits != nullptr) {
+    cudaStreamSynchronize(ctx->stream);   // what was enqueued before it failed may still write there
+  }
+  return rc;
+}
+
+// The step behind the checks; ctx->mu is held.
+static int StepTokens(gufo_cuda_decoder* d, const int* tokens, int count, int want_logits, float* host_logits) {
+  gufo_cuda_ctx* ctx = d->ctx;
   const int parity = d->conv_cur;
   const int pair = count - 1;
   const int with = want_logits != 0 ? 1 : 0;
@@ -1567,7 +1579,7 @@ int gufo_cuda_decoder_step_tokens(gufo_cuda_decoder* d, const int* tokens, int c
   // behind a pointer seen before may have been freed since.)
   float* mirror = nullptr;
   if (host_logits != nullptr && d->mirror_ok[pair] && !kernel_step && !d->timeline && !ctx->force_general) {
-    mirror = static_cast<float*>(gufo::DeviceAddress(host_logits));
+    mirror = static_cast<float*>(gufo::DeviceAddress(host_logits, static_cast<size_t>(count) * d->c.vocab * 4));
   }
   {
     const unsigned slot = d->next_slot++ % gufo::kStepSlots;

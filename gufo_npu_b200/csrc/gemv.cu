@@ -901,52 +901,58 @@ int gufo_cuda_matmul(gufo_cuda_ctx* ctx, const gufo_cuda_rows* parts, int nparts
   // thread) a kernel fetches it; more than kStagedBytes of pageable memory are left
   // to the driver's copy, whose fixed cost no longer counts there.
   constexpr size_t kStagedBytes = 1u << 20;
-  const float* from = static_cast<const float*>(gufo::DeviceAddress(host_x));
+  const float* from = static_cast<const float*>(gufo::DeviceAddress(host_x, x_bytes));
   if (from == nullptr && x_bytes <= kStagedBytes &&
       ctx->ReserveHost(&ctx->host_x, &ctx->host_x_bytes, x_bytes) == GUFO_CUDA_OK) {
     std::memcpy(ctx->host_x, host_x, x_bytes);
-    from = static_cast<const float*>(gufo::DeviceAddress(ctx->host_x));
-  }
-  if (from != nullptr && reinterpret_cast<uintptr_t>(from) % 16 == 0 && x_bytes <= kStagedBytes) {
-    const int blocks = static_cast<int>((x_values + 1023) / 1024);
-    GUFO_CUDA_TRY(gufo::LaunchOverlapped(gufo::FetchKernel, dim3(blocks), dim3(256), 0, ctx->stream, 1, from,
-                                         ctx->stage_x, static_cast<int64_t>(x_values)));
-    ctx->launches.fetch_add(1);
-  } else {
-    GUFO_CUDA_TRY(cudaMemcpyAsync(ctx->stage_x, host_x, x_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    from = static_cast<const float*>(gufo::DeviceAddress(ctx->host_x, x_bytes));
   }
   // y: the GEMV kernels store up to kDirectValues straight into pinned memory
   // (posted writes, hidden behind the weights); more go through device memory and a
   // copy, as single rows are a poor fit for PCIe.
   constexpr size_t kDirectValues = 16384;
-  float* to = static_cast<float*>(gufo::DeviceAddress(host_y));
+  float* to = static_cast<float*>(gufo::DeviceAddress(host_y, y_bytes));
   float* stage = nullptr;   // pinned memory that stands for a pageable y
   if (to == nullptr && y_bytes <= kStagedBytes &&
       ctx->ReserveHost(&ctx->host_y, &ctx->host_y_bytes, y_bytes) == GUFO_CUDA_OK) {
     stage = ctx->host_y;
-    to = static_cast<float*>(gufo::DeviceAddress(stage));
+    to = static_cast<float*>(gufo::DeviceAddress(stage, y_bytes));
   }
-  args.x = ctx->stage_x;
-  if (to != nullptr && tokens <= gufo::kMaxTokens && y_values <= kDirectValues) {
-    args.y = to;
-    rc = gufo::LaunchGemv(ctx, args, tokens);
-    if (rc != GUFO_CUDA_OK) {
-      return rc;
+  const bool direct = to != nullptr && tokens <= gufo::kMaxTokens && y_values <= kDirectValues;
+  auto enqueue = [&]() -> int {
+    if (from != nullptr && reinterpret_cast<uintptr_t>(from) % 16 == 0 && x_bytes <= kStagedBytes) {
+      const int blocks = static_cast<int>((x_values + 1023) / 1024);
+      GUFO_CUDA_TRY(gufo::LaunchOverlapped(gufo::FetchKernel, dim3(blocks), dim3(256), 0, ctx->stream, 1, from,
+                                           ctx->stage_x, static_cast<int64_t>(x_values)));
+      ctx->launches.fetch_add(1);
+    } else {
+      GUFO_CUDA_TRY(cudaMemcpyAsync(ctx->stage_x, host_x, x_bytes, cudaMemcpyHostToDevice, ctx->stream));
     }
-  } else {
-    rc = ctx->Reserve(&ctx->stage_y, &ctx->stage_y_bytes, y_bytes);
-    if (rc != GUFO_CUDA_OK) {
-      return rc;
+    args.x = ctx->stage_x;
+    if (direct) {
+      args.y = to;
+      return gufo::LaunchGemv(ctx, args, tokens);
+    }
+    int status = ctx->Reserve(&ctx->stage_y, &ctx->stage_y_bytes, y_bytes);
+    if (status != GUFO_CUDA_OK) {
+      return status;
     }
     args.y = ctx->stage_y;
-    rc = gufo::LaunchGemv(ctx, args, tokens);
-    if (rc != GUFO_CUDA_OK) {
-      return rc;
+    status = gufo::LaunchGemv(ctx, args, tokens);
+    if (status != GUFO_CUDA_OK) {
+      return status;
     }
     GUFO_CUDA_TRY(cudaMemcpyAsync(stage != nullptr ? stage : host_y, ctx->stage_y, y_bytes, cudaMemcpyDeviceToHost,
                                   ctx->stream));
+    return GUFO_CUDA_OK;
+  };
+  rc = enqueue();
+  // Also where it failed half way: the caller's buffers are its own again.
+  const cudaError_t waited = cudaStreamSynchronize(ctx->stream);
+  if (rc != GUFO_CUDA_OK) {
+    return rc;
   }
-  GUFO_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  GUFO_CUDA_TRY(waited);
   if (stage != nullptr) {
     std::memcpy(host_y, stage, y_bytes);
   }

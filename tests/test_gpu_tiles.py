@@ -228,6 +228,50 @@ def test_host_rows_pinned_and_pageable(ctx, tokens, rows, cols):
     ctx.matrix_free(m)
 
 
+@pytest.mark.parametrize("tokens,rows,cols", [(1, 9000, 256), (8, 9000, 512), (3, 700, 12288)])
+def test_host_rows_that_are_pinned_in_part_or_off_a_float(ctx, tokens, rows, cols):
+    """Buffers of which the first pages are registered, and ones that start inside a float: copied, the
+    same bytes. The step's logits likewise."""
+    import mmap
+    from gufo_npu_b200 import synth
+    from gufo_npu_b200.backend import CudaDecoder, CudaProjections
+    rt = torch.cuda.cudart()
+    m, w = _matrix(ctx, Q.GGML_Q4_K, rows, cols, 41)
+    x = G.normal(42, tokens, cols).astype(np.float32)
+    parts = Context._parts([(m, 0, rows)])
+    want = ctx.matmul([(m, 0, rows)], x, tokens, rows)
+    assert rel_l2(want, x.astype(np.float64) @ w.T) <= 1e-3
+    for registered, shift in ((4096, 0), (1 << 20, 2), (1 << 20, 4), (0, 1)):
+        buffers = [mmap.mmap(-1, 2 << 20) for _ in range(2)]
+        bx, by = (np.frombuffer(b, dtype=np.uint8) for b in buffers)
+        if registered:
+            assert int(rt.cudaHostRegister(bx.ctypes.data, registered, 0)) == 0
+            assert int(rt.cudaHostRegister(by.ctypes.data, registered, 0)) == 0
+        bx[shift:shift + x.nbytes] = x.view(np.uint8).ravel()
+        ctx.matmul_host(parts, 1, bx.ctypes.data + shift, tokens, by.ctypes.data + shift)
+        got = by[shift:shift + want.nbytes].tobytes()
+        if registered:
+            assert int(rt.cudaHostUnregister(bx.ctypes.data)) == 0 and int(rt.cudaHostUnregister(by.ctypes.data)) == 0
+        assert got == want.tobytes()
+    ctx.matrix_free(m)
+    if tokens == 1:
+        cfg = synth.ModelConfig(layers=4, hidden=256, ffn=512, vocab=40000, heads=2, kv_heads=1, head_dim=128, rope_dim=32,
+                                linear_key_heads=2, linear_value_heads=4, linear_head_dim=128)
+        tensors = synth.build_model(cfg, 3)
+        dec = CudaDecoder(CudaProjections(ctx, cfg, tensors), tensors, max_positions=64)
+        want = dec.Step(7)
+        for registered, shift in ((4096, 0), (1 << 20, 2)):
+            dec.Reset()
+            buffer = mmap.mmap(-1, 2 << 20)
+            b = np.frombuffer(buffer, dtype=np.uint8)
+            assert int(rt.cudaHostRegister(b.ctypes.data, registered, 0)) == 0
+            dec.Step(7, b.ctypes.data + shift)
+            got = b[shift:shift + want.nbytes].tobytes()
+            assert int(rt.cudaHostUnregister(b.ctypes.data)) == 0
+            assert got == want.tobytes()
+        dec.close()
+
+
 @pytest.mark.parametrize("vocab", [512, 40000])
 def test_step_logits_in_any_memory(ctx, vocab):
     """Logits left on the device (many steps, none waited for), in pageable, pooled
