@@ -677,8 +677,7 @@ class CudaDecoder:
 
     def close(self) -> None:
         if getattr(self, "handle", None):
-            if self.ctx.handle:   # a context closed first has taken its stream along
-                self.ctx.lib.gufo_cuda_decoder_destroy(self.handle)
+            self.ctx.lib.gufo_cuda_decoder_destroy(self.handle)
             self.handle = None
             self._address = 0
 

@@ -284,6 +284,7 @@ int LaunchGemvQ6KFast(gufo_cuda_ctx* ctx, const FastGemvArgs& args);
 bool Q6KFastFits(int cols, int tokens);
 }  // namespace gufo
 
+struct gufo_cuda_decoder;
 struct gufo_cuda_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -293,6 +294,9 @@ struct gufo_cuda_ctx {
   std::unordered_map<int64_t, gufo::Matrix> matrices;
   std::unordered_map<int64_t, gufo::DeltaNetLayer> deltanet_layers;
   int64_t next_id = 1;
+  // Decoders on this context and what gives their resources back: a context that goes
+  // first leaves them empty shells.
+  std::vector<std::pair<gufo_cuda_decoder*, void (*)(gufo_cuda_decoder*)>> decoders;
   // Staging for the host-pointer entry points.
   float* stage_x = nullptr;
   size_t stage_x_bytes = 0;

@@ -493,6 +493,9 @@ int gufo_cuda_ctx_destroy(gufo_cuda_ctx* ctx) {
   }
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();   // also work on a stream that set_stream replaced
+  for (const auto& decoder : ctx->decoders) {
+    decoder.second(decoder.first);
+  }
   for (auto& kv : ctx->matrices) {
     if (kv.second.owned) {
       cudaFree(const_cast<uint8_t*>(kv.second.data));

@@ -241,7 +241,8 @@ int gufo_cuda_attention_device(gufo_cuda_ctx* ctx, const gufo_cuda_attention_arg
 }  // extern "C"
 
 struct gufo_cuda_decoder {
-  gufo_cuda_ctx* ctx = nullptr;
+  gufo_cuda_ctx* ctx = nullptr;   // null once it has been destroyed
+  bool attached = false;          // in ctx->decoders
   gufo_cuda_decoder_config c{};
   struct Layer {
     bool attention = false;
@@ -691,6 +692,52 @@ int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens) 
   }
   Mark(d, GUFO_CUDA_TIMELINE_LM_HEAD);
   return GUFO_CUDA_OK;
+}
+
+// Gives back all that `d` holds and takes its context away; its work is done.
+void ReleaseDecoder(gufo_cuda_decoder* d) {
+  for (auto& per_count : d->graph) {
+    for (auto& per_window : per_count) {
+      for (cudaGraphExec_t& g : per_window) {
+        if (g != nullptr) {
+          cudaGraphExecDestroy(g);
+        }
+        g = nullptr;
+      }
+    }
+  }
+  for (void* p : d->owned) {
+    cudaFree(p);
+  }
+  d->owned.clear();
+  for (cudaEvent_t e : d->marks) {
+    cudaEventDestroy(e);
+  }
+  d->marks.clear();
+  if (d->slots != nullptr) {
+    cudaFreeHost(d->slots);
+    d->slots = nullptr;
+  }
+  for (cudaEvent_t& read : d->slot_read) {
+    if (read != nullptr) {
+      cudaEventDestroy(read);
+    }
+    read = nullptr;
+  }
+  if (d->plan.error_pinned != nullptr) {
+    cudaFreeHost(d->plan.error_pinned);
+    d->plan.error_pinned = nullptr;
+  }
+  d->ctx = nullptr;
+}
+
+// A decoder that a call may use; its context may have been destroyed before it.
+int CheckDecoder(const gufo_cuda_decoder* d, const char* what) {
+  if (d == nullptr) {
+    return Fail(GUFO_CUDA_BAD_ARGUMENT, std::string(what) + ": null decoder");
+  }
+  return d->ctx != nullptr ? GUFO_CUDA_OK
+                           : Fail(GUFO_CUDA_BAD_ARGUMENT, std::string(what) + ": the decoder's context has been destroyed");
 }
 
 // Describes the one-token step of `d` as a program for the persistent kernel.
@@ -1465,6 +1512,8 @@ int gufo_cuda_decoder_create(gufo_cuda_ctx* ctx, const gufo_cuda_decoder_config*
     return fail(rc);
   }
   *out = d;
+  ctx->decoders.emplace_back(d, gufo::ReleaseDecoder);
+  d->attached = true;
   // Zero states (the lock is already held: reset's body inline).
   if (d->conv_all_bytes > 0) {
     cudaMemsetAsync(d->conv_all[0], 0, d->conv_all_bytes, ctx->stream);
@@ -1481,41 +1530,28 @@ int gufo_cuda_decoder_destroy(gufo_cuda_decoder* d) {
   if (d == nullptr) {
     return GUFO_CUDA_OK;
   }
-  cudaSetDevice(d->ctx->device);
-  cudaStreamSynchronize(d->ctx->stream);
-  for (auto& per_count : d->graph) {
-    for (auto& per_window : per_count) {
-      for (cudaGraphExec_t g : per_window) {
-        if (g != nullptr) {
-          cudaGraphExecDestroy(g);
+  if (d->ctx != nullptr) {
+    cudaSetDevice(d->ctx->device);
+    cudaStreamSynchronize(d->ctx->stream);
+    if (d->attached) {
+      std::lock_guard<std::mutex> lock(d->ctx->mu);
+      auto& all = d->ctx->decoders;
+      for (size_t i = 0; i < all.size(); ++i) {
+        if (all[i].first == d) {
+          all.erase(all.begin() + i);
+          break;
         }
       }
     }
-  }
-  for (void* p : d->owned) {
-    cudaFree(p);
-  }
-  for (cudaEvent_t e : d->marks) {
-    cudaEventDestroy(e);
-  }
-  if (d->slots != nullptr) {
-    cudaFreeHost(d->slots);
-  }
-  for (cudaEvent_t read : d->slot_read) {
-    if (read != nullptr) {
-      cudaEventDestroy(read);
-    }
-  }
-  if (d->plan.error_pinned != nullptr) {
-    cudaFreeHost(d->plan.error_pinned);
+    gufo::ReleaseDecoder(d);
   }
   delete d;
   return GUFO_CUDA_OK;
 }
 
 int gufo_cuda_decoder_reset(gufo_cuda_decoder* d) {
-  if (d == nullptr) {
-    return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_reset: null decoder");
+  if (const int gone = gufo::CheckDecoder(d, "decoder_reset"); gone != GUFO_CUDA_OK) {
+    return gone;
   }
   gufo_cuda_ctx* ctx = d->ctx;
   std::lock_guard<std::mutex> lock(ctx->mu);
@@ -1536,6 +1572,9 @@ static int StepTokens(gufo_cuda_decoder* d, const int* tokens, int count, int wa
 
 int gufo_cuda_decoder_step_tokens(gufo_cuda_decoder* d, const int* tokens, int count, int want_logits,
                                   float* host_logits) {
+  if (const int gone = gufo::CheckDecoder(d, "decoder_step_tokens"); gone != GUFO_CUDA_OK) {
+    return gone;
+  }
   if (d == nullptr || tokens == nullptr) {
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_step: null pointer");
   }
@@ -1666,8 +1705,8 @@ static int StepTokens(gufo_cuda_decoder* d, const int* tokens, int count, int wa
 }
 
 int gufo_cuda_decoder_status(gufo_cuda_decoder* d) {
-  if (d == nullptr) {
-    return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_status: null decoder");
+  if (const int gone = gufo::CheckDecoder(d, "decoder_status"); gone != GUFO_CUDA_OK) {
+    return gone;
   }
   gufo_cuda_ctx* ctx = d->ctx;
   std::lock_guard<std::mutex> lock(ctx->mu);
@@ -1678,6 +1717,9 @@ int gufo_cuda_decoder_status(gufo_cuda_decoder* d) {
 
 int gufo_cuda_decoder_step_profile(gufo_cuda_decoder* d, int capacity, int* stages, int64_t* bytes, double* us,
                                    int* count) {
+  if (const int gone = gufo::CheckDecoder(d, "decoder_step_profile"); gone != GUFO_CUDA_OK) {
+    return gone;
+  }
   if (d == nullptr || count == nullptr) {
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_step_profile: null pointer");
   }
@@ -1714,8 +1756,8 @@ int gufo_cuda_decoder_step(gufo_cuda_decoder* d, int token, float* host_logits) 
 }
 
 int gufo_cuda_decoder_resolve(gufo_cuda_decoder* d, int keep_second) {
-  if (d == nullptr) {
-    return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_resolve: null decoder");
+  if (const int gone = gufo::CheckDecoder(d, "decoder_resolve"); gone != GUFO_CUDA_OK) {
+    return gone;
   }
   if (d->pending != 2) {
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_resolve: the last step was not a two-token step");
@@ -1746,6 +1788,9 @@ int gufo_cuda_decoder_resolve(gufo_cuda_decoder* d, int keep_second) {
 }
 
 int gufo_cuda_decoder_hidden_device(gufo_cuda_decoder* d, int t, const float** hidden) {
+  if (const int gone = gufo::CheckDecoder(d, "decoder_hidden_device"); gone != GUFO_CUDA_OK) {
+    return gone;
+  }
   if (d == nullptr || hidden == nullptr || t < 0 || t >= gufo::kStepTokens || d->final_h == nullptr) {
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_hidden_device: no such row");
   }
@@ -1754,6 +1799,9 @@ int gufo_cuda_decoder_hidden_device(gufo_cuda_decoder* d, int t, const float** h
 }
 
 int gufo_cuda_decoder_logits_device(gufo_cuda_decoder* d, const float** device_logits) {
+  if (const int gone = gufo::CheckDecoder(d, "decoder_logits_device"); gone != GUFO_CUDA_OK) {
+    return gone;
+  }
   if (d == nullptr || device_logits == nullptr) {
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_logits_device: null pointer");
   }
@@ -1762,8 +1810,8 @@ int gufo_cuda_decoder_logits_device(gufo_cuda_decoder* d, const float** device_l
 }
 
 int gufo_cuda_decoder_timeline(gufo_cuda_decoder* d, int enable, double* stage_ms, int* steps) {
-  if (d == nullptr) {
-    return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_timeline: null decoder");
+  if (const int gone = gufo::CheckDecoder(d, "decoder_timeline"); gone != GUFO_CUDA_OK) {
+    return gone;
   }
   std::lock_guard<std::mutex> lock(d->ctx->mu);
   if (stage_ms != nullptr) {
@@ -1787,6 +1835,9 @@ int gufo_cuda_decoder_timeline(gufo_cuda_decoder* d, int enable, double* stage_m
 int gufo_cuda_decoder_position(const gufo_cuda_decoder* d) { return d == nullptr ? -1 : d->position; }
 
 int gufo_cuda_decoder_linear_state(gufo_cuda_decoder* d, int layer, float* host_conv, float* host_ssm) {
+  if (const int gone = gufo::CheckDecoder(d, "decoder_linear_state"); gone != GUFO_CUDA_OK) {
+    return gone;
+  }
   if (d == nullptr || layer < 0 || layer >= static_cast<int>(d->layers.size()) || d->layers[layer].attention) {
     return Fail(GUFO_CUDA_BAD_ARGUMENT, "decoder_linear_state: not a DeltaNet layer");
   }

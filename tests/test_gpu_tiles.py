@@ -272,6 +272,33 @@ def test_host_rows_that_are_pinned_in_part_or_off_a_float(ctx, tokens, rows, col
         dec.close()
 
 
+@pytest.mark.parametrize("context_first", [False, True])
+def test_decoder_and_context_closed_in_either_order(context_first):
+    """All memory comes back, and a decoder whose context has gone refuses to step."""
+    from gufo_npu_b200 import _capi, synth
+    from gufo_npu_b200.backend import CudaDecoder, CudaProjections
+    cfg = synth.ModelConfig(layers=4, hidden=256, ffn=512, vocab=512, heads=2, kv_heads=1, head_dim=128, rope_dim=32,
+                            linear_key_heads=2, linear_value_heads=4, linear_head_dim=128)
+    tensors = synth.build_model(cfg, 3)
+    free = []
+    for _ in range(4):
+        own = Context(0)
+        dec = CudaDecoder(CudaProjections(own, cfg, tensors), tensors, max_positions=1 << 17)   # 64 MB of cache
+        for token in (5, 6, 7, 8):
+            dec.Step(token)
+        if context_first:
+            own.close()
+            for call in (lambda: dec.Step(9), lambda: dec.StepTokens([9, 10]), dec.Reset, lambda: dec.Resolve(True),
+                         lambda: dec.step_device(9)):
+                with pytest.raises(_capi.GufoCudaError, match="context"):
+                    call()
+        dec.close()
+        dec.close()
+        own.close()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[-1] < 16 << 20, free
+
+
 @pytest.mark.parametrize("vocab", [512, 40000])
 def test_step_logits_in_any_memory(ctx, vocab):
     """Logits left on the device (many steps, none waited for), in pageable, pooled
