@@ -88,7 +88,10 @@ constexpr int kTcThreads = (kMmaWarp + 1) * 32;
 constexpr int kMaxStages = 10;
 constexpr long long kWaitCycles = 1ll << 31;           // about a second of SM clocks
 constexpr int kHeaderBytes = 4096;                     // of the scratch: error word, counters of cut tiles
-constexpr size_t kScratchFloor = 48u << 20;            // of the scratch: one allocation serves most shapes
+// Token rows a pass: eight of the widest groups. Their fp16 tiles and the partial sums
+// are scratch that stays allocated, so it is bounded (90 MB for rows of 9728 values),
+// whatever the prompt; a pass dequantizes the weights once per group anyway.
+constexpr int kPassTokens = 8 * 192;
 constexpr int kSharedLimit = 227 * 1024;
 
 // The raw bytes of one block of 128 rows in shared memory.
@@ -989,8 +992,17 @@ int ReserveTc(gufo_cuda_ctx* ctx, size_t bytes) {
     return GUFO_CUDA_OK;
   }
   // An outgrown block is kept (a captured graph may hold it); its error word
-  // is not carried over: a failure is read from the current block.
-  const int rc = ctx->GrowScratch(&ctx->tc_scratch, &ctx->tc_scratch_bytes, bytes, kScratchFloor, "tcgen05 gemm");
+  // is not carried over: a failure is read from the current block. In few steps, so
+  // that little is outgrown: one allocation serves most shapes of a model.
+  constexpr size_t kSteps[] = {1u << 20, 8u << 20, 48u << 20};
+  size_t floor = (bytes + kSteps[2] - 1) / kSteps[2] * kSteps[2];
+  for (size_t step : kSteps) {
+    if (bytes <= step) {
+      floor = step;
+      break;
+    }
+  }
+  const int rc = ctx->GrowScratch(&ctx->tc_scratch, &ctx->tc_scratch_bytes, bytes, floor, "tcgen05 gemm");
   if (rc != GUFO_CUDA_OK) {
     return rc;
   }
@@ -1181,6 +1193,20 @@ int LaunchGemmTc(gufo_cuda_ctx* ctx, const GemvArgs& base, int tokens) {
     if ((reinterpret_cast<uintptr_t>(base.parts[p].data) & 15) != 0 || base.parts[p].row_bytes % 16 != 0) {
       return Fail(GUFO_CUDA_BAD_ARGUMENT, "tcgen05 gemm: weight rows must be 16-byte aligned");
     }
+  }
+  if (tokens > kPassTokens) {
+    const int passes = (tokens + kPassTokens - 1) / kPassTokens;
+    const int each = ((tokens + passes - 1) / passes + 15) / 16 * 16;
+    for (int t0 = 0; t0 < tokens; t0 += each) {
+      GemvArgs pass = base;
+      pass.x = base.x + static_cast<size_t>(t0) * base.cols;
+      pass.y = base.y + static_cast<size_t>(t0) * base.y_stride;
+      const int rc = LaunchGemmTc(ctx, pass, tokens - t0 < each ? tokens - t0 : each);
+      if (rc != GUFO_CUDA_OK) {
+        return rc;
+      }
+    }
+    return GUFO_CUDA_OK;
   }
   // Parts of one block format share a launch, up to kTcMaxParts each.
   for (int type : {GUFO_CUDA_Q4_K, GUFO_CUDA_Q6_K}) {

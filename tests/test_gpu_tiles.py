@@ -54,6 +54,31 @@ def test_gemm_tiles_groups_and_cuts(ctx, ggml_type, tokens, rows, cols):
     ctx.matrix_free(m)
 
 
+def test_gemm_scratch_is_bounded(ctx):
+    """A product of a few rows takes little, one of many no more for ever more rows; those in passes
+    are right."""
+    own = Context(0)
+    dev = torch.device("cuda:0")
+    small, _ = _matrix(own, Q.GGML_Q4_K, 16, 256, 1)
+    wide, w = _matrix(own, Q.GGML_Q4_K, 16, 9728, 2)
+    x = torch.randn(12000, 9728, device=dev, generator=torch.Generator(device=dev).manual_seed(1))
+    y = torch.empty(12000, 16, device=dev)
+
+    def taken(m, tokens, cols):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        own.matmul_device([(m, 0, 16)], None, x, tokens, y)
+        own.synchronize()
+        return (before - torch.cuda.mem_get_info()[0]) >> 20
+    assert taken(small, 17, 256) <= 4
+    first = [taken(wide, tokens, 9728) for tokens in (1537, 3100)]
+    assert sum(first) <= 200
+    want = x[:3100].double() @ torch.from_numpy(w).to(dev).T
+    assert rel_l2(y[:3100].cpu().numpy(), want.cpu().numpy()) <= 5e-4
+    assert [taken(wide, tokens, 9728) for tokens in (4000, 6000, 9000, 12000)] == [0, 0, 0, 0]
+    own.close()
+
+
 @pytest.mark.parametrize("ggml_type", [Q.GGML_Q4_K, Q.GGML_Q6_K])
 @pytest.mark.parametrize("tokens,rows,cols", [
     (2, 40, 2048), (3, 4752, 1280), (3, 33, 1536), (4, 4736, 2560), (5, 16, 2048), (8, 17, 256), (8, 4753, 1280), (6, 31, 1792),
