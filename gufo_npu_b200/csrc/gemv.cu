@@ -319,6 +319,17 @@ GemvRowsF32(const __grid_constant__ GemvArgs args, int tokens) {
 template <int ROWS>
 int LaunchRowsF32(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
   const unsigned rows = (args.total_rows + ROWS - 1) / ROWS;
+  constexpr int kMost = 65535 * 8;   // what a grid's second dimension holds of the tiles below
+  if (tokens > kMost) {
+    const int rc = LaunchRowsF32<ROWS>(ctx, args, kMost);
+    if (rc != GUFO_CUDA_OK) {
+      return rc;
+    }
+    GemvArgs rest = args;
+    rest.x += static_cast<size_t>(kMost) * args.cols;
+    rest.y += static_cast<size_t>(kMost) * args.y_stride;
+    return LaunchRowsF32<ROWS>(ctx, rest, tokens - kMost);
+  }
   auto launch = [&](auto kernel, int tok) {
     return LaunchOverlapped(kernel, dim3(rows, (tokens + tok - 1) / tok), dim3(256), 0, ctx->stream, 1, args, tokens);
   };

@@ -54,6 +54,20 @@ def test_gemm_tiles_groups_and_cuts(ctx, ggml_type, tokens, rows, cols):
     ctx.matrix_free(m)
 
 
+def test_f32_rows_of_more_tokens_than_a_grid_holds(ctx):
+    dev = torch.device("cuda:0")
+    tokens = 65535 * 8 + 3
+    w = G.normal(5, 2, 4).astype(np.float32)
+    m = ctx.matrix_upload(Q.GGML_F32, w.view(np.uint8), 2, 4)
+    x, y = torch.randn(tokens, 4, device=dev), torch.empty(tokens, 2, device=dev)
+    torch.cuda.synchronize()
+    ctx.matmul_device([(m, 0, 2)], None, x, tokens, y)
+    ctx.synchronize()
+    want = x.double() @ torch.from_numpy(w).to(dev).double().T
+    assert (y - want).abs().max() <= 1e-5
+    ctx.matrix_free(m)
+
+
 def test_gemm_scratch_is_bounded(ctx):
     """A product of a few rows takes little, one of many no more for ever more rows; those in passes
     are right."""
