@@ -289,6 +289,7 @@ struct gufo_cuda_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  bool stream_replaced = false;   // a caller's stream, by set_stream: work may be left on it
   int sm_count = 0;
   std::mutex mu;
   std::unordered_map<int64_t, gufo::Matrix> matrices;

@@ -492,7 +492,10 @@ int gufo_cuda_ctx_destroy(gufo_cuda_ctx* ctx) {
     return GUFO_CUDA_OK;
   }
   cudaSetDevice(ctx->device);
-  cudaDeviceSynchronize();   // also work on a stream that set_stream replaced
+  // Scratch goes to the pool only where nothing can still use it: not where a caller's
+  // stream was replaced, on which work may be left (its handle may be gone, and waiting
+  // for the device would end a capture of another thread). cudaFree waits by itself.
+  const bool idle = cudaStreamSynchronize(ctx->stream) == cudaSuccess && !ctx->stream_replaced;
   for (const auto& decoder : ctx->decoders) {
     decoder.second(decoder.first);
   }
@@ -515,8 +518,10 @@ int gufo_cuda_ctx_destroy(gufo_cuda_ctx* ctx) {
   ctx->retired.emplace_back(ctx->image, ctx->image_bytes);
   ctx->retired.emplace_back(ctx->tc_scratch, ctx->tc_scratch_bytes);
   for (const auto& block : ctx->retired) {
-    if (block.first != nullptr) {
+    if (block.first != nullptr && idle) {
       gufo::Pool().Give(ctx->device, block.first, block.second);
+    } else {
+      cudaFree(block.first);
     }
   }
   gufo::Pool().Leave(ctx->device);
@@ -556,6 +561,8 @@ int gufo_cuda_ctx_set_stream(gufo_cuda_ctx* ctx, void* stream) {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
     ctx->own_stream = false;
+  } else if (ctx->stream != stream) {
+    ctx->stream_replaced = true;
   }
   ctx->stream = static_cast<cudaStream_t>(stream);
   ctx->NameStream();

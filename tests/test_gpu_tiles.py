@@ -54,6 +54,28 @@ def test_gemm_tiles_groups_and_cuts(ctx, ggml_type, tokens, rows, cols):
     ctx.matrix_free(m)
 
 
+@pytest.mark.parametrize("replaced", [False, True])
+def test_scratch_of_a_context_that_changed_streams_is_not_handed_on(ctx, replaced):
+    """Work may be left on the stream it was given first; of others the next context takes it over."""
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    x, y = torch.randn(512, 2560, device="cuda:0"), torch.empty(512, 16, device="cuda:0")
+    free = []
+    for _ in range(2):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        own = Context(0, streams[0].cuda_stream)
+        m, _ = _matrix(own, Q.GGML_Q4_K, 4096, 2560, 1)
+        y = torch.empty(512, 4096, device="cuda:0")
+        torch.cuda.synchronize()
+        own.matmul_device([(m, 0, 4096)], None, x, 512, y)
+        if replaced:
+            own.set_stream(streams[1].cuda_stream)
+        own.close()
+        del y
+        free.append((before - torch.cuda.mem_get_info()[0]) >> 20)
+    assert free[1] <= 8 and (not replaced or free[0] <= 24), free
+
+
 def test_f32_rows_of_more_tokens_than_a_grid_holds(ctx):
     dev = torch.device("cuda:0")
     tokens = 65535 * 8 + 3
