@@ -192,31 +192,43 @@ SIGNATURES = {
 }
 
 _lib = None
-native = None   # the extension module _native once load() has bound it
+native = None   # the extension module _native once load_native() has bound it
 
 
 def load(path: str = LIB_PATH) -> C.CDLL:
     """Loads the library and declares every entry point; raises if it is not built."""
-    global _lib, native
+    global _lib
     if _lib is not None:
         return _lib
     if not os.path.exists(path):
         raise FileNotFoundError(
             f"{path} is not built: run `python -m gufo_npu_b200.build` (this backend has no CPU path)")
-    import torch  # noqa: F401  (its libraries have to be in the process before the extension's)
-    try:
-        from . import _native
-    except ImportError as e:
-        raise ImportError(f"gufo_npu_b200._native is not built: run `python -m gufo_npu_b200.build` ({e})") from e
     lib = C.CDLL(path)
     for name, (restype, argtypes) in SIGNATURES.items():
         fn = getattr(lib, name)
         fn.restype = restype
         fn.argtypes = argtypes
-    _native.bind(lib._handle)
-    native = _native
     _lib = lib
     return lib
+
+
+def load_native():
+    """Binds the extension that makes the per-token calls to the loaded library; needs torch, which
+    load() does not."""
+    global native
+    if native is None:
+        lib = load()
+        import torch   # its libraries have to be in the process before the extension's
+        try:
+            from . import _native
+        except ImportError as e:
+            raise ImportError(f"gufo_npu_b200._native is not built: run `python -m gufo_npu_b200.build` ({e})") from e
+        if _native.torch_version != torch.__version__:
+            raise ImportError(f"gufo_npu_b200._native was built for torch {_native.torch_version}, this is "
+                              f"{torch.__version__}: run `python -m gufo_npu_b200.build`")
+        _native.bind(lib._handle)
+        native = _native
+    return native
 
 
 def check(lib: C.CDLL, ctx, status: int) -> None:

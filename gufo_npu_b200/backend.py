@@ -81,6 +81,7 @@ class Context:
 
     def __init__(self, device: int = 0, stream: Optional[int] = None):
         self.lib = _capi.load()
+        _capi.load_native()
         handle = C.c_void_p()
         status = self.lib.gufo_cuda_ctx_create(device, C.c_void_p(stream or 0), C.byref(handle))
         _capi.check(self.lib, None, status)

@@ -1,9 +1,10 @@
-"""Builds libgufo_cuda.so (the C-ABI library, nvcc for sm_100a) and _native.so (the Python side's
-per-call work, the host compiler) in-tree."""
+"""Builds libgufo_cuda.so (the C-ABI library, nvcc for sm_100a) and the extension module _native (the
+Python side's per-call work, the host compiler) in-tree."""
 from __future__ import annotations
 
 import importlib.util
 import os
+import runpy
 import subprocess
 import sys
 import sysconfig
@@ -12,7 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgufo_cuda.so")
-NATIVE = os.path.join(HERE, "_native.so")
+NATIVE = os.path.join(HERE, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))   # of this interpreter
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -34,11 +35,18 @@ def _stale(target: str = LIB, suffixes=(".cu", ".cuh")) -> bool:
 
 def build_native(force: bool = False) -> str:
     """Compiles csrc/native.cpp against the interpreter's and torch's headers; returns its path."""
-    if not force and not _stale(NATIVE, (".cpp",)):
-        return NATIVE
     torch = os.path.dirname(importlib.util.find_spec("torch").origin)
+    version = runpy.run_path(os.path.join(torch, "version.py"))["__version__"]
+    if not force and not _stale(NATIVE, (".cpp",)):
+        with open(NATIVE, "rb") as f:
+            if version.encode() + b"\0" in f.read():   # built for this torch
+                return NATIVE
+    untagged = os.path.join(HERE, "_native.so")
+    if os.path.exists(untagged):   # any interpreter would take it
+        os.remove(untagged)
     include = os.path.join(torch, "include")
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-fvisibility=hidden",
+           f'-DGUFO_TORCH_VERSION="{version}"',
            "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"], "-isystem", include,
            "-isystem", os.path.join(include, "torch", "csrc", "api", "include"), "-isystem", "/usr/local/cuda/include",
            os.path.join(CSRC, "native.cpp"), "-o", NATIVE,

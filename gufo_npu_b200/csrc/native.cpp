@@ -16,6 +16,7 @@
 
 #include <dlfcn.h>
 
+#include <memory>
 #include <vector>
 
 #include "gufo_cuda.h"
@@ -98,12 +99,15 @@ T* Ptr(PyObject* o) {
   }
   if (PyObject_HasAttrString(o, "__array_interface__")) {   // numpy
     Py_buffer view;
-    if (PyObject_GetBuffer(o, &view, PyBUF_STRIDED_RO) != 0) {
-      throw Failed();
+    if (PyObject_GetBuffer(o, &view, PyBUF_STRIDED_RO) == 0) {
+      void* p = view.buf;
+      PyBuffer_Release(&view);   // the array outlives the call: the caller holds it
+      return static_cast<T*>(p);
     }
-    void* p = view.buf;
-    PyBuffer_Release(&view);   // the array outlives the call: the caller holds it
-    return static_cast<T*>(p);
+    PyErr_Clear();   // an element type that the buffer protocol has no name for
+    Ref ctypes(PyObject_GetAttrString(o, "ctypes"));
+    Ref data(PyObject_GetAttrString(ctypes.o, "data"));
+    return static_cast<T*>(PyLong_AsVoidPtr(data.o));
   }
   Ref data(PyObject_CallMethod(o, "data_ptr", nullptr));
   return static_cast<T*>(PyLong_AsVoidPtr(data.o));
@@ -120,28 +124,52 @@ int64_t RowStride(PyObject* o) {
 // The keys of the per-sequence dicts, interned once.
 struct Keys {
   PyObject *state, *state_out, *q, *k, *v, *decay, *beta, *y, *in, *h, *conv_in, *conv_out, *conv_saved, *ssm,
-      *ssm_out, *ssm_spec, *n_tokens;
+      *ssm_out, *ssm_spec, *n_tokens, *get;
 } keys;
 
-// A required entry (KeyError as from `seq[key]`). The dict keeps the value alive.
-PyObject* Item(PyObject* dict, PyObject* key) {
-  PyObject* o = PyDict_GetItemWithError(dict, key);
-  if (o == nullptr) {
-    if (!PyErr_Occurred()) {
-      PyErr_SetObject(PyDict_Check(dict) ? PyExc_KeyError : PyExc_TypeError, key);
+// One sequence's description: a dict, which keeps its values alive, or any other
+// mapping, whose values are held here.
+struct Entries {
+  explicit Entries(PyObject* o) : o(o), plain(PyDict_CheckExact(o)) {}
+  ~Entries() {
+    for (PyObject* v : held) {
+      Py_DECREF(v);
     }
-    throw Failed();
   }
-  return o;
-}
-
-PyObject* Optional(PyObject* dict, PyObject* key) {
-  PyObject* o = PyDict_GetItemWithError(dict, key);
-  if (o == nullptr && PyErr_Occurred()) {
-    throw Failed();
+  Entries(const Entries&) = delete;
+  Entries& operator=(const Entries&) = delete;
+  PyObject* Hold(PyObject* v) {
+    held.push_back(Must(v));
+    return v;
   }
-  return o == nullptr ? Py_None : o;
-}
+  // A required entry (KeyError as from `seq[key]`).
+  PyObject* Item(PyObject* key) {
+    if (!plain) {
+      return Hold(PyObject_GetItem(o, key));
+    }
+    PyObject* v = PyDict_GetItemWithError(o, key);
+    if (v == nullptr) {
+      if (!PyErr_Occurred()) {
+        PyErr_SetObject(PyExc_KeyError, key);
+      }
+      throw Failed();
+    }
+    return v;
+  }
+  PyObject* Optional(PyObject* key) {
+    if (!plain) {
+      return Hold(PyObject_CallMethodObjArgs(o, keys.get, key, nullptr));
+    }
+    PyObject* v = PyDict_GetItemWithError(o, key);
+    if (v == nullptr && PyErr_Occurred()) {
+      throw Failed();
+    }
+    return v == nullptr ? Py_None : v;
+  }
+  PyObject* o;
+  bool plain;
+  std::vector<PyObject*> held;
+};
 
 gufo_cuda_ctx* Context(PyObject* o) { return static_cast<gufo_cuda_ctx*>(PyLong_AsVoidPtr(o)); }
 
@@ -150,13 +178,16 @@ gufo_cuda_ctx* Context(PyObject* o) { return static_cast<gufo_cuda_ctx*>(PyLong_
 struct Parts {
   explicit Parts(PyObject* o) {
     if (PyObject_CheckBuffer(o)) {
-      if (PyObject_GetBuffer(o, &view, PyBUF_SIMPLE) != 0) {
-        throw Failed();
+      if (PyObject_GetBuffer(o, &view, PyBUF_ND) == 0) {
+        if (view.itemsize == sizeof(gufo_cuda_rows)) {
+          held = true;
+          data = static_cast<const gufo_cuda_rows*>(view.buf);
+          count = static_cast<int>(view.len / sizeof(gufo_cuda_rows));
+          return;
+        }
+        PyBuffer_Release(&view);
       }
-      held = true;
-      data = static_cast<const gufo_cuda_rows*>(view.buf);
-      count = static_cast<int>(view.len / sizeof(gufo_cuda_rows));
-      return;
+      PyErr_Clear();   // an array of numbers: a sequence like any other
     }
     Ref list(PySequence_Fast(o, "gufo_cuda: parts must be a sequence"));
     count = static_cast<int>(PySequence_Fast_GET_SIZE(list.o));
@@ -188,23 +219,30 @@ struct Parts {
 };
 
 // One C array element per dict of a sequence of dicts.
-template <typename Seq, typename Fill>
-std::vector<Seq> Gather(PyObject* seqs, Fill fill) {
-  Ref list(PySequence_Fast(seqs, "gufo_cuda: a sequence of dicts is needed"));
-  const Py_ssize_t n = PySequence_Fast_GET_SIZE(list.o);
-  std::vector<Seq> out;
-  out.reserve(n > 0 ? n : 1);
-  for (Py_ssize_t i = 0; i < n; ++i) {
-    PyObject* d = PySequence_Fast_GET_ITEM(list.o, i);
-    if (!PyDict_Check(d)) {
-      PyErr_SetString(PyExc_TypeError, "gufo_cuda: a sequence is described by a dict");
-      throw Failed();
+template <typename Seq>
+struct Gathered {
+  template <typename Fill>
+  Gathered(PyObject* seqs, Fill fill) : list(PySequence_Fast(seqs, "gufo_cuda: a sequence of dicts is needed")) {
+    const Py_ssize_t n = PySequence_Fast_GET_SIZE(list.o);
+    all.reserve(n > 0 ? n : 1);
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      PyObject* d = PySequence_Fast_GET_ITEM(list.o, i);
+      all.emplace_back();
+      if (PyDict_CheckExact(d)) {
+        Entries plain(d);
+        fill(plain, &all.back());
+      } else {
+        mappings.emplace_back(std::make_unique<Entries>(d));
+        fill(*mappings.back(), &all.back());
+      }
     }
-    out.emplace_back();
-    fill(d, &out.back());
   }
-  return out;
-}
+  const Seq* data() const { return all.data(); }
+  int count() const { return static_cast<int>(all.size()); }
+  Ref list;
+  std::vector<Seq> all;
+  std::vector<std::unique_ptr<Entries>> mappings;
+};
 
 template <typename Call>
 PyObject* Unlocked(Call call) {
@@ -265,18 +303,18 @@ PyObject* MatmulDevice(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* DeltaRule(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return Guarded(n, 5, [&] {
     gufo_cuda_ctx* ctx = Context(a[0]);
-    const auto seqs = Gather<gufo_cuda_delta_seq>(a[1], [](PyObject* d, gufo_cuda_delta_seq* s) {
-      s->state = Ptr<float>(Item(d, keys.state));
-      s->state_out = Ptr<float>(Optional(d, keys.state_out));
-      s->q = Ptr<const float>(Item(d, keys.q));
-      s->k = Ptr<const float>(Item(d, keys.k));
-      s->v = Ptr<const float>(Item(d, keys.v));
-      s->decay = Ptr<const float>(Item(d, keys.decay));
-      s->beta = Ptr<const float>(Item(d, keys.beta));
-      s->y = Ptr<float>(Item(d, keys.y));
+    const Gathered<gufo_cuda_delta_seq> seqs(a[1], [](Entries& d, gufo_cuda_delta_seq* s) {
+      s->state = Ptr<float>(d.Item(keys.state));
+      s->state_out = Ptr<float>(d.Optional(keys.state_out));
+      s->q = Ptr<const float>(d.Item(keys.q));
+      s->k = Ptr<const float>(d.Item(keys.k));
+      s->v = Ptr<const float>(d.Item(keys.v));
+      s->decay = Ptr<const float>(d.Item(keys.decay));
+      s->beta = Ptr<const float>(d.Item(keys.beta));
+      s->y = Ptr<float>(d.Item(keys.y));
     });
     const int hk = SmallInt(a[2]), hv = SmallInt(a[3]), dk = SmallInt(a[4]);
-    const int count = static_cast<int>(seqs.size());
+    const int count = seqs.count();
     return Unlocked([&] { return api.delta_rule(ctx, seqs.data(), count, hk, hv, dk); });
   });
 }
@@ -286,15 +324,15 @@ PyObject* DeltaNetLinear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return Guarded(n, 3, [&] {
     gufo_cuda_ctx* ctx = Context(a[0]);
     const long long layer = Int(a[1]);
-    const auto seqs = Gather<gufo_cuda_linear_seq>(a[2], [](PyObject* d, gufo_cuda_linear_seq* s) {
-      s->in = Ptr<const float>(Item(d, keys.in));
-      s->conv_in = Ptr<const float>(Item(d, keys.conv_in));
-      s->conv_out = Ptr<float>(Item(d, keys.conv_out));
-      s->ssm = Ptr<float>(Item(d, keys.ssm));
-      s->ssm_out = Ptr<float>(Optional(d, keys.ssm_out));
-      s->y = Ptr<float>(Item(d, keys.y));
+    const Gathered<gufo_cuda_linear_seq> seqs(a[2], [](Entries& d, gufo_cuda_linear_seq* s) {
+      s->in = Ptr<const float>(d.Item(keys.in));
+      s->conv_in = Ptr<const float>(d.Item(keys.conv_in));
+      s->conv_out = Ptr<float>(d.Item(keys.conv_out));
+      s->ssm = Ptr<float>(d.Item(keys.ssm));
+      s->ssm_out = Ptr<float>(d.Optional(keys.ssm_out));
+      s->y = Ptr<float>(d.Item(keys.y));
     });
-    const int count = static_cast<int>(seqs.size());
+    const int count = seqs.count();
     return Unlocked([&] { return api.deltanet_linear(ctx, layer, seqs.data(), count); });
   });
 }
@@ -306,22 +344,22 @@ PyObject* DeltaNetStep(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const long long layer = Int(a[1]), alpha = Int(a[2]), beta = Int(a[3]);
     const float* norm = Ptr<const float>(a[4]);
     const float eps = Float(a[5]);
-    const auto seqs = Gather<gufo_cuda_deltanet_step_seq>(a[6], [](PyObject* d, gufo_cuda_deltanet_step_seq* s) {
-      PyObject *in = Item(d, keys.in), *h = Item(d, keys.h), *y = Item(d, keys.y);
-      s->n_tokens = SmallInt(Item(d, keys.n_tokens));
+    const Gathered<gufo_cuda_deltanet_step_seq> seqs(a[6], [](Entries& d, gufo_cuda_deltanet_step_seq* s) {
+      PyObject *in = d.Item(keys.in), *h = d.Item(keys.h), *y = d.Item(keys.y);
+      s->n_tokens = SmallInt(d.Item(keys.n_tokens));
       s->in = Ptr<const float>(in);
       s->in_stride = RowStride(in);
       s->h = Ptr<const float>(h);
       s->h_stride = RowStride(h);
-      s->conv_in = Ptr<const float>(Item(d, keys.conv_in));
-      s->conv_out = Ptr<float>(Item(d, keys.conv_out));
-      s->conv_saved = Ptr<float>(Optional(d, keys.conv_saved));
-      s->ssm = Ptr<float>(Item(d, keys.ssm));
-      s->ssm_spec = Ptr<float>(Optional(d, keys.ssm_spec));
+      s->conv_in = Ptr<const float>(d.Item(keys.conv_in));
+      s->conv_out = Ptr<float>(d.Item(keys.conv_out));
+      s->conv_saved = Ptr<float>(d.Optional(keys.conv_saved));
+      s->ssm = Ptr<float>(d.Item(keys.ssm));
+      s->ssm_spec = Ptr<float>(d.Optional(keys.ssm_spec));
       s->y = Ptr<float>(y);
       s->y_stride = RowStride(y);
     });
-    const int count = static_cast<int>(seqs.size());
+    const int count = seqs.count();
     return Unlocked([&] { return api.deltanet_step(ctx, layer, alpha, beta, norm, eps, seqs.data(), count); });
   });
 }
@@ -528,7 +566,8 @@ PyMODINIT_FUNC PyInit__native() {
                      {&keys.v, "v"}, {&keys.decay, "decay"}, {&keys.beta, "beta"}, {&keys.y, "y"}, {&keys.in, "in"},
                      {&keys.h, "h"}, {&keys.conv_in, "conv_in"}, {&keys.conv_out, "conv_out"},
                      {&keys.conv_saved, "conv_saved"}, {&keys.ssm, "ssm"}, {&keys.ssm_out, "ssm_out"},
-                     {&keys.ssm_spec, "ssm_spec"}, {&keys.n_tokens, "n_tokens"}};
+                     {&keys.ssm_spec, "ssm_spec"}, {&keys.n_tokens, "n_tokens"},
+                     {&keys.get, "get"}};
   for (const auto& n : names) {
     if ((*n.key = PyUnicode_InternFromString(n.name)) == nullptr) {
       return nullptr;
@@ -542,5 +581,11 @@ PyMODINIT_FUNC PyInit__native() {
   if (PyType_Ready(&host_buffer_type) != 0) {
     return nullptr;
   }
-  return PyModule_Create(&module);
+  PyObject* m = PyModule_Create(&module);
+  // torch's C++ classes differ from release to release: load_native compares.
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", GUFO_TORCH_VERSION) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
 }

@@ -3,7 +3,10 @@ refuses to work without a device (no CPU fallback)."""
 import ctypes as C
 import os
 import re
+import subprocess
+import sys
 
+import numpy as np
 import pytest
 
 from gufo_npu_b200 import _capi, build
@@ -51,3 +54,29 @@ def test_no_cpu_fallback(lib):
     from gufo_npu_b200.backend import Context
     with pytest.raises(_capi.GufoCudaError):
         Context(0)
+
+
+def test_library_loads_without_torch(lib):
+    code = "import sys; sys.modules['torch'] = None; from gufo_npu_b200 import _capi; assert _capi.load().gufo_cuda_launch_count(None) == 0"
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT)
+
+
+def test_extension_takes_mappings_and_arrays(lib):
+    """Sequences described by any mapping, parts as rows of numbers: they reach the library, which has
+    no context to run them on (status 1)."""
+    import collections
+    native = _capi.load_native()
+    entries = {k: 16 for k in ("state", "q", "k", "v", "decay", "beta", "y")}
+
+    class Computed(dict):
+        def __missing__(self, key):
+            return np.zeros(4, dtype=np.float32)
+    for seq in (entries, collections.UserDict(entries), collections.ChainMap({}, entries), Computed()):
+        assert native.delta_rule(0, [seq], 1, 1, 32) == 1
+    with pytest.raises(KeyError):
+        native.delta_rule(0, [collections.UserDict()], 1, 1, 32)
+    for parts in ([(1, 0, 5)], np.array([[1, 0, 5]], dtype=np.int32), np.array([[1, 0, 5, 9]])[:, :3],
+                  (_capi.Rows * 1)(_capi.Rows(1, 0, 5))):
+        assert native.matmul_device(0, parts, 1, 16, 1, 16) == 1
+        with pytest.raises(ValueError):
+            native.matmul_device(0, parts, 2, 16, 1, 16)
