@@ -27,8 +27,9 @@ constexpr int kDeltaThreads = kMaxHeadDim;            // one thread per column
 constexpr int kMaxSeqs = 64;                          // descriptors per launch
 constexpr int kMaxRunTokens = 4;                      // tokens of a sequence per launch
 
+template <int SEQS>
 struct DeltaRuleArgs {
-  gufo_cuda_delta_seq seq[kMaxSeqs];
+  gufo_cuda_delta_seq seq[SEQS];
   int key_heads;
   int value_heads;
   int head_dim;
@@ -219,53 +220,104 @@ __device__ __forceinline__ void TileUpdate(NarrowTile<COLS>& tile, const float (
 }
 
 constexpr int kStepCols = 16;   // columns per warp in the decode step's kernel
-constexpr int kRuleCols = 16;   // columns per warp in the stand-alone delta rule (8: 4.9 us for config 3, 16: 4.1, 32: 4.6)
+constexpr int kRuleCols = 16;   // columns per warp in the stand-alone delta rule
 
 // Gates given: one warp per thread block, grid = (dk / 16, value_heads,
 // sequences). The tiles of a head need nothing from one another here, and
 // many small blocks per SM let one tile's stores overlap another's loads
 // (16-column tiles: 1024 warps for eight sequences of sixteen heads).
-template <int DK>
-__global__ void __launch_bounds__(32)
-DeltaRuleKernel(const __grid_constant__ DeltaRuleArgs args) {
-  __shared__ __align__(16) Pair q2[kMaxHeadDim], k2[kMaxHeadDim];
-  __shared__ __align__(16) float v[kMaxHeadDim], y[kMaxHeadDim];
+//
+// What bounds it: HBM from some hundred heads on, below that the chain from a launch's
+// arguments over the loads to the last store. So the arguments hold as many sequences
+// as the launch needs (64 always: their kilobytes come through the constant cache ahead
+// of a block's first load), the update follows the retrieval in a second pass over the
+// registers instead of taking both sums in one (TileSums: eight values through the
+// shuffles ahead of the first store, and k . q before them), and the head dim is a
+// run-time value (built in, one sequence takes 1.2 us longer: the compiler then orders
+// the loads otherwise). Sixteen warps an SM may have 128 registers each; with 96, for
+// twenty warps, the loads spill. Us, states from HBM, heads x dk: 16 x 128 4.1 -> 3.2,
+// 128 x 128 6.8 -> 5.7, 256 x 128 8.1 -> 6.9, 1536 x 128 36.8 -> 34.5.
+template <int SEQS>
+__global__ void __launch_bounds__(32, 16)
+DeltaRuleKernel(const __grid_constant__ DeltaRuleArgs<SEQS> args) {
+  using T = NarrowTile<kRuleCols>;
+  __shared__ float q[kMaxHeadDim], k[kMaxHeadDim];
   const gufo_cuda_delta_seq& seq = args.seq[blockIdx.z];
   const int head = blockIdx.y;
-  const int tile = blockIdx.x;
-  const int dk = DK > 0 ? DK : args.head_dim;
+  const int dk = args.head_dim;
   const int kh = head % args.key_heads;
   const int lane = threadIdx.x;
-  const size_t state_at = static_cast<size_t>(head) * dk * dk;
-  NarrowTile<kRuleCols> state;
+  const int col = blockIdx.x * kRuleCols + 4 * (lane % T::kGroups);
+  const int ig = lane / T::kGroups;
+  const int rows = dk / T::kRowGroups;
+  const size_t at = static_cast<size_t>(head) * dk * dk + static_cast<size_t>(ig) * dk + col;
+  float4 s[T::kRowsPerLane];
+  auto load = [&]() {
+    const float* src = seq.state + at;
+#pragma unroll
+    for (int r = 0; r < T::kRowsPerLane; ++r) {
+      if (r < rows) {
+        s[r] = *reinterpret_cast<const float4*>(src + r * T::kRowGroups * dk);
+      }
+    }
+  };
   GridLaunchDependents();
   if (args.early_state) {
-    LoadNarrowTile<DK>(state, seq.state + state_at, dk, tile);
+    load();
   }
   GridDependencyWait();
   if (!args.early_state) {
-    LoadNarrowTile<DK>(state, seq.state + state_at, dk, tile);
+    load();
   }
-  float kq = 0.f;
   for (int i = lane; i < dk; i += 32) {
-    const float q = seq.q[kh * dk + i], k = seq.k[kh * dk + i];
-    q2[i] = MakePair(q, q);
-    k2[i] = MakePair(k, k);
-    kq = fmaf(k, q, kq);
+    q[i] = seq.q[kh * dk + i];
+    k[i] = seq.k[kh * dk + i];
   }
-  if (lane < kRuleCols) {
-    v[tile * kRuleCols + lane] = seq.v[head * dk + tile * kRuleCols + lane];
-  }
+  const float* v = seq.v + head * dk + col;
+  const float v0 = v[0], v1 = v[1], v2 = v[2], v3 = v[3];
   const float decay = seq.decay[head], beta = seq.beta[head];
-  const DeltaCoef coef{decay, beta, 1.0f, 1.0f, WarpSum(kq)};
   __syncwarp();
-  float* dst = (seq.state_out != nullptr ? seq.state_out : seq.state) + state_at;
-  float sums[8];
-  TileSums<DK>(state, dk, q2, k2, sums);
-  TileUpdate<DK>(state, sums, dst, dk, tile, k2, v, coef, y);
-  __syncwarp();
-  if (lane < kRuleCols) {
-    seq.y[head * dk + tile * kRuleCols + lane] = y[tile * kRuleCols + lane];
+  auto over_rows = [](float4& x) {
+#pragma unroll
+    for (int o = T::kGroups; o <= 16; o <<= 1) {
+      x.x += __shfl_xor_sync(0xFFFFFFFFu, x.x, o);
+      x.y += __shfl_xor_sync(0xFFFFFFFFu, x.y, o);
+      x.z += __shfl_xor_sync(0xFFFFFFFFu, x.z, o);
+      x.w += __shfl_xor_sync(0xFFFFFFFFu, x.w, o);
+    }
+  };
+  float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < T::kRowsPerLane; ++r) {
+    if (r < rows) {
+      const float ki = k[r * T::kRowGroups + ig] * decay;
+      u.x = fmaf(s[r].x, ki, u.x);
+      u.y = fmaf(s[r].y, ki, u.y);
+      u.z = fmaf(s[r].z, ki, u.z);
+      u.w = fmaf(s[r].w, ki, u.w);
+    }
+  }
+  over_rows(u);
+  const float d0 = beta * (v0 - u.x), d1 = beta * (v1 - u.y), d2 = beta * (v2 - u.z), d3 = beta * (v3 - u.w);
+  float* dst = (seq.state_out != nullptr ? seq.state_out : seq.state) + at;
+  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < T::kRowsPerLane; ++r) {
+    if (r < rows) {
+      const float ki = k[r * T::kRowGroups + ig], qi = q[r * T::kRowGroups + ig];
+      const float4 n = make_float4(fmaf(s[r].x, decay, ki * d0), fmaf(s[r].y, decay, ki * d1),
+                                   fmaf(s[r].z, decay, ki * d2), fmaf(s[r].w, decay, ki * d3));
+      *reinterpret_cast<float4*>(dst + r * T::kRowGroups * dk) = n;
+      y.x = fmaf(n.x, qi, y.x);
+      y.y = fmaf(n.y, qi, y.y);
+      y.z = fmaf(n.z, qi, y.z);
+      y.w = fmaf(n.w, qi, y.w);
+    }
+  }
+  over_rows(y);
+  if (ig == 0) {
+    float* out = seq.y + head * dk + col;
+    out[0] = y.x, out[1] = y.y, out[2] = y.z, out[3] = y.w;
   }
 }
 
@@ -692,6 +744,20 @@ DeltaNetGatesKernel(const __grid_constant__ GatesArgs a) {
   }
 }
 
+template <int SEQS>
+cudaError_t LaunchRule(gufo_cuda_ctx* ctx, const gufo_cuda_delta_seq* seqs, int n, int key_heads, int value_heads,
+                       int head_dim) {
+  DeltaRuleArgs<SEQS> args;
+  for (int s = 0; s < n; ++s) {
+    args.seq[s] = seqs[s];
+  }
+  args.key_heads = key_heads;
+  args.value_heads = value_heads;
+  args.head_dim = head_dim;
+  args.early_state = ctx->early_state ? 1 : 0;
+  return LaunchOverlapped(DeltaRuleKernel<SEQS>, dim3(head_dim / kRuleCols, value_heads, n), dim3(32), 0, ctx->stream, 1, args);
+}
+
 int CheckHeads(int key_heads, int value_heads, int head_dim) {
   if (key_heads <= 0 || value_heads <= 0 || value_heads % key_heads != 0) {
     return Fail(GUFO_CUDA_SHAPE, "deltanet: value heads must tile the key heads");
@@ -735,17 +801,9 @@ int gufo_cuda_delta_rule_device(gufo_cuda_ctx* ctx,
   GUFO_CUDA_TRY(cudaSetDevice(ctx->device));
   for (int s0 = 0; s0 < nseq; s0 += gufo::kMaxSeqs) {
     const int n = nseq - s0 < gufo::kMaxSeqs ? nseq - s0 : gufo::kMaxSeqs;
-    gufo::DeltaRuleArgs args{};
-    for (int s = 0; s < n; ++s) {
-      args.seq[s] = seqs[s0 + s];
-    }
-    args.key_heads = key_heads;
-    args.value_heads = value_heads;
-    args.head_dim = head_dim;
-    args.early_state = ctx->early_state ? 1 : 0;
-    const dim3 grid(head_dim / gufo::kRuleCols, value_heads, n);
-    GUFO_CUDA_TRY(gufo::LaunchOverlapped(head_dim == 128 ? gufo::DeltaRuleKernel<128> : gufo::DeltaRuleKernel<0>, grid, dim3(32),
-                                         0, ctx->stream, 1, args));
+    GUFO_CUDA_TRY(n <= 2    ? gufo::LaunchRule<2>(ctx, seqs + s0, n, key_heads, value_heads, head_dim)
+                  : n <= 16 ? gufo::LaunchRule<16>(ctx, seqs + s0, n, key_heads, value_heads, head_dim)
+                            : gufo::LaunchRule<gufo::kMaxSeqs>(ctx, seqs + s0, n, key_heads, value_heads, head_dim));
     ctx->launches.fetch_add(1);
   }
   return GUFO_CUDA_OK;
