@@ -24,6 +24,7 @@ int Fail(int status, const std::string& text) {
 }
 
 int CudaFail(cudaError_t e, const char* what) {
+  cudaGetLastError();   // reported here: not the next launch's
   g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
   return e == cudaErrorMemoryAllocation ? GUFO_CUDA_OUT_OF_MEMORY
                                         : GUFO_CUDA_RUNTIME;

