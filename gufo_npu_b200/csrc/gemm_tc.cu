@@ -99,13 +99,12 @@ template <int TYPE>
 struct Quant;
 template <>
 struct Quant<GUFO_CUDA_Q4_K> {
-  static constexpr int kMaps = 1;
   static constexpr int kRawBytes = kTileRows * kQ4KBytes;
   static constexpr int kRawStride = kRawBytes;
 };
 template <>
 struct Quant<GUFO_CUDA_Q6_K> {
-  static constexpr int kMaps = 3;   // boxes 128, 64 and 16 bytes wide
+  // Boxes 128, 64 and 16 bytes wide.
   static constexpr int kQl = 0, kQh = kTileRows * 128, kSc = kQh + kTileRows * 64, kD = kSc + kTileRows * 16;
   static constexpr int kRawBytes = kD + kTileRows * 16;
   static constexpr int kRawStride = kRawBytes;   // 28 KiB: a multiple of 1024
@@ -138,11 +137,7 @@ struct TcGemmArgs {
   int* error;              // device int: 0, or the code of the first wait that ran out
 };
 
-__device__ __forceinline__ void MbarArrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-// The same test, suspended by the hardware for up to kSuspendNs first: most warps
+// MbarTryWait's test, suspended by the hardware for up to kSuspendNs first: most warps
 // of the kernel wait most of the time, and polling took as many issue slots as the
 // dequantization.
 constexpr uint32_t kSuspendNs = 20000;

@@ -65,34 +65,33 @@ struct Slab<GUFO_CUDA_Q6_K> {
 
 constexpr int kMaxStages = 3;
 constexpr int kExchange = 2;
+constexpr int kTileFloats = 16;   // a warp's row sums in an exchange buffer
+constexpr int kPerSm = 3;         // resident blocks the registers are for
 
 // ONE: every block of the launch multiplies a single slab, so the ring is one
 // slot (a third or half of the shared memory: more blocks fit an SM, which lets a
 // cluster of three split a three-slab row where two-slot blocks allowed two).
-template <int TYPE, int TOKENS, bool ONE = false>
+template <int TYPE, bool ONE = false>
 size_t SharedBytes(int cols) {
-  const ImageLayout l = MakeImageLayout(TOKENS, cols, Slab<TYPE>::kGroup);
+  const ImageLayout l = MakeImageLayout(1, cols, Slab<TYPE>::kGroup);
   return static_cast<size_t>(l.bytes) + (Slab<TYPE>::kZeros ? l.plane_stride : 0) +
-         static_cast<size_t>(kExchange) * kFastWarps * 16 * TOKENS * 4 +
+         static_cast<size_t>(kExchange) * kFastWarps * kTileFloats * 4 +
          static_cast<size_t>(ONE ? 1 : Slab<TYPE>::kStages) * Slab<TYPE>::kBytes;
 }
 
-// GROUPED: the routed experts' products, one token a group (FastGemvArgs).
+// GROUPED: the routed experts' products, a group's own input each (FastGemvArgs).
 // PAIRS: a block may take several (gate tile, up tile) pairs; else one, tiles blockIdx.x
 // and blockIdx.x + gridDim.x (the decode step's kernel stays 1 % faster without).
-template <int TYPE, int TOKENS, int PER_SM, bool ONE = false, bool GROUPED = false, bool PAIRS = GROUPED>
-__global__ void __launch_bounds__(kFastThreads, PER_SM)
+template <int TYPE, bool ONE = false, bool GROUPED = false, bool PAIRS = GROUPED>
+__global__ void __launch_bounds__(kFastThreads, kPerSm)
 GemvMma(const __grid_constant__ FastGemvArgs a) {
   using S = Slab<TYPE>;
   constexpr bool kQ4 = TYPE == GUFO_CUDA_Q4_K;
   constexpr int kStages = ONE ? 1 : S::kStages;
-  constexpr int kNCols = TOKENS * kLimbs;
-  constexpr int kNB = (kNCols + 7) / 8;
-  constexpr int kTileFloats = 16 * TOKENS;   // per warp in an exchange buffer: row sums per token
   extern __shared__ __align__(16) uint8_t smem[];
-  // Where the blocks of a cluster leave their sums for block 0: [2][8][16][TOKENS].
-  __shared__ float peers[2 * 8 * 16 * TOKENS];
-  __shared__ float squares[kFastWarps * TOKENS];         // a fused norm's (FillImage)
+  // Where the blocks of a cluster leave their sums for block 0: [2][8][16].
+  __shared__ float peers[2 * 8 * kTileFloats];
+  __shared__ float squares[kFastWarps];                  // a fused norm's (FillImage)
   __shared__ float* mirror;                              // the second copy of y, if any
   __shared__ __align__(8) uint64_t landed[kMaxStages];   // a slab's bytes have arrived
   // The barriers need no kernel argument: set up first, while the arguments' first
@@ -105,13 +104,13 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  const ImageLayout l = MakeImageLayout(TOKENS, a.cols, S::kGroup);
+  const ImageLayout l = MakeImageLayout(1, a.cols, S::kGroup);
   const int blocks = a.cols / kSuperBlock;
   const int slabs_per_tile = (blocks + 7) / 8;
   const float* col_scale = reinterpret_cast<const float*>(smem + l.scale_at);
   const float* sums = reinterpret_cast<const float*>(smem + l.sums_at);
   // After the image: (Q6_K) a plane of zeros, the exchange buffers
-  // [kExchange][warps][16 rows][TOKENS], then the slab ring.
+  // [kExchange][warps][16 rows], then the slab ring.
   uint8_t* zeros = smem + l.bytes;
   float* exchange = reinterpret_cast<float*>(zeros + (S::kZeros ? l.plane_stride : 0));
   uint8_t* ring = reinterpret_cast<uint8_t*>(exchange + kExchange * kFastWarps * kTileFloats);
@@ -121,14 +120,11 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   const int g = lane >> 2;
   const int t = lane & 3;
   // Lane planes of the two unit kinds (q4k_unit.cuh, q6k_unit.cuh): column g of
-  // the first MMA column group; lanes past the last token's planes wrap onto
-  // live ones, whose sums meet a zero column factor.
-  const uint8_t* lane_plane = smem + (g % kNCols) * l.plane_stride + 8 * t;
-  const uint8_t* none = zeros + 8 * t;
-  const bool one_live = (g & 3) < kNCols && ((g < 4) == (t < 2));
-  const uint8_t* lane_first = TOKENS == 1 ? (one_live ? smem + (g & 3) * l.plane_stride + 8 * t : none)
-                                          : (t < 2 ? lane_plane : none);
-  const uint8_t* lane_second = t < 2 ? none : lane_plane;
+  // the MMA's; lanes past the planes wrap onto live ones (Q4_K: their sums meet a
+  // zero column factor) or read zeros (Q6_K).
+  const uint8_t* lane_plane = smem + (g % kLimbs) * l.plane_stride + 8 * t;
+  const bool one_live = (g & 3) < kLimbs && ((g < 4) == (t < 2));
+  const uint8_t* lane_first = (one_live ? smem + (g & 3) * l.plane_stride : zeros) + 8 * t;
   const int row_tiles = TotalTiles(a);
   // With ksplit > 1 a cluster of ksplit blocks shares each tile.
   // (No division here: a block's first slabs cannot be requested before these
@@ -239,14 +235,9 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
       ++req_n;
     }
   };
-  // One token: a warp reads its fragments ahead of the block's barrier, so the
-  // slot is free for the slab kStages on as soon as the barrier has passed.
-  // More tokens hold too many registers for that to pay (the two-token step ran
-  // 7 % slower with it): the barrier comes first and frees the slot of the slab
-  // before, for the slab kStages - 1 on.
-  constexpr bool kEarly = TOKENS == 1;
-  constexpr int kAhead = kEarly || ONE ? kStages : kStages - 1;
-  const int requested = min(kAhead, my_slabs);
+  // A warp reads its fragments ahead of the block's barrier, so the slot is free for
+  // the slab kStages on as soon as the barrier has passed.
+  const int requested = min(kStages, my_slabs);
   for (int q = 0; q < requested; ++q) {
     advance();
   }
@@ -261,10 +252,10 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     }
   }
   if (a.prologue != kPrologueImage) {
-    ZeroIdleColumns<TOKENS>(l, blocks, smem);
+    ZeroIdleColumns<1>(l, blocks, smem);
   }
   float norm_ahead[8];
-  LoadNormAhead<TOKENS>(a, norm_ahead);
+  LoadNormAhead<1>(a, norm_ahead);
   const float inv_n = 1.0f / static_cast<float>(a.cols);
   if constexpr (!GROUPED) {
     GridLaunchDependents();
@@ -285,9 +276,9 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
   } else {
-    FillImage<TOKENS>(a, l, smem, S::kExtra,
-                      a.x + static_cast<size_t>(group / (a.x_group_div > 1 ? a.x_group_div : 1)) * a.x_group_stride,
-                      rank, ks, norm_ahead, squares, inv_n);
+    FillImage<1>(a, l, smem, S::kExtra,
+                 a.x + static_cast<size_t>(group / (a.x_group_div > 1 ? a.x_group_div : 1)) * a.x_group_stride,
+                 rank, ks, norm_ahead, squares, inv_n);
   }
   if (GROUPED && a.early_input) {
     if (!choose()) {
@@ -295,24 +286,14 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     }
     issue_first(requested);
   }
-  // The norm's 1 / rms of the token whose row sums this thread stores.
-  const float row_scale = threadIdx.x < kTileFloats ? RowScale<TOKENS>(a, squares, threadIdx.x % TOKENS, inv_n) : 1.f;
+  // The norm's 1 / rms, for the threads that store row sums.
+  const float row_scale = threadIdx.x < kTileFloats ? RowScale<1>(a, squares, 0, inv_n) : 1.f;
 
-  float out[kNB][4];
-  float off[TOKENS];
-  auto clear = [&]() {
-#pragma unroll
-    for (int nb = 0; nb < kNB; ++nb) {
-      out[nb][0] = out[nb][1] = out[nb][2] = out[nb][3] = 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < TOKENS; ++k) {
-      off[k] = 0.f;
-    }
-  };
+  float out[4], off;
+  auto clear = [&]() { out[0] = out[1] = out[2] = out[3] = off = 0.f; };
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   // The output rows of tile n from the eight warps' row sums in exchange buffer
-  // x: thread o of the callers takes (row o / TOKENS, token o % TOKENS).
+  // x: thread o of the callers takes row o.
   auto total_of = [&](int x, int o) {
     const float* from = exchange + x * kFastWarps * kTileFloats + o;
     float total = 0.f;
@@ -325,11 +306,9 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
   auto store = [&](int n, int o, float total) {
     int part, local;
     locate(n, &part, &local);
-    const int k = o % TOKENS;
-    const int row = local * 16 + o / TOKENS;
+    const int row = local * 16 + o;
     if (row < a.parts[part].rows) {
-      const size_t at = static_cast<size_t>(group) * a.y_group_stride + static_cast<size_t>(k) * a.y_stride +
-                        (a.epilogue == kEpilogueSwiGlu ? 0 : a.parts[part].y_offset) + row;
+      const size_t at = static_cast<size_t>(group) * a.y_group_stride + (a.epilogue == kEpilogueSwiGlu ? 0 : a.parts[part].y_offset) + row;
       if (a.peer_out.world > 0) {
         // Row-split ranks: this rank's rows go straight into every rank's copy
         // of the full vector (plain stores over NVLink for the peers).
@@ -404,9 +383,9 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
     // before are in the exchange buffer. Warp q % 8 requests the next slab.
     auto meet = [&]() {
       __syncthreads();
-      if (q + kAhead < my_slabs) {
+      if (q + kStages < my_slabs) {
         if (warp == (q & 7)) {
-          issue(q + kAhead, req_n, req_s);
+          issue(q + kStages, req_n, req_s);
         }
         advance();
       }
@@ -414,9 +393,6 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
         gather(n - 1);
       }
     };
-    if constexpr (!kEarly) {
-      meet();
-    }
     if (mine) {
       if constexpr (kQ4) {
         q4k::LoadUnit(unit, data, warp, g, t);
@@ -424,85 +400,40 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
         q6k::LoadUnit(unit, data, warp, nblk, g, t);
       }
     }
-    if constexpr (kEarly) {
-      meet();
-    }
+    meet();
     if (mine) {
+      typename std::conditional<kQ4, q4k::Accum<1>, q6k::Accum<1>>::type acc;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc.out[0][j] = out[j];
+      }
       if constexpr (kQ4) {
-        q4k::Accum<TOKENS> acc;
-#pragma unroll
-        for (int nb = 0; nb < kNB; ++nb) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc.out[nb][j] = out[nb][j];
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < TOKENS; ++k) {
-          acc.off[k] = off[k];
-        }
-        q4k::MultiplyUnit<TOKENS>(unit, b, g, t, lane_plane, l, col_scale, sums, acc);
-#pragma unroll
-        for (int nb = 0; nb < kNB; ++nb) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            out[nb][j] = acc.out[nb][j];
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < TOKENS; ++k) {
-          off[k] = acc.off[k];
-        }
+        acc.off[0] = off;
+        q4k::MultiplyUnit<1>(unit, b, g, t, lane_plane, l, col_scale, sums, acc);
+        off = acc.off[0];
       } else {
-        q6k::Accum<TOKENS> acc;
+        q6k::MultiplyUnit<1>(unit, b, g, t, lane_first, lane_first, l, col_scale, sums, acc);
+      }
 #pragma unroll
-        for (int nb = 0; nb < kNB; ++nb) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc.out[nb][j] = out[nb][j];
-          }
-        }
-        q6k::MultiplyUnit<TOKENS>(unit, b, g, t, lane_first, lane_second, l, col_scale, sums, acc);
-#pragma unroll
-        for (int nb = 0; nb < kNB; ++nb) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            out[nb][j] = acc.out[nb][j];
-          }
-        }
+      for (int j = 0; j < 4; ++j) {
+        out[j] = acc.out[0][j];
       }
     }
     if (s == slabs_mine - 1) {
-      // This warp's row sums of the tile: the columns of token k are 3k .. 3k + 2
-      // (one token: every column; dead ones carry a zero factor), the Q4_K
-      // offsets sit in lanes t < 2 for row g and t >= 2 for row g + 8; summed
-      // over the quad.
-      const int x = n % kExchange;
-      float* tile = exchange + (x * kFastWarps + warp) * kTileFloats;
+      // This warp's row sums of the tile: every column (dead ones carry a zero
+      // factor); the Q4_K offsets sit in lanes t < 2 for row g and t >= 2 for row
+      // g + 8; summed over the quad.
+      float* tile = exchange + ((n % kExchange) * kFastWarps + warp) * kTileFloats;
+      float lo = out[0] + out[1] - (t < 2 ? off : 0.f);
+      float hi = out[2] + out[3] - (t < 2 ? 0.f : off);
 #pragma unroll
-      for (int k = 0; k < TOKENS; ++k) {
-        float lo = 0.f, hi = 0.f;
-#pragma unroll
-        for (int nb = 0; nb < kNB; ++nb) {
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const int col = nb * 8 + 2 * t + j;
-            const bool of_k = TOKENS == 1 || (col < kNCols && col / kLimbs == k);
-            lo += of_k ? out[nb][j] : 0.f;
-            hi += of_k ? out[nb][2 + j] : 0.f;
-          }
-        }
-        lo -= t < 2 ? off[k] : 0.f;
-        hi -= t < 2 ? 0.f : off[k];
-#pragma unroll
-        for (int o = 1; o <= 2; o <<= 1) {
-          lo += __shfl_xor_sync(0xFFFFFFFFu, lo, o);
-          hi += __shfl_xor_sync(0xFFFFFFFFu, hi, o);
-        }
-        if (t == 0) {
-          tile[g * TOKENS + k] = lo;
-          tile[(g + 8) * TOKENS + k] = hi;
-        }
+      for (int o = 1; o <= 2; o <<= 1) {
+        lo += __shfl_xor_sync(0xFFFFFFFFu, lo, o);
+        hi += __shfl_xor_sync(0xFFFFFFFFu, hi, o);
+      }
+      if (t == 0) {
+        tile[g] = lo;
+        tile[g + 8] = hi;
       }
       clear();
       s = 0;
@@ -521,11 +452,11 @@ GemvMma(const __grid_constant__ FastGemvArgs a) {
 }
 
 // Lets the kernel use all the shared memory a block may have (once per device).
-template <int TYPE, int TOKENS, int PER_SM, bool ONE = false, bool GROUPED = false, bool PAIRS = GROUPED>
+template <int TYPE, bool ONE = false, bool GROUPED = false, bool PAIRS = GROUPED>
 int Configure(const gufo_cuda_ctx* ctx) {
   static bool configured[16] = {};
   if (!configured[ctx->device & 15]) {
-    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemvMma<TYPE, TOKENS, PER_SM, ONE, GROUPED, PAIRS>,
+    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemvMma<TYPE, ONE, GROUPED, PAIRS>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kFastMaxShared));
     configured[ctx->device & 15] = true;
   }
@@ -556,14 +487,14 @@ void PlanFastGrid(Kernel kernel, int device, int threads, size_t smem, int row_t
 // LaunchVariant leaves the launch to gemv_units.cu.
 constexpr int kNotTaken = -1;
 
-template <int TYPE, int TOKENS, int PER_SM>
+template <int TYPE>
 int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
-  const size_t smem = SharedBytes<TYPE, TOKENS>(args.cols);
+  const size_t smem = SharedBytes<TYPE>(args.cols);
   if (smem > static_cast<size_t>(kFastMaxShared)) {
     return kNotTaken;
   }
   {
-    const int rc = Configure<TYPE, TOKENS, PER_SM>(ctx);
+    const int rc = Configure<TYPE>(ctx);
     if (rc != GUFO_CUDA_OK) {
       return rc;
     }
@@ -580,7 +511,7 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
     if (TYPE != GUFO_CUDA_Q4_K) {
       return Fail(GUFO_CUDA_UNSUPPORTED_TYPE, "fast gemv: grouped launches run Q4_K only");
     }
-    if (args.groups <= 0 || TOKENS != 1 || args.prologue == kPrologueImage || args.prologue == kPrologueResNorm) {
+    if (args.groups <= 0 || args.tokens != 1 || args.prologue == kPrologueImage || args.prologue == kPrologueResNorm) {
       return Fail(GUFO_CUDA_BAD_ARGUMENT, "fast gemv: a grouped launch takes one token and a fused input");
     }
     launch.ksplit = 1;
@@ -595,17 +526,17 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
     }
     launch.ksplit = 1;
     grid = row_tiles / 2;
-    if (grid > ResidentBlocks(GemvMma<TYPE, TOKENS, PER_SM>, ctx->device, kFastThreads, smem, 1)) {
+    if (grid > ResidentBlocks(GemvMma<TYPE>, ctx->device, kFastThreads, smem, 1)) {
       // More tile pairs than resident blocks: several a block (2 x 8192 x 2048: a step of
       // twelve layers 387 -> 349 us against the unit kernel).
       if (slabs > 1 && args.cols % (8 * kSuperBlock) != 0) {
         return kNotTaken;
       }
-      const int rc = Configure<TYPE, TOKENS, PER_SM, false, false, true>(ctx);
+      const int rc = Configure<TYPE, false, false, true>(ctx);
       if (rc != GUFO_CUDA_OK) {
         return rc;
       }
-      auto* many = GemvMma<TYPE, TOKENS, PER_SM, false, false, true>;
+      auto* many = GemvMma<TYPE, false, false, true>;
       const int items = grid;
       grid = std::max(1, std::min(items, ResidentBlocks(many, ctx->device, kFastThreads, smem, 1)));
       launch.tiles_each = items / grid;
@@ -616,7 +547,7 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
     }
   } else {
     // Few rows and several slabs per tile: split the tiles' slabs over a cluster.
-    PlanFastGrid(GemvMma<TYPE, TOKENS, PER_SM>, ctx->device, kFastThreads, smem, row_tiles, slabs, &launch.ksplit,
+    PlanFastGrid(GemvMma<TYPE>, ctx->device, kFastThreads, smem, row_tiles, slabs, &launch.ksplit,
                  &grid);
     if (launch.ksplit == 1 && slabs > 1 && args.cols % (8 * kSuperBlock) != 0) {
       return kNotTaken;
@@ -630,9 +561,9 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
       // (the same launches ran 0.4 us slower when products that gain no wider
       // split went to this form too).
       if (slabs >= 2 && slabs <= 4 && launch.ksplit < slabs) {
-        const size_t smem_one = SharedBytes<TYPE, TOKENS, true>(args.cols);
-        auto* one = GemvMma<TYPE, TOKENS, PER_SM, true>;
-        if (Configure<TYPE, TOKENS, PER_SM, true>(ctx) == GUFO_CUDA_OK &&
+        const size_t smem_one = SharedBytes<TYPE, true>(args.cols);
+        auto* one = GemvMma<TYPE, true>;
+        if (Configure<TYPE, true>(ctx) == GUFO_CUDA_OK &&
             row_tiles * slabs <= ResidentBlocks(one, ctx->device, kFastThreads, smem_one, slabs)) {
           launch.ksplit = slabs;
           launch.tiles_each = 1;
@@ -645,9 +576,9 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
       }
     }
   }
-  if constexpr (TYPE == GUFO_CUDA_Q4_K && TOKENS == 1) {
+  if constexpr (TYPE == GUFO_CUDA_Q4_K) {
     if (args.group_ids != nullptr) {
-      const int rc = Configure<TYPE, TOKENS, PER_SM, false, true>(ctx);
+      const int rc = Configure<TYPE, false, true>(ctx);
       if (rc != GUFO_CUDA_OK) {
         return rc;
       }
@@ -655,7 +586,7 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
       // of tiles (pairs): a block converts its group's input once for all of its tiles
       // and streams their weights through its ring (one block per pair: 1024 blocks
       // for 32 experts of 512 rows, each with a start and a conversion of its own).
-      auto* kernel = GemvMma<TYPE, TOKENS, PER_SM, false, true>;
+      auto* kernel = GemvMma<TYPE, false, true>;
       const int resident = std::max(1, ResidentBlocks(kernel, ctx->device, kFastThreads, smem, 1));
       const int items = args.epilogue == kEpilogueSwiGlu ? row_tiles / 2 : row_tiles;
       const int64_t all = static_cast<int64_t>(items) * args.groups;
@@ -674,7 +605,7 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
     launch.tiles_each = row_tiles / grid;
     launch.tiles_more = row_tiles % grid;
   }
-  GUFO_CUDA_TRY(LaunchOverlapped(GemvMma<TYPE, TOKENS, PER_SM>, dim3(grid), dim3(kFastThreads), smem, ctx->stream,
+  GUFO_CUDA_TRY(LaunchOverlapped(GemvMma<TYPE>, dim3(grid), dim3(kFastThreads), smem, ctx->stream,
                                  launch.ksplit, launch));
   ctx->launches.fetch_add(1);
   return GUFO_CUDA_OK;
@@ -685,7 +616,7 @@ int LaunchVariant(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
 // the line stand there).
 template <int TYPE>
 int LaunchTokens(gufo_cuda_ctx* ctx, const FastGemvArgs& args) {
-  const int rc = args.tokens == 1 ? LaunchVariant<TYPE, 1, 3>(ctx, args) : kNotTaken;   // three blocks per SM
+  const int rc = args.tokens == 1 ? LaunchVariant<TYPE>(ctx, args) : kNotTaken;
   return rc == kNotTaken ? LaunchGemvUnits(ctx, TYPE, args) : rc;
 }
 

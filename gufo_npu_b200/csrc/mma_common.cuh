@@ -85,31 +85,6 @@ __device__ __forceinline__ void MmaS8S8(int (&d)[4], const uint32_t (&a)[4],
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
 }
 
-// Streaming loads of weight bytes: read once, keep them out of L1.
-__device__ __forceinline__ uint2 LoadStream8(const void* p) {
-  uint2 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];"
-               : "=r"(v.x), "=r"(v.y) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint4 LoadStream16(const void* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint32_t LoadStream4(const void* p) {
-  uint32_t v;
-  asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-
-// Asks the memory system to bring `bytes` (a multiple of 16, 16-byte aligned
-// start) into L2 without occupying registers or shared memory.
-__device__ __forceinline__ void PrefetchL2(const void* p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
 // ---- bulk copies completing on a shared-memory barrier ------------------------
 
 __device__ __forceinline__ uint32_t SharedAddress(const void* p) {
@@ -142,19 +117,6 @@ __device__ __forceinline__ void BulkCopy(uint32_t dst, const void* src, uint32_t
 // SM clock cycles a block waits for bytes it requested itself before giving the
 // slab up (about a second; a copy that has not landed by then never will).
 constexpr long long kLandLimit = 2000000000ll;
-
-// Copies `bytes` (a multiple of 16) from global to shared memory with 16-byte
-// asynchronous copies spread over the block, then waits and synchronizes.
-__device__ __forceinline__ void CopyImageToShared(uint8_t* dst, const uint8_t* src,
-                                                  int bytes) {
-  const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-  for (int at = threadIdx.x * 16; at < bytes; at += blockDim.x * 16) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(base + at), "l"(src + at)
-                 : "memory");
-  }
-  asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
-}
 
 // Converts one 256-value block of one token into the image at `image` (shared
 // or global memory): the calling warp's lane holds values 8 * lane .. + 7 of the
