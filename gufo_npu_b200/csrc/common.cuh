@@ -185,8 +185,8 @@ struct FastGemvArgs {
   // kEpilogueSwiGlu: the two parts are the gate and up rows of an FFN (equal row
   // counts, whole tiles); every block multiplies tile t of both and stores
   // act[t] = silu(gate[t]) * up[t] as rows/part outputs per token, y_stride
-  // apart (npu::Epilogue::kSwiGlu, src/npu/gemv.hpp:64-68). The launcher gives
-  // every tile pair a block of its own.
+  // apart (npu::Epilogue::kSwiGlu, src/npu/gemv.hpp:64-68). A block may take
+  // several tile pairs.
   int epilogue;
   PeerOut peer_out;       // world == 0: an ordinary product
   // Device word with the address of a second copy of y (mapped host memory; null

@@ -539,9 +539,11 @@ FetchKernel(const float* __restrict__ src, float* __restrict__ dst, int64_t n) {
 
 }  // namespace
 
-// Enqueues y = [W_0 x | W_1 x | ...]: Q4_K and Q6_K parts on the tensor-core
-// kernels (x staged once per block format, one launch per part), the rest
-// together on the general kernel; at most kMaxTokens tokens per pass.
+// Enqueues y = [W_0 x | W_1 x | ...]: many rows of Q4_K and Q6_K parts on the tcgen05
+// GEMM, F32 parts in one launch for all tokens; then, at most kMaxTokens tokens a
+// pass, Q4_K and Q6_K parts on the tensor-core GEMV kernels (up to kFastMaxParts of a
+// format a launch; x converted in them, or once ahead of them), Q5_K and Q8_0 rows of
+// whole blocks on GemvSplit and whatever is left together on the general kernel.
 int LaunchGemv(gufo_cuda_ctx* ctx, const GemvArgs& base, int tokens) {
   if (tokens >= 16 && (reinterpret_cast<uintptr_t>(base.x) & 15) == 0) {
     // Many token rows: the parts the tcgen05 GEMM runs read their weights once

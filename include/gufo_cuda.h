@@ -69,6 +69,8 @@ typedef int64_t gufo_cuda_deltanet_layer;
  * 100); fails with GUFO_CUDA_RUNTIME when no sm_100 device is usable, as the
  * reference's stub runtime throws (src/npu/gemv_stub.cpp:8-10). */
 int gufo_cuda_ctx_create(int device, void* stream, gufo_cuda_ctx** out);
+/* Also releases what the decoders on it hold; they then answer
+ * GUFO_CUDA_BAD_ARGUMENT until they are destroyed themselves. */
 int gufo_cuda_ctx_destroy(gufo_cuda_ctx* ctx);
 /* Replaces the stream later work is enqueued on (not owned). */
 int gufo_cuda_ctx_set_stream(gufo_cuda_ctx* ctx, void* stream);
@@ -165,11 +167,14 @@ typedef struct gufo_cuda_rows {
  * x is `tokens` rows of `cols` fp32 (all parts share cols), y is `tokens` rows
  * of sum(parts[p].rows) fp32. Each output is one row dot, so results do not
  * depend on how rows are stacked or how many tokens come together.
+ * Host buffers may be pinned or not; the GPU reads and writes them itself where
+ * all of a buffer is pinned and it starts on a float.
  * The _device forms only enqueue on the context's stream. Products of two or
  * more tokens stage their input in scratch memory the context owns; the first
  * product of a larger shape makes it grow (a cudaMalloc, no wait, the outgrown
  * block is kept until gufo_cuda_ctx_destroy so that CUDA graphs captured
- * earlier stay valid). A stream capture cannot allocate: while the stream is
+ * earlier stay valid; destroyed contexts' blocks, 256 MB of them at most, are
+ * kept for the next one while the process has a context on the device). A stream capture cannot allocate: while the stream is
  * being captured such a product returns GUFO_CUDA_BAD_ARGUMENT instead, so run
  * every shape once before capturing it. */
 int gufo_cuda_matmul(gufo_cuda_ctx* ctx, const gufo_cuda_rows* parts,
@@ -218,7 +223,7 @@ typedef struct gufo_cuda_fused_input {
                              /*   (two parts, equal whole 16-row tiles, one of Q4_K / Q6_K) and y    */
                              /*   receives silu(gate) * up, [tokens][rows / 2], from the product's   */
                              /*   own kernel (npu::Epilogue::kSwiGlu, src/npu/gemv.hpp:64-68). Where  */
-                             /*   the kernel cannot (more tile pairs than resident thread blocks,    */
+                             /*   the kernel cannot (rows whose image does not fit shared memory,    */
                              /*   other formats) the call returns GUFO_CUDA_UNSUPPORTED_TYPE and      */
                              /*   enqueues nothing: ask for plain rows and a SWIGLU input instead.   */
 } gufo_cuda_fused_input;
@@ -454,9 +459,10 @@ int gufo_cuda_expert_ffn_device(gufo_cuda_ctx* ctx,
  * x_stride; a slot with ids < 0 adds nothing. Equal to
  * gufo_cuda_expert_ffn_device (pairs = tokens * k, pairs_per_input = k) followed
  * by gufo_cuda_moe_combine_device up to the rounding of the row sums' order;
- * for Q4_K banks with expert_ffn 256 or 512 and k <= 8 it runs as two launches
- * (gate / up with the SwiGLU; the down rows of a token's experts with the
- * weighted sum) and touches neither ffn nor expert_out. Scratch as for
+ * for Q4_K banks whose k * expert_ffn values fit a thread block's shared memory
+ * (some 25000) it runs as two launches (gate / up with the SwiGLU; the down rows
+ * of a token's experts with the weighted sum) and touches neither ffn nor
+ * expert_out. Scratch as for
  * gufo_cuda_expert_ffn_device plus expert_out [tokens][k][hidden]. out may be
  * shared. */
 int gufo_cuda_moe_ffn_device(gufo_cuda_ctx* ctx,
