@@ -87,7 +87,9 @@ __device__ __forceinline__ void Ldmatrix2Trans(uint32_t& r0, uint32_t& r1, const
 // d = a b of sixteen values. The tensor core cuts off what does not fit its adder, so
 // sums over more than that are taken with fp32 adds, which round: accumulated by the
 // instruction, the outputs were up to three times as far from a float64 result as with
-// fp32 arithmetic throughout (16384 positions: 7.7e-7 against 2.6e-7; now 2.4e-7).
+// fp32 arithmetic throughout (16384 positions: 7.7e-7 against 2.6e-7; now 2.4e-7). It
+// costs 3 % of the time at 16000 positions and nothing up to 4096 (loops rolled to make
+// up for the longer code: no faster in a step, 3 % slower at 16000).
 __device__ __forceinline__ void MmaF16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
