@@ -24,34 +24,46 @@
 //     arithmetic, as d*sc*(q - 8) + (8*d*sc - dmin*m), or w = d*sc*(q - 32)
 //     (DequantQ6_K, :98-125). While the tensor core reads a slot, its group is at
 //     the arithmetic of the next block;
-//   - one thread brings the raw blocks of 128 rows with tiled TMA (Q4_K: one box
+//   - one warp brings the raw blocks of 128 rows with tiled TMA (Q4_K: one box
 //     of 144 bytes a row, whose row pitch is free of bank conflicts as it is;
 //     Q6_K: boxes of its four planes, the wide ones swizzled);
-//   - one thread brings the activation tiles, converted once per product into
+//   - one brings the activation tiles, converted once per product into
 //     fp16 tile images that already carry the swizzle (StageHalfKernel);
-//   - one thread issues tcgen05.mma and hands the slots back with
+//   - one issues tcgen05.mma and hands the slots back with
 //     tcgen05.commit;
 //   - four epilogue warps read the accumulators with tcgen05.ld (lane = weight
 //     row, column = token: a store instruction of a warp covers 32 adjacent
 //     rows of one token) while the others are on the next tile: tensor memory
 //     holds two accumulators beside the four weight slots.
 //
+// The loaders and the MMA warp walk their loops as whole warps, and the warp's number and
+// the tensor memory's address pass through a shuffle: what such a warp computes is then the
+// same in all lanes for the compiler too and stays in uniform registers, where the
+// asynchronous instructions take their operands from. With the whole role behind one
+// thread's predicate an MMA or commit took 47 cycles to issue (1040 of a step's 1880 at 32
+// tokens), now 13.
+//
 // Work split. A unit is a tile of 128 weight rows against one group of tokens; it
-// takes `blocks` steps of one 256-value block. The launch's units times steps are
+// takes `blocks` steps of one 256-value block. Few units are shared by clusters of two to
+// eight thread blocks each, whose accumulators meet in distributed shared memory
+// (ReduceCluster). Otherwise the launch's units times steps are
 // cut into equal contiguous ranges, one per thread block, so the SMs finish
 // together whatever the number of tiles (2 x 9728 rows are 152 tiles for 148 SMs)
 // where that saves more than the cuts cost (PlanTc). A tile that a cut goes through
 // is finished by whichever of its thread blocks comes last, which adds the others'
 // partial sums (left in scratch) to its own in block order, so the result does not
-// depend on who that is. Nobody waits for another block.
+// depend on who that is. Nobody waits for another block but for those of its cluster.
 //
-// What bounds it: the dequantization's instructions (about 4500 warp instructions
-// a step, issue slots 60-65 % busy) up to about 100 tokens, then the activation
-// tiles' shared memory (a step of 128 tokens holds 64 KB of them: two and a half
-// steps in flight) and the tensor core. Measured (activation staging included): 2 x
-// 9728 x 2560 Q4_K, 32 / 128 / 512 tokens 29 / 33 / 131 -> 17 / 24 / 58 us (875
-// TFLOP/s at 512); 248320 x 2560 Q6_K, 32 / 79 / 128 tokens 229 / 245 / 266 -> 127 /
-// 144 / 190 us (4.4 TB/s at 32).
+// What bounds it: a step takes about 1100 cycles and 9 more a token column, the
+// dequantization's instructions and hand-overs, and the tensor core and the traffic of the
+// activation tiles, which do not quite overlap them; a product of few steps the chain of
+// staging kernel (2-3 us), hand-over (1), first tiles (1) and the sum over a cluster (3).
+// Measured (activation staging included), us at 32 / 79 / 128 / 512 tokens, with every role
+// behind one thread, shares summed by the last block alone and staging in blocks of up to
+// 1024 threads -> now: 19456 x 2560 Q4_K 15.9 / 18.8 / 23.3 / 57.3 -> 14.5 / 16.7 / 19.2 /
+// 49.9; 2560 x 9728 Q6_K 18.0 / 24.8 / 32.5 / 45.2 -> 13.4 / 16.2 / 18.4 / 32.4; 2560 x 4096
+// Q4_K 13.3 / 16.5 / 18.3 / 22.7 -> 8.5 / 10.5 / 12.4 / 18.4; 248320 x 2560 Q6_K at 32 / 79 /
+// 128 tokens 122 / 155 / 222 -> 115 / 142 / 177 (outputs of 128 tokens are 127 MB).
 //
 // Each activation row is scaled by a power of two into fp16 range first and the
 // outputs scaled back, so range never costs precision. Rounding w and x to
@@ -65,6 +77,8 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <mutex>
 #include <vector>
 
 namespace gufo {
@@ -126,11 +140,12 @@ struct TcGemmArgs {
   int groups;              // token groups
   int n;                   // token columns of a group, a multiple of 16
   int units;               // tiles * groups
-  int per, extra;          // steps of a thread block: per, one more for the first `extra`
+  int cluster;             // thread blocks that share every unit as a cluster (1: none do)
+  int per, extra;          // steps of a thread block otherwise: per, one more for the first `extra`
   int raw_stages, x_stages;
   const uint8_t* xh;       // activation tile images [group][blocks * 4][n][64] fp16, swizzled
   const float* unscale;    // [groups * n]: factor that undoes a row's power-of-two scale
-  float* partial;          // [thread block][2][n][128]: sums of tiles that a cut goes through
+  float* partial;          // [thread block][2][n * 128]: sums of tiles that a cut goes through (PartialChunk)
   unsigned* counters;      // [thread block]: arrivals at the tile that starts there
   int tokens;
   int out_stride;          // floats between token rows of y
@@ -154,25 +169,32 @@ __device__ __forceinline__ bool MbarTrySuspended(uint32_t bar, uint32_t parity) 
 // Waits for the phase with `parity` to complete, for at most kWaitCycles and
 // only while no thread of the block has given up. Returns false when it did
 // not see the phase complete. PATIENT: suspended in between (loaders and
-// epilogue, whose waits are long; waking up takes longer).
+// epilogue, whose waits are long; waking up takes longer). Called by whole warps,
+// which leave it converged: what follows are instructions of the warp as one
+// (tcgen05.st, tcgen05.ld, elect.sync), and lanes that had seen the phase complete
+// at different polls reached them apart.
 template <bool PATIENT = false>
 __device__ __forceinline__ bool BoundedWait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                             int* error, int code) {
-  if (MbarTryWait(bar, parity)) {
-    return true;
+  bool done = MbarTryWait(bar, parity);
+  if (!done) {
+    const long long start = clock64();
+    do {
+#pragma unroll 1
+      for (int i = 0; i < 32 && !done; ++i) {
+        done = PATIENT ? MbarTrySuspended(bar, parity) : MbarTryWait(bar, parity);
+      }
+      if (!done && *abort_flag != 0) {
+        break;
+      }
+      if (!done && clock64() - start >= kWaitCycles) {
+        *abort_flag = 1;
+        atomicCAS(error, 0, code);
+      }
+    } while (!done);
   }
-  const long long start = clock64();
-  while (clock64() - start < kWaitCycles) {
-    if (PATIENT ? MbarTrySuspended(bar, parity) : MbarTryWait(bar, parity)) {
-      return true;
-    }
-    if (*abort_flag != 0) {
-      return false;
-    }
-  }
-  *abort_flag = 1;
-  atomicCAS(error, 0, code);
-  return false;
+  __syncwarp();
+  return done;
 }
 
 // One thread of a converged warp. Instructions of the asynchronous units take
@@ -307,6 +329,10 @@ struct Pair;
 template <>
 struct Pair<GUFO_CUDA_Q4_K> {
   uint4 head, q0, q1;
+  // A word that takes all of them.
+  __device__ __forceinline__ uint32_t Any() const {
+    return (head.x ^ head.y ^ head.z) ^ (head.w ^ q0.x ^ q0.y) ^ (q0.z ^ q0.w ^ q1.x) ^ (q1.y ^ q1.z ^ q1.w);
+  }
   __device__ __forceinline__ void Load(const uint8_t* raw, int row, int p, int b) {
     (void)b;
     const uint8_t* block = raw + row * kQ4KBytes;
@@ -348,6 +374,10 @@ struct Pair<GUFO_CUDA_Q6_K> {
   uint4 l0, l1, h0, h1;
   uint2 sc8;
   uint32_t d;
+  __device__ __forceinline__ uint32_t Any() const {
+    return (l0.x ^ l0.y ^ l0.z) ^ (l0.w ^ l1.x ^ l1.y) ^ (l1.z ^ l1.w ^ h0.x) ^ (h0.y ^ h0.z ^ h0.w) ^
+           (h1.x ^ h1.y ^ h1.z) ^ (h1.w ^ sc8.x ^ sc8.y) ^ d;
+  }
   __device__ __forceinline__ void Load(const uint8_t* raw, int row, int p, int b) {
     const int h = p >> 1;
     const uint8_t* ql = raw + Q::kQl + row * 128;
@@ -381,8 +411,15 @@ struct Pair<GUFO_CUDA_Q6_K> {
   }
 };
 
-// First step of thread block c's range: the first `extra` ranges are a step longer.
-__device__ __forceinline__ int RangeStart(const TcGemmArgs& a, int c) { return c * a.per + min(c, a.extra); }
+// First step of thread block c's range: the first `extra` ranges are a step longer, or a
+// cluster's blocks take a unit's steps in even shares.
+__device__ __forceinline__ int RangeStart(const TcGemmArgs& a, int c) {
+  if (a.cluster > 1) {
+    const int u = c / a.cluster;
+    return u * a.blocks + (c - u * a.cluster) * a.blocks / a.cluster;
+  }
+  return c * a.per + min(c, a.extra);
+}
 
 // Where a unit works: its part, first weight row and token group.
 struct Unit {
@@ -407,6 +444,58 @@ __device__ __forceinline__ Unit LocateUnit(const TcGemmArgs& a, int u) {
   return unit;
 }
 
+// Brings the raw blocks of the steps [step, until) into the ring; the calling warp's lanes
+// agree on everything, one of them issues the copies.
+template <int TYPE>
+struct RawLoader {
+  const TcGemmArgs& a;
+  uint32_t full, empty;   // barriers of stage 0
+  uint32_t to;            // stage 0
+  volatile int* abort_flag;
+  int step, last;
+  int stage = 0;
+  uint32_t phase = 0;
+
+  __device__ __forceinline__ void Run(int until) {
+    using Q = Quant<TYPE>;
+    while (step < until) {
+      const int u = step / a.blocks;
+      const Unit unit = LocateUnit(a, u);
+      const CUtensorMap* map = &a.maps[unit.part * 3];
+      const int row = unit.row0;
+      const int end = min((u + 1) * a.blocks, until);
+      for (int b = step - u * a.blocks; step < end; ++b, ++step) {
+        BoundedWait<true>(empty + 8u * stage, phase ^ 1u, abort_flag, a.error, 1);
+        const uint32_t at_shared = to + stage * Q::kRawStride;
+        const uint32_t bar = full + 8u * stage;
+        if (ElectOne()) {
+          MbarArriveExpectTx(bar, Q::kRawBytes);
+          // Rows past the end of the part arrive as zeros.
+          if constexpr (TYPE == GUFO_CUDA_Q4_K) {
+            TileCopy(at_shared, map, b * kQ4KBytes, row, bar);
+          } else {
+            // The planar device arrangement (Q6KBlockAt): a slab of n blocks stores
+            // ql n x 128 | qh n x 64 | scales n x 16 | d n x 2.
+            const int slab = b / kQ6KSlabBlocks;
+            const int j = b - slab * kQ6KSlabBlocks;
+            const int n = min(a.blocks - slab * kQ6KSlabBlocks, kQ6KSlabBlocks);
+            const int at = slab * kQ6KSlabBlocks * kQ6KBytes;
+            TileCopy(at_shared + Q::kQl, map, at + 128 * j, row, bar);
+            TileCopy(at_shared + Q::kQh, map + 1, at + 128 * n + 64 * j, row, bar);
+            TileCopy(at_shared + Q::kSc, map + 2, at + 192 * n + 16 * j, row, bar);
+            TileCopy(at_shared + Q::kD, map + 2, at + 208 * n, row, bar);   // the slab's d values
+          }
+        }
+        __syncwarp();
+        if (++stage == a.raw_stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+  }
+};
+
 // The thread blocks that share a cut tile (the unit of `blocks` steps from step
 // `begin` on), from one of them.
 struct CutTile {
@@ -428,47 +517,195 @@ __device__ __forceinline__ int CutSlot(const TcGemmArgs& a, const CutTile& cut, 
   return c == cut.from && RangeStart(a, c) < begin ? 1 : 0;
 }
 
-// Column `col` (128 rows) of a thread block's partial sums.
-__device__ __forceinline__ float* PartialColumn(const TcGemmArgs& a, int block, int slot, int col) {
-  return a.partial + ((static_cast<size_t>(block) * 2 + slot) * a.n + col) * kTileRows;
+// A thread block's share of a cut tile in scratch: chunks of sixteen columns, in which a
+// row's four quads of columns lie 128 rows apart, so that a warp writes and reads 512
+// adjacent bytes an instruction.
+constexpr int kChunk = 16;
+__device__ __forceinline__ float4* PartialChunk(const TcGemmArgs& a, int block, int slot, int chunk, int row) {
+  return reinterpret_cast<float4*>(a.partial + ((static_cast<size_t>(block) * 2 + slot) * a.n + chunk * kChunk) * kTileRows) +
+         row;
 }
 
-// A cut tile whose shares are all in scratch, by the first twenty warps: a column
-// of 128 rows a warp, in block order.
-__device__ __noinline__ void AddShares(const TcGemmArgs& a, int u, const CutTile& cut) {
+__device__ __forceinline__ void LeaveChunk(float4* to, const float (&v)[kChunk]) {
+#pragma unroll
+  for (int q = 0; q < kChunk / 4; ++q) {
+    __stcg(to + q * kTileRows, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+  }
+}
+
+// The outputs of a row in sixteen columns from `col0` of the unit on; `to` is the unit's
+// first token row (the same for all lanes, which keeps the addresses in uniform registers).
+__device__ __forceinline__ void StoreChunk(const TcGemmArgs& a, float* to, uint32_t row, int col0, int columns,
+                                           const float* factor, const float (&v)[kChunk]) {
+  to += static_cast<size_t>(col0) * a.out_stride;
+  if (col0 + kChunk <= columns) {
+#pragma unroll
+    for (int q = 0; q < kChunk / 4; ++q) {
+      const float4 f = *reinterpret_cast<const float4*>(&factor[col0 + 4 * q]);
+      to[row] = v[4 * q] * f.x;
+      to += a.out_stride;
+      to[row] = v[4 * q + 1] * f.y;
+      to += a.out_stride;
+      to[row] = v[4 * q + 2] * f.z;
+      to += a.out_stride;
+      to[row] = v[4 * q + 3] * f.w;
+      to += a.out_stride;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kChunk; ++j) {
+      if (col0 + j < columns) {
+        to[static_cast<size_t>(j) * a.out_stride + row] = v[j] * factor[col0 + j];
+      }
+    }
+  }
+}
+
+// Four outputs of a row, of four tokens from `to` on (the same for all lanes, which keeps
+// the addresses in uniform registers).
+__device__ __forceinline__ void StoreQuad(const TcGemmArgs& a, float* to, uint32_t row, int col, int columns,
+                                          const float* factor, const float4& v) {
+  if (col + 4 <= columns) {
+    const float4 f = *reinterpret_cast<const float4*>(&factor[col]);
+    to[row] = v.x * f.x;
+    to += a.out_stride;
+    to[row] = v.y * f.y;
+    to += a.out_stride;
+    to[row] = v.z * f.z;
+    to += a.out_stride;
+    to[row] = v.w * f.w;
+  } else {
+    const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      if (col + j < columns) {
+        to[static_cast<size_t>(j) * a.out_stride + row] = w[j] * factor[col + j];
+      }
+    }
+  }
+}
+
+// Adds up a cut tile whose shares are all at hand and stores its rows: by the first
+// twenty warps, four (of 32 rows each) a chunk. The shares are added in block order, two
+// on their way at a time; block `self`'s is read from tensor memory at `tmem` (self < 0:
+// every share is in scratch). `factor` holds the unit's factors.
+__device__ __noinline__ void AddShares(const TcGemmArgs& a, int u, int from, int to, int self, uint32_t tmem,
+                                       const float* factor) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int begin = u * a.blocks;
-  __threadfence();
+  const CutTile cut{from, to};
   const Unit unit = LocateUnit(a, u);
   const TcPart& part = a.parts[unit.part];
   const int token0 = unit.group * a.n;
   const int columns = min(a.n, a.tokens - token0);
-  const bool vectors = a.out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(part.out) & 15) == 0;
-#pragma unroll 4
-  for (int col = warp; col < columns; col += kDequantWarps + 4) {
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float f = __ldcg(a.unscale + token0 + col);
-#pragma unroll 4
-    for (int c = cut.from; c <= cut.to; ++c) {
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(PartialColumn(a, c, CutSlot(a, cut, c, begin), col)) + lane);
-      sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
-    }
-    const int row = unit.row0 + 4 * lane;
-    float* to = part.out + static_cast<size_t>(token0 + col) * a.out_stride + row;
-    if (vectors && row + 4 <= part.rows) {
-      *reinterpret_cast<float4*>(to) = make_float4(sum.x * f, sum.y * f, sum.z * f, sum.w * f);
-    } else {
-      const float v[4] = {sum.x * f, sum.y * f, sum.z * f, sum.w * f};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (row + i < part.rows) {
-          to[i] = v[i];
-        }
+  const int local = (warp & 3) * 32 + lane;
+  const bool live = unit.row0 + local < part.rows;
+  float* out = part.out + static_cast<size_t>(token0) * a.out_stride;
+#pragma unroll 1
+  for (int chunk = warp >> 2; chunk * kChunk < columns; chunk += kGroups + 1) {
+    auto share = [&](int c, float (&v)[kChunk]) {
+      if (c == self) {
+        TmemLoad16(tmem + chunk * kChunk, v);
+        return;
       }
+      const float4* at = PartialChunk(a, c, CutSlot(a, cut, c, begin), chunk, local);
+#pragma unroll
+      for (int q = 0; q < kChunk / 4; ++q) {
+        const float4 w = __ldcg(at + q * kTileRows);
+        v[4 * q] = w.x, v[4 * q + 1] = w.y, v[4 * q + 2] = w.z, v[4 * q + 3] = w.w;
+      }
+    };
+    float sum[kChunk];
+    share(from, sum);
+    int c = from + 1;
+#pragma unroll 1
+    for (; c + 1 <= to; c += 2) {
+      float v[kChunk], w[kChunk];
+      share(c, v);
+      share(c + 1, w);
+#pragma unroll
+      for (int j = 0; j < kChunk; ++j) {
+        sum[j] = (sum[j] + v[j]) + w[j];
+      }
+    }
+    if (c <= to) {
+      float v[kChunk];
+      share(c, v);
+#pragma unroll
+      for (int j = 0; j < kChunk; ++j) {
+        sum[j] += v[j];
+      }
+    }
+    if (live) {
+      StoreChunk(a, out, static_cast<uint32_t>(unit.row0 + local), chunk * kChunk, columns, factor, sum);
     }
   }
   if (threadIdx.x == 0) {
-    a.counters[cut.from] = 0;   // for the next launch
+    a.counters[from] = 0;   // for the next launch
+  }
+}
+
+__device__ __forceinline__ void ClusterBarrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The end of a unit that a cluster has shared, by all threads: every block's accumulator
+// goes to the blocks that own its columns (four columns, a quad, in turn to each), through
+// distributed shared memory into what was the pipeline's, and each owner adds the shares
+// of its columns in rank order and stores them. All blocks are at it together, where one
+// block used to read the others' shares from scratch at the end: 2560 x 9728 Q6_K in seven
+// shares, 32 / 128 tokens 7 / 14 us of its 18 / 31.
+__device__ __forceinline__ void ReduceCluster(const TcGemmArgs& a, uint32_t tmem_acc, uint32_t buffer, const uint8_t* local_buffer,
+                                              const float* factor, const volatile int* abort_flag) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(blockIdx.x) % a.cluster;
+  const Unit unit = LocateUnit(a, static_cast<int>(blockIdx.x) / a.cluster);
+  const TcPart& part = a.parts[unit.part];
+  const int token0 = unit.group * a.n;
+  const int columns = min(a.n, a.tokens - token0);
+  const int quads = (columns + 3) / 4;
+  const int each = (a.n / 4 + a.cluster - 1) / a.cluster;   // quads of an owner, at most
+  ClusterBarrier();   // nobody's pipeline needs its shared memory any more
+  if (warp < kDequantWarps + 4) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int row = (warp & 3) * 32 + lane;
+    for (int col0 = 16 * (warp >> 2); col0 < columns; col0 += 16 * (kGroups + 1)) {
+      float v[16];
+      TmemLoad16(tmem_acc + (static_cast<uint32_t>((warp & 3) * 32) << 16) + col0, v);
+      int owner = col0 / 4 % a.cluster, slot = col0 / 4 / a.cluster;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t to;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;"
+            : "=r"(to) : "r"(buffer + static_cast<uint32_t>(((rank * each + slot) * kTileRows + row) * 16)), "r"(owner));
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+                     ::"r"(to), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3]) : "memory");
+        if (++owner == a.cluster) {
+          owner = 0;
+          ++slot;
+        }
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  ClusterBarrier();
+  if (warp < kDequantWarps + 4 && *abort_flag == 0) {
+    const int row = static_cast<int>(threadIdx.x & 127);
+    if (unit.row0 + row < part.rows) {
+      float* out = part.out + static_cast<size_t>(token0) * a.out_stride;
+      for (int slot = threadIdx.x >> 7; slot * a.cluster + rank < quads; slot += kGroups + 1) {
+        const float4* from = reinterpret_cast<const float4*>(local_buffer) + slot * kTileRows + row;
+        float4 sum = *from;
+        for (int r = 1; r < a.cluster; ++r) {
+          const float4 v = from[r * each * kTileRows];
+          sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+        }
+        const int col = 4 * (slot * a.cluster + rank);
+        StoreQuad(a, out + static_cast<size_t>(col) * a.out_stride, static_cast<uint32_t>(unit.row0 + row), col, columns,
+                  factor, sum);
+      }
+    }
   }
 }
 
@@ -495,8 +732,11 @@ __device__ __forceinline__ void DequantSteps(const TcGemmArgs& a, const DequantP
     BoundedWait(at.raw_full + 8 * stage, phase, abort_flag, a.error, 4);
     Pair<TYPE> pair;
     pair.Load(raw, at.row, at.p, b);
-    __syncwarp();
-    if (leader) {
+    // The stage may be overwritten once every lane has its bytes. The vote needs them, and the
+    // arrival needs the vote: behind a mere __syncwarp the loads were moved past the arrival,
+    // and now and then a row's weights were those of the block that came next.
+    const unsigned arrived = __ballot_sync(0xFFFFFFFFu, pair.Any() != 0xDEADBEEFu);
+    if (leader && arrived != 0) {
       MbarArrive(at.raw_empty + 8 * stage);
     }
     uint32_t lo[16], hi[16];
@@ -525,16 +765,18 @@ __device__ __forceinline__ void DequantSteps(const TcGemmArgs& a, const DequantP
   }
 }
 
+// (The bound is that of 72 registers a thread, which leave room for a block of
+// StageHalfKernel on the SM; kTcThreads threads are launched.)
 template <int TYPE>
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(896, 1)
 GemmTc(const __grid_constant__ TcGemmArgs a) {
   using Q = Quant<TYPE>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_mem[4 * kMaxStages + 2 * kGroups + 4];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
-  __shared__ float factor[kMaxN];    // what undoes the scales of the unit's token rows
-  __shared__ int finish;             // a cut tile whose shares are all in scratch and that is left to this block (unit + 1)
+  __shared__ __align__(16) float factor[kMaxN];    // what undoes the scales of the unit's token rows
+  __shared__ int finish;   // a cut tile whose shares are all in scratch and that is left to this block (unit + 1)
   __shared__ int others_done;
   // The swizzled tiles need a 1024-byte aligned base: activation tiles, then raw blocks.
   const uint32_t base = (SharedAddress(smem_raw) + 1023u) & ~1023u;
@@ -552,16 +794,28 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
   auto acc_empty = [&](int s) { return bars + 8u * (4 * kMaxStages + 2 * kGroups + 2 + s); };
   volatile int* abort_flag = &abort_word;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const int first = RangeStart(a, blockIdx.x);
   const int last = RangeStart(a, blockIdx.x + 1);
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < a.raw_stages; ++s) {
-      MbarInit(raw_full(s), 1);
-      MbarInit(raw_empty(s), kDequantWarps);
+  // The first raw blocks are asked for before anything else: the weights never depend on
+  // earlier kernels, and they are the longest way off.
+  RawLoader<TYPE> raw_loader{a, raw_full(0), raw_empty(0), base + raw_at, abort_flag, first, last};
+  if (warp == kRawWarp) {
+    if (ElectOne()) {
+      for (int s = 0; s < a.raw_stages; ++s) {
+        MbarInit(raw_full(s), 1);
+        MbarInit(raw_empty(s), kDequantWarps);
+      }
+      abort_word = 0;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    __syncwarp();
+    raw_loader.Run(min(first + 2, last));   // (more would hold up the others: an issue takes 100 cycles and more)
+  }
+  if (threadIdx.x == 0) {
     for (int s = 0; s < a.x_stages; ++s) {
       MbarInit(x_full(s), 1);
       MbarInit(x_empty(s), 1);
@@ -574,7 +828,6 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
       MbarInit(acc_full(s), 1);
       MbarInit(acc_empty(s), 4);
     }
-    abort_word = 0;
     finish = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -587,7 +840,7 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_slot);
+  const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *reinterpret_cast<volatile uint32_t*>(&tmem_slot), 0);
   // The weights never depend on earlier kernels; the activation tiles and the
   // outputs do.
   GridLaunchDependents();
@@ -595,69 +848,36 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
   // Every role walks the steps [first, last); the stage counters run on across
   // units, so the pipeline never drains between them.
   if (warp == kRawWarp) {
-    // ---- raw blocks ----------------------------------------------------------
-    if (ElectOne()) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int step = first; step < last;) {
-        const int u = step / a.blocks;
-        const Unit unit = LocateUnit(a, u);
-        const CUtensorMap* map = &a.maps[unit.part * 3];
-        for (int b = step - u * a.blocks; b < a.blocks && step < last; ++b, ++step) {
-          {
-            BoundedWait<true>(raw_empty(stage), phase ^ 1u, abort_flag, a.error, 1);
-            const uint32_t to = base + raw_at + stage * Q::kRawStride;
-            const uint32_t bar = raw_full(stage);
-            MbarArriveExpectTx(bar, Q::kRawBytes);
-            // Rows past the end of the part arrive as zeros.
-            const int row = unit.row0;
-            if constexpr (TYPE == GUFO_CUDA_Q4_K) {
-              TileCopy(to, map, b * kQ4KBytes, row, bar);
-            } else {
-              // The planar device arrangement (Q6KBlockAt): a slab of n blocks stores
-              // ql n x 128 | qh n x 64 | scales n x 16 | d n x 2.
-              const int slab = b / kQ6KSlabBlocks;
-              const int j = b - slab * kQ6KSlabBlocks;
-              const int n = min(a.blocks - slab * kQ6KSlabBlocks, kQ6KSlabBlocks);
-              const int at = slab * kQ6KSlabBlocks * kQ6KBytes;
-              TileCopy(to + Quant<GUFO_CUDA_Q6_K>::kQl, map, at + 128 * j, row, bar);
-              TileCopy(to + Quant<GUFO_CUDA_Q6_K>::kQh, map + 1, at + 128 * n + 64 * j, row, bar);
-              TileCopy(to + Quant<GUFO_CUDA_Q6_K>::kSc, map + 2, at + 192 * n + 16 * j, row, bar);
-              TileCopy(to + Quant<GUFO_CUDA_Q6_K>::kD, map + 2, at + 208 * n, row, bar);   // the slab's d values
-            }
-            if (++stage == a.raw_stages) {
-              stage = 0;
-              phase ^= 1u;
-            }
-          }
-        }
-      }
-    }
+    raw_loader.Run(last);
   } else if (warp == kXWarp) {
     // ---- activation tiles, two (half a step's) per stage ------------------------
     GridDependencyWait();
-    if (ElectOne()) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int step = first; step < last; ++step) {
-        const int u = step / a.blocks;
-        const int group = u % a.groups;
-        const uint8_t* from = a.xh + (static_cast<size_t>(group) * a.blocks + (step - u * a.blocks)) * 2 * x_bytes;
-        for (int t = 0; t < 2; ++t) {
-          BoundedWait<true>(x_empty(stage), phase ^ 1u, abort_flag, a.error, 2);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int step = first; step < last;) {
+      const int u = step / a.blocks;
+      const int group = u % a.groups;
+      const int end = min((u + 1) * a.blocks, last);
+      const uint8_t* from = a.xh + (static_cast<size_t>(group) * a.blocks + (step - u * a.blocks)) * 2 * x_bytes;
+      for (int half = 2 * (end - step); half > 0; --half) {
+        BoundedWait<true>(x_empty(stage), phase ^ 1u, abort_flag, a.error, 2);
+        if (ElectOne()) {
           MbarArriveExpectTx(x_full(stage), x_bytes);
-          BulkCopy(base + stage * x_bytes, from + static_cast<size_t>(t) * x_bytes, x_bytes, x_full(stage));
-          if (++stage == a.x_stages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          BulkCopy(base + stage * x_bytes, from, x_bytes, x_full(stage));
+        }
+        __syncwarp();
+        from += x_bytes;
+        if (++stage == a.x_stages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
+      step = end;
     }
   } else if (warp == kMmaWarp) {
     // ---- MMA issue ---------------------------------------------------------
     // kind::f16, fp32 accumulate, fp16 A and B, both K-major, M = 128.
-    if (ElectOne()) {
+    {
       const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(a.n >> 3) << 17) |
                              (static_cast<uint32_t>(kTileRows >> 4) << 24);
       int xs = 0;              // stage of the step's first two activation tiles
@@ -682,15 +902,20 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
               const uint32_t slot = tmem + static_cast<uint32_t>(g * kSlotColumns);
               const uint64_t desc = desc_x + static_cast<uint64_t>(t * (x_bytes >> 5));   // 16-byte units
+              if (ElectOne()) {
 #pragma unroll
-              for (int k = 0; k < kTileK / 16; ++k) {
-                // 16 values: eight columns of the slot, 32 bytes of the swizzled rows.
-                MmaF16(accumulator, slot + 8u * k, desc + 2u * k, idesc, k > 0 || g > 0 ? 1u : more);
+                for (int k = 0; k < kTileK / 16; ++k) {
+                  // 16 values: eight columns of the slot, 32 bytes of the swizzled rows.
+                  MmaF16(accumulator, slot + 8u * k, desc + 2u * k, idesc, k > 0 || g > 0 ? 1u : more);
+                }
+                // A commit arrives once everything issued so far has retired.
+                MmaCommit(w_empty(g));
+                if (t == 1) {
+                  MmaCommit(x_empty(xs));
+                }
               }
-              // A commit arrives once everything issued so far has retired.
-              MmaCommit(w_empty(g));
+              __syncwarp();
             }
-            MmaCommit(x_empty(xs));
             if (++xs == a.x_stages) {
               xs = 0;
               x_phase ^= 1u;
@@ -698,7 +923,10 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
           }
           w_phase ^= 1u;
         }
-        MmaCommit(acc_full(acc));
+        if (ElectOne()) {
+          MmaCommit(acc_full(acc));
+        }
+        __syncwarp();
         acc ^= 1;
         acc_phase ^= acc == 0 ? 1u : 0u;
       }
@@ -731,24 +959,16 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t from = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kAccColumn +
                             static_cast<uint32_t>(acc * a.n);
-      const int row = unit.row0 + local;
-      float* to = part.out + static_cast<size_t>(token0) * a.out_stride + row;
-      float* partial = PartialColumn(a, blockIdx.x, 0, 0) + local;
-      for (int col0 = 0; col0 < columns; col0 += 16) {
-        float v[16];
+      const uint32_t row = static_cast<uint32_t>(unit.row0 + local);
+      const bool live = ready && unit.row0 + local < part.rows;
+      float* to = part.out + static_cast<size_t>(token0) * a.out_stride;
+      for (int col0 = 0; col0 < columns; col0 += kChunk) {
+        float v[kChunk];
         TmemLoad16(from + col0, v);
         if (!whole) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            __stcg(partial + (col0 + j) * kTileRows, v[j]);
-          }
-        } else if (ready && row < part.rows) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            if (col0 + j < columns) {
-              to[static_cast<size_t>(col0 + j) * a.out_stride] = v[j] * factor[col0 + j];
-            }
-          }
+          LeaveChunk(PartialChunk(a, blockIdx.x, 0, col0 / kChunk, local), v);
+        } else if (live) {
+          StoreChunk(a, to, row, col0, columns, factor, v);
         }
       }
       // This accumulator may be overwritten now.
@@ -788,9 +1008,9 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
   const int tail_unit = (last - 1) / a.blocks;
   const int tail_begin = tail_unit * a.blocks;
   const bool tail_opens = first >= tail_begin;   // the block's only share
-  if ((first > tail_begin || last < tail_begin + a.blocks) && warp < kDequantWarps + 4) {
-    const Unit unit = LocateUnit(a, tail_unit);
-    const TcPart& part = a.parts[unit.part];
+  if (a.cluster > 1) {
+    ReduceCluster(a, tmem + kAccColumn, base, smem, factor, abort_flag);
+  } else if ((first > tail_begin || last < tail_begin + a.blocks) && warp < kDequantWarps + 4) {
     const CutTile cut = LocateCut(a, blockIdx.x, tail_begin);
     const unsigned others = static_cast<unsigned>(cut.to - cut.from);
     if (threadIdx.x == 0) {
@@ -800,80 +1020,45 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
     }
     asm volatile("bar.sync 2, %0;" ::"n"((kDequantWarps + 4) * 32) : "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const bool finishes = *const_cast<volatile int*>(&others_done) != 0;
-    const int token0 = unit.group * a.n;
-    const int columns = min(a.n, a.tokens - token0);
-    const int local = (warp & 3) * 32 + lane;
-    const int row = unit.row0 + local;
     const int acc = (tail_unit - first / a.blocks) & 1;
     const uint32_t from = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + kAccColumn +
                           static_cast<uint32_t>(acc * a.n);
-    for (int col0 = (warp >> 2) * 16; col0 < columns; col0 += 16 * (kGroups + 1)) {
-      float v[16];
-      TmemLoad16(from + col0, v);
-      if (!finishes) {
-        float* partial = PartialColumn(a, blockIdx.x, tail_opens ? 0 : 1, col0) + local;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          __stcg(partial + j * kTileRows, v[j]);
-        }
-        continue;
+    const int self = static_cast<int>(blockIdx.x);
+    bool finishes = *const_cast<volatile int*>(&others_done) != 0;
+    if (!finishes) {
+      const int columns = min(a.n, a.tokens - (tail_unit - tail_unit / a.groups * a.groups) * a.n);
+      for (int chunk = warp >> 2; chunk * kChunk < columns; chunk += kGroups + 1) {
+        float v[kChunk];
+        TmemLoad16(from + chunk * kChunk, v);
+        LeaveChunk(PartialChunk(a, blockIdx.x, tail_opens ? 0 : 1, chunk, (warp & 3) * 32 + lane), v);
       }
-      // In block order, this block's own share at its place.
-      float sum[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        sum[j] = 0.f;
-      }
-      for (int c = cut.from; c <= cut.to; ++c) {
-        if (c == static_cast<int>(blockIdx.x)) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            sum[j] += v[j];
-          }
-        } else {
-          const float* add = PartialColumn(a, c, CutSlot(a, cut, c, tail_begin), col0) + local;
-          float w[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            w[j] = __ldcg(add + j * kTileRows);
-          }
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            sum[j] += w[j];
-          }
-        }
-      }
-      if (*abort_flag == 0 && row < part.rows) {
-        float* to = part.out + static_cast<size_t>(token0) * a.out_stride + row;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (col0 + j < columns) {
-            to[static_cast<size_t>(col0 + j) * a.out_stride] = sum[j] * factor[col0 + j];
-          }
-        }
-      }
-    }
-    if (finishes) {
-      if (threadIdx.x == 0) {
-        a.counters[cut.from] = 0;   // for the next launch
-      }
-    } else {
       __threadfence();
       asm volatile("bar.sync 2, %0;" ::"n"((kDequantWarps + 4) * 32) : "memory");
       if (threadIdx.x == 0) {
         others_done = atomicAdd(a.counters + cut.from, 1u) == others ? 2 : 0;
       }
       asm volatile("bar.sync 2, %0;" ::"n"((kDequantWarps + 4) * 32) : "memory");
-      if (*const_cast<volatile int*>(&others_done) == 2) {
-        AddShares(a, tail_unit, cut);
-      }
+      finishes = *const_cast<volatile int*>(&others_done) == 2;
+      __threadfence();
+    }
+    if (finishes && *abort_flag == 0) {
+      AddShares(a, tail_unit, cut.from, cut.to, self, from, factor);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
   __syncthreads();
-  if (finish != 0 && warp < kDequantWarps + 4) {
-    AddShares(a, finish - 1, LocateCut(a, blockIdx.x, (finish - 1) * a.blocks));
+  if (finish != 0) {   // the share that opened this block's range came last
+    const int u = finish - 1;
+    const int token0 = (u - u / a.groups * a.groups) * a.n;
+    if (threadIdx.x < min(a.n, a.tokens - token0)) {
+      factor[threadIdx.x] = __ldcg(a.unscale + token0 + threadIdx.x);
+    }
+    __syncthreads();
+    if (warp < kDequantWarps + 4) {
+      const CutTile cut = LocateCut(a, blockIdx.x, u * a.blocks);
+      __threadfence();
+      AddShares(a, u, cut.from, cut.to, -1, 0u, factor);
+    }
   }
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -881,16 +1066,21 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
   }
 }
 
-// One block per token row: scales the row by a power of two so that its largest
-// magnitude lands in [2^13, 2^14), rounds to fp16 and writes the row into every
-// tile image of its group at its swizzled place. Rows past `tokens` are zero.
-// `six`: tile 2 h + j of a block holds Q6_K's runs j and j + 2 of half h (the
-// pair a dequant group turns out together), else values 64 t .. 64 t + 63.
-__global__ void __launch_bounds__(1024)
+// gridDim.y blocks per token row: the row is scaled by a power of two so that its
+// largest magnitude lands in [2^13, 2^14), rounded to fp16 and written into every tile
+// image of its group at its swizzled place. Rows past `tokens` are zero. `six`: tile
+// 2 h + j of a block holds Q6_K's runs j and j + 2 of half h (the pair a dequant group
+// turns out together), else values 64 t .. 64 t + 63.
+//
+// Every block of a row looks for the largest magnitude itself and converts its part. The
+// blocks are small enough to share an SM with a block of the GEMM (256 threads of at most
+// 48 registers beside 736 of 72), whose weights are under way meanwhile; beside blocks of
+// 1024 threads the GEMM's came 3 us late.
+constexpr int kStageThreads = 256;
+__global__ void __launch_bounds__(kStageThreads, 5)
 StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int group_rows, int six, uint8_t* __restrict__ xh,
                 float* __restrict__ unscale) {
-  __shared__ uint32_t warp_top[32];
-  const int threads = static_cast<int>(blockDim.x);
+  __shared__ uint32_t warp_top[kStageThreads / 32];
   GridLaunchDependents();
   GridDependencyWait();
   const int token = blockIdx.x;
@@ -899,44 +1089,22 @@ StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int group_row
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const float4* row = reinterpret_cast<const float4*>(x + static_cast<size_t>(token) * cols);
-  // A thread's first chunks of eight values stay in registers between the two passes.
-  constexpr int kKeep = 2;
-  float4 keep[kKeep][2];
   float up = 1.0f;
   if (token < tokens) {
     uint32_t top = 0;
-    auto see = [&](const float4& v) {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < cols / 4; i += kStageThreads) {
+      const float4 v = row[i];
       top = max(max(top, __float_as_uint(v.x) & 0x7FFFFFFFu), __float_as_uint(v.y) & 0x7FFFFFFFu);
       top = max(max(top, __float_as_uint(v.z) & 0x7FFFFFFFu), __float_as_uint(v.w) & 0x7FFFFFFFu);
-    };
-#pragma unroll
-    for (int i = 0; i < kKeep; ++i) {
-      const int chunk = threadIdx.x + threads * i;
-      if (chunk < cols / 8) {
-        keep[i][0] = row[2 * chunk];
-        keep[i][1] = row[2 * chunk + 1];
-      } else {
-        keep[i][0] = keep[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
     }
-    for (int i = threadIdx.x + 2 * threads * kKeep; i < cols / 4; i += threads) {
-      see(row[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < kKeep; ++i) {
-      see(keep[i][0]);
-      see(keep[i][1]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-    }
+    top = __reduce_max_sync(0xFFFFFFFFu, top);
     if (lane == 0) {
       warp_top[warp] = top;
     }
     __syncthreads();
-    top = warp_top[0];
-    for (int w = 1; w < threads / 32; ++w) {
+#pragma unroll
+    for (int w = 0; w < kStageThreads / 32; ++w) {
       top = max(top, warp_top[w]);
     }
     // Biased exponent e of the maximum: |x| < 2^(e - 126). Scale by 2^(140 - e)
@@ -946,10 +1114,10 @@ StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int group_row
     int shift = e == 255 ? 0 : 140 - e;
     shift = max(-126, min(126, shift));
     up = __uint_as_float(static_cast<uint32_t>(127 + shift) << 23);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && blockIdx.y == 0) {
       unscale[token] = __uint_as_float(static_cast<uint32_t>(127 - shift) << 23);
     }
-  } else if (threadIdx.x == 0) {
+  } else if (threadIdx.x == 0 && blockIdx.y == 0) {
     unscale[token] = 0.f;
   }
   const size_t tile_bytes = static_cast<size_t>(group_rows) * (kTileK * 2);
@@ -970,14 +1138,8 @@ StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int group_row
     *reinterpret_cast<uint4*>(image + tile * tile_bytes + ((c ^ (image_row & 7)) << 4)) = packed;
   };
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < kKeep; ++i) {
-    const int chunk = threadIdx.x + threads * i;
-    if (chunk < cols / 8) {
-      put(chunk, token < tokens ? keep[i][0] : zero, token < tokens ? keep[i][1] : zero);
-    }
-  }
-  for (int chunk = threadIdx.x + threads * kKeep; chunk < cols / 8; chunk += threads) {
+#pragma unroll 4
+  for (int chunk = blockIdx.y * kStageThreads + threadIdx.x; chunk < cols / 8; chunk += gridDim.y * kStageThreads) {
     put(chunk, token < tokens ? row[2 * chunk] : zero, token < tokens ? row[2 * chunk + 1] : zero);
   }
 }
@@ -1043,20 +1205,18 @@ int EncodeRows(CUtensorMap* map, const uint8_t* data, int rows, int row_bytes, i
                                                          std::to_string(static_cast<int>(e)));
 }
 
+constexpr int kMaxCluster = 8;   // what every device takes
+
 // How a product of `tokens` rows is cut: token groups of n columns, thread blocks.
 struct Plan {
-  int groups, n, grid, units;
+  int groups, n, grid, units, cluster;
 };
 
-// Cycles of a step (256 values of 128 rows): the slower of the tensor core (16
-// MMAs of n / 2 cycles) and the dequantization with its hand-overs (measured).
-double StepCycles(int type, int n) {
-  const double mma = 8.0 * n + 120;
-  const double dequant = (type == GUFO_CUDA_Q4_K ? 1450 : 2000) + 4.0 * n;
-  return mma > dequant ? mma : dequant;
-}
+// Cycles of a step (256 values of 128 rows), as measured: what the dequantization and its
+// hand-overs take, and the tensor core's and the activation tiles' part, which grows with n.
+double StepCycles(int type, int n) { return (type == GUFO_CUDA_Q4_K ? 1070 : 1300) + 8.7 * n; }
 
-Plan PlanTc(const GemvArgs& base, const std::vector<int>& parts, int type, int tokens, int sm_count) {
+Plan PlanTc(const GemvArgs& base, const std::vector<int>& parts, int type, int tokens, int sm_count, const int* clusters) {
   const int blocks = base.cols / kSuperBlock;
   int tiles = 0;
   for (int p : parts) {
@@ -1085,9 +1245,17 @@ Plan PlanTc(const GemvArgs& base, const std::vector<int>& parts, int type, int t
       const double cost = static_cast<double>((total + grid - 1) / grid) * StepCycles(type, n) + fix + 30.0 * n;
       if (cost < best_cost) {
         best_cost = cost;
-        best = Plan{groups, n, grid, units};
+        best = Plan{groups, n, grid, units, 1};
       }
     };
+    // A unit shared by a cluster: the exchange and two cluster barriers on top.
+    for (int k = 2; k <= kMaxCluster && k <= blocks; ++k) {
+      const double cost = static_cast<double>((blocks + k - 1) / k) * StepCycles(type, n) + 3500 + 20.0 * n;
+      if (clusters[k] >= units && cost < best_cost) {
+        best_cost = cost;
+        best = Plan{groups, n, k * units, units, k};
+      }
+    }
     consider(sm_count);
     for (int share = 1; share * units <= sm_count; ++share) {
       consider(share * units);
@@ -1104,19 +1272,38 @@ Plan PlanTc(const GemvArgs& base, const std::vector<int>& parts, int type, int t
 template <int TYPE>
 int LaunchPlan(gufo_cuda_ctx* ctx, const GemvArgs& base, const std::vector<int>& group, int tokens) {
   using Q = Quant<TYPE>;
-  static bool configured[16] = {};
-  if (!configured[ctx->device & 15]) {
-    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemmTc<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit - 3072));
-    configured[ctx->device & 15] = true;
-  }
+  // Clusters of k that run at once, each block with all of its SM's shared memory.
+  static std::once_flag configured[16];
+  static int clusters[16][kMaxCluster + 1] = {};
+  static cudaError_t failed[16] = {};
+  const int device = ctx->device & 15;
+  std::call_once(configured[device], [&] {
+    failed[device] = cudaFuncSetAttribute(GemmTc<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit - 3072);
+    for (int k = 2; k <= kMaxCluster; ++k) {
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim = {static_cast<unsigned>(k), 1, 1};
+      cudaLaunchConfig_t config = {};
+      config.gridDim = dim3(static_cast<unsigned>(k));
+      config.blockDim = dim3(kTcThreads);
+      config.dynamicSmemBytes = kSharedLimit - 3072;
+      config.attrs = &attr;
+      config.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&clusters[device][k], GemmTc<TYPE>, &config) != cudaSuccess) {
+        cudaGetLastError();
+        clusters[device][k] = 0;
+      }
+    }
+  });
+  GUFO_CUDA_TRY(failed[device]);
   const int cols = base.cols;
   const int blocks = cols / kSuperBlock;
-  const Plan plan = PlanTc(base, group, TYPE, tokens, ctx->sm_count);
+  const Plan plan = PlanTc(base, group, TYPE, tokens, ctx->sm_count, clusters[device]);
   // Scratch: header (error word, counters), tile images, unscale factors, partial sums.
   const size_t rows = static_cast<size_t>(plan.groups) * plan.n;
   const size_t unscale_at = kHeaderBytes + rows * cols * 2;
   const size_t partial_at = (unscale_at + rows * 4 + 255) / 256 * 256;
-  const bool cuts = plan.units % plan.grid != 0;
+  const bool cuts = plan.cluster == 1 && plan.units % plan.grid != 0;
   const size_t partial_bytes = cuts ? static_cast<size_t>(plan.grid) * 2 * kTileRows * plan.n * 4 : 0;
   int rc = ReserveTc(ctx, partial_at + partial_bytes);
   if (rc != GUFO_CUDA_OK) {
@@ -1127,6 +1314,7 @@ int LaunchPlan(gufo_cuda_ctx* ctx, const GemvArgs& base, const std::vector<int>&
   args.groups = plan.groups;
   args.n = plan.n;
   args.units = plan.units;
+  args.cluster = plan.cluster;
   args.per = plan.units * blocks / plan.grid;
   args.extra = plan.units * blocks % plan.grid;
   args.xh = ctx->tc_scratch + kHeaderBytes;
@@ -1162,12 +1350,15 @@ int LaunchPlan(gufo_cuda_ctx* ctx, const GemvArgs& base, const std::vector<int>&
     args.x_stages = args.x_stages < kMaxStages ? args.x_stages : kMaxStages;
   } while (args.raw_stages > 2 && args.x_stages < 2 * args.raw_stages);
   const size_t smem = 1024 + static_cast<size_t>(args.x_stages) * x_bytes + static_cast<size_t>(args.raw_stages) * Q::kRawStride;
-  // A thread for every two chunks of eight values of a row.
-  const int stage_threads = cols <= 4096 ? 256 : (cols <= 8192 ? 512 : 1024);
-  GUFO_CUDA_TRY(LaunchOverlapped(StageHalfKernel, dim3(static_cast<unsigned>(rows)), dim3(stage_threads), 0, ctx->stream, 1, base.x,
+  // As many blocks a row as leave a block an SM, up to one for every 256 chunks of eight values.
+  const int chunks = cols / 8;
+  int row_blocks = ctx->sm_count / static_cast<int>(rows);
+  row_blocks = std::max(1, std::min(row_blocks, (chunks + kStageThreads - 1) / kStageThreads));
+  GUFO_CUDA_TRY(LaunchOverlapped(StageHalfKernel, dim3(static_cast<unsigned>(rows), static_cast<unsigned>(row_blocks)),
+                                 dim3(kStageThreads), 0, ctx->stream, 1, base.x,
                                  tokens, cols, plan.n, TYPE == GUFO_CUDA_Q6_K ? 1 : 0, const_cast<uint8_t*>(args.xh),
                                  const_cast<float*>(args.unscale)));
-  GUFO_CUDA_TRY(LaunchOverlapped(GemmTc<TYPE>, dim3(plan.grid), dim3(kTcThreads), smem, ctx->stream, 1, args));
+  GUFO_CUDA_TRY(LaunchOverlapped(GemmTc<TYPE>, dim3(plan.grid), dim3(kTcThreads), smem, ctx->stream, plan.cluster, args));
   ctx->launches.fetch_add(2);
   return GUFO_CUDA_OK;
 }

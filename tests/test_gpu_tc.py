@@ -77,6 +77,28 @@ def test_gemm_agrees_with_the_eight_token_passes(ctx):
     ctx.matrix_free(m)
 
 
+@pytest.mark.parametrize("ggml_type", [Q.GGML_Q4_K, Q.GGML_Q6_K])
+@pytest.mark.parametrize("rows,blocks,tokens", [(128, 2, 17), (129, 3, 190), (200, 7, 200), (640, 13, 33), (2300, 8, 18)])
+def test_gemm_units_shared_by_clusters(ctx, oracle, ggml_type, rows, blocks, tokens):
+    """Units whose steps do not divide by the cluster, ragged last tiles, columns that do not divide
+    by the cluster's owners, two token groups; outputs in the middle of wider rows. Twice alike, bit
+    for bit: the shares are added in a fixed order."""
+    cols = 256 * blocks
+    raw = _weights(90 + blocks, rows, cols, ggml_type)
+    x = torch.from_numpy(G.normal(91, tokens, cols)).cuda()
+    m = ctx.matrix_upload(ggml_type, raw, rows, cols)
+    y = torch.full((2, tokens, rows + 3), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(2):   # a second part of three rows: the rows of y are no multiple of 16 bytes
+        ctx.matmul_device(Context._parts([(m, 0, rows), (m, 0, 3)]), 2, x, tokens, y[i])
+    ctx.synchronize()
+    assert torch.equal(y[0], y[1])
+    want = oracle.matmul([(raw, ggml_type, 0, rows)], cols, x.cpu().numpy())
+    assert rel_l2(y[0, :, :rows].cpu(), want) <= 5e-4
+    assert torch.equal(y[0, :, rows:], y[0, :, :3])
+    ctx.matrix_free(m)
+
+
 def test_gemm_stacked_parts_and_row_ranges(ctx, oracle):
     """Gate and up stacked (one Q4_K, one Q6_K: two launches), a row range inside a matrix, an
     F32 part beside them (it takes the other kernels), every output column in its place."""
@@ -134,4 +156,25 @@ def test_gemm_activation_range(ctx, oracle):
     for t in range(tokens):
         if t != 3:
             assert rel_l2(got[t], want[t]) <= GEMM_TOL, t
+    ctx.matrix_free(m)
+
+
+def test_gemm_ring_of_two_blocks_under_load(ctx):
+    """Wide token groups leave the raw blocks a ring of two stages, refilled from L2 by the groups
+    behind the first: a stage must not be overwritten while lanes still read it. Many launches,
+    all alike bit for bit (a row of weights from the next block differs in every token)."""
+    rows, cols, tokens = 19456, 2560, 352   # two groups of 176
+    raw = torch.randint(0, 256, (rows, cols // 256, 144), device="cuda", dtype=torch.uint8,
+                        generator=torch.Generator("cuda").manual_seed(3))
+    raw[:, :, 0:4] = torch.tensor([1e-3, 1e-3], device="cuda").half().view(torch.uint8)
+    x = torch.randn(tokens, cols, device="cuda", generator=torch.Generator("cuda").manual_seed(4))
+    y = torch.empty(12, tokens, rows, device="cuda")
+    torch.cuda.synchronize()
+    m = ctx.matrix_from_device(Q.GGML_Q4_K, raw.data_ptr(), rows, cols)
+    for _ in range(8):
+        for i in range(12):
+            ctx.matmul_device(Context._parts([(m, 0, rows)]), 1, x, tokens, y[i])
+        ctx.synchronize()
+        for i in range(1, 12):
+            assert torch.equal(y[0], y[i])
     ctx.matrix_free(m)
