@@ -405,6 +405,10 @@ struct Input {
   float* h_out = nullptr;
   int* advance = nullptr;
   float* const* mirror = nullptr;  // FastGemvArgs::mirror
+  // residual + norm: nobody reads the normed rows behind the product. Block 0 writes them
+  // once the row's 1 / rms is known, a round trip behind the other blocks' conversion, and
+  // the product is not over before it is.
+  bool normed_unread = false;
 };
 
 // One stage's product for `tokens` rows with its input fused into the GEMV
@@ -434,7 +438,7 @@ int FusedProduct(gufo_cuda_ctx* ctx, float rms_eps, const GemvArgs& stage, const
     args.norm_w = in.norm_w;
     args.eps = rms_eps;
     args.h_out = in.h_out;
-    args.normed_out = in.prologue == kPrologueResNorm ? scratch : nullptr;
+    args.normed_out = in.prologue == kPrologueResNorm && !in.normed_unread ? scratch : nullptr;
     args.advance = in.advance;
     args.epilogue = kEpilogueSwiGlu;
     if (peer_wait != nullptr) {
@@ -517,7 +521,7 @@ int FusedProduct(gufo_cuda_ctx* ctx, float rms_eps, const GemvArgs& stage, const
     args.norm_w = in.norm_w;
     args.eps = rms_eps;
     args.h_out = in.h_out;
-    args.normed_out = in.prologue == kPrologueResNorm ? scratch : nullptr;
+    args.normed_out = in.prologue == kPrologueResNorm && !(in.normed_unread && fast_parts == stage.nparts) ? scratch : nullptr;
     for (int p = 0; p < stage.nparts; ++p) {
       const GemvPart& part = stage.parts[p];
       if (part.type != type) {
@@ -615,6 +619,7 @@ int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens) 
     norm1.delta = pending;
     norm1.norm_w = l.attn_norm;
     norm1.h_out = d->h[cur ^ 1];
+    norm1.normed_unread = l.attention;   // the DeltaNet gates read them
     GUFO_STEP_TRY(FusedProduct(d, l.in, norm1, d->normed, d->in, tokens));
     Mark(d, GUFO_CUDA_TIMELINE_IN);
     cur ^= 1;
@@ -646,6 +651,7 @@ int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens) 
     norm2.delta = d->out;
     norm2.norm_w = l.post_norm;
     norm2.h_out = d->h[cur ^ 1];
+    norm2.normed_unread = c.experts == 0;
     // Where it can, the gate / up product leaves silu(gate) * up (its kernel's
     // epilogue) and the down product starts from plain rows; else the
     // activation is the down product's fused input.
@@ -676,6 +682,7 @@ int EnqueueStep(gufo_cuda_decoder* d, int parity, bool want_logits, int tokens) 
   last.delta = pending;
   last.norm_w = d->output_norm;
   last.h_out = d->h[cur ^ 1];
+  last.normed_unread = true;
   last.advance = d->position_dev;
   d->final_h = last.h_out;
   if (want_logits) {
