@@ -518,4 +518,32 @@ __device__ __forceinline__ float WarpSum(float v) {
   return v;
 }
 
+// WarpSum of each of N values (a power of two), by the same additions: at every step a
+// lane keeps half of its values and adds the other lane's half to it. Returns how many
+// sums are left in a lane's v[0 ..] (all lanes in groups of 32 / N hold the same where N is
+// below 32) and sets *first to the number of the first.
+template <int N>
+__device__ __forceinline__ void Fold(float (&v)[N], int lane, int* first) {
+  int n = N, at = 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (n > 1) {
+      n >>= 1;
+      const bool upper = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i) {
+        if (i < n) {
+          const float keep = upper ? v[i + n] : v[i];
+          const float give = upper ? v[i] : v[i + n];
+          v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, o);
+        }
+      }
+      at += upper ? n : 0;
+    } else {
+      v[0] += __shfl_xor_sync(0xFFFFFFFFu, v[0], o);
+    }
+  }
+  *first = at;
+}
+
 }  // namespace gufo

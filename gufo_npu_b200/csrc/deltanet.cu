@@ -677,7 +677,7 @@ DeltaNetGatesKernel(const __grid_constant__ GatesArgs a) {
   }
   GridLaunchDependents();
   GridDependencyWait();
-  float acc[kGateTile][kGateTile] = {}, sq[kGateTile] = {};
+  float acc[kGateTile * kGateTile] = {}, sq[kGateTile] = {};
   const float4* norm = reinterpret_cast<const float4*>(a.rows.norm_w);
   for (int i = threadIdx.x; i < a.rows.cols / 4; i += blockDim.x) {
     float4 x[kGateTile];
@@ -692,27 +692,16 @@ DeltaNetGatesKernel(const __grid_constant__ GatesArgs a) {
       const float4 v = Times4(w[r][i], nw);
 #pragma unroll
       for (int t = 0; t < kGateTile; ++t) {
-        acc[r][t] = Dot4(v, x[t], acc[r][t]);
+        acc[r * kGateTile + t] = Dot4(v, x[t], acc[r * kGateTile + t]);
       }
     }
   }
-#pragma unroll
-  for (int r = 0; r < kGateTile; ++r) {
-#pragma unroll
-    for (int t = 0; t < kGateTile; ++t) {
-      const float total = WarpSum(acc[r][t]);
-      if (lane == 0) {
-        partial[warp][r * kGateTile + t] = total;
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < kGateTile; ++t) {
-    const float total = WarpSum(sq[t]);
-    if (lane == 0) {
-      partial[warp][kGateTile * kGateTile + t] = total;
-    }
-  }
+  int first;
+  Fold<kGateTile * kGateTile>(acc, lane, &first);
+  partial[warp][first] = acc[0];
+  partial[warp][first + 1] = acc[1];
+  Fold<kGateTile>(sq, lane, &first);
+  partial[warp][kGateTile * kGateTile + first] = sq[0];   // several lanes the same
   __syncthreads();
   const int r = threadIdx.x / kGateTile, t = threadIdx.x % kGateTile;
   if (r >= kGateTile || r0 + r >= count || t0 + t >= a.tokens) {

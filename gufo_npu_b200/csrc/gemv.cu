@@ -240,8 +240,13 @@ GemvRows(const __grid_constant__ GemvArgs args) {
 // values: 512 tokens were 64 launches of the kernel above (1.2 ms with the gaps).
 // Where eight rows a block would leave SMs without one (a router: 257 rows, 33
 // blocks) a block takes two.
+//
+// What bounds it with many tokens: the sums over the lanes and too few warps. A block's 64
+// sums a warp are folded (Fold), 62 shuffles instead of 320, and two blocks share an SM:
+// 64 rows x 2560 values, 8 / 79 / 512 tokens 2.9 / 5.0 / 16.6 -> 2.4 / 4.3 / 12.0 us, 257 rows x
+// 2048 (a router), 4 / 128 tokens 2.6 / 15.2 -> 2.1 / 9.6.
 template <int kF32Rows, int TOK>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kF32Rows * TOK >= 64 ? 2 : 1)
 GemvRowsF32(const __grid_constant__ GemvArgs args, int tokens) {
   __shared__ float partial[8][kF32Rows * TOK];
   const int lane = threadIdx.x & 31;
@@ -261,13 +266,11 @@ GemvRowsF32(const __grid_constant__ GemvArgs args, int tokens) {
   }
   GridLaunchDependents();
   GridDependencyWait();
-  float acc[kF32Rows][TOK];
+  constexpr int kSums = kF32Rows * TOK;
+  float acc[kSums];
 #pragma unroll
-  for (int r = 0; r < kF32Rows; ++r) {
-#pragma unroll
-    for (int t = 0; t < TOK; ++t) {
-      acc[r][t] = 0.f;
-    }
+  for (int j = 0; j < kSums; ++j) {
+    acc[j] = 0.f;
   }
   for (int i = warp * 32 + lane; i < args.cols / 4; i += 256) {
     float4 v[kF32Rows], xv[TOK];
@@ -283,19 +286,16 @@ GemvRowsF32(const __grid_constant__ GemvArgs args, int tokens) {
     for (int r = 0; r < kF32Rows; ++r) {
 #pragma unroll
       for (int t = 0; t < TOK; ++t) {
-        acc[r][t] += v[r].x * xv[t].x + v[r].y * xv[t].y + v[r].z * xv[t].z + v[r].w * xv[t].w;
+        acc[r * TOK + t] += v[r].x * xv[t].x + v[r].y * xv[t].y + v[r].z * xv[t].z + v[r].w * xv[t].w;
       }
     }
   }
+  int first;
+  Fold<kSums>(acc, lane, &first);
+  constexpr int kLeft = kSums > 32 ? kSums / 32 : 1;
 #pragma unroll
-  for (int r = 0; r < kF32Rows; ++r) {
-#pragma unroll
-    for (int t = 0; t < TOK; ++t) {
-      const float total = WarpSum(acc[r][t]);
-      if (lane == 0) {
-        partial[warp][r * TOK + t] = total;
-      }
-    }
+  for (int j = 0; j < kLeft; ++j) {
+    partial[warp][first + j] = acc[j];   // below 32 sums several lanes store the same
   }
   __syncthreads();
   const int r = threadIdx.x / TOK, t = threadIdx.x % TOK;
@@ -371,124 +371,186 @@ __device__ __forceinline__ void SplitWeights5(const uint4& head, uint32_t h, uin
   }
 }
 
-template <int TYPE, int M>
-__global__ void __launch_bounds__(256)
+// Q5_K and Q8_0 rows of whole blocks against up to M tokens. A block takes a group of four
+// rows, or every gridDim.x-th where there are many; AHEAD: a warp's first unit is asked for
+// ahead of the dependency wait and the next one while it multiplies, across the groups. The
+// sums over the lanes are folded (Fold).
+//
+// What bounds it: issue slots for long matrices (a value's conversion and its FMAs), a
+// block's start and one load for short ones. Against loads behind the wait, a block for
+// every group and a butterfly per sum, us at 1 / 2 / 4 / 8 tokens: Q5_K 2048 x 2048 4.2 /
+// 4.6 / 5.9 / 9.3 -> 4.1 / 4.4 / 5.0 / 6.6, 24576 x 2560 46 / 50 / 78 / 101 -> 46 / 51 / 62 /
+// 83; Q8_0 3.3 / 4.5 / 5.8 / 8.6 -> 2.6 / 4.1 / 4.7 / 6.1, 31 / 40 / 64 / 90 -> 27 / 33 / 43 / 64.
+// Registers are kept to what lets three blocks share an SM (four for Q8_0 and one token:
+// 2048 rows are one round then).
+template <int TYPE, int M, bool AHEAD>
+__global__ void __launch_bounds__(256, M == 1 && TYPE == GUFO_CUDA_Q8_0 ? 4 : (M <= 2 ? 3 : 2))
 GemvSplit(const __grid_constant__ GemvArgs args, int tokens) {
   constexpr bool kQ5 = TYPE == GUFO_CUDA_Q5_K;
   constexpr int kBlockBytes = kQ5 ? kQ5KBytes : kSuperBlock / kQ8Block * kQ8Bytes;
-  __shared__ float partial[8][kSplitRows * M];
+  constexpr int kSums = kSplitRows * M;
+  __shared__ float partial[2][8][kSums];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  // Rows past the end repeat the last one, tokens past the end the last token.
+  const int groups = (args.total_rows + kSplitRows - 1) / kSplitRows;
+  const int blocks = args.cols / kSuperBlock;
+  // The rows of a group; rows past the end repeat the last one.
   const uint8_t* row[kSplitRows];
+  auto enter = [&](int group) {
 #pragma unroll
-  for (int r = 0; r < kSplitRows; ++r) {
-    int local = min(static_cast<int>(blockIdx.x) * kSplitRows + r, args.total_rows - 1);
-    int p = 0;
-    while (p + 1 < args.nparts && local >= args.parts[p].rows) {
-      local -= args.parts[p].rows;
-      ++p;
+    for (int r = 0; r < kSplitRows; ++r) {
+      int local = min(group * kSplitRows + r, args.total_rows - 1);
+      int p = 0;
+      while (p + 1 < args.nparts && local >= args.parts[p].rows) {
+        local -= args.parts[p].rows;
+        ++p;
+      }
+      row[r] = args.parts[p].data + static_cast<size_t>(local) * args.parts[p].row_bytes;
     }
-    row[r] = args.parts[p].data + static_cast<size_t>(local) * args.parts[p].row_bytes;
-  }
+  };
   // Where this lane's eight inputs sit: two groups of four.
   const int at = kQ5 ? 64 * (lane >> 3) + 4 * (lane & 7) : 8 * lane;
   constexpr int kApart = kQ5 ? 32 : 4;
   // Q8_0: eight codes at a 2-byte boundary, out of aligned words.
   const int code = 34 * (lane >> 2) + 2 + 8 * (lane & 3);
   const bool odd = (code & 2) != 0;
+  struct Raw {
+    uint4 head[kQ5 ? kSplitRows : 1];
+    uint32_t h[kQ5 ? kSplitRows : 1];
+    uint32_t q[kSplitRows][kQ5 ? 1 : 3];
+    uint16_t d[kQ5 ? 1 : kSplitRows];
+  } raw;
+  auto load = [&](int b) {
+#pragma unroll
+    for (int r = 0; r < kSplitRows; ++r) {
+      const uint8_t* block = row[r] + static_cast<size_t>(b) * kBlockBytes;
+      if constexpr (kQ5) {
+        raw.head[r] = __ldg(reinterpret_cast<const uint4*>(block));
+        raw.h[r] = __ldg(reinterpret_cast<const uint32_t*>(block + 16) + (lane & 7));
+        raw.q[r][0] = __ldg(reinterpret_cast<const uint32_t*>(block + 48) + lane);
+      } else {
+        const uint32_t* words = reinterpret_cast<const uint32_t*>(block + (code & ~3));
+        raw.q[r][0] = __ldg(words);
+        raw.q[r][1] = __ldg(words + 1);
+        raw.q[r][2] = odd ? __ldg(words + 2) : 0u;
+        raw.d[r] = __ldg(reinterpret_cast<const uint16_t*>(block + 34 * (lane >> 2)));
+      }
+    }
+  };
+  enter(static_cast<int>(blockIdx.x));
+  if (AHEAD && warp < blocks) {
+    load(warp);
+  }
   GridLaunchDependents();
   GridDependencyWait();
-  float acc[kSplitRows][M];
-#pragma unroll
-  for (int r = 0; r < kSplitRows; ++r) {
-#pragma unroll
-    for (int t = 0; t < M; ++t) {
-      acc[r][t] = 0.f;
+  int buffer = 0;
+#pragma unroll 1
+  for (int group = static_cast<int>(blockIdx.x); group < groups; group += static_cast<int>(gridDim.x), buffer ^= 1) {
+    if (!AHEAD) {
+      enter(group);
     }
-  }
-  for (int b = warp; b < args.cols / kSuperBlock; b += 8) {
-    float w[kSplitRows][8];
-    if constexpr (kQ5) {
-      uint4 head[kSplitRows];
-      uint32_t h[kSplitRows], q[kSplitRows];
+    float acc[kSums];
 #pragma unroll
-      for (int r = 0; r < kSplitRows; ++r) {
-        const uint8_t* block = row[r] + static_cast<size_t>(b) * kBlockBytes;
-        head[r] = __ldg(reinterpret_cast<const uint4*>(block));
-        h[r] = __ldg(reinterpret_cast<const uint32_t*>(block + 16) + (lane & 7));
-        q[r] = __ldg(reinterpret_cast<const uint32_t*>(block + 48) + lane);
+    for (int j = 0; j < kSums; ++j) {
+      acc[j] = 0.f;
+    }
+    for (int b = warp; b < blocks; b += 8) {
+      // The next unit: of this group, or the first of the block's next one.
+      if constexpr (!AHEAD) {
+        load(b);
       }
+      auto ahead = [&]() {
+        if (!AHEAD) {
+          return;
+        }
+        if (b + 8 < blocks) {
+          load(b + 8);
+        } else if (group + static_cast<int>(gridDim.x) < groups) {
+          enter(group + static_cast<int>(gridDim.x));
+          load(warp);
+        }
+      };
+      auto weights = [&](int r, float (&w)[8]) {
+        if constexpr (kQ5) {
+          SplitWeights5(raw.head[r], raw.h[r], raw.q[r][0], lane >> 3, w);
+        } else {
+          const uint32_t pick = odd ? 0x5432u : 0x3210u;
+          // Codes + 128 as bytes under the exponent of 2^23.
+          const uint32_t lo = __byte_perm(raw.q[r][0], raw.q[r][1], pick) ^ 0x80808080u;
+          const uint32_t hi = __byte_perm(raw.q[r][1], raw.q[r][2], pick) ^ 0x80808080u;
+          const float scale = HalfBitsToFloat(raw.d[r]);
 #pragma unroll
-      for (int r = 0; r < kSplitRows; ++r) {
-        SplitWeights5(head[r], h[r], q[r], lane >> 3, w[r]);
-      }
-    } else {
-      uint32_t q[kSplitRows][3];
-      uint16_t d[kSplitRows];
+          for (int i = 0; i < 4; ++i) {
+            w[i] = scale * (__uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7440u | i)) - 8388736.0f);
+            w[4 + i] = scale * (__uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7440u | i)) - 8388736.0f);
+          }
+        }
+      };
+      auto inputs = [&](int t, float4& x0, float4& x1) {
+        const float* x = args.x + static_cast<size_t>(min(t, tokens - 1)) * args.cols + b * kSuperBlock + at;
+        x0 = *reinterpret_cast<const float4*>(x);
+        x1 = *reinterpret_cast<const float4*>(x + kApart);
+      };
+      auto add = [&](float& to, const float (&w)[8], const float4& x0, const float4& x1) {
+        float sum = fmaf(w[0], x0.x, fmaf(w[1], x0.y, fmaf(w[2], x0.z, w[3] * x0.w)));
+        sum = fmaf(w[4], x1.x, fmaf(w[5], x1.y, fmaf(w[6], x1.z, fmaf(w[7], x1.w, sum))));
+        to += sum;
+      };
+      if constexpr (AHEAD && M <= 2) {
+        // The inputs in registers, a row's weights at a time: three blocks an SM.
+        float4 x0[M], x1[M];
 #pragma unroll
-      for (int r = 0; r < kSplitRows; ++r) {
-        const uint8_t* block = row[r] + static_cast<size_t>(b) * kBlockBytes;
-        const uint32_t* words = reinterpret_cast<const uint32_t*>(block + (code & ~3));
-        q[r][0] = __ldg(words);
-        q[r][1] = __ldg(words + 1);
-        q[r][2] = odd ? __ldg(words + 2) : 0u;
-        d[r] = __ldg(reinterpret_cast<const uint16_t*>(block + 34 * (lane >> 2)));
-      }
+        for (int t = 0; t < M; ++t) {
+          inputs(t, x0[t], x1[t]);
+        }
 #pragma unroll
-      for (int r = 0; r < kSplitRows; ++r) {
-        const uint32_t pick = odd ? 0x5432u : 0x3210u;
-        // Codes + 128 as bytes under the exponent of 2^23.
-        const uint32_t lo = __byte_perm(q[r][0], q[r][1], pick) ^ 0x80808080u;
-        const uint32_t hi = __byte_perm(q[r][1], q[r][2], pick) ^ 0x80808080u;
-        const float scale = HalfBitsToFloat(d[r]);
+        for (int r = 0; r < kSplitRows; ++r) {
+          float w[8];
+          weights(r, w);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          w[r][i] = scale * (__uint_as_float(__byte_perm(lo, 0x4B000000u, 0x7440u | i)) - 8388736.0f);
-          w[r][4 + i] = scale * (__uint_as_float(__byte_perm(hi, 0x4B000000u, 0x7440u | i)) - 8388736.0f);
+          for (int t = 0; t < M; ++t) {
+            add(acc[r * M + t], w, x0[t], x1[t]);
+          }
+        }
+        ahead();
+      } else {
+        float w[kSplitRows][8];
+#pragma unroll
+        for (int r = 0; r < kSplitRows; ++r) {
+          weights(r, w[r]);
+        }
+        ahead();
+#pragma unroll
+        for (int t = 0; t < M; ++t) {
+          float4 x0, x1;
+          inputs(t, x0, x1);
+#pragma unroll
+          for (int r = 0; r < kSplitRows; ++r) {
+            add(acc[r * M + t], w[r], x0, x1);
+          }
         }
       }
     }
+    int first;
+    Fold<kSums>(acc, lane, &first);
+    partial[buffer][warp][first] = acc[0];   // several lanes the same, below 32 sums
+    __syncthreads();
+    const int r = threadIdx.x / M, t = threadIdx.x % M;
+    int local = group * kSplitRows + r;
+    if (threadIdx.x < kSums && local < args.total_rows && t < tokens) {
+      float total = 0.f;
 #pragma unroll
-    for (int t = 0; t < M; ++t) {
-      const float* x = args.x + static_cast<size_t>(min(t, tokens - 1)) * args.cols + b * kSuperBlock + at;
-      const float4 x0 = *reinterpret_cast<const float4*>(x);
-      const float4 x1 = *reinterpret_cast<const float4*>(x + kApart);
-#pragma unroll
-      for (int r = 0; r < kSplitRows; ++r) {
-        float sum = fmaf(w[r][0], x0.x, fmaf(w[r][1], x0.y, fmaf(w[r][2], x0.z, w[r][3] * x0.w)));
-        sum = fmaf(w[r][4], x1.x, fmaf(w[r][5], x1.y, fmaf(w[r][6], x1.z, fmaf(w[r][7], x1.w, sum))));
-        acc[r][t] += sum;
+      for (int k = 0; k < 8; ++k) {
+        total += partial[buffer][k][threadIdx.x];
       }
+      int p = 0;
+      while (p + 1 < args.nparts && local >= args.parts[p].rows) {
+        local -= args.parts[p].rows;
+        ++p;
+      }
+      args.y[static_cast<size_t>(t) * args.y_stride + args.parts[p].out_offset + local] = total;
     }
   }
-#pragma unroll
-  for (int r = 0; r < kSplitRows; ++r) {
-#pragma unroll
-    for (int t = 0; t < M; ++t) {
-      const float total = WarpSum(acc[r][t]);
-      if (lane == 0) {
-        partial[warp][r * M + t] = total;
-      }
-    }
-  }
-  __syncthreads();
-  const int r = threadIdx.x / M, t = threadIdx.x % M;
-  int local = static_cast<int>(blockIdx.x) * kSplitRows + r;
-  if (threadIdx.x >= kSplitRows * M || local >= args.total_rows || t >= tokens) {
-    return;
-  }
-  float total = 0.f;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    total += partial[k][threadIdx.x];
-  }
-  int p = 0;
-  while (p + 1 < args.nparts && local >= args.parts[p].rows) {
-    local -= args.parts[p].rows;
-    ++p;
-  }
-  args.y[static_cast<size_t>(t) * args.y_stride + args.parts[p].out_offset + local] = total;
 }
 
 // Whether GemvSplit runs a part: whole 256-value blocks at the alignment of its loads.
@@ -500,12 +562,21 @@ bool SplitRuns(const GemvPart& part, int cols) {
 
 template <int TYPE>
 int LaunchSplit(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
-  const dim3 grid((args.total_rows + kSplitRows - 1) / kSplitRows);
-  auto launch = [&](auto kernel) { return LaunchOverlapped(kernel, grid, dim3(256), 0, ctx->stream, 1, args, tokens); };
-  GUFO_CUDA_TRY(tokens == 1   ? launch(GemvSplit<TYPE, 1>)
-                : tokens == 2 ? launch(GemvSplit<TYPE, 2>)
-                : tokens <= 4 ? launch(GemvSplit<TYPE, 4>)
-                              : launch(GemvSplit<TYPE, 8>));
+  const int groups = static_cast<int>((args.total_rows + kSplitRows - 1) / kSplitRows);
+  auto launch = [&](auto kernel) {
+    // A few rounds of blocks are dealt out by the hardware as they finish.
+    const int resident = std::max(1, ResidentBlocks(kernel, ctx->device, 256, 0, 1));
+    const int grid = groups <= 3 * resident ? groups : resident;
+    return LaunchOverlapped(kernel, dim3(grid), dim3(256), 0, ctx->stream, 1, args, tokens);
+  };
+  // Long Q5_K rows of one or two tokens hold too much at once for a further unit a warp:
+  // 2560 x 9728 16.5 / 18.2 us without, 17.4 / 19.8 with it.
+  constexpr bool kShort = TYPE != GUFO_CUDA_Q5_K;
+  const bool ahead = kShort || args.cols <= 8 * kSuperBlock;
+  GUFO_CUDA_TRY(tokens == 1   ? (ahead ? launch(GemvSplit<TYPE, 1, true>) : launch(GemvSplit<TYPE, 1, kShort>))
+                : tokens == 2 ? (ahead ? launch(GemvSplit<TYPE, 2, true>) : launch(GemvSplit<TYPE, 2, kShort>))
+                : tokens <= 4 ? launch(GemvSplit<TYPE, 4, true>)
+                              : launch(GemvSplit<TYPE, 8, true>));
   ctx->launches.fetch_add(1);
   return GUFO_CUDA_OK;
 }

@@ -830,3 +830,33 @@ def test_mixture_of_given_experts(ctx, tokens, k, hidden, ffn, experts):
     assert rel_l2(t_sh.cpu().numpy(), want) <= 7e-7
     for m in mats:
         ctx.matrix_free(m)
+
+
+@pytest.mark.parametrize("ggml_type", [Q.GGML_Q5_K, Q.GGML_Q8_0])
+@pytest.mark.parametrize("rows,cols", [(5, 256), (1024, 2304), (5999, 256), (5501, 2560)])
+def test_split_rows_over_many_groups(ctx, ggml_type, rows, cols):
+    """Q5_K and Q8_0 rows in two parts: groups of four rows past the end and across the parts, more
+    groups than three rounds of blocks (each takes several), warps without a block, one unit a warp
+    and several; against float64 over the dequantized rows."""
+    gen = torch.Generator("cuda").manual_seed(rows + cols)
+    per, size = Q.BLOCK_ELEMENTS[ggml_type], Q.BLOCK_BYTES[ggml_type]
+    raw = torch.randint(0, 256, (rows * cols // per, size), device="cuda", generator=gen, dtype=torch.uint8)
+    for at in ((0, 2) if ggml_type == Q.GGML_Q5_K else (0,)):
+        raw[:, at:at + 2] = (1e-4 * (1.0 + torch.rand(raw.shape[0], device="cuda", generator=gen))).half().view(torch.uint8).reshape(-1, 2)
+    m = ctx.matrix_from_device(ggml_type, raw.data_ptr(), rows, cols)
+    w = torch.empty(rows, cols, device="cuda")
+    torch.cuda.synchronize()
+    ctx.dequantize_device(m, 0, rows, w)
+    ctx.synchronize()
+    parts = Context._parts([(m, 0, rows), (m, 1, 3)])
+    for tokens in (1, 2, 3, 5, 8):
+        x = torch.randn(tokens, cols, device="cuda", generator=gen)
+        y = torch.full((tokens, rows + 3), 7.0, device="cuda")
+        torch.cuda.synchronize()
+        ctx.matmul_device(parts, 2, x, tokens, y)
+        ctx.synchronize()
+        want = x.double() @ w.double().T
+        scale = x.double().abs() @ w.double().abs().T   # fp32 sums of cols terms: a few roundings of it
+        assert ((y[:, :rows].double() - want).abs() <= 2e-6 * scale).all()
+        assert torch.equal(y[:, rows:], y[:, 1:4])
+    ctx.matrix_free(m)
