@@ -1237,18 +1237,20 @@ Plan PlanTc(const GemvArgs& base, const std::vector<int>& parts, int type, int t
         return;
       }
       // Thread blocks that share a tile: one more than the even share where the cuts
-      // do not fall on tile ends. Two shares of which one is complete early cost
-      // little; others end together, and their sums go through scratch (measured
-      // for 96 tiles on 148 blocks and 20 tiles on 40 to 148).
+      // do not fall on tile ends. Shares of which one is complete early cost the sums
+      // behind the last step all the same (12288 x 2560, 128 tokens: 96 whole tiles 14.6
+      // us, two groups cut over 148 blocks 18.7; 384 tokens 24.8 and 27.5); others end
+      // together, and their sums go through scratch.
       const int sharing = units % grid == 0 ? 1 : (grid % units == 0 ? grid / units : (grid + units - 1) / units + 1);
-      const double fix = sharing <= 1 ? 0 : (units > grid ? 1500 : 9000 + 60.0 * n + 500.0 * sharing);
+      const double fix = sharing <= 1 ? 0 : (units > grid ? 5000 + 15.0 * n : 9000 + 60.0 * n + 500.0 * sharing);
       const double cost = static_cast<double>((total + grid - 1) / grid) * StepCycles(type, n) + fix + 30.0 * n;
       if (cost < best_cost) {
         best_cost = cost;
         best = Plan{groups, n, grid, units, 1};
       }
     };
-    // A unit shared by a cluster: the exchange and two cluster barriers on top.
+    // A unit shared by a cluster: the exchange and two cluster barriers on top (2560 x
+    // 9728, 79 tokens: 22.1 / 21.9 / 17.6 / 15.9 / 15.4 / 16.5 us in clusters of one to six).
     for (int k = 2; k <= kMaxCluster && k <= blocks; ++k) {
       const double cost = static_cast<double>((blocks + k - 1) / k) * StepCycles(type, n) + 3500 + 20.0 * n;
       if (clusters[k] >= units && cost < best_cost) {
