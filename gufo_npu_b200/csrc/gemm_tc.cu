@@ -54,16 +54,17 @@
 // partial sums (left in scratch) to its own in block order, so the result does not
 // depend on who that is. Nobody waits for another block but for those of its cluster.
 //
-// What bounds it: a step takes about 1100 cycles and 9 more a token column, the
-// dequantization's instructions and hand-overs, and the tensor core and the traffic of the
-// activation tiles, which do not quite overlap them; a product of few steps the chain of
-// staging kernel (2-3 us), hand-over (1), first tiles (1) and the sum over a cluster (3).
+// What bounds it: small products the chain of staging kernel (2-3 us), hand-over (1), first
+// tiles (1) and the sum over a cluster (3); large ones a step's 1000 cycles of
+// dequantization and hand-overs and, in a loop of more than about 100 tokens, the board's
+// power limit (1.3-1.4 GHz then). An MMA with A in tensor memory takes 9.5 + n / 2 cycles.
 // Measured (activation staging included), us at 32 / 79 / 128 / 512 tokens, with every role
 // behind one thread, shares summed by the last block alone and staging in blocks of up to
-// 1024 threads -> now: 19456 x 2560 Q4_K 15.9 / 18.8 / 23.3 / 57.3 -> 14.5 / 16.7 / 19.2 /
-// 49.9; 2560 x 9728 Q6_K 18.0 / 24.8 / 32.5 / 45.2 -> 13.4 / 16.2 / 18.4 / 32.4; 2560 x 4096
-// Q4_K 13.3 / 16.5 / 18.3 / 22.7 -> 8.5 / 10.5 / 12.4 / 18.4; 248320 x 2560 Q6_K at 32 / 79 /
-// 128 tokens 122 / 155 / 222 -> 115 / 142 / 177 (outputs of 128 tokens are 127 MB).
+// 1024 threads -> now: 19456 x 2560 Q4_K 15.9 / 18.8 / 23.3 / 57.3 -> 14.9 / 17.0 / 19.5 /
+// 49.5; 12288 x 2560 Q4_K 12.8 / 15.3 / 18.7 / 36.0 -> 11.4 / 12.9 / 14.5 / 29.7; 2560 x 4096
+// Q4_K 13.3 / 16.5 / 18.3 / 22.7 -> 8.5 / 10.6 / 12.4 / 18.5; 2560 x 9728 Q6_K 18.0 / 24.8 /
+// 32.5 / 45.2 -> 13.6 / 16.5 / 18.6 / 32.7; 248320 x 2560 Q6_K at 32 / 79 / 128 tokens 122 /
+// 155 / 222 -> 119 / 145 / 187 (outputs of 128 tokens are 127 MB).
 //
 // Each activation row is scaled by a power of two into fp16 range first and the
 // outputs scaled back, so range never costs precision. Rounding w and x to
