@@ -60,9 +60,9 @@
 // power limit (1.3-1.4 GHz then). An MMA with A in tensor memory takes 9.5 + n / 2 cycles.
 // Measured (activation staging included), us at 32 / 79 / 128 / 512 tokens, with every role
 // behind one thread, shares summed by the last block alone and staging in blocks of up to
-// 1024 threads -> now: 19456 x 2560 Q4_K 15.9 / 18.8 / 23.3 / 57.3 -> 14.9 / 17.0 / 19.5 /
-// 49.5; 12288 x 2560 Q4_K 12.8 / 15.3 / 18.7 / 36.0 -> 11.4 / 12.9 / 14.5 / 29.7; 2560 x 4096
-// Q4_K 13.3 / 16.5 / 18.3 / 22.7 -> 8.5 / 10.6 / 12.4 / 18.5; 2560 x 9728 Q6_K 18.0 / 24.8 /
+// 1024 threads -> now: 19456 x 2560 Q4_K 15.9 / 18.8 / 23.3 / 57.3 -> 14.0 / 16.2 / 18.6 /
+// 49.5; 12288 x 2560 Q4_K 12.8 / 15.3 / 18.7 / 36.0 -> 10.8 / 12.0 / 13.6 / 28.9; 2560 x 4096
+// Q4_K 13.3 / 16.5 / 18.3 / 22.7 -> 8.3 / 9.4 / 11.2 / 17.5; 2560 x 9728 Q6_K 18.0 / 24.8 /
 // 32.5 / 45.2 -> 13.6 / 16.5 / 18.6 / 32.7; 248320 x 2560 Q6_K at 32 / 79 / 128 tokens 122 /
 // 155 / 222 -> 119 / 145 / 187 (outputs of 128 tokens are 127 MB).
 //
@@ -1090,14 +1090,44 @@ StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int group_row
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const float4* row = reinterpret_cast<const float4*>(x + static_cast<size_t>(token) * cols);
+  // A thread's first chunks of eight values stay in registers between the two passes: a
+  // round trip less (2560 x 4096, 32 / 79 / 512 tokens 8.6 / 10.6 / 18.6 -> 8.3 / 9.4 / 17.5 us;
+  // 12288 x 2560 11.5 / 12.9 / 29.3 -> 10.8 / 12.0 / 28.8). Rows past the end are zeros.
+  constexpr int kKeep = 2;
+  const int chunks = cols / 8;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 keep[kKeep][2];
+#pragma unroll
+  for (int i = 0; i < kKeep; ++i) {
+    keep[i][0] = keep[i][1] = zero;
+  }
   float up = 1.0f;
   if (token < tokens) {
     uint32_t top = 0;
-#pragma unroll 8
-    for (int i = threadIdx.x; i < cols / 4; i += kStageThreads) {
-      const float4 v = row[i];
+    auto see = [&](const float4& v) {
       top = max(max(top, __float_as_uint(v.x) & 0x7FFFFFFFu), __float_as_uint(v.y) & 0x7FFFFFFFu);
       top = max(max(top, __float_as_uint(v.z) & 0x7FFFFFFFu), __float_as_uint(v.w) & 0x7FFFFFFFu);
+    };
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i) {
+      const int chunk = threadIdx.x + kStageThreads * i;
+      if (chunk < chunks) {
+        keep[i][0] = row[2 * chunk];
+        keep[i][1] = row[2 * chunk + 1];
+      }
+    }
+    if (chunks > kKeep * kStageThreads) {
+#pragma unroll 4
+      for (int i = threadIdx.x + 2 * kStageThreads * kKeep; i < cols / 4; i += kStageThreads) {
+        see(row[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i) {
+      if (i * kStageThreads < chunks) {
+        see(keep[i][0]);
+        see(keep[i][1]);
+      }
     }
     top = __reduce_max_sync(0xFFFFFFFFu, top);
     if (lane == 0) {
@@ -1138,9 +1168,24 @@ StageHalfKernel(const float* __restrict__ x, int tokens, int cols, int group_row
     }
     *reinterpret_cast<uint4*>(image + tile * tile_bytes + ((c ^ (image_row & 7)) << 4)) = packed;
   };
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  // The row's blocks take every gridDim.y-th run of kStageThreads chunks.
+  const int each = static_cast<int>(gridDim.y);
+  int run = static_cast<int>(blockIdx.y);
+#pragma unroll
+  for (int i = 0; i < kKeep; ++i) {
+    const int chunk = threadIdx.x + kStageThreads * i;
+    if (run == i) {
+      if (chunk < chunks) {
+        put(chunk, keep[i][0], keep[i][1]);
+      }
+      run += each;
+    }
+  }
+  if (chunks <= kKeep * kStageThreads) {
+    return;
+  }
 #pragma unroll 4
-  for (int chunk = blockIdx.y * kStageThreads + threadIdx.x; chunk < cols / 8; chunk += gridDim.y * kStageThreads) {
+  for (int chunk = run * kStageThreads + threadIdx.x; chunk < chunks; chunk += each * kStageThreads) {
     put(chunk, token < tokens ? row[2 * chunk] : zero, token < tokens ? row[2 * chunk + 1] : zero);
   }
 }
