@@ -134,7 +134,9 @@ int gufo_cuda_matrix_upload(gufo_cuda_ctx* ctx, int ggml_type,
                             gufo_cuda_matrix* out);
 /* The same over bytes already on the device; they are borrowed, not copied,
  * and must outlive the handle (GgufProjections keeps pointers into the mapped
- * file the same way, src/models/qwen35/gguf_projections.hpp:28). */
+ * file the same way, src/models/qwen35/gguf_projections.hpp:28). They must be
+ * complete when a product is enqueued: the kernels ask for quantized weights ahead
+ * of what is still running on the stream. */
 int gufo_cuda_matrix_from_device(gufo_cuda_ctx* ctx, int ggml_type,
                                  const void* device_bytes, int64_t rows,
                                  int64_t cols, gufo_cuda_matrix* out);
