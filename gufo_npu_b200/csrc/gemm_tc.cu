@@ -733,11 +733,9 @@ __device__ __forceinline__ void DequantSteps(const TcGemmArgs& a, const DequantP
     BoundedWait(at.raw_full + 8 * stage, phase, abort_flag, a.error, 4);
     Pair<TYPE> pair;
     pair.Load(raw, at.row, at.p, b);
-    // The stage may be overwritten once every lane has its bytes. The vote needs them, and the
-    // arrival needs the vote: behind a mere __syncwarp the loads were moved past the arrival,
-    // and now and then a row's weights were those of the block that came next.
-    const unsigned arrived = __ballot_sync(0xFFFFFFFFu, pair.Any() != 0xDEADBEEFu);
-    if (leader && arrived != 0) {
+    // The stage may be overwritten once every lane has its bytes, whatever they are.
+    const bool loaded = LoadsDone(pair.Any());
+    if (leader && loaded) {
       MbarArrive(at.raw_empty + 8 * stage);
     }
     uint32_t lo[16], hi[16];

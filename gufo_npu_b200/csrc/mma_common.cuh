@@ -96,6 +96,14 @@ __device__ __forceinline__ void MbarInit(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void MbarArrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// True, for every word: none is both 0 and ~0. But only the votes of the whole warp tell, and
+// they need the word of every lane, so what depends on the answer comes behind the loads that
+// went into the words. A ring slot that asynchronous copies refill is handed back behind it:
+// behind a mere __syncwarp the arrival passed loads of the slot that were still under way, and
+// now and then a row's weights were those of the block that came next.
+__device__ __forceinline__ bool LoadsDone(uint32_t word) {
+  return __any_sync(0xFFFFFFFFu, word != 0u) != 0 || __any_sync(0xFFFFFFFFu, word != ~0u) != 0;
+}
 __device__ __forceinline__ void MbarArriveExpectTx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }

@@ -178,3 +178,53 @@ def test_gemm_ring_of_two_blocks_under_load(ctx):
         for i in range(1, 12):
             assert torch.equal(y[0], y[i])
     ctx.matrix_free(m)
+
+
+def _rows_whose_words_cancel(ggml_type, blocks, word, seed):
+    """One row of `blocks` blocks whose bytes, as a dequantizing lane loads them for 64 of the values
+    of a block (its head or its scales and d, and the words of the codes), have `word` as their xor."""
+    rng = np.random.default_rng(seed)
+    size = Q.BLOCK_BYTES[ggml_type]
+    raw = rng.integers(0, 256, (blocks, size), dtype=np.uint8)
+    d = np.float16(1e-3).tobytes()
+    words = lambda a: np.ascontiguousarray(a).view(np.uint32)
+    for block in raw:
+        if ggml_type == Q.GGML_Q4_K:
+            block[0:4] = np.frombuffer(d + d, np.uint8)
+        else:
+            block[208:210] = np.frombuffer(d, np.uint8)
+        for p in range(4):
+            if ggml_type == Q.GGML_Q4_K:
+                codes = block[16 + 32 * p:48 + 32 * p]
+                rest = words(block[0:16])
+            else:
+                h = p >> 1
+                codes = block[64 * h + 32 * (p & 1):64 * h + 32 * (p & 1) + 32]
+                rest = np.concatenate([words(block[128 + 32 * h:160 + 32 * h]), words(block[192 + 8 * h:200 + 8 * h]),
+                                       np.array([int.from_bytes(d, "little")], np.uint32)])
+            last = np.uint32(word) ^ np.bitwise_xor.reduce(rest) ^ np.bitwise_xor.reduce(words(codes[:28]))
+            codes[28:32] = np.frombuffer(np.uint32(last).tobytes(), np.uint8)
+            assert np.bitwise_xor.reduce(np.concatenate([rest, words(codes)])) == word
+    return raw.reshape(-1)
+
+
+@pytest.mark.parametrize("ggml_type", [Q.GGML_Q4_K, Q.GGML_Q6_K])
+@pytest.mark.parametrize("word", [0x00000000, 0xFFFFFFFF, 0xDEADBEEF])
+def test_gemm_raw_stages_are_released_whatever_the_bytes(ctx, ggml_type, word):
+    """Equal rows, so that all lanes of a warp load the same words, with the xors a release could
+    mistake for nothing loaded: 152 tiles of ten blocks, more steps a thread block than raw stages."""
+    rows, blocks, tokens = 152 * 128, 10, 32
+    cols = 256 * blocks
+    one = _rows_whose_words_cancel(ggml_type, blocks, word, word & 0xFF)
+    raw = torch.from_numpy(one).cuda().repeat(rows, 1)
+    x = torch.randn(tokens, cols, device="cuda", generator=torch.Generator("cuda").manual_seed(5))
+    w = torch.empty(1, cols, device="cuda")
+    y = torch.full((tokens, rows), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    m = ctx.matrix_from_device(ggml_type, raw.data_ptr(), rows, cols)
+    ctx.dequantize_device(m, 0, 1, w)
+    ctx.matmul_device(Context._parts([(m, 0, rows)]), 1, x, tokens, y)
+    ctx.synchronize()
+    want = (x.double() @ w.double().T).expand(tokens, rows)
+    assert float((y.double() - want).norm() / want.norm()) <= GEMM_TOL
+    ctx.matrix_free(m)
