@@ -48,6 +48,20 @@ __device__ __forceinline__ void LoadUnit(Q4KUnit& u, const uint8_t* slab, int bl
   LoadFragments(u, b0, b0 + 8 * kSlabRowBytes, t);
 }
 
+// A word that takes all of them (LoadsDone).
+__device__ __forceinline__ uint32_t AllWords(const Q4KUnit& u) {
+  uint32_t all = 0;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    all ^= u.head[r].x ^ u.head[r].y ^ u.head[r].z ^ u.head[r].w;
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    all ^= u.code[i].x ^ u.code[i].y;
+  }
+  return all;
+}
+
 // The eight 6-bit scales and mins of a block as bytes of two words each
 // (quant::ScaleMinK4, src/core/quant.cpp:158-167, four sub-blocks at a time).
 __device__ __forceinline__ void ScaleBytes(const uint4& h, uint32_t (&sc)[2],

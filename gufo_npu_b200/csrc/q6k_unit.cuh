@@ -70,6 +70,21 @@ __device__ __forceinline__ void LoadUnit(Q6KUnit& u, const uint8_t* slab, int j,
   }
 }
 
+// A word that takes all of them (LoadsDone).
+__device__ __forceinline__ uint32_t AllWords(const Q6KUnit& u) {
+  uint32_t all = 0;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      all ^= u.ql[r][half][0].x ^ u.ql[r][half][0].y ^ u.ql[r][half][1].x ^ u.ql[r][half][1].y ^ u.qh[r][half].x ^
+             u.qh[r][half].y;
+    }
+    all ^= u.sc[r].x ^ u.sc[r].y ^ u.sc[r].z ^ u.sc[r].w ^ u.d[r];
+  }
+  return all;
+}
+
 template <int TOKENS>
 struct Accum {
   static constexpr int kNB = (TOKENS * kLimbs + 7) / 8;

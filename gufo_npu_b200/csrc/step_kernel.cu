@@ -369,11 +369,12 @@ __device__ __noinline__ void TeamGemv(const StepShared& sh, const StepOp& op, co
       const int b = s * 8 + warp;
       if constexpr (kQ4) {
         q4k::Q4KUnit unit;
+        uint32_t loaded = 0;
         if (warp < nblk) {
           q4k::LoadUnit(unit, slab, warp, g, t);
+          loaded = q4k::AllWords(unit);
         }
-        __syncwarp();
-        if (lane == 0) {
+        if (LoadsDone(loaded) && lane == 0) {
           MbarArrive(sh.empty(team, slot));
         }
         if (warp < nblk && landed) {
@@ -404,11 +405,12 @@ __device__ __noinline__ void TeamGemv(const StepShared& sh, const StepOp& op, co
         }
       } else {
         q6k::Q6KUnit unit;
+        uint32_t loaded = 0;
         if (warp < nblk) {
           q6k::LoadUnit(unit, slab, warp, nblk, g, t);
+          loaded = q6k::AllWords(unit);
         }
-        __syncwarp();
-        if (lane == 0) {
+        if (LoadsDone(loaded) && lane == 0) {
           MbarArrive(sh.empty(team, slot));
         }
         if (warp < nblk && landed) {
@@ -682,12 +684,13 @@ __device__ __noinline__ void TeamDelta(const StepShared& sh, const StepOp& op, c
     const bool landed = sh.Wait(sh.full(team, slot), (n / kStepSlots) & 1u, kStepErrSlotFull);
     const float* tile = reinterpret_cast<const float*>(sh.slot(team, slot));
     float s[kDeltaMaxDim / kTeamWarps];
+    uint32_t loaded = 0;
 #pragma unroll
     for (int r = 0; r < kDeltaMaxDim / kTeamWarps; ++r) {
       s[r] = r < rows ? tile[(warp + kTeamWarps * r) * kDeltaTileCols + lane] : 0.f;
+      loaded ^= __float_as_uint(s[r]);
     }
-    __syncwarp();
-    if (lane == 0) {
+    if (LoadsDone(loaded) && lane == 0) {
       MbarArrive(sh.empty(team, slot));
     }
     ++n;

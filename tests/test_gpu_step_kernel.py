@@ -97,6 +97,22 @@ def test_step_kernel_matches_the_launch_chain(shape):
     assert rel_l2(states[1][1], states[0][1]) <= 1e-5
 
 
+def test_step_kernel_repeats_bit_for_bit(ctx):
+    """Rows of nine blocks refill every slot of a team's ring many times a product: a slot handed back
+    ahead of a lane's loads would give that lane bytes of a later slab. Three runs, all alike."""
+    cfg = synth.ModelConfig(**dict(G.DENSE, hidden=2304, ffn=4608, vocab=4096))
+    tensors = synth.build_model(cfg, 22)
+    dec = CudaDecoder(CudaProjections(ctx, cfg, tensors), tensors, max_positions=32, use_graph=True)
+    tokens = [int(t) for t in np.random.default_rng(4).integers(0, cfg.vocab, size=24)]
+    runs = []
+    for _ in range(3):
+        runs.append(np.stack([np.array(dec.Step(t)) for t in tokens]))
+        dec.Reset()
+    assert len(dec.step_profile()) > 0
+    assert np.array_equal(runs[0], runs[1]) and np.array_equal(runs[0], runs[2])
+    dec.close()
+
+
 def test_step_kernel_wait_that_runs_out_is_reported(ctx, golden):
     """Block 0 stays away from one grid barrier (a test hook): the other blocks' waits run out
     after the two milliseconds set here, the kernel ends by itself, the step reports
