@@ -373,7 +373,8 @@ __device__ __forceinline__ void SplitWeights5(const uint4& head, uint32_t h, uin
 
 // Q5_K and Q8_0 rows of whole blocks against up to M tokens. A block takes a group of four
 // rows, or every gridDim.x-th where there are many; AHEAD: a warp's first unit is asked for
-// ahead of the dependency wait and the next one while it multiplies, across the groups. The
+// ahead of the dependency wait (`early`: no bytes are borrowed) and the next one while it
+// multiplies, across the groups. The
 // sums over the lanes are folded (Fold).
 //
 // What bounds it: issue slots for long matrices (a value's conversion and its FMAs), a
@@ -385,7 +386,7 @@ __device__ __forceinline__ void SplitWeights5(const uint4& head, uint32_t h, uin
 // 2048 rows are one round then).
 template <int TYPE, int M, bool AHEAD>
 __global__ void __launch_bounds__(256, M == 1 && TYPE == GUFO_CUDA_Q8_0 ? 4 : (M <= 2 ? 3 : 2))
-GemvSplit(const __grid_constant__ GemvArgs args, int tokens) {
+GemvSplit(const __grid_constant__ GemvArgs args, int tokens, bool early) {
   constexpr bool kQ5 = TYPE == GUFO_CUDA_Q5_K;
   constexpr int kBlockBytes = kQ5 ? kQ5KBytes : kSuperBlock / kQ8Block * kQ8Bytes;
   constexpr int kSums = kSplitRows * M;
@@ -395,17 +396,20 @@ GemvSplit(const __grid_constant__ GemvArgs args, int tokens) {
   const int groups = (args.total_rows + kSplitRows - 1) / kSplitRows;
   const int blocks = args.cols / kSuperBlock;
   // The rows of a group; rows past the end repeat the last one.
+  auto row_of = [&](int group, int r) {
+    int local = min(group * kSplitRows + r, args.total_rows - 1);
+    int p = 0;
+    while (p + 1 < args.nparts && local >= args.parts[p].rows) {
+      local -= args.parts[p].rows;
+      ++p;
+    }
+    return args.parts[p].data + static_cast<size_t>(local) * args.parts[p].row_bytes;
+  };
   const uint8_t* row[kSplitRows];
   auto enter = [&](int group) {
 #pragma unroll
     for (int r = 0; r < kSplitRows; ++r) {
-      int local = min(group * kSplitRows + r, args.total_rows - 1);
-      int p = 0;
-      while (p + 1 < args.nparts && local >= args.parts[p].rows) {
-        local -= args.parts[p].rows;
-        ++p;
-      }
-      row[r] = args.parts[p].data + static_cast<size_t>(local) * args.parts[p].row_bytes;
+      row[r] = row_of(group, r);
     }
   };
   // Where this lane's eight inputs sit: two groups of four.
@@ -438,6 +442,18 @@ GemvSplit(const __grid_constant__ GemvArgs args, int tokens) {
     }
   };
   enter(static_cast<int>(blockIdx.x));
+  if (!early) {
+    // Borrowed bytes may be what a kernel is writing that let this one start already: ahead of
+    // the wait nothing but the L2, where its stores arrive too, may hold them. (Q8_0, one token:
+    // 2048 x 2048 3.3 us instead of 3.5, 2048 x 6144 6.4 instead of 7.0; rows of one block and
+    // Q5_K only pay for it. Read ahead they take 2.6 and 5.9.)
+    GridLaunchDependents();
+    if (!kQ5 && blocks >= 8 && threadIdx.x < kSplitRows) {
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row_of(static_cast<int>(blockIdx.x), threadIdx.x)),
+                   "r"(blocks * kBlockBytes) : "memory");
+    }
+    GridDependencyWait();
+  }
   if (AHEAD && warp < blocks) {
     load(warp);
   }
@@ -563,11 +579,15 @@ bool SplitRuns(const GemvPart& part, int cols) {
 template <int TYPE>
 int LaunchSplit(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
   const int groups = static_cast<int>((args.total_rows + kSplitRows - 1) / kSplitRows);
+  bool early = true;
+  for (int p = 0; p < args.nparts; ++p) {
+    early = early && !args.parts[p].borrowed;
+  }
   auto launch = [&](auto kernel) {
     // A few rounds of blocks are dealt out by the hardware as they finish.
     const int resident = std::max(1, ResidentBlocks(kernel, ctx->device, 256, 0, 1));
     const int grid = groups <= 3 * resident ? groups : resident;
-    return LaunchOverlapped(kernel, dim3(grid), dim3(256), 0, ctx->stream, 1, args, tokens);
+    return LaunchOverlapped(kernel, dim3(grid), dim3(256), 0, ctx->stream, 1, args, tokens, early);
   };
   // Long Q5_K rows of one or two tokens hold too much at once for a further unit a warp:
   // 2560 x 9728 16.5 / 18.2 us without, 17.4 / 19.8 with it.
@@ -920,6 +940,7 @@ int BuildGemvArgs(gufo_cuda_ctx* ctx, const gufo_cuda_rows* parts, int nparts,
     out.out_offset = static_cast<int>(total);
     out.type = m->type;
     out.row_bytes = static_cast<int>(m->row_bytes);
+    out.borrowed = !m->owned;
     total += parts[p].rows;
   }
   if (total > INT32_MAX || cols > INT32_MAX) {

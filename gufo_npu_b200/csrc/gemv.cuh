@@ -15,6 +15,7 @@ struct GemvPart {
   int out_offset;       // column of y where this part starts
   int type;
   int row_bytes;
+  bool borrowed = false;   // bytes that are the caller's (gufo_cuda_matrix_from_device)
 };
 
 struct GemvArgs {

@@ -134,9 +134,11 @@ int gufo_cuda_matrix_upload(gufo_cuda_ctx* ctx, int ggml_type,
                             gufo_cuda_matrix* out);
 /* The same over bytes already on the device; they are borrowed, not copied,
  * and must outlive the handle (GgufProjections keeps pointers into the mapped
- * file the same way, src/models/qwen35/gguf_projections.hpp:28). They must be
- * complete when a product is enqueued: the kernels ask for quantized weights ahead
- * of what is still running on the stream. */
+ * file the same way, src/models/qwen35/gguf_projections.hpp:28). Work enqueued on
+ * the context's stream ahead of a product may write them, but for Q4_K bytes written
+ * by a kernel that lets its dependents start early (griddepcontrol.launch_dependents,
+ * as this library's own kernels do): products ask for Q4_K weights ahead of what is
+ * still running then. */
 int gufo_cuda_matrix_from_device(gufo_cuda_ctx* ctx, int ggml_type,
                                  const void* device_bytes, int64_t rows,
                                  int64_t cols, gufo_cuda_matrix* out);

@@ -860,3 +860,38 @@ def test_split_rows_over_many_groups(ctx, ggml_type, rows, cols):
         assert ((y[:, :rows].double() - want).abs() <= 2e-6 * scale).all()
         assert torch.equal(y[:, rows:], y[:, 1:4])
     ctx.matrix_free(m)
+
+
+@pytest.mark.parametrize("ggml_type", [Q.GGML_Q5_K, Q.GGML_Q8_0])
+def test_borrowed_bytes_that_the_kernel_before_writes(ctx, ggml_type):
+    """A product's outputs are the borrowed weights of the next one: rows of 524288 values keep the
+    first busy long after it has let the second start, which must not have read them by then."""
+    rows, cols, wide = 4, 256, 524288
+    gen = torch.Generator("cuda").manual_seed(7)
+    size = rows * cols // Q.BLOCK_ELEMENTS[ggml_type] * Q.BLOCK_BYTES[ggml_type]
+    # Bytes of 1 to 63 are normal floats and halves wherever a word or a scale falls.
+    want = torch.randint(1, 64, (size,), device="cuda", generator=gen, dtype=torch.uint8)
+    source = torch.zeros(size // 4, wide, device="cuda")
+    source[:, 0] = want.view(torch.float32)
+    one = torch.zeros(wide, device="cuda")
+    one[0] = 1.0
+    target = torch.zeros(size // 4, device="cuda")
+    x = torch.randn(1, cols, device="cuda", generator=gen)
+    w = torch.empty(rows, cols, device="cuda")
+    y = torch.empty(5, rows, device="cuda")
+    torch.cuda.synchronize()
+    writer = Context._parts([(ctx.matrix_from_device(Q.GGML_F32, source.data_ptr(), size // 4, wide), 0, size // 4)])
+    m = ctx.matrix_from_device(ggml_type, target.data_ptr(), rows, cols)
+    for i in range(5):
+        target.zero_()
+        torch.cuda.synchronize()
+        ctx.matmul_device(writer, 1, one, 1, target)
+        ctx.matmul_device(Context._parts([(m, 0, rows)]), 1, x, 1, y[i])
+        ctx.synchronize()
+    assert torch.equal(target.view(torch.uint8), want)
+    ctx.dequantize_device(m, 0, rows, w)
+    ctx.synchronize()
+    exact = x.double() @ w.double().T
+    scale = x.double().abs() @ w.double().abs().T
+    assert ((y.double() - exact).abs() <= 2e-6 * scale).all()
+    ctx.matrix_free(m)
