@@ -375,7 +375,7 @@ __device__ __forceinline__ void SplitWeights5(const uint4& head, uint32_t h, uin
 // rows, or every gridDim.x-th where there are many; AHEAD: a warp's first unit is asked for
 // ahead of the dependency wait (`early`: no bytes are borrowed) and the next one while it
 // multiplies, across the groups. The
-// sums over the lanes are folded (Fold).
+// sums over the lanes are folded (Fold). Without LOOP the grid has a block for every group.
 //
 // What bounds it: issue slots for long matrices (a value's conversion and its FMAs), a
 // block's start and one load for short ones. Against loads behind the wait, a block for
@@ -384,7 +384,7 @@ __device__ __forceinline__ void SplitWeights5(const uint4& head, uint32_t h, uin
 // 83; Q8_0 3.3 / 4.5 / 5.8 / 8.6 -> 2.6 / 4.1 / 4.7 / 6.1, 31 / 40 / 64 / 90 -> 27 / 33 / 43 / 64.
 // Registers are kept to what lets three blocks share an SM (four for Q8_0 and one token:
 // 2048 rows are one round then).
-template <int TYPE, int M, bool AHEAD>
+template <int TYPE, int M, bool AHEAD, bool LOOP = AHEAD>
 __global__ void __launch_bounds__(256, M == 1 && TYPE == GUFO_CUDA_Q8_0 ? 4 : (M <= 2 ? 3 : 2))
 GemvSplit(const __grid_constant__ GemvArgs args, int tokens, bool early) {
   constexpr bool kQ5 = TYPE == GUFO_CUDA_Q5_K;
@@ -445,10 +445,10 @@ GemvSplit(const __grid_constant__ GemvArgs args, int tokens, bool early) {
   if (!early) {
     // Borrowed bytes may be what a kernel is writing that let this one start already: ahead of
     // the wait nothing but the L2, where its stores arrive too, may hold them. (Q8_0, one token:
-    // 2048 x 2048 3.3 us instead of 3.5, 2048 x 6144 6.4 instead of 7.0; rows of one block and
-    // Q5_K only pay for it. Read ahead they take 2.6 and 5.9.)
+    // 2048 x 2048 3.3 us instead of 3.5, 2048 x 6144 6.4 instead of 7.0; rows of one or two
+    // blocks and Q5_K only pay for it. Read ahead they take 2.6 and 5.9.)
     GridLaunchDependents();
-    if (!kQ5 && blocks >= 8 && threadIdx.x < kSplitRows) {
+    if (!kQ5 && blocks >= 4 && threadIdx.x < kSplitRows) {
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(row_of(static_cast<int>(blockIdx.x), threadIdx.x)),
                    "r"(blocks * kBlockBytes) : "memory");
     }
@@ -461,8 +461,9 @@ GemvSplit(const __grid_constant__ GemvArgs args, int tokens, bool early) {
   GridDependencyWait();
   int buffer = 0;
 #pragma unroll 1
-  for (int group = static_cast<int>(blockIdx.x); group < groups; group += static_cast<int>(gridDim.x), buffer ^= 1) {
-    if (!AHEAD) {
+  for (int group = static_cast<int>(blockIdx.x); group < groups;
+       group = LOOP ? group + static_cast<int>(gridDim.x) : groups, buffer ^= 1) {
+    if (LOOP && !AHEAD) {
       enter(group);
     }
     float acc[kSums];
@@ -512,7 +513,7 @@ GemvSplit(const __grid_constant__ GemvArgs args, int tokens, bool early) {
         sum = fmaf(w[4], x1.x, fmaf(w[5], x1.y, fmaf(w[6], x1.z, fmaf(w[7], x1.w, sum))));
         to += sum;
       };
-      if constexpr (AHEAD && M <= 2) {
+      if constexpr (M <= 2 && (AHEAD || (kQ5 && M == 2))) {
         // The inputs in registers, a row's weights at a time: three blocks an SM.
         float4 x0[M], x1[M];
 #pragma unroll
@@ -576,6 +577,21 @@ bool SplitRuns(const GemvPart& part, int cols) {
          reinterpret_cast<uintptr_t>(part.data) % align == 0 && part.row_bytes % align == 0;
 }
 
+// Which form of GemvSplit. Three tokens and more read ahead, and where there are more groups
+// than three rounds of blocks (fewer are dealt out by the hardware as they finish) a block
+// takes several. One or two tokens:
+//   - many groups of short rows (2048 values of Q5_K, 1280 with two tokens, 5120 of Q8_0): the
+//     same, a block's start and its first load are much of it. A block for every group / several,
+//     us: Q5_K 24576 x 1024 25.4 / 20.9, x 3072 48.9 / 49.2, x 9728 121 / 130; two tokens x 1280
+//     (20000 rows) 24.6 / 23.3, x 1536 25.7 / 28.1; Q8_0 24576 x 1024 17.8 / 13.3, x 5120 43.7 /
+//     44.6, x 9728 71 / 79.
+//   - fewer, or longer rows: a block a group. Read ahead is what the library holds: Q8_0, but
+//     not for two tokens and long rows in more than one round (4096 x 9728 19.4 us, 18.8
+//     without); short Q5_K rows of one token in more than one and a half (4096 x 2048 6.9,
+//     7.3 without; 2048 x 1536 3.7, 3.5 without). One token's Q8_0 rows in more than one round
+//     take that form for its prefetch even where they are borrowed (5000 x 1280 5.7 us, 6.2
+//     without). Many long ones keep the loop over one group, with which the compiler's code
+//     is faster (24576 x 9728 80 us without it, 71 with it).
 template <int TYPE>
 int LaunchSplit(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
   const int groups = static_cast<int>((args.total_rows + kSplitRows - 1) / kSplitRows);
@@ -583,20 +599,31 @@ int LaunchSplit(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
   for (int p = 0; p < args.nparts; ++p) {
     early = early && !args.parts[p].borrowed;
   }
-  auto launch = [&](auto kernel) {
-    // A few rounds of blocks are dealt out by the hardware as they finish.
-    const int resident = std::max(1, ResidentBlocks(kernel, ctx->device, 256, 0, 1));
-    const int grid = groups <= 3 * resident ? groups : resident;
+  auto resident = [&](auto kernel) { return std::max(1, ResidentBlocks(kernel, ctx->device, 256, 0, 1)); };
+  auto launch = [&](auto kernel, int grid) {
     return LaunchOverlapped(kernel, dim3(grid), dim3(256), 0, ctx->stream, 1, args, tokens, early);
   };
-  // Long Q5_K rows of one or two tokens hold too much at once for a further unit a warp:
-  // 2560 x 9728 16.5 / 18.2 us without, 17.4 / 19.8 with it.
-  constexpr bool kShort = TYPE != GUFO_CUDA_Q5_K;
-  const bool ahead = kShort || args.cols <= 8 * kSuperBlock;
-  GUFO_CUDA_TRY(tokens == 1   ? (ahead ? launch(GemvSplit<TYPE, 1, true>) : launch(GemvSplit<TYPE, 1, kShort>))
-                : tokens == 2 ? (ahead ? launch(GemvSplit<TYPE, 2, true>) : launch(GemvSplit<TYPE, 2, kShort>))
-                : tokens <= 4 ? launch(GemvSplit<TYPE, 4, true>)
-                              : launch(GemvSplit<TYPE, 8, true>));
+  auto ahead = [&](auto kernel) {
+    const int round = resident(kernel);
+    return launch(kernel, groups <= 3 * round ? groups : round);
+  };
+  constexpr bool kQ5 = TYPE == GUFO_CUDA_Q5_K;
+  if (tokens == 1) {
+    const int round = resident(GemvSplit<TYPE, 1, true>);
+    const bool many = groups > 3 * round;
+    const bool shorter = args.cols <= (kQ5 ? 2048 : 5120);
+    const bool read_ahead = many ? shorter : kQ5 ? shorter && early && 2 * groups > 3 * round : early || groups > round;
+    GUFO_CUDA_TRY(read_ahead     ? ahead(GemvSplit<TYPE, 1, true>)
+                  : kQ5 || !many ? launch(GemvSplit<TYPE, 1, false>, groups)
+                                 : launch(GemvSplit<TYPE, 1, false, !kQ5>, groups));
+  } else if (tokens == 2) {
+    const int round = resident(GemvSplit<TYPE, 2, true>);
+    const bool shorter = args.cols <= (kQ5 ? 1280 : 5120);
+    const bool read_ahead = groups > 3 * round ? shorter : !kQ5 && early && (shorter || groups <= round);
+    GUFO_CUDA_TRY(read_ahead ? ahead(GemvSplit<TYPE, 2, true>) : launch(GemvSplit<TYPE, 2, false>, groups));
+  } else {
+    GUFO_CUDA_TRY(tokens <= 4 ? ahead(GemvSplit<TYPE, 4, true>) : ahead(GemvSplit<TYPE, 8, true>));
+  }
   ctx->launches.fetch_add(1);
   return GUFO_CUDA_OK;
 }

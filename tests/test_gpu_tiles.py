@@ -833,17 +833,23 @@ def test_mixture_of_given_experts(ctx, tokens, k, hidden, ffn, experts):
 
 
 @pytest.mark.parametrize("ggml_type", [Q.GGML_Q5_K, Q.GGML_Q8_0])
-@pytest.mark.parametrize("rows,cols", [(5, 256), (1024, 2304), (5999, 256), (5501, 2560)])
-def test_split_rows_over_many_groups(ctx, ggml_type, rows, cols):
+@pytest.mark.parametrize("held", [False, True])
+@pytest.mark.parametrize("rows,cols", [(5, 256), (1024, 2304), (3001, 1280), (5999, 256), (5501, 2560), (7301, 512),
+                                       (7301, 5376), (2001, 5376)])
+def test_split_rows_over_many_groups(ctx, ggml_type, held, rows, cols):
     """Q5_K and Q8_0 rows in two parts: groups of four rows past the end and across the parts, more
-    groups than three rounds of blocks (each takes several), warps without a block, one unit a warp
-    and several; against float64 over the dequantized rows."""
+    groups than three rounds of blocks (1332 groups, 1776 for one token of Q8_0) of short and of long
+    rows, more than one round and one and a half, warps without a block, one unit a warp and several,
+    bytes that are borrowed and bytes that the library holds; against float64 over the dequantized
+    rows."""
     gen = torch.Generator("cuda").manual_seed(rows + cols)
     per, size = Q.BLOCK_ELEMENTS[ggml_type], Q.BLOCK_BYTES[ggml_type]
     raw = torch.randint(0, 256, (rows * cols // per, size), device="cuda", generator=gen, dtype=torch.uint8)
     for at in ((0, 2) if ggml_type == Q.GGML_Q5_K else (0,)):
         raw[:, at:at + 2] = (1e-4 * (1.0 + torch.rand(raw.shape[0], device="cuda", generator=gen))).half().view(torch.uint8).reshape(-1, 2)
-    m = ctx.matrix_from_device(ggml_type, raw.data_ptr(), rows, cols)
+    torch.cuda.synchronize()
+    m = (ctx.matrix_upload(ggml_type, raw.cpu().numpy(), rows, cols) if held else
+         ctx.matrix_from_device(ggml_type, raw.data_ptr(), rows, cols))
     w = torch.empty(rows, cols, device="cuda")
     torch.cuda.synchronize()
     ctx.dequantize_device(m, 0, rows, w)
