@@ -79,6 +79,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <iterator>
 #include <mutex>
 #include <vector>
 
@@ -1315,16 +1316,22 @@ Plan PlanTc(const GemvArgs& base, const std::vector<int>& parts, int type, int t
   return best;
 }
 
+// Prepares the kernel on the context's device and says how many clusters of k blocks run at
+// once, each block with all of its SM's shared memory (0: not known). What the driver refuses
+// is asked for again at the next product.
 template <int TYPE>
-int LaunchPlan(gufo_cuda_ctx* ctx, const GemvArgs& base, const std::vector<int>& group, int tokens) {
-  using Q = Quant<TYPE>;
-  // Clusters of k that run at once, each block with all of its SM's shared memory.
-  static std::once_flag configured[16];
-  static int clusters[16][kMaxCluster + 1] = {};
-  static cudaError_t failed[16] = {};
-  const int device = ctx->device & 15;
-  std::call_once(configured[device], [&] {
-    failed[device] = cudaFuncSetAttribute(GemmTc<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit - 3072);
+int ConfigureTc(const gufo_cuda_ctx* ctx, int (&clusters)[kMaxCluster + 1]) {
+  struct Device {
+    bool done = false;
+    int clusters[kMaxCluster + 1] = {};
+  };
+  static std::mutex mu;
+  static Device devices[16];
+  std::lock_guard<std::mutex> lock(mu);
+  Device& device = devices[ctx->device & 15];
+  if (!device.done) {
+    GUFO_CUDA_TRY(cudaFuncSetAttribute(GemmTc<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit - 3072));
+    device.done = true;
     for (int k = 2; k <= kMaxCluster; ++k) {
       cudaLaunchAttribute attr;
       attr.id = cudaLaunchAttributeClusterDimension;
@@ -1335,23 +1342,35 @@ int LaunchPlan(gufo_cuda_ctx* ctx, const GemvArgs& base, const std::vector<int>&
       config.dynamicSmemBytes = kSharedLimit - 3072;
       config.attrs = &attr;
       config.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&clusters[device][k], GemmTc<TYPE>, &config) != cudaSuccess) {
+      if (cudaOccupancyMaxActiveClusters(&device.clusters[k], GemmTc<TYPE>, &config) != cudaSuccess) {
         cudaGetLastError();
-        clusters[device][k] = 0;
+        device.clusters[k] = 0;
+        device.done = false;
       }
     }
-  });
-  GUFO_CUDA_TRY(failed[device]);
+  }
+  std::copy(std::begin(device.clusters), std::end(device.clusters), clusters);
+  return GUFO_CUDA_OK;
+}
+
+template <int TYPE>
+int LaunchPlan(gufo_cuda_ctx* ctx, const GemvArgs& base, const std::vector<int>& group, int tokens) {
+  using Q = Quant<TYPE>;
+  int clusters[kMaxCluster + 1];
+  int rc = ConfigureTc<TYPE>(ctx, clusters);
+  if (rc != GUFO_CUDA_OK) {
+    return rc;
+  }
   const int cols = base.cols;
   const int blocks = cols / kSuperBlock;
-  const Plan plan = PlanTc(base, group, TYPE, tokens, ctx->sm_count, clusters[device]);
+  const Plan plan = PlanTc(base, group, TYPE, tokens, ctx->sm_count, clusters);
   // Scratch: header (error word, counters), tile images, unscale factors, partial sums.
   const size_t rows = static_cast<size_t>(plan.groups) * plan.n;
   const size_t unscale_at = kHeaderBytes + rows * cols * 2;
   const size_t partial_at = (unscale_at + rows * 4 + 255) / 256 * 256;
   const bool cuts = plan.cluster == 1 && plan.units % plan.grid != 0;
   const size_t partial_bytes = cuts ? static_cast<size_t>(plan.grid) * 2 * kTileRows * plan.n * 4 : 0;
-  int rc = ReserveTc(ctx, partial_at + partial_bytes);
+  rc = ReserveTc(ctx, partial_at + partial_bytes);
   if (rc != GUFO_CUDA_OK) {
     return rc;
   }
