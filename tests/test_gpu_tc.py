@@ -39,8 +39,8 @@ def _weights(seed, rows, cols, ggml_type=Q.GGML_Q4_K):
 @pytest.mark.parametrize("rows,cols", [(256, 512), (130, 256), (1000, 2560), (2560, 9728)])
 @pytest.mark.parametrize("tokens", [16, 17, 33, 128, 131])
 def test_gemm_matches_oracle(ctx, oracle, ggml_type, rows, cols, tokens):
-    """One Q4_K or Q6_K part: row counts off the 256-row tile, K split over thread blocks
-    (2560 x 9728), block counts that leave a partial slab in the Q6_K device arrangement (10, 38),
+    """One Q4_K or Q6_K part: row counts off the 128-row tile, K shared by a cluster's thread blocks
+    (1000 x 2560, 2560 x 9728), block counts that leave a partial slab in the Q6_K device arrangement (10, 38),
     token counts off the tile granule and past one pass."""
     if rows * cols * tokens > 1.5e9:
         tokens = min(tokens, 33)
@@ -159,10 +159,54 @@ def test_gemm_activation_range(ctx, oracle):
     ctx.matrix_free(m)
 
 
+def _near_float64(y, x, w):
+    """y = x w^T to the rounding of weights and inputs to fp16: as a whole, and in every row and token.
+
+    An output's size is taken as |w row| |x row| / sqrt(cols), what it is on average for inputs that
+    are random: the outputs of a row at 17 tokens may by chance be small together (chi-squared of 17
+    degrees, a sixth of its mean in the smallest of 19400 rows), its errors may not be large together
+    (three times the mean in the largest: 1.7 x 4e-4)."""
+    error = (y.double() - x.double() @ w.double().T) ** 2
+    size = (x.double() ** 2).sum(1)[:, None] * (w.double() ** 2).sum(1)[None] / x.shape[1]
+    assert float((error.sum() / size.sum()).sqrt()) <= 5e-4
+    for d in (0, 1):
+        assert float((error.sum(d) / size.sum(d)).sqrt().max()) <= GEMM_TOL, d
+
+
+@pytest.mark.parametrize("ggml_type", [Q.GGML_Q4_K, Q.GGML_Q6_K])
+@pytest.mark.parametrize("rows,cols,tokens", [
+    (2560, 4096, 79), (2560, 9728, 128),        # clusters of six, 80 and 128 columns
+    (2560, 9728, 352),                          # clusters of three, two groups of 176
+    (2560, 4096, 512), (9000, 2560, 190),       # clusters of two, 176 and 192 columns; a ragged tile
+    (12288, 2560, 128), (12288, 2560, 512),     # whole tiles, one round and two
+    (19400, 2560, 17), (19400, 2560, 79),       # 152 tiles cut over 148 blocks, the last one ragged
+    (19400, 2560, 352), (19456, 2560, 512),     # the same with two and three groups, ragged columns
+    (12000, 9728, 17), (12000, 9728, 128),      # 94 tiles cut over 148 blocks: up to three shares a tile
+])
+def test_gemm_plans_against_float64(ctx, ggml_type, rows, cols, tokens):
+    """Every way the planner cuts a product on 148 SMs, at narrow and wide token groups (few raw
+    stages); twice, as the second run meets the counters and partial sums the first has left."""
+    gen = torch.Generator("cuda").manual_seed(rows + tokens)
+    raw = Q.quantize(ggml_type, torch.randn(rows, cols, device="cuda", generator=gen) * 0.02)
+    x = torch.randn(tokens, cols, device="cuda", generator=gen)
+    w = torch.empty(rows, cols, device="cuda")
+    y = torch.full((2, tokens, rows), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    m = ctx.matrix_from_device(ggml_type, raw.data_ptr(), rows, cols)
+    ctx.dequantize_device(m, 0, rows, w)
+    for i in range(2):
+        ctx.matmul_device(Context._parts([(m, 0, rows)]), 1, x, tokens, y[i])
+    ctx.synchronize()
+    assert torch.equal(y[0], y[1])
+    _near_float64(y[0], x, w)
+    ctx.matrix_free(m)
+
+
 def test_gemm_ring_of_two_blocks_under_load(ctx):
     """Wide token groups leave the raw blocks a ring of two stages, refilled from L2 by the groups
     behind the first: a stage must not be overwritten while lanes still read it. Many launches,
-    all alike bit for bit (a row of weights from the next block differs in every token)."""
+    all alike bit for bit (a row of weights from the next block differs in every token), and the
+    first against float64."""
     rows, cols, tokens = 19456, 2560, 352   # two groups of 176
     raw = torch.randint(0, 256, (rows, cols // 256, 144), device="cuda", dtype=torch.uint8,
                         generator=torch.Generator("cuda").manual_seed(3))
@@ -177,6 +221,11 @@ def test_gemm_ring_of_two_blocks_under_load(ctx):
         ctx.synchronize()
         for i in range(1, 12):
             assert torch.equal(y[0], y[i])
+    w = torch.empty(rows, cols, device="cuda")
+    torch.cuda.synchronize()
+    ctx.dequantize_device(m, 0, rows, w)
+    ctx.synchronize()
+    _near_float64(y[0], x, w)
     ctx.matrix_free(m)
 
 
