@@ -103,6 +103,7 @@ constexpr int kMmaWarp = kXWarp + 1;
 constexpr int kTcThreads = (kMmaWarp + 1) * 32;
 constexpr int kMaxStages = 10;
 constexpr long long kWaitCycles = 1ll << 31;           // about a second of SM clocks
+constexpr long long kDrainCycles = 1ll << 27;          // the same for what a block that gave up has under way
 constexpr int kHeaderBytes = 4096;                     // of the scratch: error word, counters of cut tiles
 // Token rows a pass: eight of the widest groups. Their fp16 tiles and the partial sums
 // are scratch that stays allocated, so it is bounded (90 MB for rows of 9728 values),
@@ -197,6 +198,31 @@ __device__ __forceinline__ bool BoundedWait(uint32_t bar, uint32_t parity, volat
   }
   __syncwarp();
   return done;
+}
+
+// After a wait that ran out: waits, with a limit, for the phase of an asynchronous operation
+// that this warp has started. A block must not end before these: copies would land in the
+// shared memory of the next one, and MMAs use tensor memory that is given back.
+__device__ __forceinline__ void Drain(uint32_t bar, uint32_t parity) {
+  const long long start = clock64();
+#pragma unroll 1
+  while (!MbarTryWait(bar, parity) && clock64() - start < kDrainCycles) {
+  }
+  __syncwarp();
+}
+
+// The same for the fills of a ring of `stages` stages, `issued` so far, the next one to go to
+// `stage` at `phase`; `full` is the barrier of stage 0.
+__device__ __forceinline__ void DrainRing(uint32_t full, int stages, int stage, uint32_t phase, int issued) {
+#pragma unroll 1
+  for (int left = min(issued, stages); left > 0; --left) {
+    if (stage == 0) {
+      stage = stages;
+      phase ^= 1u;
+    }
+    --stage;
+    Drain(full + 8u * stage, phase);
+  }
 }
 
 // One thread of a converged warp. Instructions of the asynchronous units take
@@ -446,8 +472,8 @@ __device__ __forceinline__ Unit LocateUnit(const TcGemmArgs& a, int u) {
   return unit;
 }
 
-// Brings the raw blocks of the steps [step, until) into the ring; the calling warp's lanes
-// agree on everything, one of them issues the copies.
+// Brings the raw blocks of the steps [step, until) into the ring, up to the first wait that
+// runs out; the calling warp's lanes agree on everything, one of them issues the copies.
 template <int TYPE>
 struct RawLoader {
   const TcGemmArgs& a;
@@ -467,7 +493,9 @@ struct RawLoader {
       const int row = unit.row0;
       const int end = min((u + 1) * a.blocks, until);
       for (int b = step - u * a.blocks; step < end; ++b, ++step) {
-        BoundedWait<true>(empty + 8u * stage, phase ^ 1u, abort_flag, a.error, 1);
+        if (!__all_sync(0xFFFFFFFFu, BoundedWait<true>(empty + 8u * stage, phase ^ 1u, abort_flag, a.error, 1))) {
+          return;
+        }
         const uint32_t at_shared = to + stage * Q::kRawStride;
         const uint32_t bar = full + 8u * stage;
         if (ElectOne()) {
@@ -772,7 +800,7 @@ __global__ void __launch_bounds__(896, 1)
 GemmTc(const __grid_constant__ TcGemmArgs a) {
   using Q = Quant<TYPE>;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bar_mem[4 * kMaxStages + 2 * kGroups + 4];
+  __shared__ __align__(8) uint64_t bar_mem[4 * kMaxStages + 2 * kGroups + 5];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
   __shared__ __align__(16) float factor[kMaxN];    // what undoes the scales of the unit's token rows
@@ -792,6 +820,7 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
   auto w_empty = [&](int g) { return bars + 8u * (4 * kMaxStages + kGroups + g); };
   auto acc_full = [&](int s) { return bars + 8u * (4 * kMaxStages + 2 * kGroups + s); };
   auto acc_empty = [&](int s) { return bars + 8u * (4 * kMaxStages + 2 * kGroups + 2 + s); };
+  const uint32_t mma_done = bars + 8u * (4 * kMaxStages + 2 * kGroups + 4);   // after a wait that ran out
   volatile int* abort_flag = &abort_word;
 
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0);
@@ -828,6 +857,7 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
       MbarInit(acc_full(s), 1);
       MbarInit(acc_empty(s), 4);
     }
+    MbarInit(mma_done, 1);
     finish = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -849,30 +879,40 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
   // units, so the pipeline never drains between them.
   if (warp == kRawWarp) {
     raw_loader.Run(last);
+    if (__any_sync(0xFFFFFFFFu, *abort_flag != 0)) {
+      DrainRing(raw_full(0), a.raw_stages, raw_loader.stage, raw_loader.phase, raw_loader.step - first);
+    }
   } else if (warp == kXWarp) {
     // ---- activation tiles, two (half a step's) per stage ------------------------
     GridDependencyWait();
-    int stage = 0;
+    int stage = 0, issued = 0;
     uint32_t phase = 0;
     for (int step = first; step < last;) {
       const int u = step / a.blocks;
       const int group = u % a.groups;
       const int end = min((u + 1) * a.blocks, last);
       const uint8_t* from = a.xh + (static_cast<size_t>(group) * a.blocks + (step - u * a.blocks)) * 2 * x_bytes;
-      for (int half = 2 * (end - step); half > 0; --half) {
-        BoundedWait<true>(x_empty(stage), phase ^ 1u, abort_flag, a.error, 2);
+      int half = 2 * (end - step);
+      for (step = end; half > 0; --half) {
+        if (!__all_sync(0xFFFFFFFFu, BoundedWait<true>(x_empty(stage), phase ^ 1u, abort_flag, a.error, 2))) {
+          step = last;
+          break;
+        }
         if (ElectOne()) {
           MbarArriveExpectTx(x_full(stage), x_bytes);
           BulkCopy(base + stage * x_bytes, from, x_bytes, x_full(stage));
         }
         __syncwarp();
         from += x_bytes;
+        ++issued;
         if (++stage == a.x_stages) {
           stage = 0;
           phase ^= 1u;
         }
       }
-      step = end;
+    }
+    if (__any_sync(0xFFFFFFFFu, *abort_flag != 0)) {
+      DrainRing(x_full(0), a.x_stages, stage, phase, issued);
     }
   } else if (warp == kMmaWarp) {
     // ---- MMA issue ---------------------------------------------------------
@@ -929,6 +969,13 @@ GemmTc(const __grid_constant__ TcGemmArgs a) {
         __syncwarp();
         acc ^= 1;
         acc_phase ^= acc == 0 ? 1u : 0u;
+      }
+      if (__any_sync(0xFFFFFFFFu, *abort_flag != 0)) {
+        if (ElectOne()) {
+          MmaCommit(mma_done);
+        }
+        __syncwarp();
+        Drain(mma_done, 0);
       }
     }
   } else if (warp >= kEpilogueWarp && warp < kEpilogueWarp + 4) {
