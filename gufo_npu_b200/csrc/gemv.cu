@@ -245,8 +245,16 @@ GemvRows(const __grid_constant__ GemvArgs args) {
 // sums a warp are folded (Fold), 62 shuffles instead of 320, and two blocks share an SM:
 // 64 rows x 2560 values, 8 / 79 / 512 tokens 2.9 / 5.0 / 16.6 -> 2.4 / 4.3 / 12.0 us, 257 rows x
 // 2048 (a router), 4 / 128 tokens 2.6 / 15.2 -> 2.1 / 9.6.
-template <int kF32Rows, int TOK>
-__global__ void __launch_bounds__(256, kF32Rows * TOK >= 64 ? 2 : 1)
+//
+// PER_SM, the blocks an SM that registers are kept to: few, for loads in flight and the folded
+// sums of several tokens. But one token's blocks that would need another round, with rows of one
+// chunk a warp or in tiles of two, are better all there (us: 65536 x 1024 44 with two an SM, 38
+// with five, but 12288 x 2048 12.8 and 15.1; 1024 x 2048 in tiles of two 2.8 with three, 2.3
+// with six, but 600 x 4096 2.3 and 2.7); and where the matrix does not stay in the L2, tiles of
+// 64 sums have an SM to themselves (8 tokens: 12288 x 2560 69 with two, 45 with one, but 4096 x
+// 2048 9.5 and 10.2).
+template <int kF32Rows, int TOK, int PER_SM>
+__global__ void __launch_bounds__(256, PER_SM)
 GemvRowsF32(const __grid_constant__ GemvArgs args, int tokens) {
   __shared__ float partial[8][kF32Rows * TOK];
   const int lane = threadIdx.x & 31;
@@ -333,10 +341,22 @@ int LaunchRowsF32(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
   auto launch = [&](auto kernel, int tok) {
     return LaunchOverlapped(kernel, dim3(rows, (tokens + tok - 1) / tok), dim3(256), 0, ctx->stream, 1, args, tokens);
   };
-  GUFO_CUDA_TRY(tokens == 1   ? launch(GemvRowsF32<ROWS, 1>, 1)
-                : tokens == 2 ? launch(GemvRowsF32<ROWS, 2>, 2)
-                : tokens <= 4 ? launch(GemvRowsF32<ROWS, 4>, 4)
-                              : launch(GemvRowsF32<ROWS, 8>, 8));
+  const bool beyond_l2 = static_cast<int64_t>(args.total_rows) * args.cols * 4 > (64ll << 20);
+  if constexpr (ROWS == 2) {
+    const bool rounds = static_cast<int>(rows) > 3 * ctx->sm_count;
+    GUFO_CUDA_TRY(tokens > 4   ? launch(GemvRowsF32<2, 8, 2>, 8)
+                  : tokens > 2 ? launch(GemvRowsF32<2, 4, 4>, 4)
+                  : tokens > 1 ? launch(GemvRowsF32<2, 2, 4>, 2)
+                  : rounds     ? launch(GemvRowsF32<2, 1, 6>, 1)
+                               : launch(GemvRowsF32<2, 1, 3>, 1));
+  } else {
+    const bool rounds = static_cast<int>(rows) > 2 * ctx->sm_count;
+    GUFO_CUDA_TRY(tokens > 4                     ? (beyond_l2 ? launch(GemvRowsF32<8, 8, 1>, 8) : launch(GemvRowsF32<8, 8, 2>, 8))
+                  : tokens > 2                   ? launch(GemvRowsF32<8, 4, 2>, 4)
+                  : tokens > 1                   ? launch(GemvRowsF32<8, 2, 2>, 2)
+                  : rounds && args.cols <= 1024 ? launch(GemvRowsF32<8, 1, 5>, 1)
+                                                 : launch(GemvRowsF32<8, 1, 2>, 1));
+  }
   ctx->launches.fetch_add(1);
   return GUFO_CUDA_OK;
 }

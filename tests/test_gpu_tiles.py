@@ -901,3 +901,23 @@ def test_borrowed_bytes_that_the_kernel_before_writes(ctx, ggml_type):
     scale = x.double().abs() @ w.double().abs().T
     assert ((y.double() - exact).abs() <= 2e-6 * scale).all()
     ctx.matrix_free(m)
+
+
+@pytest.mark.parametrize("rows,cols,tokens", [(601, 2052, 1), (1001, 2052, 1), (2371, 1024, 1), (2371, 1028, 1), (2371, 516, 2),
+                                              (2371, 516, 3), (1183, 2048, 8), (8199, 2564, 5), (8199, 2564, 17)])
+def test_f32_rows_in_every_form(ctx, rows, cols, tokens):
+    """Tiles of two rows in one round of blocks and more, of eight rows of one chunk a warp and more,
+    matrices beyond the L2; ragged rows, chunks and tokens, two parts; against float64."""
+    gen = torch.Generator("cuda").manual_seed(rows + cols)
+    w = torch.randn(rows, cols, device="cuda", generator=gen)
+    x = torch.randn(tokens, cols, device="cuda", generator=gen)
+    y = torch.full((tokens, rows + 3), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    m = ctx.matrix_from_device(Q.GGML_F32, w.data_ptr(), rows, cols)
+    ctx.matmul_device(Context._parts([(m, 0, rows), (m, 1, 3)]), 2, x, tokens, y)
+    ctx.synchronize()
+    want = x.double() @ w.double().T
+    scale = x.double().abs() @ w.double().abs().T   # fp32 sums of cols terms: a few roundings of it
+    assert ((y[:, :rows].double() - want).abs() <= 2e-6 * scale).all()
+    assert torch.equal(y[:, rows:], y[:, 1:4])
+    ctx.matrix_free(m)
