@@ -518,12 +518,17 @@ __device__ __forceinline__ float WarpSum(float v) {
   return v;
 }
 
+// Sums that Fold leaves in every lane.
+template <int N>
+constexpr int kFoldLeft = N > 32 ? N / 32 : 1;
+
 // WarpSum of each of N values (a power of two), by the same additions: at every step a
-// lane keeps half of its values and adds the other lane's half to it. Returns how many
-// sums are left in a lane's v[0 ..] (all lanes in groups of 32 / N hold the same where N is
-// below 32) and sets *first to the number of the first.
+// lane keeps half of its values and adds the other lane's half to it. kFoldLeft<N> sums
+// are left in a lane's v[0 ..], from number *first on (below 32 values several lanes hold
+// the same one).
 template <int N>
 __device__ __forceinline__ void Fold(float (&v)[N], int lane, int* first) {
+  static_assert(N > 0 && (N & (N - 1)) == 0, "halves at every step");
   int n = N, at = 0;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {

@@ -698,9 +698,12 @@ DeltaNetGatesKernel(const __grid_constant__ GatesArgs a) {
   }
   int first;
   Fold<kGateTile * kGateTile>(acc, lane, &first);
-  partial[warp][first] = acc[0];
-  partial[warp][first + 1] = acc[1];
+#pragma unroll
+  for (int j = 0; j < kFoldLeft<kGateTile * kGateTile>; ++j) {
+    partial[warp][first + j] = acc[j];
+  }
   Fold<kGateTile>(sq, lane, &first);
+  static_assert(kFoldLeft<kGateTile> == 1, "one sum a lane");
   partial[warp][kGateTile * kGateTile + first] = sq[0];   // several lanes the same
   __syncthreads();
   const int r = threadIdx.x / kGateTile, t = threadIdx.x % kGateTile;

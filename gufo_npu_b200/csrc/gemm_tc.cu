@@ -55,16 +55,13 @@
 // depend on who that is. Nobody waits for another block but for those of its cluster.
 //
 // What bounds it: small products the chain of staging kernel (2-3 us), hand-over (1), first
-// tiles (1) and the sum over a cluster (3); large ones a step's 1000 cycles of
-// dequantization and hand-overs and, in a loop of more than about 100 tokens, the board's
-// power limit (1.3-1.4 GHz then). An MMA with A in tensor memory takes 9.5 + n / 2 cycles.
-// Measured (activation staging included), us at 32 / 79 / 128 / 512 tokens, with every role
-// behind one thread, shares summed by the last block alone and staging in blocks of up to
-// 1024 threads -> now: 19456 x 2560 Q4_K 15.9 / 18.8 / 23.3 / 57.3 -> 14.0 / 16.2 / 18.6 /
-// 49.5; 12288 x 2560 Q4_K 12.8 / 15.3 / 18.7 / 36.0 -> 10.8 / 12.0 / 13.6 / 28.9; 2560 x 4096
-// Q4_K 13.3 / 16.5 / 18.3 / 22.7 -> 8.3 / 9.4 / 11.2 / 17.5; 2560 x 9728 Q6_K 18.0 / 24.8 /
-// 32.5 / 45.2 -> 13.6 / 16.5 / 18.6 / 32.7; 248320 x 2560 Q6_K at 32 / 79 / 128 tokens 122 /
-// 155 / 222 -> 119 / 145 / 187 (outputs of 128 tokens are 127 MB).
+// tiles (1) and the sum over a cluster (3); large ones a step, which takes the 1000 cycles of
+// dequantization and hand-overs and the tensor core's time (an MMA with A in tensor memory:
+// 9.5 + n / 2 cycles) nearly one after the other (StepCycles), and, in a loop of more than
+// about 100 tokens, the board's power limit (1.3-1.4 GHz then). Measured, staging included, us
+// at 32 / 79 / 128 / 512 tokens, with the roles behind one thread each and shares summed by the
+// last block alone, and now: 19456 x 2560 Q4_K 15.9 / 18.8 / 23.3 / 57.3 and 13.9 / 16.2 / 18.8 /
+// 48.9; 2560 x 9728 Q6_K 18.0 / 24.8 / 32.5 / 45.2 and 13.9 / 16.3 / 18.3 / 32.3.
 //
 // Each activation row is scaled by a power of two into fp16 range first and the
 // outputs scaled back, so range never costs precision. Rounding w and x to
@@ -225,11 +222,8 @@ __device__ __forceinline__ void DrainRing(uint32_t full, int stages, int stage, 
   }
 }
 
-// One thread of a converged warp. Instructions of the asynchronous units take
-// their operands from uniform registers; behind this predicate the compiler knows
-// that there is one thread, behind `lane == 0` it does not and walks the warp for
-// every operand (measured: 112 cycles to issue an MMA or a commit, whatever its
-// size, against N / 2 and about 25).
+// One thread of a converged warp, for the instructions of the asynchronous units alone: the
+// loops around them stay the whole warp's (see the head of this file).
 __device__ __forceinline__ bool ElectOne() {
   uint32_t elected;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));

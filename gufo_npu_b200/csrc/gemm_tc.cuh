@@ -1,4 +1,4 @@
-// Launch interface of the tcgen05 small-M GEMM (16 or more token rows).
+// Launch interface of the tcgen05 small-M GEMM (kTcMinTokens or more token rows).
 #pragma once
 
 #include "gemv.cuh"

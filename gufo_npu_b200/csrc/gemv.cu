@@ -300,9 +300,8 @@ GemvRowsF32(const __grid_constant__ GemvArgs args, int tokens) {
   }
   int first;
   Fold<kSums>(acc, lane, &first);
-  constexpr int kLeft = kSums > 32 ? kSums / 32 : 1;
 #pragma unroll
-  for (int j = 0; j < kLeft; ++j) {
+  for (int j = 0; j < kFoldLeft<kSums>; ++j) {
     partial[warp][first + j] = acc[j];   // below 32 sums several lanes store the same
   }
   __syncthreads();
@@ -361,11 +360,7 @@ int LaunchRowsF32(gufo_cuda_ctx* ctx, const GemvArgs& args, int tokens) {
   return GUFO_CUDA_OK;
 }
 
-// Q5_K and Q8_0 rows of whole 256-value blocks, up to M tokens: a thread block takes
-// kSplitRows rows, its warps the 256-value blocks of K round-robin, a lane eight
-// values of each. The rows' loads of a block are in flight together and a row of
-// 2048 values is one round trip deep, where one warp per row walks eight (Q8_0:
-// sixty-four, a byte a lane); a token's inputs are read once for the rows.
+// Rows of a group of GemvSplit.
 constexpr int kSplitRows = 4;
 
 // Eight weights of a Q5_K block: values 64 p + c .. + 3 and the same 32 further on
@@ -391,19 +386,21 @@ __device__ __forceinline__ void SplitWeights5(const uint4& head, uint32_t h, uin
   }
 }
 
-// Q5_K and Q8_0 rows of whole blocks against up to M tokens. A block takes a group of four
-// rows, or every gridDim.x-th where there are many; AHEAD: a warp's first unit is asked for
-// ahead of the dependency wait (`early`: no bytes are borrowed) and the next one while it
-// multiplies, across the groups. The
-// sums over the lanes are folded (Fold). Without LOOP the grid has a block for every group.
+// Q5_K and Q8_0 rows of whole 256-value blocks against up to M tokens. A thread block takes a
+// group of four rows (LOOP: every gridDim.x-th), its warps the 256-value blocks of K
+// round-robin, a lane eight values of each: the rows' loads of a block are in flight together
+// and a row of 2048 values is one round trip deep, where one warp per row walks eight (Q8_0:
+// sixty-four, a byte a lane); a token's inputs are read once for the rows. AHEAD: a warp's
+// first unit is asked for ahead of the dependency wait (`early`: no bytes are borrowed) and the
+// next one while it multiplies, across the groups. The sums over the lanes are folded (Fold).
 //
-// What bounds it: issue slots for long matrices (a value's conversion and its FMAs), a
-// block's start and one load for short ones. Against loads behind the wait, a block for
-// every group and a butterfly per sum, us at 1 / 2 / 4 / 8 tokens: Q5_K 2048 x 2048 4.2 /
-// 4.6 / 5.9 / 9.3 -> 4.1 / 4.4 / 5.0 / 6.6, 24576 x 2560 46 / 50 / 78 / 101 -> 46 / 51 / 62 /
-// 83; Q8_0 3.3 / 4.5 / 5.8 / 8.6 -> 2.6 / 4.1 / 4.7 / 6.1, 31 / 40 / 64 / 90 -> 27 / 33 / 43 / 64.
-// Registers are kept to what lets three blocks share an SM (four for Q8_0 and one token:
-// 2048 rows are one round then).
+// What bounds it: issue slots for long matrices (a value's conversion and its FMAs), a block's
+// start and one load for short ones. With loads behind the wait, a block for every group and a
+// butterfly per sum, and now, us at 1 / 2 / 4 / 8 tokens, held by the library: Q5_K 2048 x 2048
+// 4.2 / 4.6 / 5.9 / 9.3 and 4.0 / 4.2 / 5.0 / 6.6, 24576 x 2560 46 / 50 / 78 / 101 and 45 / 48 /
+// 62 / 83; Q8_0 3.3 / 4.5 / 5.8 / 8.6 and 2.6 / 4.1 / 4.7 / 6.1, 31 / 40 / 64 / 90 and 27 / 33 /
+// 43 / 64. Registers are kept to what lets two blocks share an SM, three with one or two tokens
+// (four for Q8_0 and one token: 2048 rows are one round then).
 template <int TYPE, int M, bool AHEAD, bool LOOP = AHEAD>
 __global__ void __launch_bounds__(256, M == 1 && TYPE == GUFO_CUDA_Q8_0 ? 4 : (M <= 2 ? 3 : 2))
 GemvSplit(const __grid_constant__ GemvArgs args, int tokens, bool early) {
@@ -570,6 +567,7 @@ GemvSplit(const __grid_constant__ GemvArgs args, int tokens, bool early) {
     }
     int first;
     Fold<kSums>(acc, lane, &first);
+    static_assert(kFoldLeft<kSums> == 1, "one sum a lane");
     partial[buffer][warp][first] = acc[0];   // several lanes the same, below 32 sums
     __syncthreads();
     const int r = threadIdx.x / M, t = threadIdx.x % M;
