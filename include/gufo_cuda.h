@@ -126,8 +126,8 @@ int gufo_cuda_host_give(void* host);
  * Types: Q4_K, Q6_K and F32 (the alpha/beta and router rows,
  * src/models/qwen35/gguf_projections.cpp:126-131,162-170) on every path; Q8_0
  * and Q5_K (the other row formats of real UD-Q4_K_XL files,
- * src/models/qwen35/gguf_dot.hpp:31-69,190-193) for products on the general
- * kernel and dequantization; F16 and BF16 for dequantization only
+ * src/models/qwen35/gguf_dot.hpp:31-69,190-193) for products in fp32 arithmetic
+ * and dequantization; F16 and BF16 for dequantization only
  * (src/core/quant.cpp:221-260). */
 int gufo_cuda_matrix_upload(gufo_cuda_ctx* ctx, int ggml_type,
                             const void* host_bytes, int64_t rows, int64_t cols,
